@@ -93,6 +93,23 @@ int b200proj_project_3d_to_2d_forw(const float* rec, int64_t B, int64_t R,
                                    double fourier_radius_cutoff, float* out,
                                    const int32_t* pose_order, void* stream);
 
+/* The 3D projections with scratch: large calls (many slices through each region of the volume) run
+ * brick by brick -- a block keeps a piece of the volume in shared memory and handles the pixels of
+ * all slices that fall into it -- which needs a workspace for the slices' records and the list of
+ * work items.  b200proj_project_workspace_bytes gives its size, 0 when the call would not gain
+ * (small calls; the workspace may then be NULL; records != 0: of _forw_records below).  With too small a workspace, or NULL, the plain
+ * kernels run: the results are the same to rounding.  The workspace must be 16-byte aligned and
+ * is free again when the call's work has run. */
+size_t b200proj_project_workspace_bytes(int64_t B, int64_t P, int64_t N, int interpolation, int records,
+                                        double oversampling, double fourier_radius_cutoff);
+int b200proj_project_3d_to_2d_forw_ws(const float* rec, int64_t B, int64_t R,
+                                      const float* rot, int64_t B_rot,
+                                      const float* shifts, int64_t B_shift,
+                                      int64_t P, int64_t N, int interpolation, double oversampling,
+                                      double fourier_radius_cutoff, float* out,
+                                      const int32_t* pose_order, void* workspace,
+                                      size_t workspace_bytes, void* stream);
+
 /* ---- forward projection with packed output ------------------------------------------------
  * No counterpart in the reference.  For callers that move the projections off the device: only
  * the pixels inside the cutoff are produced, side by side, out_packed [B, P, pack_count] complex
@@ -352,6 +369,22 @@ int b200proj_project_3d_to_2d_back_saved(const float* grad_proj, const float* ou
                                          int interpolation, double oversampling,
                                          double fourier_radius_cutoff, float* grad_rec, float* grad_rot,
                                          float* grad_shifts, const int32_t* pose_order, void* stream);
+
+/* The 3D pair with one 32-byte record (d/dc, d/dr, d/dd, projection; complex each) per pixel in place of
+ * the planes, records = [B,P,N,Nh,4] complex, 32-byte aligned: whole sectors, which is what the
+ * brick-by-brick kernel (workspace as for b200proj_project_3d_to_2d_forw_ws) writes best. */
+int b200proj_project_3d_to_2d_forw_records(const float* rec, int64_t B, int64_t R, const float* rot,
+                                           int64_t B_rot, const float* shifts, int64_t B_shift, int64_t P,
+                                           int64_t N, int interpolation, double oversampling,
+                                           double fourier_radius_cutoff, float* out, float* records,
+                                           const int32_t* pose_order, void* workspace,
+                                           size_t workspace_bytes, void* stream);
+int b200proj_project_3d_to_2d_back_records(const float* grad_proj, const float* out, const float* records,
+                                           int64_t B, int64_t R, const float* rot, int64_t B_rot,
+                                           const float* shifts, int64_t B_shift, int64_t P, int64_t N,
+                                           int interpolation, double oversampling,
+                                           double fourier_radius_cutoff, float* grad_rec, float* grad_rot,
+                                           float* grad_shifts, const int32_t* pose_order, void* stream);
 
 /* ---- backward of back-projection (gather) ----------------------------------------------
  * grad_proj [B,P,N,Nh] complex is fully written.  grad_weights [B,P,N,Nh] float is written

@@ -1,0 +1,72 @@
+"""The brick-by-brick 3D kernels (a block keeps a piece of the volume in shared memory and walks over the slices)
+against the CPU oracle, at sizes and poses where the walk can go wrong: one brick and several, ragged boxes and pose
+counts, lattice poses, matrices that are no rotations, cutoffs inside and beyond Nyquist, batches."""
+import os
+import subprocess
+import sys
+from pathlib import Path
+
+import pytest
+import torch
+
+from cases import Case, TOL_ATOMIC, TOL_FORWARD, axis_aligned_rotations, make_inputs, rel_err
+
+pytestmark = pytest.mark.gpu
+ROOT = Path(__file__).resolve().parent.parent
+
+#      B  P   N   R   os    cutoff  B_rot  B_shift
+SIZES = [(1, 40, 4, 8, 2.0, None, 1, 1),
+         (1, 45, 18, 36, 2.0, None, 1, 1),
+         (2, 33, 20, 30, 1.5, 7.3, 2, 0),
+         (2, 9, 34, 34, 1.0, 20.0, 1, 2),
+         (1, 37, 26, 34, 1.3, None, 1, 1),
+         (1, 3, 48, 120, 2.5, 17.0, 1, 1)]
+
+
+def _inputs(size, seed):
+    B, P, N, R, os_, cutoff, B_rot, B_shift = size
+    t = make_inputs(Case("bricks", 3, "cubic", B, P, N, R, os_, cutoff, B_rot, B_shift, shift_range=5.0, seed=seed))
+    lattice = axis_aligned_rotations(torch.Generator().manual_seed(seed))
+    if P >= len(lattice):
+        t["rot"][0, : len(lattice)] = lattice
+        t["rot"][0, len(lattice)] *= 1.2                    # not rotations: these slices take the plain path
+    if P > 2:
+        t["rot"][0, 2, :, 1] = t["rot"][0, 2, :, 0]
+    return t, dict(output_shape=(N, N), oversampling=os_, fourier_radius_cutoff=cutoff)
+
+
+def check(names):
+    """Run in a fresh process with the bricks forced on (the library reads the switch once)."""
+    sys.path[:0] = [str(ROOT), str(ROOT / "torch-projectors_b200"), str(ROOT / "tests")]
+    import torch_projectors_b200 as tp
+    from oracle import port
+    for seed, size in enumerate(SIZES):
+        for interp in ("linear", "cubic"):
+            t, kw = _inputs(size, seed)
+            N, os_, cutoff = size[2], size[4], size[5]
+            want = port.project_3d_to_2d_forw(t["rec"], t["rot"], t["shifts"], [N, N], interp, os_, cutoff)
+            shifts = t["shifts"].cuda() if t["shifts"] is not None else None
+            if "forward" in names:
+                got = tp.project_3d_to_2d_forw(t["rec"].cuda(), t["rot"].cuda(), shifts, interpolation=interp, **kw)
+                assert rel_err(got, want) <= TOL_FORWARD, (size, interp, rel_err(got, want))
+            if "gradients" in names:
+                tp.set_save_derivatives(True, min_volume_bytes=0)
+                for fixed in (False, True):
+                    rec, rot = t["rec"].cuda().requires_grad_(not fixed), t["rot"].cuda().requires_grad_(True)
+                    sh = shifts.clone().requires_grad_(True) if shifts is not None else None
+                    out = tp.project_3d_to_2d_forw(rec, rot, sh, interpolation=interp, **kw)
+                    assert rel_err(out, want) <= TOL_FORWARD, (size, interp)
+                    out.backward(t["proj"].cuda())
+                    grads = port.project_3d_to_2d_back(t["proj"], t["rec"], t["rot"], t["shifts"], interp, os_, cutoff,
+                                                       need_rot_grad=True, need_shift_grad=shifts is not None)
+                    for have, ref, what in ((rec.grad, grads[0], "volume"), (rot.grad, grads[1], "rotations"), (sh.grad if sh is not None else None, grads[2], "shifts")):
+                        if have is not None:
+                            assert rel_err(have, ref) <= TOL_ATOMIC, (size, interp, what, rel_err(have, ref))
+
+
+@pytest.mark.parametrize("names", ["forward", "gradients"])
+def test_bricks_match_the_oracle(names):
+    env = dict(os.environ, B200PROJ_BRICKS="1")
+    r = subprocess.run([sys.executable, "-c", f"import sys; sys.path.insert(0, {str(ROOT / 'tests')!r}); import test_gpu_bricks as t; t.check({names!r})"],
+                       env=env, cwd=ROOT, capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]

@@ -12,7 +12,7 @@
 #include <mutex>
 #include <type_traits>
 
-#include "fourier_slice_kernels.cuh"
+#include "brick_kernels.cuh"
 
 namespace {
 
@@ -79,6 +79,9 @@ int prepare(Launch& L, int dim, int64_t B, int64_t R, int64_t B_rot, const void*
     g.cutoff_sq_d = cutoff * cutoff;
     g.os = oversampling;
     g.phase_scale = -2.0 * M_PI / (double)(float)N;
+    g.n_f = (float)N;
+    g.inv_n = (float)(1.0 / (double)N);
+    g.phase_scale_f = (float)g.phase_scale;
     g.shift_scale = -2.0 * M_PI / (double)N;
     g.vol_elems = vol;
     g.order = nullptr;
@@ -176,17 +179,110 @@ bool linear_rows2() {
     return on;
 }
 
+
+// ---- brick-stationary kernels: plan and launch ---------------------------------------------------------
+struct BrickLaunch {
+    BrickPlan plan;
+    int64_t bricks;          // of one batch item
+    size_t items;            // capacity of the item list
+    size_t item_bytes, rec_bytes;
+    size_t bytes;            // workspace
+    bool use;
+};
+
+// Pixels of a slice inside the cutoff.
+double pixels_inside(int64_t N, double cutoff) {
+    const double r = cutoff < 0.0 ? 0.0 : cutoff, n = (double)N / 2.0;
+    const double all = (double)N * (double)(N / 2 + 1);
+    if (r >= n * 1.4143) return all;
+    const double disc = M_PI / 2.0 * r * r + r;
+    return disc < all ? disc : all;
+}
+
+BrickLaunch brick_plan(int64_t B, int64_t P, int64_t N, bool cubic, bool records, double os, double cutoff) {
+    BrickLaunch L{};
+    static const int force = [] { const char* e = getenv("B200PROJ_BRICKS"); return e ? atoi(e) : -1; }();   // 0 / 1: never / always, for tests
+    if (force == 0 || os < 1.0 || !(cutoff >= 0.0) || P < 1) return L;
+    const double corner = sqrt((double)N * N / 2.0);
+    const double reach = (cutoff < corner ? cutoff : corner) * os;
+    if (reach > 1000.0) return L;
+    const double pixels = pixels_inside(N, cutoff) * (double)B * (double)P;
+    L.plan.ball = (float)(reach + 1.0);
+    const int span = 2 * ((int)ceil(reach) + 2);
+    const int dims[3] = {kBrickX, kBrickY, kBrickZ};
+    L.bricks = 1;
+    for (int a = 0; a < 3; ++a) {
+        L.plan.n[a] = (span + dims[a] - 1) / dims[a];
+        L.plan.lo[a] = -((L.plan.n[a] * dims[a]) / 2);
+        L.bricks *= L.plan.n[a];
+    }
+    if (L.bricks * B > (1 << 26) || B * P > (1 << 26)) return L;
+    L.plan.density = (float)((double)kBrickX * kBrickY * kBrickZ / (4.0 * os * os));
+    double target = pixels / (148.0 * 3.0 * 8.0);
+    if (target < 3000.0) target = 3000.0;
+    L.plan.target = (float)target;
+    L.plan.max_extra = (int)(1.5 * pixels / target) + 64;
+    L.items = (size_t)(L.bricks * B) + (size_t)L.plan.max_extra;
+    L.item_bytes = (L.items * sizeof(int4) + 255) & ~(size_t)255;
+    L.rec_bytes = (size_t)(B * P) * 3 * sizeof(float4);
+    L.bytes = 256 + L.item_bytes + L.rec_bytes + (size_t)(N * (N / 2 + 1)) * sizeof(int);
+    // Bricks pay once their pixels outweigh staging them, whatever their number, and a fixed cost (measured: 20 us and
+    // 26 ns per brick against 33 ps saved per cubic pixel at oversampling 2; dense samples are cheaper for the plain
+    // kernels, linear taps save only some 2 ps).
+    const double in_ball = 4.19 * pow(reach + 12.0, 3) / ((double)kBrickX * kBrickY * kBrickZ) * (double)B;
+    const double need = cubic ? (1.2e6 + 900.0 * in_ball) * (os < 2.0 ? 2.0 / os : 1.0)
+                              : (10e6 + 4000.0 * in_ball) * (records ? 0.6 : 1.0);
+    L.use = force == 1 || pixels > need;
+    return L;
+}
+
+BrickWork brick_work(const BrickLaunch& L, void* workspace) {
+    BrickWork w;
+    w.header = (int*)workspace;
+    w.items = (int4*)((char*)workspace + 256);
+    w.recs = (float4*)((char*)workspace + 256 + L.item_bytes);
+    w.outside = (int*)((char*)workspace + 256 + L.item_bytes + L.rec_bytes);
+    return w;
+}
+
+int brick_setup(const BrickLaunch& bl, const BrickWork& w, const Launch& L, const float* rot, const float* shifts, cudaStream_t s) {
+    if (int rc = zero_async(w.header, 16, s)) return rc;
+    const int64_t clusters = (int64_t)((bl.plan.n[0] + 7) / 8) * ((bl.plan.n[1] + 7) / 8) * ((bl.plan.n[2] + 3) / 4) * L.B;
+    const int64_t slices = (L.B * L.P + 255) / 256;
+    brick_setup_kernel<<<(unsigned)(clusters > slices ? clusters : slices) + 1u, 256, 0, s>>>(rot, shifts, w, L.g, bl.plan, (int)L.B);
+    return check_launch("brick_setup launch");
+}
+
+template <bool CUBIC, bool SAVE>
+int launch_brick_forw(const Launch& L, const BrickLaunch& bl, void* workspace, const float* rec, const float* rot, const float* shifts,
+                      float* out, float* derivs, cudaStream_t s) {
+    const BrickWork w = brick_work(bl, workspace);
+    if (int rc = brick_setup(bl, w, L, rot, shifts, s)) return rc;
+    constexpr size_t smem = sizeof(float2) * BrickShape<CUBIC>::kVoxels + sizeof(BrickBlock);
+    const cudaError_t e = cudaFuncSetAttribute(brick_forw_kernel<CUBIC, SAVE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return cuda_fail(e, "brick_forw shared memory");
+    brick_forw_kernel<CUBIC, SAVE><<<148 * 3, kBlockThreads, smem, s>>>((const float2*)rec, rot, shifts, (float2*)out, (float2*)derivs, w, L.g, bl.plan);
+    return check_launch("brick_forw launch");
+}
+
 // ---- operator bodies, templated on the dimensionality and the real type (float | double) ------------------------------------
 template <int DIM, typename Real>
 int project_forw(const Real* rec, int64_t B, int64_t R, const Real* rot, int64_t B_rot,
                  const Real* shifts, int64_t B_shift, int64_t P, int64_t N, int interpolation,
-                 double os, double cutoff, Real* out, const int32_t* pose_order, void* stream) {
+                 double os, double cutoff, Real* out, const int32_t* pose_order, void* stream,
+                 void* workspace = nullptr, size_t workspace_bytes = 0) {
     Launch L;
     if (int rc = prepare(L, DIM, B, R, B_rot, rot, shifts, B_shift, P, N, interpolation, os, cutoff)) return rc;
     if (rec == nullptr || out == nullptr) return fail(B200PROJ_ERR_ARGUMENT, "reconstruction / output pointer is NULL");
     L.g.order = pose_order;
     if (P == 0) return B200PROJ_OK;
     cudaStream_t s = (cudaStream_t)stream;
+    if constexpr (DIM == 3 && std::is_same<Real, float>::value) {
+        const BrickLaunch bl = workspace != nullptr ? brick_plan(B, P, N, interpolation == B200PROJ_CUBIC, false, os, cutoff) : BrickLaunch{};
+        if (bl.use && workspace_bytes >= bl.bytes)
+            return interpolation == B200PROJ_CUBIC ? launch_brick_forw<true, false>(L, bl, workspace, rec, rot, shifts, out, nullptr, s)
+                                                   : launch_brick_forw<false, false>(L, bl, workspace, rec, rot, shifts, out, nullptr, s);
+    }
     const C2<Real>* v = (const C2<Real>*)rec;
     C2<Real>* o = (C2<Real>*)out;
     if (interpolation == B200PROJ_CUBIC) {
@@ -215,12 +311,12 @@ void launch_project_back(const Launch& L, cudaStream_t s, const C2<Real>* gp, co
 #undef B200PROJ_PB
 }
 
-template <int DIM, bool CUBIC, bool NEED_REC>
+template <int DIM, bool CUBIC, bool NEED_REC, bool RECORDS>
 void launch_project_back_saved(const Launch& L, cudaStream_t s, const float2* gp, const float2* out, const float2* derivs,
                                const float* rot, const float* shifts, float2* grad_rec, float* grad_rot, float* grad_shift) {
     const bool nr = grad_rot != nullptr, ns = grad_shift != nullptr;
 #define B200PROJ_PBS(NR, NS) \
-    project_back_saved_kernel<DIM, CUBIC, NR, NS, NEED_REC><<<L.grid, kBlockThreads, 0, s>>>(gp, out, derivs, rot, shifts, grad_rec, grad_rot, grad_shift, L.g)
+    project_back_saved_kernel<DIM, CUBIC, NR, NS, NEED_REC, RECORDS><<<L.grid, kBlockThreads, 0, s>>>(gp, out, derivs, rot, shifts, grad_rec, grad_rot, grad_shift, L.g)
     if (nr && ns) B200PROJ_PBS(true, true);
     else if (nr) B200PROJ_PBS(true, false);
     else if (ns) B200PROJ_PBS(false, true);
@@ -228,25 +324,34 @@ void launch_project_back_saved(const Launch& L, cudaStream_t s, const float2* gp
 #undef B200PROJ_PBS
 }
 
-// Forward projection that also writes the pixels' derivatives, and the backward pass from them (fp32).
-template <int DIM>
+// Forward projection that also writes the pixels' derivatives (as planes, or as one record per pixel), and the
+// backward pass from them (fp32).
+template <int DIM, bool RECORDS = false>
 int project_forw_saving(const float* rec, int64_t B, int64_t R, const float* rot, int64_t B_rot, const float* shifts,
                         int64_t B_shift, int64_t P, int64_t N, int interpolation, double os, double cutoff,
-                        float* out, float* derivatives, const int32_t* pose_order, void* stream) {
+                        float* out, float* derivatives, const int32_t* pose_order, void* stream,
+                        void* workspace = nullptr, size_t workspace_bytes = 0) {
     Launch L;
     if (int rc = prepare(L, DIM, B, R, B_rot, rot, shifts, B_shift, P, N, interpolation, os, cutoff)) return rc;
     if (rec == nullptr || out == nullptr || derivatives == nullptr) return fail(B200PROJ_ERR_ARGUMENT, "reconstruction / output / derivatives pointer is NULL");
     L.g.order = pose_order;
     if (P == 0) return B200PROJ_OK;
     cudaStream_t s = (cudaStream_t)stream;
+    if constexpr (RECORDS) {
+        if ((reinterpret_cast<uintptr_t>(derivatives) & 31u) != 0) return fail(B200PROJ_ERR_ARGUMENT, "records must be 32-byte aligned");
+        const BrickLaunch bl = workspace != nullptr ? brick_plan(B, P, N, interpolation == B200PROJ_CUBIC, true, os, cutoff) : BrickLaunch{};
+        if (bl.use && workspace_bytes >= bl.bytes)
+            return interpolation == B200PROJ_CUBIC ? launch_brick_forw<true, true>(L, bl, workspace, rec, rot, shifts, out, derivatives, s)
+                                                   : launch_brick_forw<false, true>(L, bl, workspace, rec, rot, shifts, out, derivatives, s);
+    }
     if (interpolation == B200PROJ_CUBIC)
-        project_forw_saving_kernel<DIM, true><<<L.grid, kBlockThreads, 0, s>>>((const float2*)rec, rot, shifts, (float2*)out, (float2*)derivatives, L.g);
+        project_forw_saving_kernel<DIM, true, RECORDS><<<L.grid, kBlockThreads, 0, s>>>((const float2*)rec, rot, shifts, (float2*)out, (float2*)derivatives, L.g);
     else
-        project_forw_saving_kernel<DIM, false><<<L.grid, kBlockThreads, 0, s>>>((const float2*)rec, rot, shifts, (float2*)out, (float2*)derivatives, L.g);
+        project_forw_saving_kernel<DIM, false, RECORDS><<<L.grid, kBlockThreads, 0, s>>>((const float2*)rec, rot, shifts, (float2*)out, (float2*)derivatives, L.g);
     return check_launch("project_forw (saving derivatives) launch");
 }
 
-template <int DIM>
+template <int DIM, bool RECORDS = false>
 int project_back_saved(const float* grad_proj, const float* out, const float* derivatives, int64_t B, int64_t R,
                        const float* rot, int64_t B_rot, const float* shifts, int64_t B_shift, int64_t P, int64_t N,
                        int interpolation, double os, double cutoff, float* grad_rec, float* grad_rot, float* grad_shifts,
@@ -269,10 +374,10 @@ int project_back_saved(const float* grad_proj, const float* out, const float* de
     const float2* d = (const float2*)derivatives;
     const bool cubic = interpolation == B200PROJ_CUBIC;
     if (grad_rec != nullptr) {
-        if (cubic) launch_project_back_saved<DIM, true, true>(L, s, gp, o, d, rot, shifts, (float2*)grad_rec, grad_rot, grad_shifts);
-        else launch_project_back_saved<DIM, false, true>(L, s, gp, o, d, rot, shifts, (float2*)grad_rec, grad_rot, grad_shifts);
+        if (cubic) launch_project_back_saved<DIM, true, true, RECORDS>(L, s, gp, o, d, rot, shifts, (float2*)grad_rec, grad_rot, grad_shifts);
+        else launch_project_back_saved<DIM, false, true, RECORDS>(L, s, gp, o, d, rot, shifts, (float2*)grad_rec, grad_rot, grad_shifts);
     } else {
-        launch_project_back_saved<DIM, false, false>(L, s, gp, o, d, rot, shifts, nullptr, grad_rot, grad_shifts);
+        launch_project_back_saved<DIM, false, false, RECORDS>(L, s, gp, o, d, rot, shifts, nullptr, grad_rot, grad_shifts);
     }
     return check_launch("project_back (saved derivatives) launch");
 }
@@ -589,6 +694,31 @@ int b200proj_project_3d_to_2d_forw(const float* rec, int64_t B, int64_t R, const
                                    int64_t N, int interpolation, double oversampling, double cutoff,
                                    float* out, const int32_t* pose_order, void* stream) {
     return project_forw<3>(rec, B, R, rot, B_rot, shifts, B_shift, P, N, interpolation, oversampling, cutoff, out, pose_order, stream);
+}
+
+size_t b200proj_project_workspace_bytes(int64_t B, int64_t P, int64_t N, int interpolation, int records, double oversampling, double cutoff) {
+    const BrickLaunch bl = brick_plan(B, P, N, interpolation == B200PROJ_CUBIC, records != 0, oversampling, cutoff);
+    return bl.use ? bl.bytes : 0;
+}
+int b200proj_project_3d_to_2d_forw_ws(const float* rec, int64_t B, int64_t R, const float* rot,
+                                      int64_t B_rot, const float* shifts, int64_t B_shift, int64_t P,
+                                      int64_t N, int interpolation, double oversampling, double cutoff,
+                                      float* out, const int32_t* pose_order, void* workspace, size_t workspace_bytes, void* stream) {
+    return project_forw<3>(rec, B, R, rot, B_rot, shifts, B_shift, P, N, interpolation, oversampling, cutoff, out, pose_order, stream, workspace, workspace_bytes);
+}
+int b200proj_project_3d_to_2d_forw_records(const float* rec, int64_t B, int64_t R, const float* rot,
+                                           int64_t B_rot, const float* shifts, int64_t B_shift, int64_t P,
+                                           int64_t N, int interpolation, double oversampling, double cutoff, float* out,
+                                           float* records, const int32_t* pose_order, void* workspace, size_t workspace_bytes, void* stream) {
+    return project_forw_saving<3, true>(rec, B, R, rot, B_rot, shifts, B_shift, P, N, interpolation, oversampling, cutoff, out, records, pose_order, stream, workspace, workspace_bytes);
+}
+int b200proj_project_3d_to_2d_back_records(const float* grad_proj, const float* out, const float* records,
+                                           int64_t B, int64_t R, const float* rot, int64_t B_rot,
+                                           const float* shifts, int64_t B_shift, int64_t P, int64_t N,
+                                           int interpolation, double oversampling, double cutoff,
+                                           float* grad_rec, float* grad_rot, float* grad_shifts,
+                                           const int32_t* pose_order, void* stream) {
+    return project_back_saved<3, true>(grad_proj, out, records, B, R, rot, B_rot, shifts, B_shift, P, N, interpolation, oversampling, cutoff, grad_rec, grad_rot, grad_shifts, pose_order, stream);
 }
 
 int b200proj_project_2d_back(const float* grad_proj, const float* rec, int64_t B, int64_t R,

@@ -1,0 +1,562 @@
+// Brick-stationary kernels of the 3D operators (fp32): the volume is cut into bricks that fit shared
+// memory, a block keeps one brick and walks over the slices, handling the pixels whose sample position
+// lies in its brick.  The plain kernels (fourier_slice_kernels.cuh) keep the pixels and fetch the taps
+// of every pixel through L1: 16 rows of a cubic footprint are 13 cache lines per pixel, and the L1TEX
+// data pipe retires about one a clock.  Here a brick is staged once per work item and the taps of all
+// its pixels, of all slices, come from shared memory without bank conflicts, 16 lanes = 128 bytes a
+// wavefront: 4 wavefronts per cubic pixel instead of 13-18.  Measured on B200: 10,000 slices of 128 x 65
+// from a box-256 volume, cubic, 3.95 -> 1.77 ms (62 -> 27 ps per pixel; data pipe 75 %, issue 69 %), with
+// records 8.9 -> 4.0 ms for 4,096 slices of 256 x 129 from a box-512 volume; linear 1.09 -> 1.02 ms.
+//
+// Bricks of 17 x 17 x 16 sample positions: with the halo of cubic taps 20 x 20 x 19 voxels = 61 KB, three
+// blocks (24 warps, 80 registers) per SM.  Smaller bricks meet a slice in too few pixels (here 40) to
+// pay for finding them.
+//
+// A call runs as two launches:
+//   brick_setup_kernel   per slice a 48-byte record (matrix, shift, plane normal); per brick its work items
+//   brick_*_kernel       persistent blocks take items (brick, range of slices) from a ticket counter
+// Nothing waits on another block.
+#pragma once
+
+#include "fourier_slice_kernels.cuh"
+
+namespace b200proj {
+
+constexpr int kBrickX = 17, kBrickY = 17, kBrickZ = 16;     // sample positions of a brick (units of voxels)
+constexpr int kBrickHits = 1024;                            // slices in the list of hits
+constexpr int kBrickSlots = 8;                              // slices a warp takes at a time
+constexpr float kBrickSlack = 0.06f;                        // slack of the linear estimates, in voxels
+
+// What the host derives from the sizes (see brick_plan in b200proj.cu).
+struct BrickPlan {
+    int n[3];               // bricks along x (column), y (row), z (plane)
+    int lo[3];              // first sample position of the grid
+    float ball;             // sample positions of a rotated slice lie inside this radius
+    float density;          // expected pixels per brick and slice at radius r: density / max(r, ...)
+    float target;           // pixels a work item should hold
+    int max_extra;          // items beyond one per brick that fit the list
+};
+
+// Workspace layout: int header[4] {items, extra, ticket, pixels outside the cutoff}, int4 items[bricks * B + max_extra],
+// float4 records[3 * B * P], int outside[N * Nh].
+struct BrickWork {
+    int* header;
+    int4* items;
+    float4* recs;
+    int* outside;
+};
+
+struct SliceRec {           // 48 bytes
+    float4 a;               // n.x, n.y, n.z (plane normal; NaN: the slice is not for the bricks), m00
+    float4 b;               // m10, m20, m01, m11
+    float4 c;               // m21, s0, s1, -
+};
+
+// A slice goes through the bricks when the two columns of its matrix that matter are orthonormal to 2e-5
+// (then its pixels stay inside the ball, and plane and half-plane tests with slack hold).
+__device__ __forceinline__ bool brick_slice_ok(const float* __restrict__ rm) {
+    const float a0 = __ldg(rm + 0), a1 = __ldg(rm + 3), a2 = __ldg(rm + 6);
+    const float b0 = __ldg(rm + 1), b1 = __ldg(rm + 4), b2 = __ldg(rm + 7);
+    const float aa = a0 * a0 + a1 * a1 + a2 * a2, bb = b0 * b0 + b1 * b1 + b2 * b2, ab = a0 * b0 + a1 * b1 + a2 * b2;
+    return fabsf(aa - 1.f) < 2e-5f && fabsf(bb - 1.f) < 2e-5f && fabsf(ab) < 2e-5f;
+}
+
+__device__ __forceinline__ bool brick_in_ball(const BrickPlan& pl, int bx, int by, int bz, float& r_center) {
+    const float x0 = (float)(pl.lo[0] + bx * kBrickX), y0 = (float)(pl.lo[1] + by * kBrickY), z0 = (float)(pl.lo[2] + bz * kBrickZ);
+    const float nx = fmaxf(fmaxf(x0, -(x0 + kBrickX)), 0.f), ny = fmaxf(fmaxf(y0, -(y0 + kBrickY)), 0.f), nz = fmaxf(fmaxf(z0, -(z0 + kBrickZ)), 0.f);
+    const float cx = x0 + 0.5f * kBrickX, cy = y0 + 0.5f * kBrickY, cz = z0 + 0.5f * kBrickZ;
+    r_center = sqrtf(cx * cx + cy * cy + cz * cz);
+    return nx * nx + ny * ny + nz * nz <= pl.ball * pl.ball;
+}
+
+// The pixels outside the cutoff, by one block: their offsets in a slice, row by row.
+__device__ __forceinline__ void brick_list_outside(const SliceGeom& g, BrickWork ws) {
+    __shared__ int row_at[2049];
+    // first column outside: rad is monotonic in j, the estimate is at most one column late
+    auto first_out = [&](int i) {
+        const float kr = (float)((i <= g.N / 2) ? i : i - g.N), kr2 = mul_rn(kr, kr), room = g.cutoff_sq - kr2;
+        int j = room > 0.f ? max(0, (int)fminf(sqrtf(room), (float)g.Nh) - 1) : 0;
+        while (j < g.Nh && !(add_rn(kr2, mul_rn((float)j, (float)j)) > g.cutoff_sq)) ++j;
+        return j;
+    };
+    for (int i = threadIdx.x; i < g.N; i += blockDim.x) row_at[i + 1] = g.Nh - first_out(i);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        row_at[0] = 0;
+        for (int i = 0; i < g.N; ++i) row_at[i + 1] += row_at[i];
+        ws.header[3] = row_at[g.N];
+    }
+    __syncthreads();
+    for (int i = threadIdx.x >> 5; i < g.N; i += (int)blockDim.x >> 5) {
+        const int at = row_at[i], n = row_at[i + 1] - at;
+        for (int q = threadIdx.x & 31; q < n; q += 32) ws.outside[at + q] = i * g.Nh + g.Nh - n + q;
+    }
+}
+
+// Slice records (one thread per slice) and work items (one thread per brick and batch item).  header[0..2]
+// are zero on entry.  A brick's slices are split over as many items as bring one near pl.target pixels for
+// uniformly distributed poses (the density of pixels falls as 1 / r); the list has room for one item per
+// brick plus max_extra, and a brick that finds no room for its extra items keeps a single one.
+// Neighbouring bricks are neighbours in the list, so that they run at the same time: the runs of pixels that
+// they write into a row of a slice then meet in L2 before the row's sectors leave it.
+__global__ void __launch_bounds__(256)
+brick_setup_kernel(const float* __restrict__ rot, const float* __restrict__ shifts, BrickWork ws, const SliceGeom g,
+                   const BrickPlan pl, int B) {
+    const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (t < g.BP) {
+        const int b = t / g.P, p = t - b * g.P;
+        const float* rm = pose_rot<3>(g, rot, b, p);
+        const float m00 = __ldg(rm + 0), m01 = __ldg(rm + 1), m10 = __ldg(rm + 3), m11 = __ldg(rm + 4), m20 = __ldg(rm + 6), m21 = __ldg(rm + 7);
+        float s0 = 0.f, s1 = 0.f;
+        if (g.has_shift) {
+            const float* s = pose_shift(g, shifts, b, p);
+            s0 = __ldg(s);
+            s1 = __ldg(s + 1);
+        }
+        float nx = m10 * m21 - m20 * m11;
+        const float ny = m20 * m01 - m00 * m21, nz = m00 * m11 - m10 * m01;
+        if (!brick_slice_ok(rm)) nx = __int_as_float(0x7fffffff);
+        ws.recs[3 * t + 0] = make_float4(nx, ny, nz, m00);
+        ws.recs[3 * t + 1] = make_float4(m10, m20, m01, m11);
+        ws.recs[3 * t + 2] = make_float4(m21, s0, s1, 0.f);
+    }
+    if (blockIdx.x == gridDim.x - 1) {
+        brick_list_outside(g, ws);
+        return;
+    }
+    // work items: a block takes a cluster of 8 x 8 x 4 neighbouring bricks of one batch item
+    __shared__ int warp_sum[8], block_at;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int cx = (pl.n[0] + 7) / 8, cy = (pl.n[1] + 7) / 8, cz = (pl.n[2] + 3) / 4;
+    if ((int)blockIdx.x >= cx * cy * cz * B) return;
+    const int b = (int)blockIdx.x / (cx * cy * cz), k = (int)blockIdx.x - b * (cx * cy * cz);
+    const int bx = k % cx * 8 + (threadIdx.x & 7), by = k / cx % cy * 8 + (threadIdx.x >> 3 & 7), bz = k / (cx * cy) * 4 + (threadIdx.x >> 6);
+    int parts = 0;
+    float r;
+    if (bx < pl.n[0] && by < pl.n[1] && bz < pl.n[2] && brick_in_ball(pl, bx, by, bz, r)) {
+        const float expected = pl.density / fmaxf(r, 0.42f * kBrickX) * (float)g.P;
+        parts = max(1, min((int)(expected / pl.target + 0.5f), (g.P + 31) / 32));
+        if (parts > 1 && atomicAdd(ws.header + 1, parts - 1) + parts - 1 > pl.max_extra) parts = 1;
+    }
+    int incl = parts;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += up;
+    }
+    if (lane == 31) warp_sum[warp] = incl;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int sum = 0;
+        for (int w = 0; w < 8; ++w) { const int n = warp_sum[w]; warp_sum[w] = sum; sum += n; }
+        block_at = atomicAdd(ws.header, sum);
+    }
+    __syncthreads();
+    const int at = block_at + warp_sum[warp] + incl - parts;
+    for (int q = 0; q < parts; ++q)
+        ws.items[at + q] = make_int4(bx | by << 10 | bz << 20, b, b * g.P + (int)((long long)g.P * q / parts), b * g.P + (int)((long long)g.P * (q + 1) / parts));
+}
+
+// Shared-memory layout of a staged brick: 4 x 4 cells of (x, y) are contiguous, so that the place of a voxel
+// modulo 16 is its class (x & 3) + 4 (y & 3).  A cubic footprint holds every class once per plane; lane l takes
+// the columns and rows of its footprint in an order that starts at class (l & 3, (l >> 2) & 3), so that at
+// every step the 16 lanes of a half-warp hold 16 different classes = 16 different 8-byte banks, wherever
+// their pixels lie.
+template <bool CUBIC>
+struct BrickShape {
+    static constexpr int T = CUBIC ? 4 : 2;
+    static constexpr int TX = ((kBrickX + T - 1) + 3) / 4 * 4, TY = ((kBrickY + T - 1) + 3) / 4 * 4, TZ = kBrickZ + T - 1;
+    static constexpr int kRowCells = TX / 4 * 16;            // voxels of four rows
+    static constexpr int kPlane = TX * TY;
+    static constexpr int kVoxels = kPlane * TZ;
+};
+__device__ __forceinline__ int brick_off_x(int x) { return x + 12 * (x >> 2); }
+template <bool CUBIC>
+__device__ __forceinline__ int brick_off_y(int y) { return 4 * (y & 3) + BrickShape<CUBIC>::kRowCells * (y >> 2); }
+
+// Stage the brick: voxel (x, y, z) of it is tap (X0 - o + x, Y0 - o + y, Z0 - o + z), o = 1 for cubic, read with
+// the gather's rules (Friedel mirror with conjugation, clamping), so that edges need no further care.
+template <bool CUBIC>
+__device__ __forceinline__ void brick_stage(const SliceGeom& g, const float2* __restrict__ vol, float2* sm, int X0, int Y0, int Z0) {
+    using S = BrickShape<CUBIC>;
+    constexpr int o = CUBIC ? 1 : 0, kRows = kBlockThreads / S::TX;      // rows staged at a time
+    const int x = (int)threadIdx.x % S::TX, first = (int)threadIdx.x / S::TX;
+    if (first >= kRows) return;
+    bool m;
+    const int col = gather_col<CUBIC>(g, X0 - o + x, m);
+    const int ox = brick_off_x(x);
+    int y = first, z = 0;
+#pragma unroll 4
+    for (int n = first; n < S::TY * S::TZ; n += kRows) {
+        const int row = gather_line<CUBIC>(g, Y0 - o + y, m), pln = gather_line<CUBIC>(g, Z0 - o + z, m);
+        float2 v = __ldg(vol + ((pln * g.R + row) * g.Rh + col));
+        if (m) v.y = -v.y;
+        sm[z * S::kPlane + brick_off_y<CUBIC>(y) + ox] = v;
+        y += kRows;
+        if (y >= S::TY) { y -= S::TY; ++z; }
+    }
+}
+
+template <typename F>
+__device__ __forceinline__ void rotate4(F (&w)[4], int t0) {      // w[s] <- w[(s + t0) & 3]
+    if (t0 & 1) { const F x = w[0]; w[0] = w[1]; w[1] = w[2]; w[2] = w[3]; w[3] = x; }
+    if (t0 & 2) { F x = w[0]; w[0] = w[2]; w[2] = x; x = w[1]; w[1] = w[3]; w[3] = x; }
+}
+
+__device__ __forceinline__ unsigned long long fmul2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// Value (and derivatives) at (lx + fx, ly + fy, lz + fz) of the staged brick, all of it in this lane.
+template <bool CUBIC, bool WITH_DERIV>
+__device__ __forceinline__ void brick_gather(const float2* sm, int lx, int ly, int lz, float fx, float fy, float fz,
+                                             float2& val, float2& gc, float2& gr, float2& gd) {
+    using S = BrickShape<CUBIC>;
+    using u64 = unsigned long long;
+    const int lane = threadIdx.x & 31;
+    constexpr int T = S::T;
+    int ox[T], oy[T];                // byte offsets of the columns and rows, in this lane's order
+    u64 wx[T], wy[T], wz[T], dx[T], dy[T], dz[T];
+    const int base = (lz * S::kPlane + (ly >> 2) * S::kRowCells + (lx >> 2) * 16) * 8;
+    if constexpr (CUBIC) {
+        // the tap of class a lies in the first cell of the footprint when a >= (first tap's class), else in the next one
+        float w[4];
+        const int rx = lx & 3, ry = ly & 3, tx = (lane - lx) & 3, ty = ((lane >> 2) - ly) & 3;
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            const int ax = (lane + s) & 3, ay = ((lane >> 2) + s) & 3;
+            ox[s] = ax * 8 + (ax < rx ? 128 : 0) + base;
+            oy[s] = ay * 32 + (ay < ry ? S::kRowCells * 8 : 0);
+        }
+        cubic_weights(fx, w);
+        rotate4(w, tx);
+#pragma unroll
+        for (int s = 0; s < 4; ++s) wx[s] = pack2(w[s], w[s]);
+        cubic_weights(fy, w);
+        rotate4(w, ty);
+#pragma unroll
+        for (int s = 0; s < 4; ++s) wy[s] = pack2(w[s], w[s]);
+        cubic_weights(fz, w);
+#pragma unroll
+        for (int s = 0; s < 4; ++s) wz[s] = pack2(w[s], w[s]);
+        if (WITH_DERIV) {
+            cubic_dweights(fx, w);
+            rotate4(w, tx);
+#pragma unroll
+            for (int s = 0; s < 4; ++s) dx[s] = pack2(w[s], w[s]);
+            cubic_dweights(fy, w);
+            rotate4(w, ty);
+#pragma unroll
+            for (int s = 0; s < 4; ++s) dy[s] = pack2(w[s], w[s]);
+            cubic_dweights(fz, w);
+#pragma unroll
+            for (int s = 0; s < 4; ++s) dz[s] = pack2(w[s], w[s]);
+        }
+    } else {
+        ox[0] = base + (lx & 3) * 8;
+        ox[1] = ox[0] + ((lx & 3) == 3 ? 128 - 24 : 8);
+        oy[0] = (ly & 3) * 32;
+        oy[1] = oy[0] + ((ly & 3) == 3 ? S::kRowCells * 8 - 96 : 32);
+        wx[0] = pack2(1.f - fx, 1.f - fx); wx[1] = pack2(fx, fx);
+        wy[0] = pack2(1.f - fy, 1.f - fy); wy[1] = pack2(fy, fy);
+        wz[0] = pack2(1.f - fz, 1.f - fz); wz[1] = pack2(fz, fz);
+        dx[0] = dy[0] = dz[0] = pack2(-1.f, -1.f);
+        dx[1] = dy[1] = dz[1] = pack2(1.f, 1.f);
+    }
+    const char* smb = reinterpret_cast<const char*>(sm);
+    u64 v2 = 0ull, c2 = 0ull, r2 = 0ull, d2 = 0ull;
+#pragma unroll
+    for (int a = 0; a < T; ++a) {
+        u64 A = 0ull, Bq = 0ull, Dq = 0ull;
+#pragma unroll
+        for (int b = 0; b < T; ++b) {
+            const char* col = smb + (ox[a] + oy[b]);
+            u64 s = 0ull, sd = 0ull;
+#pragma unroll
+            for (int k = 0; k < T; ++k) {
+                const u64 v = *reinterpret_cast<const u64*>(col + k * S::kPlane * 8);
+                s = fma2(wz[k], v, s);
+                if (WITH_DERIV) sd = fma2(dz[k], v, sd);
+            }
+            A = fma2(wy[b], s, A);
+            if (WITH_DERIV) {
+                Bq = fma2(dy[b], s, Bq);
+                Dq = fma2(wy[b], sd, Dq);
+            }
+        }
+        v2 = fma2(wx[a], A, v2);
+        if (WITH_DERIV) {
+            c2 = fma2(dx[a], A, c2);
+            r2 = fma2(wx[a], Bq, r2);
+            d2 = fma2(wx[a], Dq, d2);
+        }
+    }
+    unpack2(v2, val.x, val.y);
+    if (WITH_DERIV) {
+        unpack2(c2, gc.x, gc.y);
+        unpack2(r2, gr.x, gr.y);
+        unpack2(d2, gd.x, gd.y);
+    }
+}
+
+// A warp's working set of the slice walk.
+struct BrickWarp {
+    uint2 segs[64];                 // rows of slices: {slot << 16 | (kr & 0xffff), ja << 16 | length}
+    float4 slots[kBrickSlots][3];   // the slices' records
+    int slice[kBrickSlots];         // and their indices
+};
+
+struct BrickBlock {
+    int nhits, next, item;
+    int hits[kBrickHits];           // slices whose half-plane meets the brick
+    BrickWarp warp[kWarps];
+};
+
+// The slice walk of one work item: calls body(active, slice record slot, i, j, pixel, lx, ly, lz) with all 32
+// lanes for windows of 32 candidate pixels; `active` lanes hold a pixel whose sample position lies in the brick.
+// Every pixel of the item's slices inside the brick is visited exactly once.
+//   1. all threads test the slices' planes (and half-planes: columns j >= 0 only) against the brick,
+//   2. a warp takes a few slices from the list of hits and flattens their rows, one row per lane: row kr meets the
+//      brick in one run of columns, clipped with linear estimates plus slack,
+//   3. the non-empty runs of 32 rows are flattened into one index space, so that the windows are full although
+//      a slice has only some 40 pixels in a brick and a row 5; each candidate is then tested exactly.
+template <typename Body>
+__device__ __forceinline__ void brick_walk(const SliceGeom& g, const float4* __restrict__ recs, BrickBlock& sb,
+                                           int X0, int Y0, int Z0, int first, int last, Body body) {
+    constexpr unsigned kFull = 0xffffffffu;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned upto = 0xffffffffu >> (31 - lane);               // lanes up to this one
+    BrickWarp& sw = sb.warp[warp];
+    const float hx = 0.5f * kBrickX, hy = 0.5f * kBrickY, hz = 0.5f * kBrickZ;
+    const float cx = (float)X0 + hx, cy = (float)Y0 + hy, cz = (float)Z0 + hz;
+    const float osf = (float)g.os, inv_os = 1.f / osf;
+    const int grab = max(1, min(kBrickSlots, (int)(2.f * osf)));       // slices with about 32 rows in the brick
+    for (int k_next = first; k_next < last;) {
+        __syncthreads();
+        if (threadIdx.x == 0) { sb.nhits = 0; sb.next = 0; }
+        __syncthreads();
+        int nhits = 0;
+        do {            // as many slices as the list of hits has room for, whatever the tests say
+            const int k_end = min(last, k_next + (kBrickHits - nhits) / kBlockThreads * kBlockThreads);
+            for (; k_next < k_end; k_next += kBlockThreads) {
+                const int k = k_next + (int)threadIdx.x;
+                bool hit = false;
+                if (k < k_end) {
+                    const float4 a = __ldg(recs + 3 * (size_t)k);
+                    hit = fabsf(a.x * cx + a.y * cy + a.z * cz) <= fabsf(a.x) * hx + fabsf(a.y) * hy + fabsf(a.z) * hz + kBrickSlack;
+                    if (hit) {
+                        const float2 e = __ldg(reinterpret_cast<const float2*>(recs + 3 * (size_t)k + 1));
+                        hit = a.w * cx + e.x * cy + e.y * cz + fabsf(a.w) * hx + fabsf(e.x) * hy + fabsf(e.y) * hz >= -kBrickSlack;
+                    }
+                }
+                const unsigned m = __ballot_sync(kFull, hit);
+                int pos = 0;
+                if (lane == 0 && m) pos = atomicAdd(&sb.nhits, __popc(m));
+                pos = __shfl_sync(kFull, pos, 0);
+                if (hit) sb.hits[pos + __popc(m & upto) - 1] = k;
+            }
+            k_next = k_end;
+            __syncthreads();
+            nhits = sb.nhits;
+            __syncthreads();
+        } while (k_next < last && nhits + kBlockThreads <= kBrickHits);
+        while (true) {
+            int h = 0;
+            if (lane == 0) h = atomicAdd(&sb.next, grab);
+            h = __shfl_sync(kFull, h, 0);
+            if (h >= nhits) break;
+            const int slices = min(grab, nhits - h);
+            int row_count = 0, k_lo = 0;
+            if (lane < slices) {
+                const int slice = sb.hits[h + lane];
+                const float4 a = __ldg(recs + 3 * (size_t)slice), e = __ldg(recs + 3 * (size_t)slice + 1), f = __ldg(recs + 3 * (size_t)slice + 2);
+                sw.slice[lane] = slice;
+                sw.slots[lane][0] = a;
+                sw.slots[lane][1] = e;
+                sw.slots[lane][2] = f;
+                const float mid = e.z * cx + e.w * cy + f.x * cz, reach = fabsf(e.z) * hx + fabsf(e.w) * hy + fabsf(f.x) * hz + kBrickSlack;
+                k_lo = max((int)ceilf((mid - reach) * inv_os), 1 - g.N / 2);
+                row_count = max(1, min((int)floorf((mid + reach) * inv_os), g.N / 2) - k_lo + 1);
+            }
+            int row_incl = row_count;
+#pragma unroll
+            for (int o = 1; o < kBrickSlots; o <<= 1) {
+                const int up = __shfl_up_sync(kFull, row_incl, o);
+                if (lane >= o) row_incl += up;
+            }
+            const int row_start = row_incl - row_count, rows = __shfl_sync(kFull, row_incl, kBrickSlots - 1);
+            const int kr_start = k_lo - row_start;
+            __syncwarp();
+            int nseg = 0, row0 = 0, slots_before = 0;
+            while (true) {
+            while (row0 < rows && nseg < 32) {
+                const unsigned starts = __reduce_or_sync(kFull, (lane < slices && row_start >= row0 && row_start < row0 + 32) ? 1u << (row_start - row0) : 0u);
+                const int slot = slots_before + __popc(starts & upto) - 1;
+                slots_before += __popc(starts);
+                const int kr = row0 + lane + __shfl_sync(kFull, kr_start, slot);
+                const float krf = (float)kr;
+                const float4 ra = sw.slots[slot][0], rb = sw.slots[slot][1];
+                const float m21 = sw.slots[slot][2].x;
+                const float room = g.cutoff_sq - krf * krf;
+                int ja_i = 0, len = 0;
+                if (row0 + lane < rows && room >= 0.f) {
+                    float ja = 0.f, jb = fminf((float)(g.Nh - 1), sqrtf(room) + 0.01f);
+                    auto clip = [&](float a, float b, float lo, float n) {
+                        a *= osf;
+                        b *= osf * krf;
+                        if (fabsf(a) < 1e-5f) {
+                            if (b < lo - kBrickSlack || b > lo + n + kBrickSlack) jb = -1.f;
+                        } else {
+                            const float ia = __fdividef(1.f, a);
+                            const float x0 = (lo - kBrickSlack - b) * ia, x1 = (lo + n + kBrickSlack - b) * ia;
+                            ja = fmaxf(ja, fminf(x0, x1));
+                            jb = fminf(jb, fmaxf(x0, x1));
+                        }
+                    };
+                    clip(ra.w, rb.z, (float)X0, (float)kBrickX);
+                    clip(rb.x, rb.w, (float)Y0, (float)kBrickY);
+                    clip(rb.y, m21, (float)Z0, (float)kBrickZ);
+                    ja_i = (int)ceilf(ja);
+                    len = jb >= ja ? (int)floorf(jb) - ja_i + 1 : 0;
+                }
+                const unsigned have = __ballot_sync(kFull, len > 0);
+                if (len > 0) sw.segs[nseg + __popc(have & upto) - 1] = make_uint2((unsigned)slot << 16 | ((unsigned)kr & 0xffffu), (unsigned)ja_i << 16 | (unsigned)len);
+                nseg += __popc(have);
+                row0 += 32;
+            }
+            if (nseg == 0) break;
+            __syncwarp();
+            const int take = min(nseg, 32);
+            const uint2 seg = lane < take ? sw.segs[lane] : make_uint2(0u, 0u);
+            const int len = (int)(seg.y & 0xffffu);
+            int incl = len;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int up = __shfl_up_sync(kFull, incl, o);
+                if (lane >= o) incl += up;
+            }
+            const int total = __shfl_sync(kFull, incl, 31), start = incl - len;
+            const int ja_start = (int)(seg.y >> 16) - start;
+            int before = 0;                                           // segments that start before the window
+            for (int k0 = 0; k0 < total; k0 += 32) {
+                const unsigned bit = (len > 0 && start >= k0 && start < k0 + 32) ? 1u << (start - k0) : 0u;
+                const unsigned starts = __reduce_or_sync(kFull, bit);
+                const int src = before + __popc(starts & upto) - 1;
+                before += __popc(starts);
+                const unsigned sk = __shfl_sync(kFull, seg.x, src);
+                const int j = k0 + lane + __shfl_sync(kFull, ja_start, src);
+                const int kr = (int)(short)(sk & 0xffffu), slot = (int)(sk >> 16);
+                const float4 ra = sw.slots[slot][0], rb = sw.slots[slot][1];
+                const float m21 = sw.slots[slot][2].x;
+                Pixel px;
+                px.kr = (float)kr;
+                px.kc = (float)j;
+                if (g.os_is_float) {
+                    px.sc = mul_rn(px.kc, g.os_f);
+                    px.sr = mul_rn(px.kr, g.os_f);
+                } else {
+                    px.sc = (float)((double)px.kc * g.os);
+                    px.sr = (float)((double)px.kr * g.os);
+                }
+                px.c = add_rn(mul_rn(ra.w, px.sc), mul_rn(rb.z, px.sr));
+                px.r = add_rn(mul_rn(rb.x, px.sc), mul_rn(rb.w, px.sr));
+                px.d = add_rn(mul_rn(rb.y, px.sc), mul_rn(m21, px.sr));
+                int lx = (int)floorf(px.c) - X0, ly = (int)floorf(px.r) - Y0, lz = (int)floorf(px.d) - Z0;
+                const float rad = add_rn(mul_rn(px.kr, px.kr), mul_rn(px.kc, px.kc));
+                const bool active = k0 + lane < total && (unsigned)lx < (unsigned)kBrickX && (unsigned)ly < (unsigned)kBrickY &&
+                                    (unsigned)lz < (unsigned)kBrickZ && !(rad > g.cutoff_sq);
+                if (!active) lx = ly = lz = 0;
+                body(active, slot, kr < 0 ? kr + g.N : kr, j, px, lx, ly, lz);
+            }
+            nseg -= take;
+            const uint2 rest = lane < nseg ? sw.segs[take + lane] : make_uint2(0u, 0u);
+            __syncwarp();
+            if (lane < nseg) sw.segs[lane] = rest;
+            __syncwarp();
+            }
+        }
+    }
+}
+
+// What the bricks leave of a slice: zeros outside the cutoff, or -- when its matrix is not (nearly) a rotation, so
+// that its pixels may lie anywhere -- the whole slice, by the plain gather.
+template <bool CUBIC, bool SAVE>
+__device__ __forceinline__ void brick_rest(const SliceGeom& g, const BrickWork& ws, int k, const float2* __restrict__ rec, const float* __restrict__ rot,
+                                           const float* __restrict__ shifts, float2* __restrict__ out, float2* __restrict__ derivs) {
+    const int b = k / g.P, p = k - b * g.P;
+    const float* rm = pose_rot<3>(g, rot, b, p);
+    const size_t base = (size_t)k * (size_t)g.slice_pixels;
+    if (brick_slice_ok(rm)) {
+        const int n = __ldg(ws.header + 3);
+        for (int q = threadIdx.x; q < n; q += kBlockThreads) __stcs(out + (base + (size_t)__ldg(ws.outside + q)), make_float2(0.f, 0.f));
+        return;
+    }
+    for (int tile = 0; tile < g.tiles_i * g.tiles_j; ++tile) {
+        int i, j;
+        tile_pixel(g, tile, i, j);
+        Pixel px;
+        px.c = px.r = px.d = 0.f;
+        const bool in_image = i < g.N && j < g.Nh;
+        const bool valid = in_image && pixel_setup<3>(g, rm, i, j, px);
+        float2 v, gc, gr, gd;
+        interpolate_any<3, CUBIC, SAVE>(g, rec + (size_t)b * g.vol_elems, px, valid, v, gc, gr, gd);
+        if (!in_image) continue;
+        float2 ph = make_float2(1.f, 0.f);
+        if (valid && g.has_shift) {
+            const float* s = pose_shift(g, shifts, b, p);
+            ph = phase_ramp(g, px, __ldg(s), __ldg(s + 1));
+            v = cmul(v, ph);
+        }
+        const size_t pix = base + (size_t)(i * g.Nh + j);
+        __stcs(out + pix, v);
+        if (SAVE && valid) store_record(derivs + 4 * pix, g.has_shift ? cmul(gc, ph) : gc, g.has_shift ? cmul(gr, ph) : gr, g.has_shift ? cmul(gd, ph) : gd, v);
+    }
+}
+
+// Forward projection (SAVE: with the records of project_forw_saving_kernel).
+template <bool CUBIC, bool SAVE>
+__global__ void __launch_bounds__(kBlockThreads, 3)
+brick_forw_kernel(const float2* __restrict__ rec, const float* __restrict__ rot, const float* __restrict__ shifts,
+                  float2* __restrict__ out, float2* __restrict__ derivs, BrickWork ws, const SliceGeom g, const BrickPlan pl) {
+    extern __shared__ __align__(16) unsigned char dyn[];
+    float2* sm = reinterpret_cast<float2*>(dyn);
+    BrickBlock& sb = *reinterpret_cast<BrickBlock*>(dyn + sizeof(float2) * BrickShape<CUBIC>::kVoxels);
+    const int items = __ldg(ws.header);
+    while (true) {
+        __syncthreads();
+        if (threadIdx.x == 0) sb.item = atomicAdd(ws.header + 2, 1);
+        __syncthreads();
+        const int item = sb.item;
+        if (item >= items) return;
+        // beside its brick an item does its share of the slices' rest, whose stores overlap the brick's staging
+        for (int k = (int)((long long)g.BP * item / items), k_end = (int)((long long)g.BP * (item + 1) / items); k < k_end; ++k)
+            brick_rest<CUBIC, SAVE>(g, ws, k, rec, rot, shifts, out, derivs);
+        const int4 it = __ldg(ws.items + item);
+        const int X0 = pl.lo[0] + (it.x & 1023) * kBrickX, Y0 = pl.lo[1] + ((it.x >> 10) & 1023) * kBrickY, Z0 = pl.lo[2] + (it.x >> 20) * kBrickZ;
+        brick_stage<CUBIC>(g, rec + (size_t)it.y * g.vol_elems, sm, X0, Y0, Z0);
+        const BrickWarp& sw = sb.warp[threadIdx.x >> 5];
+        brick_walk(g, ws.recs, sb, X0, Y0, Z0, it.z, it.w,
+                   [&](bool active, int slot, int i, int j, const Pixel& px, int lx, int ly, int lz) {
+            float2 v, gc, gr, gd;
+            brick_gather<CUBIC, SAVE>(sm, lx, ly, lz, px.c - floorf(px.c), px.r - floorf(px.r), px.d - floorf(px.d), v, gc, gr, gd);
+            if (!active) return;
+            if (g.has_shift) {
+                const float4 rc = sw.slots[slot][2];
+                const float2 ph = phase_ramp(g, px, rc.y, rc.z);
+                v = cmul(v, ph);
+                if (SAVE) {
+                    gc = cmul(gc, ph);
+                    gr = cmul(gr, ph);
+                    gd = cmul(gd, ph);
+                }
+            }
+            const size_t pix = (size_t)sw.slice[slot] * (size_t)g.slice_pixels + (size_t)(i * g.Nh + j);
+            __stcg(out + pix, v);
+            if (SAVE) store_record(derivs + 4 * pix, gc, gr, gd, v);
+        });
+    }
+}
+
+}  // namespace b200proj

@@ -8,10 +8,9 @@
 //    (csrc/cpu/3d/projection_3d_to_2d_kernels.cpp:163-188): k*os is formed in double and
 //    rounded once, the rotation is separately rounded fp32 multiplies and adds (no FMA),
 //    so floor() and the fractional parts agree bit for bit with the CPU result;
-//  * the phase of the shift ramp is float(double(float(kr*s0 + kc*s1)) * (-2*pi/N))
-//    (csrc/cpu/common/projection_utils.h:82-94); fp32: reduced to about [-pi, pi] by a
-//    two-constant Cody-Waite step in fp32 and evaluated with the hardware sin/cos
-//    (see phase_sincos); fp64: the library sincos;
+//  * the phase of the shift ramp is (kr*s0 + kc*s1) * (-2*pi/N) with the dot product rounded to float
+//    (csrc/cpu/common/projection_utils.h:82-94); fp32: reduced by whole periods, exactly, and
+//    evaluated with the hardware sin/cos (see phase_of_dot); fp64: the library sincos;
 //  * tap sums are re-associated (separable form); that moves results by ~1e-7 relative.
 #pragma once
 
@@ -74,6 +73,7 @@ struct SliceGeom {
     float cutoff_sq;        // (float(cutoff))^2, the fp32 path compares in float as the reference does
     double cutoff_sq_d;     // cutoff^2 for the fp64 path
     double os;              // oversampling factor
+    float n_f, inv_n, phase_scale_f;    // N, 1 / N and -2*pi / N in single precision
     double phase_scale;     // -2*pi / float(N)
     double shift_scale;     // -2*pi / N   (d phase / d shift per unit frequency)
     long long vol_elems;    // voxels per batch item
@@ -137,30 +137,24 @@ __device__ __forceinline__ bool pixel_setup(const SliceGeom& g, const R* __restr
     return true;
 }
 
-// sin and cos of a phase of tens of radians.  fp32: the phase (already rounded to float as the
-// reference rounds it) is reduced to about [-pi, pi] with a two-constant Cody-Waite step in
-// fp32 (2*pi = 6.28125 + 1.9353072e-3: the first product is exact for |k| < 2^16, so the
-// reduced argument is good to ~1e-7), then evaluated with the hardware approximations, whose
-// absolute error there (< 5e-7) is below the fp32 noise of the interpolated value it
-// multiplies; this replaces ~40 instructions of sincosf's full-range path by 6.  fp64: the
-// accurate library routine.
-__device__ __forceinline__ void phase_sincos(float ph, float* sn, float* cs) {
-    const float k = rintf(ph * 0.15915494309189535f);               // 1 / (2*pi)
-    float r = fmaf(k, -6.28125f, ph);
-    r = fmaf(k, -1.9353071795864769e-3f, r);
-    *sn = __sinf(r);
-    *cs = __cosf(r);
+// exp(-2*pi*i*(kr*s0 + kc*s1)/N) as (cos, sin).  fp32: the dot product (rounded as the reference rounds it)
+// is reduced by whole periods, which one fused multiply-add does exactly (k * N and the difference are
+// representable), so the only rounding is that of the angle in [-pi, pi]; sine and cosine are the hardware
+// approximations, whose absolute error there (< 5e-7) is below the fp32 noise of the interpolated value
+// that they multiply.  fp64: the library's sincos of the unreduced phase.
+__device__ __forceinline__ float2 phase_of_dot(const SliceGeom& g, float dot) {
+    const float k = rintf(dot * g.inv_n);
+    const float angle = fmaf(-k, g.n_f, dot) * g.phase_scale_f;
+    return make_float2(__cosf(angle), __sinf(angle));
 }
-__device__ __forceinline__ void phase_sincos(double ph, double* sn, double* cs) { sincos(ph, sn, cs); }
-
-// exp(-2*pi*i*(kr*s0 + kc*s1)/N) as (cos, sin).
+__device__ __forceinline__ double2 phase_of_dot(const SliceGeom& g, double dot) {
+    double sn, cs;
+    sincos(dot * g.phase_scale, &sn, &cs);
+    return make_double2(cs, sn);
+}
 template <typename R>
 __device__ __forceinline__ C2<R> phase_ramp(const SliceGeom& g, const PixelT<R>& px, R s0, R s1) {
-    const R dot = add_rn(mul_rn(px.kr, s0), mul_rn(px.kc, s1));
-    const R ph = (R)((double)dot * g.phase_scale);
-    R sn, cs;
-    phase_sincos(ph, &sn, &cs);
-    return make2<R>(cs, sn);
+    return phase_of_dot(g, add_rn(mul_rn(px.kr, s0), mul_rn(px.kc, s1)));
 }
 
 template <typename V>

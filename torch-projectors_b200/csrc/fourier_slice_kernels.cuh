@@ -119,7 +119,12 @@ project_forw_kernel(const C2<R>* __restrict__ rec, const R* __restrict__ rot,
 // gather (project_back_saved_kernel): the rotation gradient of a pixel is
 // Re(grad * conj(derivative)) * sample frequency, the same numbers project_back_kernel forms from a
 // second gather of the volume.  Pixels outside the cutoff are not written (and never read).
-template <int DIM, bool CUBIC>
+// RECORDS: one 32-byte record (d/dc, d/dr, d/dd, pixel) per pixel instead, [B, P, N, Nh, 4]: a whole
+// sector, so that writers whose pixels lie in short runs (brick_forw_kernel) never leave part of one.
+__device__ __forceinline__ void store_record(float2* p, float2 a, float2 b, float2 c, float2 d) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y), "f"(d.x), "f"(d.y) : "memory");
+}
+template <int DIM, bool CUBIC, bool RECORDS = false>
 __global__ void __launch_bounds__(kBlockThreads)
 project_forw_saving_kernel(const float2* __restrict__ rec, const float* __restrict__ rot,
                            const float* __restrict__ shifts, float2* __restrict__ out,
@@ -140,7 +145,9 @@ project_forw_saving_kernel(const float2* __restrict__ rec, const float* __restri
         if (DIM == 3) gd = cmul(gd, ph);
     }
     __stcs(out + w.pix, v);
-    if (valid) {
+    if (RECORDS) {
+        if (valid) store_record(derivs + 4 * w.pix, gc, gr, gd, v);
+    } else if (valid) {
         const size_t plane = (size_t)g.BP * (size_t)g.slice_pixels;
         __stcs(derivs + w.pix, gc);
         __stcs(derivs + plane + w.pix, gr);
@@ -221,11 +228,7 @@ project_forw_rows2_kernel(const C2<R>* __restrict__ rec, const R* __restrict__ r
         interpolate_any<DIM, false, false>(g, vol, px, valid, v, gc, gr, gd);      // all 32 lanes take part
         if (!in_image) continue;
         if (valid && g.has_shift) {
-            const R dot = add_rn(mul_rn(px.kr, s0), kc_s1);
-            const R ph = (R)((double)dot * g.phase_scale);
-            R sn, cs;
-            phase_sincos(ph, &sn, &cs);
-            v = cmul(v, make2<R>(cs, sn));
+            v = cmul(v, phase_of_dot(g, add_rn(mul_rn(px.kr, s0), kc_s1)));
         }
         __stcs(out + (slice_base + (size_t)(i * g.Nh + j)), v);
     }
@@ -335,7 +338,7 @@ project_back_kernel(const C2<R>* __restrict__ grad_proj, const C2<R>* __restrict
 // Backward of project_forw_saving_kernel: pose gradients from the saved derivatives and output
 // (Re(grad * conj(derivative)) for the rotation, Im(grad * conj(output)) for the shift: the shift
 // phase cancels in both), then the same scatter of the gradient into the volume (NEED_REC).
-template <int DIM, bool CUBIC, bool NEED_ROT, bool NEED_SHIFT, bool NEED_REC>
+template <int DIM, bool CUBIC, bool NEED_ROT, bool NEED_SHIFT, bool NEED_REC, bool RECORDS = false>
 __global__ void __launch_bounds__(kBlockThreads)
 project_back_saved_kernel(const float2* __restrict__ grad_proj, const float2* __restrict__ out,
                           const float2* __restrict__ derivs, const float* __restrict__ rot,
@@ -355,9 +358,13 @@ project_back_saved_kernel(const float2* __restrict__ grad_proj, const float2* __
         u = __ldcs(grad_proj + w.pix);
         if (NEED_ROT) {
             const size_t plane = (size_t)g.BP * (size_t)g.slice_pixels;
+            const float4* rec4 = reinterpret_cast<const float4*>(derivs + 4 * w.pix);
+            const float4 cr = RECORDS ? __ldcs(rec4) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
             for (int a = 0; a < DIM; ++a) {
-                const float2 d = __ldcs(derivs + (size_t)a * plane + w.pix);
+                float2 d;
+                if (RECORDS) d = a == 0 ? make_float2(cr.x, cr.y) : a == 1 ? make_float2(cr.z, cr.w) : __ldcs(reinterpret_cast<const float2*>(rec4 + 1));
+                else d = __ldcs(derivs + (size_t)a * plane + w.pix);
                 const float dot = u.x * d.x + u.y * d.y;
                 acc[2 * a + 0] = dot * px.sc;
                 acc[2 * a + 1] = dot * px.sr;

@@ -153,6 +153,15 @@ Tensor resolve_order(int dim, const Tensor& vol, int64_t B, const Poses& p, cons
     return plane_locality_order(p.rot, B);
 }
 
+// Scratch of the brick-by-brick 3D projection (complex64), undefined when the plain kernels are the better choice.
+Tensor project_workspace(int dim, const Tensor& rec, int64_t P, int64_t N, int interp, bool records, double oversampling, double cutoff) {
+    if (dim != 3 || is_f64(rec)) return Tensor();
+    const size_t bytes = b200proj_project_workspace_bytes(rec.size(0), P, N, interp, records ? 1 : 0, oversampling, cutoff);
+    return bytes ? at::empty({(int64_t)bytes}, rec.options().dtype(at::kByte)) : Tensor();
+}
+inline void* ws_ptr(const Tensor& ws) { return ws.defined() ? ws.data_ptr() : nullptr; }
+inline size_t ws_size(const Tensor& ws) { return ws.defined() ? (size_t)ws.numel() : 0; }
+
 // ---- forward projection ---------------------------------------------------------------------------
 Tensor project_forw(int dim, const Tensor& reconstruction, const Tensor& rotations, const OptTensor& shifts, at::IntArrayRef output_shape,
                     const std::string& interpolation, double oversampling, const c10::optional<double>& cutoff, const OptTensor& pose_order) {
@@ -170,16 +179,17 @@ Tensor project_forw(int dim, const Tensor& reconstruction, const Tensor& rotatio
     c10::cuda::CUDAGuard guard(rec.device());
     Tensor out = at::empty({B, p.P, N, N / 2 + 1}, rec.options());
     if (out.numel() == 0) return out;
-    Tensor order = resolve_order(dim, rec, B, p, pose_order);
     void* s = current_stream(rec);
     const double cut = cutoff_of(cutoff, N);
+    const Tensor ws = project_workspace(dim, rec, p.P, N, interp, false, oversampling, cut);
+    Tensor order = ws.defined() ? Tensor() : resolve_order(dim, rec, B, p, pose_order);
     int rc;
     if (is_f64(rec)) {
         rc = dim == 2 ? b200proj_project_2d_forw_f64(cptr<double>(rec), B, R, cptr<double>(p.rot), p.B_rot, cptr<double>(p.shifts), p.B_shift, p.P, N, interp, oversampling, cut, mptr<double>(out), s)
                       : b200proj_project_3d_to_2d_forw_f64(cptr<double>(rec), B, R, cptr<double>(p.rot), p.B_rot, cptr<double>(p.shifts), p.B_shift, p.P, N, interp, oversampling, cut, mptr<double>(out), cptr<int32_t>(order), s);
     } else {
         rc = dim == 2 ? b200proj_project_2d_forw(cptr<float>(rec), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts), p.B_shift, p.P, N, interp, oversampling, cut, mptr<float>(out), s)
-                      : b200proj_project_3d_to_2d_forw(cptr<float>(rec), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts), p.B_shift, p.P, N, interp, oversampling, cut, mptr<float>(out), cptr<int32_t>(order), s);
+                      : b200proj_project_3d_to_2d_forw_ws(cptr<float>(rec), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts), p.B_shift, p.P, N, interp, oversampling, cut, mptr<float>(out), cptr<int32_t>(order), ws_ptr(ws), ws_size(ws), s);
     }
     status(rc, dim == 2 ? "project_2d_forw" : "project_3d_to_2d_forw");
     return out;
@@ -232,6 +242,27 @@ std::tuple<Tensor, Tensor, Tensor> project_back(int dim, const Tensor& grad_proj
     return std::make_tuple(grad_rec, need_rot ? grad_rot : empty_real0(rec, rd), need_shift ? grad_sh : empty_real0(rec, rd));
 }
 
+// The saved derivatives, [dim, B, P, H, W/2+1].  3D: a view of records [B, P, H, W/2+1, 4] (the fourth entry of a
+// record is the pixel itself), which is how the kernels write and read them; 2D: plain planes.
+Tensor empty_derivatives(int dim, int64_t B, int64_t P, int64_t N, const at::TensorOptions& opt) {
+    if (dim == 2) return at::empty({2, B, P, N, N / 2 + 1}, opt);
+    return at::empty({B, P, N, N / 2 + 1, 4}, opt).permute({4, 0, 1, 2, 3}).narrow(0, 0, 3);
+}
+// Derivatives in the layout the kernels read: as made above, or copied into it.
+Tensor kernel_derivatives(int dim, const Tensor& d) {
+    if (dim == 2) return d.contiguous();
+    int64_t stride = 4;
+    bool records = d.stride(0) == 1 && (reinterpret_cast<uintptr_t>(d.data_ptr()) & 31u) == 0;
+    for (int64_t a = 4; a >= 1; --a) {
+        records = records && (d.stride(a) == stride || d.size(a) == 1);
+        stride *= d.size(a);
+    }
+    if (records) return d;
+    Tensor made = empty_derivatives(3, d.size(1), d.size(2), d.size(3), d.options());
+    made.copy_(d);
+    return made;
+}
+
 // ---- forward projection that keeps the pixels' derivatives, and its backward pass --------------------
 // (additions; complex64 only: the step of an optimisation over poses needs no second gather of the
 // volume in its backward pass, and none of the volume's gradient when the volume is fixed)
@@ -250,15 +281,16 @@ std::tuple<Tensor, Tensor> project_forw_saving(int dim, const Tensor& reconstruc
     const Tensor rec = reconstruction.contiguous();
     c10::cuda::CUDAGuard guard(rec.device());
     Tensor out = at::empty({B, p.P, N, N / 2 + 1}, rec.options());
-    Tensor derivs = at::empty({dim, B, p.P, N, N / 2 + 1}, rec.options());
+    Tensor derivs = empty_derivatives(dim, B, p.P, N, rec.options());
     if (out.numel() == 0) return std::make_tuple(out, derivs);
-    Tensor order = resolve_order(dim, rec, B, p, pose_order);
     const double cut = cutoff_of(cutoff, N);
+    const Tensor ws = project_workspace(dim, rec, p.P, N, interp, true, oversampling, cut);
+    Tensor order = ws.defined() ? Tensor() : resolve_order(dim, rec, B, p, pose_order);
     const int rc = dim == 2
         ? b200proj_project_2d_forw_saving(cptr<float>(rec), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts), p.B_shift, p.P, N, interp,
                                           oversampling, cut, mptr<float>(out), mptr<float>(derivs), current_stream(rec))
-        : b200proj_project_3d_to_2d_forw_saving(cptr<float>(rec), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts), p.B_shift, p.P, N, interp,
-                                                oversampling, cut, mptr<float>(out), mptr<float>(derivs), cptr<int32_t>(order), current_stream(rec));
+        : b200proj_project_3d_to_2d_forw_records(cptr<float>(rec), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts), p.B_shift, p.P, N, interp,
+                                                   oversampling, cut, mptr<float>(out), mptr<float>(derivs), cptr<int32_t>(order), ws_ptr(ws), ws_size(ws), current_stream(rec));
     status(rc, dim == 2 ? "project_2d_forw_saving" : "project_3d_to_2d_forw_saving");
     return std::make_tuple(out, derivs);
 }
@@ -289,7 +321,7 @@ std::tuple<Tensor, Tensor, Tensor> project_back_saved(int dim, const Tensor& gra
     const bool need_shift = p.shifts.defined() && shifts->requires_grad();
     const Tensor gp = grad_projections.contiguous();
     const Tensor out = projections.contiguous();
-    const Tensor der = derivatives.numel() ? derivatives.contiguous() : Tensor();
+    const Tensor der = derivatives.numel() ? kernel_derivatives(dim, derivatives) : Tensor();
     const int64_t R = reconstruction.size(-2);
     c10::cuda::CUDAGuard guard(gp.device());
     Tensor grad_rec = need_rec_grad ? at::empty(reconstruction.sizes(), gp.options()) : Tensor();
@@ -304,7 +336,7 @@ std::tuple<Tensor, Tensor, Tensor> project_back_saved(int dim, const Tensor& gra
             ? b200proj_project_2d_back_saved(cptr<float>(gp), cptr<float>(out), cptr<float>(der), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts),
                                              p.B_shift, p.P, N, interp, oversampling, cut, mptr<float>(grad_rec), mptr<float>(grad_rot), mptr<float>(grad_sh),
                                              current_stream(gp))
-            : b200proj_project_3d_to_2d_back_saved(cptr<float>(gp), cptr<float>(out), cptr<float>(der), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts),
+            : b200proj_project_3d_to_2d_back_records(cptr<float>(gp), cptr<float>(out), cptr<float>(der), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts),
                                                    p.B_shift, p.P, N, interp, oversampling, cut, mptr<float>(grad_rec), mptr<float>(grad_rot), mptr<float>(grad_sh),
                                                    cptr<int32_t>(order), current_stream(gp));
         status(rc, dim == 2 ? "project_2d_back_saved" : "project_3d_to_2d_back_saved");
@@ -523,7 +555,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> meta_backproject_back_ordered(const T
 }
 std::tuple<Tensor, Tensor> meta_project_forw_saving(const Tensor& rec, const Tensor& rot, const OptTensor& sh, at::IntArrayRef shape, std::string i, double os, Cut c, const OptTensor&) {
     Tensor out = meta_project_forw(rec, rot, sh, shape, i, os, c);
-    return std::make_tuple(out, at::empty({3, out.size(0), out.size(1), out.size(2), out.size(3)}, out.options()));
+    return std::make_tuple(out, empty_derivatives(3, out.size(0), out.size(1), out.size(2), out.options()));
 }
 std::tuple<Tensor, Tensor> meta_project_2d_forw_saving(const Tensor& rec, const Tensor& rot, const OptTensor& sh, at::IntArrayRef shape, std::string i, double os, Cut c) {
     Tensor out = meta_project_forw(rec, rot, sh, shape, i, os, c);

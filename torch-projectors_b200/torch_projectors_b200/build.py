@@ -32,7 +32,7 @@ LIB_PATH = PKG_DIR / "libb200proj.so"
 BINDING_PATH = PKG_DIR / "_C.so"
 
 SOURCES = [CSRC_DIR / "b200proj.cu"]
-HEADERS = [CSRC_DIR / "fourier_slice_device.cuh", CSRC_DIR / "fourier_slice_kernels.cuh",
+HEADERS = [CSRC_DIR / "fourier_slice_device.cuh", CSRC_DIR / "fourier_slice_kernels.cuh", CSRC_DIR / "brick_kernels.cuh",
            INCLUDE_DIR / "b200proj.h"]
 BINDING_SOURCES = [CSRC_DIR / "torch_binding.cpp"]
 

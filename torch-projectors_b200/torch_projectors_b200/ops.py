@@ -125,7 +125,7 @@ def set_pose_order_thresholds(min_volume_bytes: int = 96 << 20, min_poses: int =
 
 
 # Saved derivatives: when the rotations of a cubic 3D projection need gradients, the forward pass can
-# also write every pixel's derivatives with respect to its sample position (three more tensors of
+# also write every pixel's derivatives with respect to its sample position (a record of four times
 # the projections' size), and the backward pass then forms the pose gradients from them instead of
 # gathering the volume a second time -- and skips the scatter into the volume's gradient altogether
 # when the volume needs none.  Measured on B200, box 512, 4,096 poses of 256 x 256, cubic: forward
@@ -143,7 +143,7 @@ def set_save_derivatives(enabled: bool = True, max_bytes: int = 16 << 30, min_vo
     """Whether ``project_2d_forw`` / ``project_3d_to_2d_forw`` keep their pixels' derivatives for the
     backward pass when the rotations require gradients (complex64; when the reconstruction needs a
     gradient as well: cubic interpolation and at least `min_volume_bytes` per batch item), and up to
-    which size of that extra tensor (2 or 3 x the projections)."""
+    which size of that extra tensor (2D: 2 x the projections, 3D: 4 x)."""
     global SAVE_DERIVATIVES, SAVE_DERIVATIVES_MAX_BYTES, SAVE_DERIVATIVES_MIN_VOLUME_BYTES
     SAVE_DERIVATIVES, SAVE_DERIVATIVES_MAX_BYTES = bool(enabled), int(max_bytes)
     SAVE_DERIVATIVES_MIN_VOLUME_BYTES = int(min_volume_bytes)
@@ -572,7 +572,7 @@ def _save_derivatives(dim, reconstruction, rotations, output_shape, interpolatio
     if need_rec and not (interpolation == "cubic" and reconstruction[0].numel() * 8 >= SAVE_DERIVATIVES_MIN_VOLUME_BYTES):
         return _PLAIN
     N = int(output_shape[0])
-    fits = 8 * dim * reconstruction.size(0) * rotations.size(1) * N * (N // 2 + 1) <= SAVE_DERIVATIVES_MAX_BYTES
+    fits = 8 * (2 if dim == 2 else 4) * reconstruction.size(0) * rotations.size(1) * N * (N // 2 + 1) <= SAVE_DERIVATIVES_MAX_BYTES
     return _KEEP_DERIVATIVES if fits else _PLAIN
 
 
