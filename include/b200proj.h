@@ -102,6 +102,11 @@ int b200proj_project_3d_to_2d_forw(const float* rec, int64_t B, int64_t R,
  * is free again when the call's work has run. */
 size_t b200proj_project_workspace_bytes(int64_t B, int64_t P, int64_t N, int interpolation, int records,
                                         double oversampling, double fourier_radius_cutoff);
+/* The same for the scatters of the 3D operators (b200proj_project_3d_to_2d_back_records and _back_ws with
+ * grad_rec, b200proj_backproject_2d_to_3d_accumulate_ws, b200proj_backproject_2d_to_3d_forw; 0: no gain, for
+ * the last of them see there for what else a workspace is good for). */
+size_t b200proj_scatter_workspace_bytes(int64_t B, int64_t P, int64_t N, int interpolation, int has_weights,
+                                        double oversampling, double fourier_radius_cutoff);
 int b200proj_project_3d_to_2d_forw_ws(const float* rec, int64_t B, int64_t R,
                                       const float* rot, int64_t B_rot,
                                       const float* shifts, int64_t B_shift,
@@ -109,6 +114,21 @@ int b200proj_project_3d_to_2d_forw_ws(const float* rec, int64_t B, int64_t R,
                                       double fourier_radius_cutoff, float* out,
                                       const int32_t* pose_order, void* workspace,
                                       size_t workspace_bytes, void* stream);
+
+int b200proj_project_3d_to_2d_back_ws(const float* grad_proj, const float* rec, int64_t B, int64_t R,
+                                      const float* rot, int64_t B_rot,
+                                      const float* shifts, int64_t B_shift,
+                                      int64_t P, int64_t N, int interpolation, double oversampling,
+                                      double fourier_radius_cutoff, float* grad_rec, float* grad_rot,
+                                      float* grad_shifts, const int32_t* pose_order,
+                                      void* workspace, size_t workspace_bytes, void* stream);
+int b200proj_backproject_2d_to_3d_accumulate_ws(const float* proj, const float* weights, int64_t B,
+                                                int64_t R, const float* rot, int64_t B_rot,
+                                                const float* shifts, int64_t B_shift,
+                                                int64_t P, int64_t N, int interpolation,
+                                                double oversampling, double fourier_radius_cutoff,
+                                                void* accumulator, void* workspace,
+                                                size_t workspace_bytes, void* stream);
 
 /* ---- forward projection with packed output ------------------------------------------------
  * No counterpart in the reference.  For callers that move the projections off the device: only
@@ -384,7 +404,8 @@ int b200proj_project_3d_to_2d_back_records(const float* grad_proj, const float* 
                                            const float* shifts, int64_t B_shift, int64_t P, int64_t N,
                                            int interpolation, double oversampling,
                                            double fourier_radius_cutoff, float* grad_rec, float* grad_rot,
-                                           float* grad_shifts, const int32_t* pose_order, void* stream);
+                                           float* grad_shifts, const int32_t* pose_order,
+                                           void* workspace, size_t workspace_bytes, void* stream);
 
 /* ---- backward of back-projection (gather) ----------------------------------------------
  * grad_proj [B,P,N,Nh] complex is fully written.  grad_weights [B,P,N,Nh] float is written

@@ -62,9 +62,25 @@ def check(names):
                     for have, ref, what in ((rec.grad, grads[0], "volume"), (rot.grad, grads[1], "rotations"), (sh.grad if sh is not None else None, grads[2], "shifts")):
                         if have is not None:
                             assert rel_err(have, ref) <= TOL_ATOMIC, (size, interp, what, rel_err(have, ref))
+                rec = t["rec"].cuda().requires_grad_(True)                 # the volume's gradient alone
+                tp.project_3d_to_2d_forw(rec, t["rot"].cuda(), shifts, interpolation=interp, **kw).backward(t["proj"].cuda())
+                assert rel_err(rec.grad, grads[0]) <= TOL_ATOMIC, (size, interp, "volume alone")
+            if "backprojection" in names:
+                for weights in (None, t["weights"]):
+                    data, wrec = tp.backproject_2d_to_3d_forw(t["proj"].cuda(), t["rot"].cuda(), weights.cuda() if weights is not None else None, shifts,
+                                                              interpolation=interp, oversampling=os_, fourier_radius_cutoff=cutoff)
+                    ref, wref = port.backproject_2d_to_3d_forw(t["proj"], weights, t["rot"], t["shifts"], interp, os_, cutoff)
+                    assert rel_err(data, ref) <= TOL_ATOMIC, (size, interp, "data", rel_err(data, ref))
+                    if weights is not None:
+                        acc = tp.new_backprojection_accumulator(size[0], data.shape[-2], "cuda")
+                        tp.backproject_2d_to_3d_accumulate_interleaved_(acc, t["proj"].cuda(), t["rot"].cuda(), weights.cuda(), shifts,
+                                                                        interpolation=interp, oversampling=os_, fourier_radius_cutoff=cutoff)
+                        d2, w2 = tp.fold_backprojection_accumulator(acc)
+                        assert rel_err(d2, ref) <= TOL_ATOMIC and rel_err(w2, wref) <= TOL_ATOMIC, (size, interp, "accumulator")
+                        assert rel_err(wrec, wref) <= TOL_ATOMIC, (size, interp, "weights", rel_err(wrec, wref))
 
 
-@pytest.mark.parametrize("names", ["forward", "gradients"])
+@pytest.mark.parametrize("names", ["forward", "gradients", "backprojection"])
 def test_bricks_match_the_oracle(names):
     env = dict(os.environ, B200PROJ_BRICKS="1")
     r = subprocess.run([sys.executable, "-c", f"import sys; sys.path.insert(0, {str(ROOT / 'tests')!r}); import test_gpu_bricks as t; t.check({names!r})"],

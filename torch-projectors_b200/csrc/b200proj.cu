@@ -187,7 +187,8 @@ struct BrickLaunch {
     size_t items;            // capacity of the item list
     size_t item_bytes, rec_bytes;
     size_t bytes;            // workspace
-    bool use;
+    double pixels, in_ball;  // of the call: pixels inside the cutoff, bricks that can hold some
+    bool forced, use;
 };
 
 // Pixels of a slice inside the cutoff.
@@ -199,7 +200,9 @@ double pixels_inside(int64_t N, double cutoff) {
     return disc < all ? disc : all;
 }
 
-BrickLaunch brick_plan(int64_t B, int64_t P, int64_t N, bool cubic, bool records, double os, double cutoff) {
+// Geometry and item list for bricks of D sample positions, `blocks` of them resident on the GPU.
+template <typename D>
+BrickLaunch brick_layout(int64_t B, int64_t P, int64_t N, double os, double cutoff, double blocks, double min_target, bool outside) {
     BrickLaunch L{};
     static const int force = [] { const char* e = getenv("B200PROJ_BRICKS"); return e ? atoi(e) : -1; }();   // 0 / 1: never / always, for tests
     if (force == 0 || os < 1.0 || !(cutoff >= 0.0) || P < 1) return L;
@@ -209,30 +212,50 @@ BrickLaunch brick_plan(int64_t B, int64_t P, int64_t N, bool cubic, bool records
     const double pixels = pixels_inside(N, cutoff) * (double)B * (double)P;
     L.plan.ball = (float)(reach + 1.0);
     const int span = 2 * ((int)ceil(reach) + 2);
-    const int dims[3] = {kBrickX, kBrickY, kBrickZ};
+    const int dims[3] = {D::x, D::y, D::z};
     L.bricks = 1;
     for (int a = 0; a < 3; ++a) {
+        L.plan.d[a] = dims[a];
         L.plan.n[a] = (span + dims[a] - 1) / dims[a];
         L.plan.lo[a] = -((L.plan.n[a] * dims[a]) / 2);
         L.bricks *= L.plan.n[a];
     }
     if (L.bricks * B > (1 << 26) || B * P > (1 << 26)) return L;
-    L.plan.density = (float)((double)kBrickX * kBrickY * kBrickZ / (4.0 * os * os));
-    double target = pixels / (148.0 * 3.0 * 8.0);
-    if (target < 3000.0) target = 3000.0;
+    L.plan.density = (float)((double)D::x * D::y * D::z / (4.0 * os * os));
+    double target = pixels / (blocks * 8.0);
+    if (target < min_target) target = min_target;
     L.plan.target = (float)target;
-    L.plan.max_extra = (int)(1.5 * pixels / target) + 64;
+    L.plan.per_slice = (float)pixels_inside(N, cutoff);
+    // the estimate counts bricks that stick out of the ball in full, and a few large ones may each count the whole slice
+    L.plan.max_extra = (int)((L.bricks < 64 ? (double)L.bricks : 4.0) * pixels / target) + 64;
     L.items = (size_t)(L.bricks * B) + (size_t)L.plan.max_extra;
     L.item_bytes = (L.items * sizeof(int4) + 255) & ~(size_t)255;
     L.rec_bytes = (size_t)(B * P) * 3 * sizeof(float4);
-    L.bytes = 256 + L.item_bytes + L.rec_bytes + (size_t)(N * (N / 2 + 1)) * sizeof(int);
-    // Bricks pay once their pixels outweigh staging them, whatever their number, and a fixed cost (measured: 20 us and
-    // 26 ns per brick against 33 ps saved per cubic pixel at oversampling 2; dense samples are cheaper for the plain
-    // kernels, linear taps save only some 2 ps).
-    const double in_ball = 4.19 * pow(reach + 12.0, 3) / ((double)kBrickX * kBrickY * kBrickZ) * (double)B;
-    const double need = cubic ? (1.2e6 + 900.0 * in_ball) * (os < 2.0 ? 2.0 / os : 1.0)
-                              : (10e6 + 4000.0 * in_ball) * (records ? 0.6 : 1.0);
-    L.use = force == 1 || pixels > need;
+    L.bytes = 256 + L.item_bytes + L.rec_bytes + (outside ? (size_t)(N * (N / 2 + 1)) * sizeof(int) : 0);
+    L.pixels = pixels;
+    L.in_ball = 4.19 * pow(reach + 12.0, 3) / ((double)D::x * D::y * D::z) * (double)B;
+    L.forced = force == 1;
+    L.use = true;
+    return L;
+}
+
+// Forward projection: bricks pay once their pixels outweigh staging them, whatever their number, and a fixed cost
+// (measured: 20 us and 26 ns per brick against 33 ps saved per cubic pixel at oversampling 2; dense samples are cheaper
+// for the plain kernels, linear taps save only some 2 ps).
+BrickLaunch gather_plan(int64_t B, int64_t P, int64_t N, bool cubic, bool records, double os, double cutoff) {
+    BrickLaunch L = brick_layout<GatherBrick>(B, P, N, os, cutoff, 148.0 * 3.0, 3000.0, true);
+    const double need = cubic ? (1.2e6 + 900.0 * L.in_ball) * (os < 2.0 ? 2.0 / os : 1.0)
+                              : (10e6 + 4000.0 * L.in_ball) * (records ? 0.6 : 1.0);
+    // linear taps: small volumes meet a slice in too few pixels per brick (box 38 oversampled twice: 1.8x slower)
+    L.use = L.use && (L.forced || (L.pixels > need && (cubic || L.plan.ball > 85.f)));
+    return L;
+}
+
+// Cubic scatter (measured crossings: 1.1-1.3 M pixels for box-64 and box-128 volumes, 2 M for box 256, 4.6 M for box 400).
+BrickLaunch scatter_plan(int64_t B, int64_t P, int64_t N, bool weights, double os, double cutoff) {
+    BrickLaunch L = weights ? brick_layout<Scatter<true>::Brick>(B, P, N, os, cutoff, 148.0 * Scatter<true>::kBlocks, 1500.0, false)
+                            : brick_layout<Scatter<false>::Brick>(B, P, N, os, cutoff, 148.0 * Scatter<false>::kBlocks, 1500.0, false);
+    L.use = L.use && (L.forced || L.pixels > 1.2e6 + 150.0 * L.in_ball);
     return L;
 }
 
@@ -245,11 +268,11 @@ BrickWork brick_work(const BrickLaunch& L, void* workspace) {
     return w;
 }
 
-int brick_setup(const BrickLaunch& bl, const BrickWork& w, const Launch& L, const float* rot, const float* shifts, cudaStream_t s) {
+int brick_setup(const BrickLaunch& bl, const BrickWork& w, const Launch& L, const float* rot, const float* shifts, bool outside, cudaStream_t s) {
     if (int rc = zero_async(w.header, 16, s)) return rc;
     const int64_t clusters = (int64_t)((bl.plan.n[0] + 7) / 8) * ((bl.plan.n[1] + 7) / 8) * ((bl.plan.n[2] + 3) / 4) * L.B;
     const int64_t slices = (L.B * L.P + 255) / 256;
-    brick_setup_kernel<<<(unsigned)(clusters > slices ? clusters : slices) + 1u, 256, 0, s>>>(rot, shifts, w, L.g, bl.plan, (int)L.B);
+    brick_setup_kernel<<<(unsigned)(clusters > slices ? clusters : slices) + 1u, 256, 0, s>>>(rot, shifts, w, L.g, bl.plan, (int)L.B, outside ? 1 : 0);
     return check_launch("brick_setup launch");
 }
 
@@ -257,12 +280,25 @@ template <bool CUBIC, bool SAVE>
 int launch_brick_forw(const Launch& L, const BrickLaunch& bl, void* workspace, const float* rec, const float* rot, const float* shifts,
                       float* out, float* derivs, cudaStream_t s) {
     const BrickWork w = brick_work(bl, workspace);
-    if (int rc = brick_setup(bl, w, L, rot, shifts, s)) return rc;
-    constexpr size_t smem = sizeof(float2) * BrickShape<CUBIC>::kVoxels + sizeof(BrickBlock);
+    if (int rc = brick_setup(bl, w, L, rot, shifts, true, s)) return rc;
+    constexpr size_t smem = sizeof(float2) * BrickShape<CUBIC>::kVoxels + sizeof(GatherBlock);
     const cudaError_t e = cudaFuncSetAttribute(brick_forw_kernel<CUBIC, SAVE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cuda_fail(e, "brick_forw shared memory");
     brick_forw_kernel<CUBIC, SAVE><<<148 * 3, kBlockThreads, smem, s>>>((const float2*)rec, rot, shifts, (float2*)out, (float2*)derivs, w, L.g, bl.plan);
     return check_launch("brick_forw launch");
+}
+
+template <bool WEIGHTS, bool DUP, bool INTERLEAVED = false>
+int launch_brick_scatter(const Launch& L, const BrickLaunch& bl, void* workspace, const float* proj, const float* weights, const float* rot,
+                         const float* shifts, float* vol, float* wvol, cudaStream_t s, float4* accum = nullptr) {
+    const BrickWork w = brick_work(bl, workspace);
+    if (int rc = brick_setup(bl, w, L, rot, shifts, false, s)) return rc;
+    constexpr size_t smem = sizeof(typename Scatter<WEIGHTS>::Shared);
+    static_assert((smem + 1024) * Scatter<WEIGHTS>::kBlocks <= 233472, "shared memory of an SM");
+    const cudaError_t e = cudaFuncSetAttribute(brick_scatter_kernel<WEIGHTS, DUP, INTERLEAVED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return cuda_fail(e, "brick_scatter shared memory");
+    brick_scatter_kernel<WEIGHTS, DUP, INTERLEAVED><<<148 * Scatter<WEIGHTS>::kBlocks, Scatter<WEIGHTS>::kThreads, smem, s>>>((const float2*)proj, weights, rot, shifts, (float2*)vol, wvol, accum, w, L.g, bl.plan);
+    return check_launch("brick_scatter launch");
 }
 
 // ---- operator bodies, templated on the dimensionality and the real type (float | double) ------------------------------------
@@ -278,7 +314,7 @@ int project_forw(const Real* rec, int64_t B, int64_t R, const Real* rot, int64_t
     if (P == 0) return B200PROJ_OK;
     cudaStream_t s = (cudaStream_t)stream;
     if constexpr (DIM == 3 && std::is_same<Real, float>::value) {
-        const BrickLaunch bl = workspace != nullptr ? brick_plan(B, P, N, interpolation == B200PROJ_CUBIC, false, os, cutoff) : BrickLaunch{};
+        const BrickLaunch bl = workspace != nullptr ? gather_plan(B, P, N, interpolation == B200PROJ_CUBIC, false, os, cutoff) : BrickLaunch{};
         if (bl.use && workspace_bytes >= bl.bytes)
             return interpolation == B200PROJ_CUBIC ? launch_brick_forw<true, false>(L, bl, workspace, rec, rot, shifts, out, nullptr, s)
                                                    : launch_brick_forw<false, false>(L, bl, workspace, rec, rot, shifts, out, nullptr, s);
@@ -339,7 +375,7 @@ int project_forw_saving(const float* rec, int64_t B, int64_t R, const float* rot
     cudaStream_t s = (cudaStream_t)stream;
     if constexpr (RECORDS) {
         if ((reinterpret_cast<uintptr_t>(derivatives) & 31u) != 0) return fail(B200PROJ_ERR_ARGUMENT, "records must be 32-byte aligned");
-        const BrickLaunch bl = workspace != nullptr ? brick_plan(B, P, N, interpolation == B200PROJ_CUBIC, true, os, cutoff) : BrickLaunch{};
+        const BrickLaunch bl = workspace != nullptr ? gather_plan(B, P, N, interpolation == B200PROJ_CUBIC, true, os, cutoff) : BrickLaunch{};
         if (bl.use && workspace_bytes >= bl.bytes)
             return interpolation == B200PROJ_CUBIC ? launch_brick_forw<true, true>(L, bl, workspace, rec, rot, shifts, out, derivatives, s)
                                                    : launch_brick_forw<false, true>(L, bl, workspace, rec, rot, shifts, out, derivatives, s);
@@ -355,7 +391,7 @@ template <int DIM, bool RECORDS = false>
 int project_back_saved(const float* grad_proj, const float* out, const float* derivatives, int64_t B, int64_t R,
                        const float* rot, int64_t B_rot, const float* shifts, int64_t B_shift, int64_t P, int64_t N,
                        int interpolation, double os, double cutoff, float* grad_rec, float* grad_rot, float* grad_shifts,
-                       const int32_t* pose_order, void* stream) {
+                       const int32_t* pose_order, void* stream, void* workspace = nullptr, size_t workspace_bytes = 0) {
     Launch L;
     if (int rc = prepare(L, DIM, B, R, B_rot, rot, shifts, B_shift, P, N, interpolation, os, cutoff)) return rc;
     L.g.order = pose_order;
@@ -373,6 +409,15 @@ int project_back_saved(const float* grad_proj, const float* out, const float* de
     const float2* o = (const float2*)out;
     const float2* d = (const float2*)derivatives;
     const bool cubic = interpolation == B200PROJ_CUBIC;
+    if constexpr (RECORDS) {
+        // large cubic scatter: brick by brick, the pose gradients in a streaming pass of their own
+        const BrickLaunch bl = grad_rec != nullptr && cubic && workspace != nullptr ? scatter_plan(B, P, N, false, os, cutoff) : BrickLaunch{};
+        if (bl.use && workspace_bytes >= bl.bytes) {
+            if (int rc = launch_brick_scatter<false, false>(L, bl, workspace, grad_proj, nullptr, rot, shifts, grad_rec, nullptr, s)) return rc;
+            if (grad_rot == nullptr && grad_shifts == nullptr) return B200PROJ_OK;
+            grad_rec = nullptr;
+        }
+    }
     if (grad_rec != nullptr) {
         if (cubic) launch_project_back_saved<DIM, true, true, RECORDS>(L, s, gp, o, d, rot, shifts, (float2*)grad_rec, grad_rot, grad_shifts);
         else launch_project_back_saved<DIM, false, true, RECORDS>(L, s, gp, o, d, rot, shifts, (float2*)grad_rec, grad_rot, grad_shifts);
@@ -386,7 +431,7 @@ template <int DIM, typename Real>
 int project_back(const Real* grad_proj, const Real* rec, int64_t B, int64_t R, const Real* rot,
                  int64_t B_rot, const Real* shifts, int64_t B_shift, int64_t P, int64_t N,
                  int interpolation, double os, double cutoff, Real* grad_rec, Real* grad_rot,
-                 Real* grad_shifts, const int32_t* pose_order, void* stream) {
+                 Real* grad_shifts, const int32_t* pose_order, void* stream, void* workspace = nullptr, size_t workspace_bytes = 0) {
     Launch L;
     if (int rc = prepare(L, DIM, B, R, B_rot, rot, shifts, B_shift, P, N, interpolation, os, cutoff)) return rc;
     L.g.order = pose_order;
@@ -399,6 +444,12 @@ int project_back(const Real* grad_proj, const Real* rec, int64_t B, int64_t R, c
     if (int rc = zero_async(grad_rot, (size_t)B_rot * P * DIM * DIM * sizeof(Real), s)) return rc;
     if (int rc = zero_async(grad_shifts, (size_t)(shifts ? B_shift : 0) * P * 2 * sizeof(Real), s)) return rc;
     if (P == 0) return B200PROJ_OK;
+    if constexpr (DIM == 3 && std::is_same<Real, float>::value) {
+        if (interpolation == B200PROJ_CUBIC && grad_rot == nullptr && grad_shifts == nullptr && workspace != nullptr) {
+            const BrickLaunch bl = scatter_plan(B, P, N, false, os, cutoff);
+            if (bl.use && workspace_bytes >= bl.bytes) return launch_brick_scatter<false, false>(L, bl, workspace, grad_proj, nullptr, rot, shifts, grad_rec, nullptr, s);
+        }
+    }
     if (interpolation == B200PROJ_CUBIC)
         launch_project_back<DIM, true>(L, s, (const C2<Real>*)grad_proj, (const C2<Real>*)rec, rot, shifts, (C2<Real>*)grad_rec, grad_rot, grad_shifts);
     else
@@ -425,6 +476,17 @@ int backproject_forw(const Real* proj, const Real* weights, int64_t B, int64_t R
     // Interleaved path: data and weight of a voxel share one 16-byte slot of the workspace
     // (one v4 reduction per tap), folded into the outputs afterwards.
     const size_t ws_one = L.rec_count * sizeof(float4);
+    if constexpr (DIM == 3 && std::is_same<Real, float>::value) {
+        const BrickLaunch bl = cubic && P > 0 && workspace != nullptr ? scatter_plan(B, P, N, hw, os, cutoff) : BrickLaunch{};
+        if (bl.use && workspace_bytes >= bl.bytes && (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0) {
+            if (!accumulate) {
+                if (int rc = zero_async(data_rec, L.rec_count * sizeof(C2<Real>), s)) return rc;
+                if (int rc = zero_async(weight_rec, L.rec_count * sizeof(Real), s)) return rc;
+            }
+            return hw ? launch_brick_scatter<true, true>(L, bl, workspace, proj, weights, rot, shifts, data_rec, weight_rec, s)
+                      : launch_brick_scatter<false, true>(L, bl, workspace, proj, nullptr, rot, shifts, data_rec, nullptr, s);
+        }
+    }
     constexpr bool kIsF32 = std::is_same<Real, float>::value;  // workspace and slab paths exist in fp32 only
     if constexpr (kIsF32) {
     if (hw && P > 0 && !(DIM == 3 && slab_plan(R, hw).slabs > 1) && workspace != nullptr && workspace_bytes >= ws_one &&
@@ -534,7 +596,7 @@ int backproject_back(const Real* grad_data_rec, const Real* grad_weight_rec, con
 int backproject_accumulate(const float* proj, const float* weights, int64_t B, int64_t R, const float* rot,
                            int64_t B_rot, const float* shifts, int64_t B_shift, int64_t P, int64_t N,
                            int interpolation, double os, double cutoff, void* accumulator,
-                           int slab_first, int slab_count, void* stream) {
+                           int slab_first, int slab_count, void* stream, void* workspace = nullptr, size_t workspace_bytes = 0) {
     Launch L;
     if (int rc = prepare(L, 3, B, R, B_rot, rot, shifts, B_shift, P, N, interpolation, os, cutoff)) return rc;
     if (proj == nullptr || weights == nullptr || accumulator == nullptr)
@@ -552,6 +614,10 @@ int backproject_accumulate(const float* proj, const float* weights, int64_t B, i
     cudaStream_t s = (cudaStream_t)stream;
     float4* acc = (float4*)accumulator;
     const bool cubic = interpolation == B200PROJ_CUBIC;
+    if (cubic && workspace != nullptr && slab_count == plan.slabs) {
+        const BrickLaunch bl = scatter_plan(B, P, N, true, os, cutoff);
+        if (bl.use && workspace_bytes >= bl.bytes) return launch_brick_scatter<true, true, true>(L, bl, workspace, proj, weights, rot, shifts, nullptr, nullptr, s, acc);
+    }
     if (plan.slabs > 1) {
         launch_slab_interleaved(L, s, cubic, proj, weights, rot, shifts, acc, plan, slab_first, slab_count);
         return check_launch("backproject_accumulate (slab-ordered) launch");
@@ -696,8 +762,13 @@ int b200proj_project_3d_to_2d_forw(const float* rec, int64_t B, int64_t R, const
     return project_forw<3>(rec, B, R, rot, B_rot, shifts, B_shift, P, N, interpolation, oversampling, cutoff, out, pose_order, stream);
 }
 
+size_t b200proj_scatter_workspace_bytes(int64_t B, int64_t P, int64_t N, int interpolation, int has_weights, double oversampling, double cutoff) {
+    if (interpolation != B200PROJ_CUBIC) return 0;
+    const BrickLaunch bl = scatter_plan(B, P, N, has_weights != 0, oversampling, cutoff);
+    return bl.use ? bl.bytes : 0;
+}
 size_t b200proj_project_workspace_bytes(int64_t B, int64_t P, int64_t N, int interpolation, int records, double oversampling, double cutoff) {
-    const BrickLaunch bl = brick_plan(B, P, N, interpolation == B200PROJ_CUBIC, records != 0, oversampling, cutoff);
+    const BrickLaunch bl = gather_plan(B, P, N, interpolation == B200PROJ_CUBIC, records != 0, oversampling, cutoff);
     return bl.use ? bl.bytes : 0;
 }
 int b200proj_project_3d_to_2d_forw_ws(const float* rec, int64_t B, int64_t R, const float* rot,
@@ -717,8 +788,8 @@ int b200proj_project_3d_to_2d_back_records(const float* grad_proj, const float* 
                                            const float* shifts, int64_t B_shift, int64_t P, int64_t N,
                                            int interpolation, double oversampling, double cutoff,
                                            float* grad_rec, float* grad_rot, float* grad_shifts,
-                                           const int32_t* pose_order, void* stream) {
-    return project_back_saved<3, true>(grad_proj, out, records, B, R, rot, B_rot, shifts, B_shift, P, N, interpolation, oversampling, cutoff, grad_rec, grad_rot, grad_shifts, pose_order, stream);
+                                           const int32_t* pose_order, void* workspace, size_t workspace_bytes, void* stream) {
+    return project_back_saved<3, true>(grad_proj, out, records, B, R, rot, B_rot, shifts, B_shift, P, N, interpolation, oversampling, cutoff, grad_rec, grad_rot, grad_shifts, pose_order, stream, workspace, workspace_bytes);
 }
 
 int b200proj_project_2d_back(const float* grad_proj, const float* rec, int64_t B, int64_t R,
@@ -735,6 +806,15 @@ int b200proj_project_3d_to_2d_back(const float* grad_proj, const float* rec, int
                                    float* grad_rot, float* grad_shifts, const int32_t* pose_order,
                                    void* stream) {
     return project_back<3>(grad_proj, rec, B, R, rot, B_rot, shifts, B_shift, P, N, interpolation, oversampling, cutoff, grad_rec, grad_rot, grad_shifts, pose_order, stream);
+}
+
+int b200proj_project_3d_to_2d_back_ws(const float* grad_proj, const float* rec, int64_t B, int64_t R,
+                                      const float* rot, int64_t B_rot, const float* shifts,
+                                      int64_t B_shift, int64_t P, int64_t N, int interpolation,
+                                      double oversampling, double cutoff, float* grad_rec,
+                                      float* grad_rot, float* grad_shifts, const int32_t* pose_order,
+                                      void* workspace, size_t workspace_bytes, void* stream) {
+    return project_back<3>(grad_proj, rec, B, R, rot, B_rot, shifts, B_shift, P, N, interpolation, oversampling, cutoff, grad_rec, grad_rot, grad_shifts, pose_order, stream, workspace, workspace_bytes);
 }
 
 int b200proj_project_2d_forw_saving(const float* rec, int64_t B, int64_t R, const float* rot,
@@ -867,6 +947,14 @@ int b200proj_backproject_2d_to_3d_accumulate(const float* proj, const float* wei
                                              int64_t N, int interpolation, double oversampling,
                                              double cutoff, void* accumulator, void* stream) {
     return backproject_accumulate(proj, weights, B, R, rot, B_rot, shifts, B_shift, P, N, interpolation, oversampling, cutoff, accumulator, 0, -1, stream);
+}
+
+int b200proj_backproject_2d_to_3d_accumulate_ws(const float* proj, const float* weights, int64_t B,
+                                                int64_t R, const float* rot, int64_t B_rot,
+                                                const float* shifts, int64_t B_shift, int64_t P,
+                                                int64_t N, int interpolation, double oversampling,
+                                                double cutoff, void* accumulator, void* workspace, size_t workspace_bytes, void* stream) {
+    return backproject_accumulate(proj, weights, B, R, rot, B_rot, shifts, B_shift, P, N, interpolation, oversampling, cutoff, accumulator, 0, -1, stream, workspace, workspace_bytes);
 }
 
 int b200proj_backproject_2d_to_3d_accumulate_slabs(const float* proj, const float* weights, int64_t B,

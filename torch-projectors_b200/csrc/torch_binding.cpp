@@ -159,6 +159,12 @@ Tensor project_workspace(int dim, const Tensor& rec, int64_t P, int64_t N, int i
     const size_t bytes = b200proj_project_workspace_bytes(rec.size(0), P, N, interp, records ? 1 : 0, oversampling, cutoff);
     return bytes ? at::empty({(int64_t)bytes}, rec.options().dtype(at::kByte)) : Tensor();
 }
+// The same for the 3D scatters.
+Tensor scatter_workspace(int dim, const Tensor& like, int64_t B, int64_t P, int64_t N, int interp, bool weights, double oversampling, double cutoff) {
+    if (dim != 3 || is_f64(like)) return Tensor();
+    const size_t bytes = b200proj_scatter_workspace_bytes(B, P, N, interp, weights ? 1 : 0, oversampling, cutoff);
+    return bytes ? at::empty({(int64_t)bytes}, like.options().dtype(at::kByte)) : Tensor();
+}
 inline void* ws_ptr(const Tensor& ws) { return ws.defined() ? ws.data_ptr() : nullptr; }
 inline size_t ws_size(const Tensor& ws) { return ws.defined() ? (size_t)ws.numel() : 0; }
 
@@ -225,16 +231,17 @@ std::tuple<Tensor, Tensor, Tensor> project_back(int dim, const Tensor& grad_proj
     if (p.P == 0 || gp.numel() == 0) {                     // nothing to launch: pointers of empty tensors are NULL
         grad_rec.zero_();
     } else {
-        Tensor order = resolve_order(dim, rec, B, p, pose_order);
         void* s = current_stream(rec);
         const double cut = cutoff_of(cutoff, N);
+        const Tensor ws = need_rot || need_shift ? Tensor() : scatter_workspace(dim, rec, B, p.P, N, interp, false, oversampling, cut);
+        Tensor order = ws.defined() ? Tensor() : resolve_order(dim, rec, B, p, pose_order);
         int rc;
         if (is_f64(rec)) {
             rc = dim == 2 ? b200proj_project_2d_back_f64(cptr<double>(gp), cptr<double>(rec), B, R, cptr<double>(p.rot), p.B_rot, cptr<double>(p.shifts), p.B_shift, p.P, N, interp, oversampling, cut, mptr<double>(grad_rec), mptr<double>(grad_rot), mptr<double>(grad_sh), s)
                           : b200proj_project_3d_to_2d_back_f64(cptr<double>(gp), cptr<double>(rec), B, R, cptr<double>(p.rot), p.B_rot, cptr<double>(p.shifts), p.B_shift, p.P, N, interp, oversampling, cut, mptr<double>(grad_rec), mptr<double>(grad_rot), mptr<double>(grad_sh), cptr<int32_t>(order), s);
         } else {
             rc = dim == 2 ? b200proj_project_2d_back(cptr<float>(gp), cptr<float>(rec), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts), p.B_shift, p.P, N, interp, oversampling, cut, mptr<float>(grad_rec), mptr<float>(grad_rot), mptr<float>(grad_sh), s)
-                          : b200proj_project_3d_to_2d_back(cptr<float>(gp), cptr<float>(rec), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts), p.B_shift, p.P, N, interp, oversampling, cut, mptr<float>(grad_rec), mptr<float>(grad_rot), mptr<float>(grad_sh), cptr<int32_t>(order), s);
+                          : b200proj_project_3d_to_2d_back_ws(cptr<float>(gp), cptr<float>(rec), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts), p.B_shift, p.P, N, interp, oversampling, cut, mptr<float>(grad_rec), mptr<float>(grad_rot), mptr<float>(grad_sh), cptr<int32_t>(order), ws_ptr(ws), ws_size(ws), s);
         }
         status(rc, dim == 2 ? "project_2d_back" : "project_3d_to_2d_back");
     }
@@ -330,15 +337,16 @@ std::tuple<Tensor, Tensor, Tensor> project_back_saved(int dim, const Tensor& gra
     if (p.P == 0 || gp.numel() == 0) {
         if (need_rec_grad) grad_rec.zero_();
     } else {
-        Tensor order = resolve_order(dim, reconstruction, B, p, pose_order);
         const double cut = cutoff_of(cutoff, N);
+        const Tensor ws = need_rec_grad ? scatter_workspace(dim, gp, B, p.P, N, interp, false, oversampling, cut) : Tensor();
+        Tensor order = ws.defined() ? Tensor() : resolve_order(dim, reconstruction, B, p, pose_order);
         const int rc = dim == 2
             ? b200proj_project_2d_back_saved(cptr<float>(gp), cptr<float>(out), cptr<float>(der), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts),
                                              p.B_shift, p.P, N, interp, oversampling, cut, mptr<float>(grad_rec), mptr<float>(grad_rot), mptr<float>(grad_sh),
                                              current_stream(gp))
             : b200proj_project_3d_to_2d_back_records(cptr<float>(gp), cptr<float>(out), cptr<float>(der), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts),
                                                    p.B_shift, p.P, N, interp, oversampling, cut, mptr<float>(grad_rec), mptr<float>(grad_rot), mptr<float>(grad_sh),
-                                                   cptr<int32_t>(order), current_stream(gp));
+                                                   cptr<int32_t>(order), ws_ptr(ws), ws_size(ws), current_stream(gp));
         status(rc, dim == 2 ? "project_2d_back_saved" : "project_3d_to_2d_back_saved");
     }
     const at::ScalarType rd = p.rot.scalar_type();
@@ -387,9 +395,13 @@ std::tuple<Tensor, Tensor> backproject_forw(int dim, const Tensor& projections, 
                           : b200proj_backproject_2d_to_3d_forw_f64(cptr<double>(proj), cptr<double>(weights), B, R, cptr<double>(p.rot), p.B_rot, cptr<double>(p.shifts), p.B_shift, p.P, N, interp, oversampling, cut, mptr<double>(data_rec), mptr<double>(weight_rec), 0, nullptr, 0, s);
         } else {
             // scratch for the interleaved accumulation path, from the caching allocator (nothing is freed behind the stream)
-            const size_t ws_bytes = b200proj_backproject_workspace_bytes(dim, B, R, p.P, N, interp, weights.defined() ? 1 : 0);
-            Tensor ws = ws_bytes ? at::empty({(int64_t)ws_bytes}, proj.options().dtype(at::kByte)) : Tensor();
-            void* wsp = ws.defined() ? ws.data_ptr() : nullptr;
+            Tensor ws = scatter_workspace(dim, proj, B, p.P, N, interp, weights.defined(), oversampling, cut);
+            if (!ws.defined()) {
+                const size_t bytes = b200proj_backproject_workspace_bytes(dim, B, R, p.P, N, interp, weights.defined() ? 1 : 0);
+                if (bytes) ws = at::empty({(int64_t)bytes}, proj.options().dtype(at::kByte));
+            }
+            void* wsp = ws_ptr(ws);
+            const size_t ws_bytes = ws_size(ws);
             rc = dim == 2 ? b200proj_backproject_2d_forw(cptr<float>(proj), cptr<float>(weights), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts), p.B_shift, p.P, N, interp, oversampling, cut, mptr<float>(data_rec), mptr<float>(weight_rec), 0, wsp, ws_bytes, s)
                           : b200proj_backproject_2d_to_3d_forw(cptr<float>(proj), cptr<float>(weights), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts), p.B_shift, p.P, N, interp, oversampling, cut, mptr<float>(data_rec), mptr<float>(weight_rec), 0, wsp, ws_bytes, s);
         }

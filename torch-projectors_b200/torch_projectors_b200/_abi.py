@@ -41,6 +41,7 @@ SIGNATURES = {
 SIGNATURES.update({name + "_f64": sig for name, sig in list(SIGNATURES.items()) if not name.endswith("_noalloc")})
 # fp32-only entry points of the persistent interleaved accumulator
 SIGNATURES["b200proj_backproject_2d_to_3d_accumulate"] = [_ptr, _ptr] + _COMMON + [_ptr, _ptr]
+SIGNATURES["b200proj_backproject_2d_to_3d_accumulate_ws"] = [_ptr, _ptr] + _COMMON + [_ptr, _ptr, C.c_size_t, _ptr]
 SIGNATURES["b200proj_accumulator_fold"] = [_ptr, _i64, _i64, _ptr, _ptr, _int, _ptr]
 SIGNATURES["b200proj_accumulator_fold_range"] = [_ptr, _i64, _i64, _ptr, _ptr, _int, _ptr]
 SIGNATURES["b200proj_accumulator_fold_normalized"] = [_ptr, _i64, _i64, _dbl, _ptr, _ptr]
@@ -54,7 +55,7 @@ SIGNATURES["b200proj_reduction_rate_probe_streaming"] = [_ptr, C.c_size_t, C.c_s
 SIGNATURES["b200proj_backproject_2d_to_3d_accumulate_slabs"] = [_ptr, _ptr] + _COMMON + [_ptr, _int, _int, _ptr]
 EXPORTS = list(SIGNATURES) + ["b200proj_version", "b200proj_last_error", "b200proj_rec_boxsize",
                                 "b200proj_backproject_workspace_bytes", "b200proj_accumulator_bytes",
-                                "b200proj_source_stamp", "b200proj_accumulator_slab_plan",
+                                "b200proj_source_stamp", "b200proj_accumulator_slab_plan", "b200proj_scatter_workspace_bytes",
                                 "b200proj_accumulator_slab_voxels", "b200proj_debug_index", "b200proj_cutoff_pack_index"]
 
 _lib: Optional[C.CDLL] = None
@@ -99,6 +100,8 @@ def load() -> C.CDLL:
     lib.b200proj_last_error.argtypes = []
     lib.b200proj_rec_boxsize.restype = _i64
     lib.b200proj_rec_boxsize.argtypes = [_i64, _dbl]
+    lib.b200proj_scatter_workspace_bytes.restype = C.c_size_t
+    lib.b200proj_scatter_workspace_bytes.argtypes = [_i64, _i64, _i64, _int, _int, _dbl, _dbl]
     lib.b200proj_backproject_workspace_bytes.restype = C.c_size_t
     lib.b200proj_backproject_workspace_bytes.argtypes = [_int, _i64, _i64, _i64, _i64, _int, _int]
     lib.b200proj_accumulator_bytes.restype = C.c_size_t
@@ -242,8 +245,14 @@ def backproject_accumulate(proj, weights, rot, shifts, interp, oversampling, cut
     """Add the slices into the persistent interleaved accumulator (a zero-initialised CUDA tensor
     of accumulator_bytes(B, R) bytes); see b200proj_backproject_2d_to_3d_accumulate."""
     B, P, N = proj.shape[0], proj.shape[1], proj.shape[2]
-    _call("b200proj_backproject_2d_to_3d_accumulate", proj, _p(proj), _p(weights),
-          *_geom(B, R, rot, shifts, P, N, interp, oversampling, cutoff), _p(accumulator))
+    geom = _geom(B, R, rot, shifts, P, N, interp, oversampling, cutoff)
+    if interp == CUBIC:          # large cubic chunks run brick by brick, with scratch
+        n = int(load().b200proj_scatter_workspace_bytes(B, P, N, interp, 1, float(oversampling), float(cutoff)))
+        if n:
+            workspace = torch.empty(n, dtype=torch.uint8, device=proj.device)
+            _call("b200proj_backproject_2d_to_3d_accumulate_ws", proj, _p(proj), _p(weights), *geom, _p(accumulator), _p(workspace), n)
+            return
+    _call("b200proj_backproject_2d_to_3d_accumulate", proj, _p(proj), _p(weights), *geom, _p(accumulator))
 
 
 def backproject_accumulate_slabs(proj, weights, rot, shifts, interp, oversampling, cutoff, R, accumulator,

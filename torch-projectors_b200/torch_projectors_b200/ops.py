@@ -133,10 +133,12 @@ def set_pose_order_thresholds(min_volume_bytes: int = 96 << 20, min_poses: int =
 # When the reconstruction needs a gradient too, the backward pass still scatters, and onto a small
 # reconstruction that scatter is bound by contention, not by the gather beside it (one 128 x 65
 # reference, 65,536 poses, cubic: 9.8 ms either way, while the forward pass pays 1.4 ms for the
-# derivatives): below SAVE_DERIVATIVES_MIN_VOLUME_BYTES per batch item the plain pair stays.
+# derivatives): below SAVE_DERIVATIVES_MIN_VOLUME_BYTES per batch item the plain pair stays -- in 3D only
+# up to SAVE_DERIVATIVES_MIN_PIXELS, beyond which the scatter runs brick by brick without that contention.
 SAVE_DERIVATIVES = True
 SAVE_DERIVATIVES_MAX_BYTES = 16 << 30
 SAVE_DERIVATIVES_MIN_VOLUME_BYTES = 2 << 20
+SAVE_DERIVATIVES_MIN_PIXELS = 1 << 22
 
 
 def set_save_derivatives(enabled: bool = True, max_bytes: int = 16 << 30, min_volume_bytes: int = 2 << 20) -> None:
@@ -569,9 +571,11 @@ def _save_derivatives(dim, reconstruction, rotations, output_shape, interpolatio
         return _PLAIN
     if not need_rot:
         return _KEEP_OUTPUT if need_shift else _PLAIN      # costs the forward pass nothing and spares the backward pass its gather
-    if need_rec and not (interpolation == "cubic" and reconstruction[0].numel() * 8 >= SAVE_DERIVATIVES_MIN_VOLUME_BYTES):
-        return _PLAIN
     N = int(output_shape[0])
+    if need_rec and not (interpolation == "cubic" and
+                         (reconstruction[0].numel() * 8 >= SAVE_DERIVATIVES_MIN_VOLUME_BYTES or
+                          (dim == 3 and reconstruction.size(0) * rotations.size(1) * N * N >= SAVE_DERIVATIVES_MIN_PIXELS))):
+        return _PLAIN
     fits = 8 * (2 if dim == 2 else 4) * reconstruction.size(0) * rotations.size(1) * N * (N // 2 + 1) <= SAVE_DERIVATIVES_MAX_BYTES
     return _KEEP_DERIVATIVES if fits else _PLAIN
 
