@@ -128,6 +128,31 @@ int zero_async(void* p, size_t bytes, cudaStream_t s) {
     return e == cudaSuccess ? B200PROJ_OK : cuda_fail(e, "cudaMemsetAsync");
 }
 
+// Clear up to three outputs (NULL or empty: none).  What is below a few MB goes into one launch; a memset runs at
+// full bandwidth but costs a launch per output.
+int zero_outputs(cudaStream_t s, void* a, size_t na, void* b, size_t nb, void* c = nullptr, size_t nc = 0) {
+    void* p[3] = {a, b, c};
+    const size_t n[3] = {na, nb, nc};
+    ZeroRegions z{};
+    int small = 0;
+    size_t words = 0;
+    for (int r = 0; r < 3; ++r) {
+        if (p[r] == nullptr || n[r] == 0) continue;
+        if (n[r] > (4u << 20)) {
+            if (int rc = zero_async(p[r], n[r], s)) return rc;
+            continue;
+        }
+        z.p[small] = (unsigned*)p[r];
+        z.n[small++] = n[r] / 4;
+        words += n[r] / 4;
+    }
+    if (small == 0) return B200PROJ_OK;
+    if (small == 1) return zero_async(z.p[0], z.n[0] * 4, s);
+    const size_t blocks = (words + 1023) / 1024;
+    zero_regions_kernel<<<(unsigned)(blocks < 1184 ? blocks : 1184), 256, 0, s>>>(z);
+    return check_launch("zero_regions launch");
+}
+
 // Slab plan of the slab-ordered 3D back-projection: volumes whose planes of one batch item
 // exceed 160 MB are processed in slabs of at most `slab_mb` MB of planes.  `eager` lowers the
 // threshold to 120 MB: an interleaved accumulator (16 bytes per voxel) just above L2 (box 256:
@@ -347,17 +372,27 @@ void launch_project_back(const Launch& L, cudaStream_t s, const C2<Real>* gp, co
 #undef B200PROJ_PB
 }
 
-template <int DIM, bool CUBIC, bool NEED_REC, bool RECORDS>
+template <int DIM, bool CUBIC, bool RECORDS>
 void launch_project_back_saved(const Launch& L, cudaStream_t s, const float2* gp, const float2* out, const float2* derivs,
                                const float* rot, const float* shifts, float2* grad_rec, float* grad_rot, float* grad_shift) {
     const bool nr = grad_rot != nullptr, ns = grad_shift != nullptr;
 #define B200PROJ_PBS(NR, NS) \
-    project_back_saved_kernel<DIM, CUBIC, NR, NS, NEED_REC, RECORDS><<<L.grid, kBlockThreads, 0, s>>>(gp, out, derivs, rot, shifts, grad_rec, grad_rot, grad_shift, L.g)
+    project_back_saved_kernel<DIM, CUBIC, NR, NS, RECORDS><<<L.grid, kBlockThreads, 0, s>>>(gp, out, derivs, rot, shifts, grad_rec, grad_rot, grad_shift, L.g)
     if (nr && ns) B200PROJ_PBS(true, true);
     else if (nr) B200PROJ_PBS(true, false);
     else if (ns) B200PROJ_PBS(false, true);
     else B200PROJ_PBS(false, false);
 #undef B200PROJ_PBS
+}
+
+template <int DIM, bool RECORDS>
+void launch_pose_grad_saved(const Launch& L, cudaStream_t s, const float2* gp, const float2* out, const float2* derivs, float* grad_rot, float* grad_shift) {
+    // one block per slice once that fills the GPU (8 blocks per SM), else the slice in parts of at least 1,024 pixels
+    const int64_t fill = 148 * 8 / (int64_t)L.g.BP, most = (L.g.slice_pixels + 1023) / 1024;
+    const dim3 grid((unsigned)L.g.BP, (unsigned)(fill < 1 ? 1 : fill < most ? fill : most), 1);
+    if (grad_rot != nullptr && grad_shift != nullptr) pose_grad_saved_kernel<DIM, true, true, RECORDS><<<grid, kBlockThreads, 0, s>>>(gp, out, derivs, grad_rot, grad_shift, L.g);
+    else if (grad_rot != nullptr) pose_grad_saved_kernel<DIM, true, false, RECORDS><<<grid, kBlockThreads, 0, s>>>(gp, out, derivs, grad_rot, grad_shift, L.g);
+    else pose_grad_saved_kernel<DIM, false, true, RECORDS><<<grid, kBlockThreads, 0, s>>>(gp, out, derivs, grad_rot, grad_shift, L.g);
 }
 
 // Forward projection that also writes the pixels' derivatives (as planes, or as one record per pixel), and the
@@ -401,9 +436,8 @@ int project_back_saved(const float* grad_proj, const float* out, const float* de
         return fail(B200PROJ_ERR_ARGUMENT, "grad_shifts requested but no shifts / saved projections given");
     if (grad_rec == nullptr && grad_rot == nullptr && grad_shifts == nullptr) return B200PROJ_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    if (int rc = zero_async(grad_rec, L.rec_count * sizeof(float2), s)) return rc;
-    if (int rc = zero_async(grad_rot, (size_t)B_rot * P * DIM * DIM * sizeof(float), s)) return rc;
-    if (int rc = zero_async(grad_shifts, (size_t)(shifts ? B_shift : 0) * P * 2 * sizeof(float), s)) return rc;
+    if (int rc = zero_outputs(s, grad_rec, L.rec_count * sizeof(float2), grad_rot, (size_t)B_rot * P * DIM * DIM * sizeof(float),
+                              grad_shifts, (size_t)(shifts ? B_shift : 0) * P * 2 * sizeof(float))) return rc;
     if (P == 0) return B200PROJ_OK;
     const float2* gp = (const float2*)grad_proj;
     const float2* o = (const float2*)out;
@@ -419,10 +453,10 @@ int project_back_saved(const float* grad_proj, const float* out, const float* de
         }
     }
     if (grad_rec != nullptr) {
-        if (cubic) launch_project_back_saved<DIM, true, true, RECORDS>(L, s, gp, o, d, rot, shifts, (float2*)grad_rec, grad_rot, grad_shifts);
-        else launch_project_back_saved<DIM, false, true, RECORDS>(L, s, gp, o, d, rot, shifts, (float2*)grad_rec, grad_rot, grad_shifts);
+        if (cubic) launch_project_back_saved<DIM, true, RECORDS>(L, s, gp, o, d, rot, shifts, (float2*)grad_rec, grad_rot, grad_shifts);
+        else launch_project_back_saved<DIM, false, RECORDS>(L, s, gp, o, d, rot, shifts, (float2*)grad_rec, grad_rot, grad_shifts);
     } else {
-        launch_project_back_saved<DIM, false, false, RECORDS>(L, s, gp, o, d, rot, shifts, nullptr, grad_rot, grad_shifts);
+        launch_pose_grad_saved<DIM, RECORDS>(L, s, gp, o, d, grad_rot, grad_shifts);
     }
     return check_launch("project_back (saved derivatives) launch");
 }
@@ -440,9 +474,8 @@ int project_back(const Real* grad_proj, const Real* rec, int64_t B, int64_t R, c
     if (grad_shifts != nullptr && shifts == nullptr)
         return fail(B200PROJ_ERR_ARGUMENT, "grad_shifts requested but no shifts given");
     cudaStream_t s = (cudaStream_t)stream;
-    if (int rc = zero_async(grad_rec, L.rec_count * sizeof(C2<Real>), s)) return rc;
-    if (int rc = zero_async(grad_rot, (size_t)B_rot * P * DIM * DIM * sizeof(Real), s)) return rc;
-    if (int rc = zero_async(grad_shifts, (size_t)(shifts ? B_shift : 0) * P * 2 * sizeof(Real), s)) return rc;
+    if (int rc = zero_outputs(s, grad_rec, L.rec_count * sizeof(C2<Real>), grad_rot, (size_t)B_rot * P * DIM * DIM * sizeof(Real),
+                              grad_shifts, (size_t)(shifts ? B_shift : 0) * P * 2 * sizeof(Real))) return rc;
     if (P == 0) return B200PROJ_OK;
     if constexpr (DIM == 3 && std::is_same<Real, float>::value) {
         if (interpolation == B200PROJ_CUBIC && grad_rot == nullptr && grad_shifts == nullptr && workspace != nullptr) {
@@ -480,8 +513,7 @@ int backproject_forw(const Real* proj, const Real* weights, int64_t B, int64_t R
         const BrickLaunch bl = cubic && P > 0 && workspace != nullptr ? scatter_plan(B, P, N, hw, os, cutoff) : BrickLaunch{};
         if (bl.use && workspace_bytes >= bl.bytes && (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0) {
             if (!accumulate) {
-                if (int rc = zero_async(data_rec, L.rec_count * sizeof(C2<Real>), s)) return rc;
-                if (int rc = zero_async(weight_rec, L.rec_count * sizeof(Real), s)) return rc;
+                if (int rc = zero_outputs(s, data_rec, L.rec_count * sizeof(C2<Real>), weight_rec, L.rec_count * sizeof(Real))) return rc;
             }
             return hw ? launch_brick_scatter<true, true>(L, bl, workspace, proj, weights, rot, shifts, data_rec, weight_rec, s)
                       : launch_brick_scatter<false, true>(L, bl, workspace, proj, nullptr, rot, shifts, data_rec, nullptr, s);
@@ -514,8 +546,7 @@ int backproject_forw(const Real* proj, const Real* weights, int64_t B, int64_t R
     }
     }
     if (!accumulate) {
-        if (int rc = zero_async(data_rec, L.rec_count * sizeof(C2<Real>), s)) return rc;
-        if (int rc = zero_async(weight_rec, L.rec_count * sizeof(Real), s)) return rc;
+        if (int rc = zero_outputs(s, data_rec, L.rec_count * sizeof(C2<Real>), weight_rec, L.rec_count * sizeof(Real))) return rc;
     }
     if (P == 0) return B200PROJ_OK;
     const C2<Real>* p = (const C2<Real>*)proj;
@@ -579,8 +610,7 @@ int backproject_back(const Real* grad_data_rec, const Real* grad_weight_rec, con
         return fail(B200PROJ_ERR_ARGUMENT, "grad_data_rec boxsize %lld does not match ceil(N*oversampling) rounded up to even = %lld",
                     (long long)R, (long long)b200proj_rec_boxsize(N, os));
     cudaStream_t s = (cudaStream_t)stream;
-    if (int rc = zero_async(grad_rot, (size_t)B_rot * P * DIM * DIM * sizeof(Real), s)) return rc;
-    if (int rc = zero_async(grad_shifts, (size_t)(shifts ? B_shift : 0) * P * 2 * sizeof(Real), s)) return rc;
+    if (int rc = zero_outputs(s, grad_rot, (size_t)B_rot * P * DIM * DIM * sizeof(Real), grad_shifts, (size_t)(shifts ? B_shift : 0) * P * 2 * sizeof(Real))) return rc;
     if (grad_weights != nullptr && grad_weight_rec == nullptr)   // weights given, no incoming gradient: zeros
         if (int rc = zero_async(grad_weights, L.pix_count * sizeof(Real), s)) return rc;
     if (P == 0) return B200PROJ_OK;

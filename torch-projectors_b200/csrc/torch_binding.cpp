@@ -256,7 +256,7 @@ Tensor empty_derivatives(int dim, int64_t B, int64_t P, int64_t N, const at::Ten
     return at::empty({B, P, N, N / 2 + 1, 4}, opt).permute({4, 0, 1, 2, 3}).narrow(0, 0, 3);
 }
 // Derivatives in the layout the kernels read: as made above, or copied into it.
-Tensor kernel_derivatives(int dim, const Tensor& d) {
+Tensor kernel_derivatives(int dim, const Tensor& d, const Tensor& projections) {
     if (dim == 2) return d.contiguous();
     int64_t stride = 4;
     bool records = d.stride(0) == 1 && (reinterpret_cast<uintptr_t>(d.data_ptr()) & 31u) == 0;
@@ -265,8 +265,9 @@ Tensor kernel_derivatives(int dim, const Tensor& d) {
         stride *= d.size(a);
     }
     if (records) return d;
-    Tensor made = empty_derivatives(3, d.size(1), d.size(2), d.size(3), d.options());
-    made.copy_(d);
+    Tensor made = at::empty({d.size(1), d.size(2), d.size(3), d.size(4), 4}, d.options());
+    made.narrow(4, 0, 3).copy_(d.permute({1, 2, 3, 4, 0}));
+    made.select(4, 3).copy_(projections);
     return made;
 }
 
@@ -328,7 +329,7 @@ std::tuple<Tensor, Tensor, Tensor> project_back_saved(int dim, const Tensor& gra
     const bool need_shift = p.shifts.defined() && shifts->requires_grad();
     const Tensor gp = grad_projections.contiguous();
     const Tensor out = projections.contiguous();
-    const Tensor der = derivatives.numel() ? kernel_derivatives(dim, derivatives) : Tensor();
+    const Tensor der = derivatives.numel() ? kernel_derivatives(dim, derivatives, projections) : Tensor();
     const int64_t R = reconstruction.size(-2);
     c10::cuda::CUDAGuard guard(gp.device());
     Tensor grad_rec = need_rec_grad ? at::empty(reconstruction.sizes(), gp.options()) : Tensor();
