@@ -12,7 +12,7 @@
 #include <mutex>
 #include <type_traits>
 
-#include "brick_kernels.cuh"
+#include "brick_scatter.cuh"
 
 namespace {
 
@@ -276,10 +276,11 @@ BrickLaunch gather_plan(int64_t B, int64_t P, int64_t N, bool cubic, bool record
     return L;
 }
 
-// Cubic scatter (measured crossings: 1.1-1.3 M pixels for box-64 and box-128 volumes, 2 M for box 256, 4.6 M for box 400).
-BrickLaunch scatter_plan(int64_t B, int64_t P, int64_t N, bool weights, double os, double cutoff) {
-    BrickLaunch L = weights ? brick_layout<Scatter<true>::Brick>(B, P, N, os, cutoff, 148.0 * Scatter<true>::kBlocks, 1500.0, false)
-                            : brick_layout<Scatter<false>::Brick>(B, P, N, os, cutoff, 148.0 * Scatter<false>::kBlocks, 1500.0, false);
+// Cubic scatter (linear taps keep the plain kernels, see brick_scatter.cuh).
+BrickLaunch scatter_plan(int64_t B, int64_t P, int64_t N, bool cubic, bool weights, double os, double cutoff) {
+    if (!cubic) return BrickLaunch{};
+    BrickLaunch L = weights ? brick_layout<Scatter<true>::Brick>(B, P, N, os, cutoff, 148.0 * Scatter<true>::kBlocks, 3000.0, false)
+                            : brick_layout<Scatter<false>::Brick>(B, P, N, os, cutoff, 148.0 * Scatter<false>::kBlocks, 3000.0, false);
     L.use = L.use && (L.forced || L.pixels > 1.2e6 + 150.0 * L.in_ball);
     return L;
 }
@@ -316,13 +317,14 @@ int launch_brick_forw(const Launch& L, const BrickLaunch& bl, void* workspace, c
 template <bool WEIGHTS, bool DUP, bool INTERLEAVED = false>
 int launch_brick_scatter(const Launch& L, const BrickLaunch& bl, void* workspace, const float* proj, const float* weights, const float* rot,
                          const float* shifts, float* vol, float* wvol, cudaStream_t s, float4* accum = nullptr) {
+    using C = Scatter<WEIGHTS>;
     const BrickWork w = brick_work(bl, workspace);
     if (int rc = brick_setup(bl, w, L, rot, shifts, false, s)) return rc;
-    constexpr size_t smem = sizeof(typename Scatter<WEIGHTS>::Shared);
-    static_assert((smem + 1024) * Scatter<WEIGHTS>::kBlocks <= 233472, "shared memory of an SM");
+    constexpr size_t smem = sizeof(typename C::Shared);
+    static_assert((smem + 1024) * C::kBlocks <= 233472, "shared memory of an SM");
     const cudaError_t e = cudaFuncSetAttribute(brick_scatter_kernel<WEIGHTS, DUP, INTERLEAVED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cuda_fail(e, "brick_scatter shared memory");
-    brick_scatter_kernel<WEIGHTS, DUP, INTERLEAVED><<<148 * Scatter<WEIGHTS>::kBlocks, Scatter<WEIGHTS>::kThreads, smem, s>>>((const float2*)proj, weights, rot, shifts, (float2*)vol, wvol, accum, w, L.g, bl.plan);
+    brick_scatter_kernel<WEIGHTS, DUP, INTERLEAVED><<<148 * C::kBlocks, C::kThreads, smem, s>>>((const float2*)proj, weights, rot, shifts, (float2*)vol, wvol, accum, w, L.g, bl.plan);
     return check_launch("brick_scatter launch");
 }
 
@@ -445,7 +447,7 @@ int project_back_saved(const float* grad_proj, const float* out, const float* de
     const bool cubic = interpolation == B200PROJ_CUBIC;
     if constexpr (RECORDS) {
         // large cubic scatter: brick by brick, the pose gradients in a streaming pass of their own
-        const BrickLaunch bl = grad_rec != nullptr && cubic && workspace != nullptr ? scatter_plan(B, P, N, false, os, cutoff) : BrickLaunch{};
+        const BrickLaunch bl = grad_rec != nullptr && workspace != nullptr ? scatter_plan(B, P, N, cubic, false, os, cutoff) : BrickLaunch{};
         if (bl.use && workspace_bytes >= bl.bytes) {
             if (int rc = launch_brick_scatter<false, false>(L, bl, workspace, grad_proj, nullptr, rot, shifts, grad_rec, nullptr, s)) return rc;
             if (grad_rot == nullptr && grad_shifts == nullptr) return B200PROJ_OK;
@@ -478,8 +480,9 @@ int project_back(const Real* grad_proj, const Real* rec, int64_t B, int64_t R, c
                               grad_shifts, (size_t)(shifts ? B_shift : 0) * P * 2 * sizeof(Real))) return rc;
     if (P == 0) return B200PROJ_OK;
     if constexpr (DIM == 3 && std::is_same<Real, float>::value) {
-        if (interpolation == B200PROJ_CUBIC && grad_rot == nullptr && grad_shifts == nullptr && workspace != nullptr) {
-            const BrickLaunch bl = scatter_plan(B, P, N, false, os, cutoff);
+        if (grad_rot == nullptr && grad_shifts == nullptr && workspace != nullptr) {
+            const bool cubic = interpolation == B200PROJ_CUBIC;
+            const BrickLaunch bl = scatter_plan(B, P, N, cubic, false, os, cutoff);
             if (bl.use && workspace_bytes >= bl.bytes) return launch_brick_scatter<false, false>(L, bl, workspace, grad_proj, nullptr, rot, shifts, grad_rec, nullptr, s);
         }
     }
@@ -510,7 +513,7 @@ int backproject_forw(const Real* proj, const Real* weights, int64_t B, int64_t R
     // (one v4 reduction per tap), folded into the outputs afterwards.
     const size_t ws_one = L.rec_count * sizeof(float4);
     if constexpr (DIM == 3 && std::is_same<Real, float>::value) {
-        const BrickLaunch bl = cubic && P > 0 && workspace != nullptr ? scatter_plan(B, P, N, hw, os, cutoff) : BrickLaunch{};
+        const BrickLaunch bl = P > 0 && workspace != nullptr ? scatter_plan(B, P, N, cubic, hw, os, cutoff) : BrickLaunch{};
         if (bl.use && workspace_bytes >= bl.bytes && (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0) {
             if (!accumulate) {
                 if (int rc = zero_outputs(s, data_rec, L.rec_count * sizeof(C2<Real>), weight_rec, L.rec_count * sizeof(Real))) return rc;
@@ -644,8 +647,8 @@ int backproject_accumulate(const float* proj, const float* weights, int64_t B, i
     cudaStream_t s = (cudaStream_t)stream;
     float4* acc = (float4*)accumulator;
     const bool cubic = interpolation == B200PROJ_CUBIC;
-    if (cubic && workspace != nullptr && slab_count == plan.slabs) {
-        const BrickLaunch bl = scatter_plan(B, P, N, true, os, cutoff);
+    if (workspace != nullptr && slab_count == plan.slabs) {
+        const BrickLaunch bl = scatter_plan(B, P, N, cubic, true, os, cutoff);
         if (bl.use && workspace_bytes >= bl.bytes) return launch_brick_scatter<true, true, true>(L, bl, workspace, proj, weights, rot, shifts, nullptr, nullptr, s, acc);
     }
     if (plan.slabs > 1) {
@@ -793,8 +796,7 @@ int b200proj_project_3d_to_2d_forw(const float* rec, int64_t B, int64_t R, const
 }
 
 size_t b200proj_scatter_workspace_bytes(int64_t B, int64_t P, int64_t N, int interpolation, int has_weights, double oversampling, double cutoff) {
-    if (interpolation != B200PROJ_CUBIC) return 0;
-    const BrickLaunch bl = scatter_plan(B, P, N, has_weights != 0, oversampling, cutoff);
+    const BrickLaunch bl = scatter_plan(B, P, N, interpolation == B200PROJ_CUBIC, has_weights != 0, oversampling, cutoff);
     return bl.use ? bl.bytes : 0;
 }
 size_t b200proj_project_workspace_bytes(int64_t B, int64_t P, int64_t N, int interpolation, int records, double oversampling, double cutoff) {

@@ -599,294 +599,4 @@ brick_forw_kernel(const float2* __restrict__ rec, const float* __restrict__ rot,
     }
 }
 
-// ---- scatter ------------------------------------------------------------------------------------------
-// Gradient of the projection with respect to the volume, and back-projection, with cubic taps.  The plain kernels
-// send every tap to L2 as a reduction (64 per pixel) and sit on the rate at which reductions leave the SMs, 40
-// clocks per pixel and SM.  Here a brick's sums are kept in shared memory and leave once per work item.
-//
-// Shared-memory float atomics are compare-and-swap loops (6.5 clocks per warp and float); plain read-add-write is
-// 4.3 clocks per warp and complex number, so a block has ONE warp that adds (no other warp touches the sums) and
-// four that walk over the slices and hand it the pixels through a double-buffered queue.  The adding warp takes 32
-// pixels at a time, one per lane, and every lane its taps in an order that starts at its own class
-// (x & 3, y & 3, z & 3 in pairs): at every step the 32 lanes and their two taps are 64 different classes,
-// hence 64 different voxels, whatever pixels they hold -- no two lanes ever add to the same voxel between two
-// synchronisations of the warp, and no bank conflicts arise.
-// Measured on B200: the scatter of 4,096 slices of 256 x 129 into a box-512 gradient 14.4 -> 7.8 ms, 2,501 weighted
-// slices of box 90 into box 180 1.61 -> 1.06 ms.  Bound by the adding warp's chain (load, add, store: 60 clocks per 64
-// taps) times the blocks that fit: five per SM with 13^3 sample positions (16^3 sums), four with 13 x 13 x 9 and weights.
-// Two adding warps in turn, three walking warps, or one tall brick per SM whose slabs several warps add to measured
-// slower (8.5, 8.0 and 14.8 ms).
-template <bool WEIGHTS>
-struct Scatter {
-    using Brick = BrickDims<13, 13, WEIGHTS ? 9 : 13>;
-    using Shape = BrickShape<true, Brick>;
-    static constexpr int kWalkers = 4, kThreads = (kWalkers + 1) * 32;
-    static constexpr int kBlocks = WEIGHTS ? 4 : 5;         // per SM
-    static constexpr int kQueue = WEIGHTS ? 48 : 32;        // pixels a walking warp hands over at a time
-    struct Queue {
-        float4 a[kWalkers * kQueue];        // fx, fy, fz, local position (x | y << 8 | z << 16)
-        float2 v[kWalkers * kQueue];
-        float w[WEIGHTS ? kWalkers * kQueue : 1];
-        int count[kWalkers], done[kWalkers];
-    };
-    struct Shared {
-        float2 sum[Shape::kVoxels];
-        float wsum[WEIGHTS ? Shape::kVoxels : 1];
-        Queue queue[2];
-        BrickBlock<1, 64> walk[kWalkers];
-        int item;
-    };
-};
-
-// Add 32 pixels, one per lane (a lane without one adds zeros somewhere).
-template <bool WEIGHTS>
-__device__ __forceinline__ void brick_add(typename Scatter<WEIGHTS>::Shared& sh, const float4 a, float2 v, float wv) {
-    using S = typename Scatter<WEIGHTS>::Shape;
-    using u64 = unsigned long long;
-    const int lane = threadIdx.x & 31;
-    const unsigned at = __float_as_uint(a.w);
-    const int lx = at & 255, ly = at >> 8 & 255, lz = at >> 16;
-    const int rx = lx & 3, ry = ly & 3, tx = (lane - lx) & 3, ty = ((lane >> 2) - ly) & 3, tz = (2 * (lane >> 4) - lz) & 3;
-    int ox[4], oy[4], oz[4];
-    const int base = (lz * S::kPlane + (ly >> 2) * S::kRowCells + (lx >> 2) * 16) * 8;
-    float wx[4], wy[4], wz[4];
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-        const int ax = (lane + s) & 3, ay = ((lane >> 2) + s) & 3;
-        ox[s] = ax * 8 + (ax < rx ? 128 : 0);
-        oy[s] = ay * 32 + (ay < ry ? S::kRowCells * 8 : 0);
-        oz[s] = ((tz + s) & 3) * S::kPlane * 8 + base;
-    }
-    cubic_weights(a.x, wx);
-    rotate4(wx, tx);
-    cubic_weights(a.y, wy);
-    rotate4(wy, ty);
-    cubic_weights(a.z, wz);
-    rotate4(wz, tz);
-    const u64 v2 = pack2(v.x, v.y);
-    u64 wx2[4];
-#pragma unroll
-    for (int s = 0; s < 4; ++s) wx2[s] = pack2(wx[s], wx[s]);
-    char* sums = reinterpret_cast<char*>(sh.sum);
-    char* wsums = reinterpret_cast<char*>(sh.wsum);
-#pragma unroll
-    for (int c = 0; c < 4; c += 2) {
-        const u64 p0 = fmul2(pack2(wz[c], wz[c]), v2), p1 = fmul2(pack2(wz[c + 1], wz[c + 1]), v2);
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const u64 wy2 = pack2(wy[b], wy[b]);
-            const u64 q0 = fmul2(wy2, p0), q1 = fmul2(wy2, p1);
-            const int a0 = oz[c] + oy[b], a1 = oz[c + 1] + oy[b];
-            float f0 = 0.f, f1 = 0.f;
-            if (WEIGHTS) {
-                f0 = wv * fabsf(wz[c] * wy[b]);
-                f1 = wv * fabsf(wz[c + 1] * wy[b]);
-            }
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                {
-                    u64* s0 = reinterpret_cast<u64*>(sums + a0 + ox[k]);
-                    u64* s1 = reinterpret_cast<u64*>(sums + a1 + ox[k]);
-                    const u64 u0 = *s0, u1 = *s1;
-                    *s0 = fma2(wx2[k], q0, u0);
-                    *s1 = fma2(wx2[k], q1, u1);
-                    if (WEIGHTS) {
-                        float* t0 = reinterpret_cast<float*>(wsums + ((a0 + ox[k]) >> 1));
-                        float* t1 = reinterpret_cast<float*>(wsums + ((a1 + ox[k]) >> 1));
-                        const float g0 = *t0, g1 = *t1;
-                        *t0 = fmaf(fabsf(wx[k]), f0, g0);
-                        *t1 = fmaf(fabsf(wx[k]), f1, g1);
-                    }
-                }
-                __syncwarp();
-            }
-        }
-    }
-}
-
-// Sums of a finished item to the volume, by the scatter's rules (Friedel mirror with conjugation, taps outside the
-// stored half-volume dropped, DUP: the conjugate also to the Friedel partner of a voxel on the c == 0 plane); cleared
-// for the next item.  INTERLEAVED: into 16-byte (re, im, weight, 0) voxels.
-template <bool WEIGHTS, bool DUP, bool INTERLEAVED>
-__device__ __forceinline__ void brick_flush(const SliceGeom& g, typename Scatter<WEIGHTS>::Shared& sh, float2* __restrict__ vol, float* __restrict__ wvol,
-                                            float4* __restrict__ accum, int X0, int Y0, int Z0) {
-    auto add = [&](int off, float re, float im, float w) {
-        if (INTERLEAVED) {
-            red_add_v4(accum + off, re, im, w, 0.f);
-        } else {
-            red_add_v2(vol + off, re, im);
-            if (WEIGHTS) red_add(wvol + off, w);
-        }
-    };
-    using S = typename Scatter<WEIGHTS>::Shape;
-    for (int t = (int)threadIdx.x; t < S::kVoxels; t += Scatter<WEIGHTS>::kThreads) {
-        const int x = t % S::TX, y = (t / S::TX) % S::TY, z = t / (S::TX * S::TY);
-        const int at = z * S::kPlane + brick_off_y<S>(y) + brick_off_x(x);
-        float2 v = sh.sum[at];
-        const float w = WEIGHTS ? sh.wsum[at] : 0.f;
-        if (v.x == 0.f && v.y == 0.f && w == 0.f) continue;
-        sh.sum[at] = make_float2(0.f, 0.f);
-        if (WEIGHTS) sh.wsum[at] = 0.f;
-        bool m;
-        const int c = scatter_col(g, X0 - 1 + x, m), r = scatter_line(g, Y0 - 1 + y, m), d = scatter_line(g, Z0 - 1 + z, m);
-        if (c < 0 || r < 0 || d < 0) continue;
-        if (m) v.y = -v.y;
-        const int off = (d * g.R + r) * g.Rh + c;
-        add(off, v.x, v.y, w);
-        if (DUP && c == 0) {
-            const int r2 = r == 0 ? 0 : g.R - r, d2 = d == 0 ? 0 : g.R - d;
-            if (r2 != r || d2 != d) add((d2 * g.R + r2) * g.Rh, v.x, -v.y, w);
-        }
-    }
-}
-
-template <bool WEIGHTS, bool DUP, bool INTERLEAVED>
-__global__ void __launch_bounds__(Scatter<WEIGHTS>::kThreads, Scatter<WEIGHTS>::kBlocks)
-brick_scatter_kernel(const float2* __restrict__ proj, const float* __restrict__ weights, const float* __restrict__ rot,
-                     const float* __restrict__ shifts, float2* __restrict__ vol, float* __restrict__ wvol, float4* __restrict__ accum,
-                     BrickWork ws, const SliceGeom g, const BrickPlan pl) {
-    using C = Scatter<WEIGHTS>;
-    extern __shared__ __align__(16) unsigned char dyn[];
-    typename C::Shared& sh = *reinterpret_cast<typename C::Shared*>(dyn);
-    constexpr unsigned kFull = 0xffffffffu;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int t = (int)threadIdx.x; t < C::Shape::kVoxels; t += C::kThreads) {
-        sh.sum[t] = make_float2(0.f, 0.f);
-        if (WEIGHTS) sh.wsum[t] = 0.f;
-    }
-    auto hand_over = [] { asm volatile("bar.sync 1, %0;" ::"n"(C::kThreads) : "memory"); };      // a queue is filled, the other one empty
-    auto all_done = [](const typename C::Queue& q) {
-        int n = 0;
-#pragma unroll
-        for (int w = 0; w < C::kWalkers; ++w) n += *(const volatile int*)&q.done[w];
-        return n == C::kWalkers;
-    };
-    const int items = __ldg(ws.header);
-    while (true) {
-        __syncthreads();
-        if (threadIdx.x == 0) sh.item = atomicAdd(ws.header + 2, 1);
-        __syncthreads();
-        const int item = sh.item;
-        if (item >= items) return;
-        // the item's share of the slices that are not for the bricks: plain scatter
-        for (int k = (int)((long long)g.BP * item / items), k_end = (int)((long long)g.BP * (item + 1) / items); k < k_end; ++k) {
-            const int b = k / g.P, p = k - b * g.P;
-            const float* rm = pose_rot<3>(g, rot, b, p);
-            if (brick_slice_ok(rm)) continue;
-            const int nj = (g.Nh + 7) / 8, ni = (g.N + 3) / 4;
-            for (int patch = warp; patch < ni * nj; patch += C::kThreads / 32) {
-                BlockWork w;
-                w.b = b;
-                w.p = p;
-                w.i = patch / nj * 4 + (lane >> 3);
-                w.j = patch % nj * 8 + (lane & 7);
-                w.in_image = w.i < g.N && w.j < g.Nh;
-                w.pix = (size_t)k * (size_t)g.slice_pixels + (size_t)(w.i * g.Nh + w.j);
-                Pixel px;
-                float2 v;
-                float wv;
-                const bool active = backproject_pixel<3, WEIGHTS>(g, w, proj, weights, rot, shifts, px, v, wv);
-                const size_t at = (size_t)b * g.vol_elems;
-                scatter_coop<3, true, WEIGHTS, DUP, INTERLEAVED>(g, INTERLEAVED ? nullptr : vol + at, WEIGHTS && !INTERLEAVED ? wvol + at : nullptr,
-                                                                 INTERLEAVED ? accum + at : nullptr, px, active, v, wv);
-            }
-        }
-        const int4 it = __ldg(ws.items + item);
-        const int X0 = pl.lo[0] + (it.x & 1023) * C::Brick::x, Y0 = pl.lo[1] + ((it.x >> 10) & 1023) * C::Brick::y, Z0 = pl.lo[2] + (it.x >> 20) * C::Brick::z;
-        if (warp < C::kWalkers) {
-            const BrickWarp& sw = sh.walk[warp].warp[0];
-            int buffer = 0, count = 0;
-            // the previous window's pixels, whose values are still on their way from memory
-            bool held = false;
-            float4 h_a = make_float4(0.f, 0.f, 0.f, 0.f);
-            float2 h_v = make_float2(0.f, 0.f), h_ph = make_float2(1.f, 0.f);
-            float h_w = 0.f;
-            auto put = [&] {
-                const unsigned m = __ballot_sync(kFull, held);
-                int at = held ? count + __popc(m & ((1u << lane) - 1u)) : 1 << 20;
-                count += __popc(m);
-                if (held && g.has_shift) h_v = cmul_conj(h_v, h_ph);
-                while (true) {                                              // once or twice: what does not fit waits for the other queue
-                    typename C::Queue& q = sh.queue[buffer];
-                    if (at < C::kQueue) {
-                        q.a[warp * C::kQueue + at] = h_a;
-                        q.v[warp * C::kQueue + at] = h_v;
-                        if (WEIGHTS) q.w[warp * C::kQueue + at] = h_w;
-                        at = 1 << 20;
-                    }
-                    if (count < C::kQueue) return;
-                    if (lane == 0) { q.count[warp] = C::kQueue; q.done[warp] = 0; }
-                    __syncwarp();
-                    hand_over();
-                    buffer ^= 1;
-                    count -= C::kQueue;
-                    at -= C::kQueue;
-                }
-            };
-            brick_walk<typename C::Brick>(g, ws.recs, sh.walk[warp], X0, Y0, Z0, it.z, it.w, warp, C::kWalkers,
-                                          [&](bool active, int slot, int i, int j, const Pixel& px, int lx, int ly, int lz) {
-                active = active && !(j == 0 && i >= g.N / 2);
-                float2 v = make_float2(0.f, 0.f);
-                float w = 0.f;
-                if (active) {
-                    const size_t pix = (size_t)sw.slice[slot] * (size_t)g.slice_pixels + (size_t)(i * g.Nh + j);
-                    v = __ldg(proj + pix);
-                    if (WEIGHTS) w = __ldg(weights + pix);
-                }
-                put();
-                held = active;
-                h_a = make_float4(px.c - floorf(px.c), px.r - floorf(px.r), px.d - floorf(px.d), __uint_as_float((unsigned)(lx | ly << 8 | lz << 16)));
-                h_v = v;
-                h_w = w;
-                if (g.has_shift) {
-                    const float4 rc = sw.slots[slot][2];
-                    h_ph = phase_ramp(g, px, rc.y, rc.z);
-                }
-            });
-            put();
-            while (true) {
-                typename C::Queue& q = sh.queue[buffer];
-                if (lane == 0) { q.count[warp] = count; q.done[warp] = 1; }
-                __syncwarp();
-                hand_over();
-                if (all_done(q)) break;
-                buffer ^= 1;
-                count = 0;
-            }
-        } else {
-            for (int buffer = 0;; buffer ^= 1) {
-                hand_over();
-                const typename C::Queue& q = sh.queue[buffer];
-                int n[C::kWalkers], total = 0;
-#pragma unroll
-                for (int w = 0; w < C::kWalkers; ++w) total += n[w] = *(const volatile int*)&q.count[w];
-                const bool last = all_done(q);
-                for (int k0 = 0; k0 < total; k0 += 32) {
-                    int k = k0 + lane, at = 0;
-                    const bool active = k < total;
-#pragma unroll
-                    for (int w = 0; w < C::kWalkers; ++w) {
-                        if (k >= 0 && k < n[w]) at = w * C::kQueue + k;
-                        k -= n[w];
-                    }
-                    float4 a = q.a[at];
-                    float2 v = q.v[at];
-                    float wv = WEIGHTS ? q.w[at] : 0.f;
-                    if (!active) {
-                        a = make_float4(0.f, 0.f, 0.f, 0.f);
-                        v = make_float2(0.f, 0.f);
-                        wv = 0.f;
-                    }
-                    brick_add<WEIGHTS>(sh, a, v, wv);
-                }
-                if (last) break;
-            }
-        }
-        __syncthreads();
-        const size_t at = (size_t)it.y * g.vol_elems;
-        brick_flush<WEIGHTS, DUP, INTERLEAVED>(g, sh, INTERLEAVED ? nullptr : vol + at, WEIGHTS && !INTERLEAVED ? wvol + at : nullptr,
-                                               INTERLEAVED ? accum + at : nullptr, X0, Y0, Z0);
-    }
-}
-
 }  // namespace b200proj
