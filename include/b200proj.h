@@ -107,6 +107,12 @@ size_t b200proj_project_workspace_bytes(int64_t B, int64_t P, int64_t N, int int
  * the last of them see there for what else a workspace is good for). */
 size_t b200proj_scatter_workspace_bytes(int64_t B, int64_t P, int64_t N, int interpolation, int has_weights,
                                         double oversampling, double fourier_radius_cutoff);
+/* Workspace of the backward passes of the projection (b200proj_project_{2d,3d_to_2d}_back_ws with grad_rec,
+ * b200proj_project_2d_back_saved_ws, b200proj_project_3d_to_2d_back_records): the larger calls above, and copies
+ * of a small reconstruction over which the scatter is spread (reductions onto less than ~2 MB run at
+ * half the rate).  pose_gradients != 0: of a _back_ws call that also computes grad_rot or grad_shifts. */
+size_t b200proj_gradient_workspace_bytes(int dim, int64_t B, int64_t R, int64_t P, int64_t N, int interpolation,
+                                         int pose_gradients, double oversampling, double fourier_radius_cutoff);
 int b200proj_project_3d_to_2d_forw_ws(const float* rec, int64_t B, int64_t R,
                                       const float* rot, int64_t B_rot,
                                       const float* shifts, int64_t B_shift,
@@ -115,6 +121,18 @@ int b200proj_project_3d_to_2d_forw_ws(const float* rec, int64_t B, int64_t R,
                                       const int32_t* pose_order, void* workspace,
                                       size_t workspace_bytes, void* stream);
 
+int b200proj_project_2d_back_ws(const float* grad_proj, const float* rec, int64_t B, int64_t R,
+                                const float* rot, int64_t B_rot,
+                                const float* shifts, int64_t B_shift,
+                                int64_t P, int64_t N, int interpolation, double oversampling,
+                                double fourier_radius_cutoff, float* grad_rec, float* grad_rot,
+                                float* grad_shifts, void* workspace, size_t workspace_bytes, void* stream);
+int b200proj_project_2d_back_saved_ws(const float* grad_proj, const float* out, const float* derivatives,
+                                      int64_t B, int64_t R, const float* rot, int64_t B_rot,
+                                      const float* shifts, int64_t B_shift, int64_t P, int64_t N,
+                                      int interpolation, double oversampling, double fourier_radius_cutoff,
+                                      float* grad_rec, float* grad_rot, float* grad_shifts,
+                                      void* workspace, size_t workspace_bytes, void* stream);
 int b200proj_project_3d_to_2d_back_ws(const float* grad_proj, const float* rec, int64_t B, int64_t R,
                                       const float* rot, int64_t B_rot,
                                       const float* shifts, int64_t B_shift,

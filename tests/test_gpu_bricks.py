@@ -86,3 +86,28 @@ def test_bricks_match_the_oracle(names):
     r = subprocess.run([sys.executable, "-c", f"import sys; sys.path.insert(0, {str(ROOT / 'tests')!r}); import test_gpu_bricks as t; t.check({names!r})"],
                        env=env, cwd=ROOT, capture_output=True, text=True, timeout=600)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]
+
+
+@pytest.mark.parametrize("dim,interp,P", [(2, "linear", 64), (2, "cubic", 67), (3, "linear", 130), (2, "cubic", 63)])
+def test_scatters_spread_over_copies_of_a_small_reconstruction(dim, interp, P):
+    """From 64 poses on, slices are spread over copies of a small reconstruction that are added up at the end: gradients
+    (with and without pose gradients) and back-projection without weights, against the oracle."""
+    import torch_projectors_b200 as tp
+    from oracle import port
+    t = make_inputs(Case("copies", dim, interp, 2, P, 12, 18, 1.5, None, 1, 2, shift_range=2.0, seed=P))
+    project, back = (tp.project_2d_forw, port.project_2d_back) if dim == 2 else (tp.project_3d_to_2d_forw, port.project_3d_to_2d_back)
+    want = back(t["proj"], t["rec"], t["rot"], t["shifts"], interp, 1.5, None, need_rot_grad=True, need_shift_grad=True)
+    for poses in (True, False):
+        for keep in (True, False):
+            tp.set_save_derivatives(keep, min_volume_bytes=0)
+            try:
+                rec, rot, sh = (t[k].cuda().requires_grad_(k == "rec" or poses) for k in ("rec", "rot", "shifts"))
+                project(rec, rot, sh, output_shape=(12, 12), interpolation=interp, oversampling=1.5).backward(t["proj"].cuda())
+            finally:
+                tp.set_save_derivatives(True)
+            assert rel_err(rec.grad, want[0]) <= TOL_ATOMIC
+            if poses:
+                assert rel_err(rot.grad, want[1]) <= TOL_ATOMIC and rel_err(sh.grad, want[2]) <= TOL_ATOMIC
+    forw, ref = (tp.backproject_2d_forw, port.backproject_2d_forw) if dim == 2 else (tp.backproject_2d_to_3d_forw, port.backproject_2d_to_3d_forw)
+    data, _ = forw(t["proj"].cuda(), t["rot"].cuda(), None, t["shifts"].cuda(), interpolation=interp, oversampling=1.5)
+    assert rel_err(data, ref(t["proj"], None, t["rot"], t["shifts"], interp, 1.5, None)[0]) <= TOL_ATOMIC

@@ -281,7 +281,8 @@ BrickLaunch scatter_plan(int64_t B, int64_t P, int64_t N, bool cubic, bool weigh
     if (!cubic) return BrickLaunch{};
     BrickLaunch L = weights ? brick_layout<Scatter<true>::Brick>(B, P, N, os, cutoff, 148.0 * Scatter<true>::kBlocks, 3000.0, false)
                             : brick_layout<Scatter<false>::Brick>(B, P, N, os, cutoff, 148.0 * Scatter<false>::kBlocks, 3000.0, false);
-    L.use = L.use && (L.forced || L.pixels > 1.2e6 + 150.0 * L.in_ball);
+    // measured crossings with the plain kernels, in M pixels: 0.8 / 1.7 / 5 for box-128 / 256 / 400 gradients, 0.55 / 0.8 / 0.9 with weights
+    L.use = L.use && (L.forced || L.pixels > (weights ? 0.6e6 + 45.0 * L.in_ball : 0.75e6 + 430.0 * L.in_ball));
     return L;
 }
 
@@ -326,6 +327,23 @@ int launch_brick_scatter(const Launch& L, const BrickLaunch& bl, void* workspace
     if (e != cudaSuccess) return cuda_fail(e, "brick_scatter shared memory");
     brick_scatter_kernel<WEIGHTS, DUP, INTERLEAVED><<<148 * C::kBlocks, C::kThreads, smem, s>>>((const float2*)proj, weights, rot, shifts, (float2*)vol, wvol, accum, w, L.g, bl.plan);
     return check_launch("brick_scatter launch");
+}
+
+// Copies of a small complex reconstruction over which the slices of a scatter are spread (see workspace_replicas):
+// as many as the rule wants and the workspace holds; sets the kernels' geometry.
+int scatter_copies(Launch& L, const void* workspace, size_t workspace_bytes) {
+    if (workspace == nullptr || (reinterpret_cast<uintptr_t>(workspace) & 15u) != 0) return 1;
+    const size_t one = L.rec_count * sizeof(float2);
+    int copies = workspace_replicas((double)one, L.P);
+    while (copies > 1 && (size_t)copies * one > workspace_bytes) copies /= 2;
+    L.g.replicas = copies;
+    L.g.replica_stride = copies > 1 ? (long long)L.rec_count : 0;
+    return copies;
+}
+int add_copies(const Launch& L, const void* workspace, int copies, float* rec, cudaStream_t s, bool accumulate = false) {
+    const size_t blocks = (L.rec_count + 255) / 256;
+    add_copies_kernel<<<(unsigned)(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, s>>>((const float2*)workspace, (float2*)rec, L.rec_count, copies, accumulate);
+    return check_launch("add_copies launch");
 }
 
 // ---- operator bodies, templated on the dimensionality and the real type (float | double) ------------------------------------
@@ -438,28 +456,33 @@ int project_back_saved(const float* grad_proj, const float* out, const float* de
         return fail(B200PROJ_ERR_ARGUMENT, "grad_shifts requested but no shifts / saved projections given");
     if (grad_rec == nullptr && grad_rot == nullptr && grad_shifts == nullptr) return B200PROJ_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    if (int rc = zero_outputs(s, grad_rec, L.rec_count * sizeof(float2), grad_rot, (size_t)B_rot * P * DIM * DIM * sizeof(float),
+    const bool cubic = interpolation == B200PROJ_CUBIC;
+    BrickLaunch bl{};
+    if (RECORDS && P > 0 && grad_rec != nullptr && workspace != nullptr) bl = scatter_plan(B, P, N, cubic, false, os, cutoff);
+    if (workspace_bytes < bl.bytes) bl.use = false;
+    const int copies = P > 0 && grad_rec != nullptr && !bl.use ? scatter_copies(L, workspace, workspace_bytes) : 1;
+    if (int rc = zero_outputs(s, copies > 1 ? nullptr : grad_rec, L.rec_count * sizeof(float2), grad_rot, (size_t)B_rot * P * DIM * DIM * sizeof(float),
                               grad_shifts, (size_t)(shifts ? B_shift : 0) * P * 2 * sizeof(float))) return rc;
     if (P == 0) return B200PROJ_OK;
     const float2* gp = (const float2*)grad_proj;
     const float2* o = (const float2*)out;
     const float2* d = (const float2*)derivatives;
-    const bool cubic = interpolation == B200PROJ_CUBIC;
-    if constexpr (RECORDS) {
+    if (bl.use) {
         // large cubic scatter: brick by brick, the pose gradients in a streaming pass of their own
-        const BrickLaunch bl = grad_rec != nullptr && workspace != nullptr ? scatter_plan(B, P, N, cubic, false, os, cutoff) : BrickLaunch{};
-        if (bl.use && workspace_bytes >= bl.bytes) {
-            if (int rc = launch_brick_scatter<false, false>(L, bl, workspace, grad_proj, nullptr, rot, shifts, grad_rec, nullptr, s)) return rc;
-            if (grad_rot == nullptr && grad_shifts == nullptr) return B200PROJ_OK;
-            grad_rec = nullptr;
-        }
+        if (int rc = launch_brick_scatter<false, false>(L, bl, workspace, grad_proj, nullptr, rot, shifts, grad_rec, nullptr, s)) return rc;
+        if (grad_rot == nullptr && grad_shifts == nullptr) return B200PROJ_OK;
+        grad_rec = nullptr;
     }
     if (grad_rec != nullptr) {
-        if (cubic) launch_project_back_saved<DIM, true, RECORDS>(L, s, gp, o, d, rot, shifts, (float2*)grad_rec, grad_rot, grad_shifts);
-        else launch_project_back_saved<DIM, false, RECORDS>(L, s, gp, o, d, rot, shifts, (float2*)grad_rec, grad_rot, grad_shifts);
-    } else {
-        launch_pose_grad_saved<DIM, RECORDS>(L, s, gp, o, d, grad_rot, grad_shifts);
+        if (copies > 1)
+            if (int rc = zero_async(workspace, (size_t)copies * L.rec_count * sizeof(float2), s)) return rc;
+        float2* to = copies > 1 ? (float2*)workspace : (float2*)grad_rec;
+        if (cubic) launch_project_back_saved<DIM, true, RECORDS>(L, s, gp, o, d, rot, shifts, to, grad_rot, grad_shifts);
+        else launch_project_back_saved<DIM, false, RECORDS>(L, s, gp, o, d, rot, shifts, to, grad_rot, grad_shifts);
+        if (int rc = check_launch("project_back (saved derivatives) launch")) return rc;
+        return copies > 1 ? add_copies(L, workspace, copies, grad_rec, s) : B200PROJ_OK;
     }
+    launch_pose_grad_saved<DIM, RECORDS>(L, s, gp, o, d, grad_rot, grad_shifts);
     return check_launch("project_back (saved derivatives) launch");
 }
 
@@ -476,21 +499,25 @@ int project_back(const Real* grad_proj, const Real* rec, int64_t B, int64_t R, c
     if (grad_shifts != nullptr && shifts == nullptr)
         return fail(B200PROJ_ERR_ARGUMENT, "grad_shifts requested but no shifts given");
     cudaStream_t s = (cudaStream_t)stream;
-    if (int rc = zero_outputs(s, grad_rec, L.rec_count * sizeof(C2<Real>), grad_rot, (size_t)B_rot * P * DIM * DIM * sizeof(Real),
+    BrickLaunch bl{};
+    if (DIM == 3 && std::is_same<Real, float>::value && P > 0 && grad_rot == nullptr && grad_shifts == nullptr && workspace != nullptr)
+        bl = scatter_plan(B, P, N, interpolation == B200PROJ_CUBIC, false, os, cutoff);
+    if (workspace_bytes < bl.bytes) bl.use = false;
+    const int copies = P > 0 && std::is_same<Real, float>::value && !bl.use ? scatter_copies(L, workspace, workspace_bytes) : 1;
+    if (int rc = zero_outputs(s, copies > 1 ? nullptr : grad_rec, L.rec_count * sizeof(C2<Real>), grad_rot, (size_t)B_rot * P * DIM * DIM * sizeof(Real),
                               grad_shifts, (size_t)(shifts ? B_shift : 0) * P * 2 * sizeof(Real))) return rc;
     if (P == 0) return B200PROJ_OK;
-    if constexpr (DIM == 3 && std::is_same<Real, float>::value) {
-        if (grad_rot == nullptr && grad_shifts == nullptr && workspace != nullptr) {
-            const bool cubic = interpolation == B200PROJ_CUBIC;
-            const BrickLaunch bl = scatter_plan(B, P, N, cubic, false, os, cutoff);
-            if (bl.use && workspace_bytes >= bl.bytes) return launch_brick_scatter<false, false>(L, bl, workspace, grad_proj, nullptr, rot, shifts, grad_rec, nullptr, s);
-        }
-    }
+    if constexpr (DIM == 3 && std::is_same<Real, float>::value)
+        if (bl.use) return launch_brick_scatter<false, false>(L, bl, workspace, grad_proj, nullptr, rot, shifts, grad_rec, nullptr, s);
+    if (copies > 1)
+        if (int rc = zero_async(workspace, (size_t)copies * L.rec_count * sizeof(float2), s)) return rc;
+    C2<Real>* to = copies > 1 ? (C2<Real>*)workspace : (C2<Real>*)grad_rec;
     if (interpolation == B200PROJ_CUBIC)
-        launch_project_back<DIM, true>(L, s, (const C2<Real>*)grad_proj, (const C2<Real>*)rec, rot, shifts, (C2<Real>*)grad_rec, grad_rot, grad_shifts);
+        launch_project_back<DIM, true>(L, s, (const C2<Real>*)grad_proj, (const C2<Real>*)rec, rot, shifts, to, grad_rot, grad_shifts);
     else
-        launch_project_back<DIM, false>(L, s, (const C2<Real>*)grad_proj, (const C2<Real>*)rec, rot, shifts, (C2<Real>*)grad_rec, grad_rot, grad_shifts);
-    return check_launch("project_back launch");
+        launch_project_back<DIM, false>(L, s, (const C2<Real>*)grad_proj, (const C2<Real>*)rec, rot, shifts, to, grad_rot, grad_shifts);
+    if (int rc = check_launch("project_back launch")) return rc;
+    return copies > 1 ? add_copies(L, workspace, copies, (float*)grad_rec, s) : B200PROJ_OK;
 }
 
 template <int DIM, typename Real>
@@ -547,6 +574,17 @@ int backproject_forw(const Real* proj, const Real* weights, int64_t B, int64_t R
                                                                                               replicas, L.rec_count);
         return check_launch("fold_interleaved launch");
     }
+    }
+    if constexpr (kIsF32) {
+        // a small reconstruction without weights: copies of it in the workspace
+        const int copies = !hw && P > 0 ? scatter_copies(L, workspace, workspace_bytes) : 1;
+        if (copies > 1) {
+            if (int rc = zero_async(workspace, (size_t)copies * L.rec_count * sizeof(float2), s)) return rc;
+            if (cubic) backproject_forw_kernel<DIM, true, false><<<L.grid, kBlockThreads, 0, s>>>((const float2*)proj, weights, rot, shifts, (float2*)workspace, weight_rec, L.g);
+            else backproject_forw_kernel<DIM, false, false><<<L.grid, kBlockThreads, 0, s>>>((const float2*)proj, weights, rot, shifts, (float2*)workspace, weight_rec, L.g);
+            if (int rc = check_launch("backproject_forw (copies) launch")) return rc;
+            return add_copies(L, workspace, copies, data_rec, s, accumulate != 0);
+        }
     }
     if (!accumulate) {
         if (int rc = zero_outputs(s, data_rec, L.rec_count * sizeof(C2<Real>), weight_rec, L.rec_count * sizeof(Real))) return rc;
@@ -748,15 +786,16 @@ const char* b200proj_last_error(void) { return g_error; }
 
 size_t b200proj_backproject_workspace_bytes(int dim, int64_t B, int64_t R, int64_t P, int64_t N,
                                            int interpolation, int has_weights) {
-    if (!has_weights || (dim != 2 && dim != 3) || B < 1 || R < 2 || P < 1 || N < 2) return 0;
+    if ((dim != 2 && dim != 3) || B < 1 || R < 2 || P < 1 || N < 2) return 0;
     const double voxels = (double)B * (dim == 3 ? R : 1) * R * (R / 2 + 1);
     const int t = interpolation == B200PROJ_CUBIC ? 4 : 2;
     const double taps = (double)B * P * N * (N / 2 + 1) * (dim == 3 ? t * t * t : t * t);
     // worth it once the scatter outweighs the two extra passes over the volume
     if (taps < 4.0 * voxels) return 0;
-    if (dim == 3 && slab_plan(R, true).slabs > 1) return 0;      // beyond-L2 volumes take the slab-ordered path
-    const double one = voxels * (double)sizeof(float4);
-    return (size_t)one * (size_t)workspace_replicas(one, P);       // small reconstructions: several copies
+    if (dim == 3 && slab_plan(R, has_weights != 0).slabs > 1) return 0;      // beyond-L2 volumes take the slab-ordered path
+    const double one = voxels * (double)(has_weights ? sizeof(float4) : sizeof(float2));
+    const int copies = workspace_replicas(one, P);                 // small reconstructions: several copies
+    return has_weights || copies > 1 ? (size_t)one * (size_t)copies : 0;
 }
 
 int64_t b200proj_rec_boxsize(int64_t N, double oversampling) {
@@ -799,6 +838,15 @@ size_t b200proj_scatter_workspace_bytes(int64_t B, int64_t P, int64_t N, int int
     const BrickLaunch bl = scatter_plan(B, P, N, interpolation == B200PROJ_CUBIC, has_weights != 0, oversampling, cutoff);
     return bl.use ? bl.bytes : 0;
 }
+size_t b200proj_gradient_workspace_bytes(int dim, int64_t B, int64_t R, int64_t P, int64_t N, int interpolation, int pose_gradients,
+                                         double oversampling, double cutoff) {
+    if ((dim != 2 && dim != 3) || B < 1 || R < 2 || P < 1 || N < 2) return 0;
+    if (dim == 3 && !pose_gradients)
+        if (const size_t bytes = b200proj_scatter_workspace_bytes(B, P, N, interpolation, 0, oversampling, cutoff)) return bytes;
+    const double one = (double)B * (dim == 3 ? R : 1) * R * (R / 2 + 1) * (double)sizeof(float2);
+    const int copies = workspace_replicas(one, P);
+    return copies > 1 ? (size_t)one * (size_t)copies : 0;
+}
 size_t b200proj_project_workspace_bytes(int64_t B, int64_t P, int64_t N, int interpolation, int records, double oversampling, double cutoff) {
     const BrickLaunch bl = gather_plan(B, P, N, interpolation == B200PROJ_CUBIC, records != 0, oversampling, cutoff);
     return bl.use ? bl.bytes : 0;
@@ -840,6 +888,19 @@ int b200proj_project_3d_to_2d_back(const float* grad_proj, const float* rec, int
     return project_back<3>(grad_proj, rec, B, R, rot, B_rot, shifts, B_shift, P, N, interpolation, oversampling, cutoff, grad_rec, grad_rot, grad_shifts, pose_order, stream);
 }
 
+int b200proj_project_2d_back_ws(const float* grad_proj, const float* rec, int64_t B, int64_t R,
+                                const float* rot, int64_t B_rot, const float* shifts, int64_t B_shift, int64_t P, int64_t N,
+                                int interpolation, double oversampling, double cutoff, float* grad_rec,
+                                float* grad_rot, float* grad_shifts, void* workspace, size_t workspace_bytes, void* stream) {
+    return project_back<2>(grad_proj, rec, B, R, rot, B_rot, shifts, B_shift, P, N, interpolation, oversampling, cutoff, grad_rec, grad_rot, grad_shifts, nullptr, stream, workspace, workspace_bytes);
+}
+int b200proj_project_2d_back_saved_ws(const float* grad_proj, const float* out, const float* derivatives,
+                                      int64_t B, int64_t R, const float* rot, int64_t B_rot,
+                                      const float* shifts, int64_t B_shift, int64_t P, int64_t N,
+                                      int interpolation, double oversampling, double cutoff, float* grad_rec,
+                                      float* grad_rot, float* grad_shifts, void* workspace, size_t workspace_bytes, void* stream) {
+    return project_back_saved<2>(grad_proj, out, derivatives, B, R, rot, B_rot, shifts, B_shift, P, N, interpolation, oversampling, cutoff, grad_rec, grad_rot, grad_shifts, nullptr, stream, workspace, workspace_bytes);
+}
 int b200proj_project_3d_to_2d_back_ws(const float* grad_proj, const float* rec, int64_t B, int64_t R,
                                       const float* rot, int64_t B_rot, const float* shifts,
                                       int64_t B_shift, int64_t P, int64_t N, int interpolation,

@@ -165,6 +165,12 @@ Tensor scatter_workspace(int dim, const Tensor& like, int64_t B, int64_t P, int6
     const size_t bytes = b200proj_scatter_workspace_bytes(B, P, N, interp, weights ? 1 : 0, oversampling, cutoff);
     return bytes ? at::empty({(int64_t)bytes}, like.options().dtype(at::kByte)) : Tensor();
 }
+// The same for the backward passes of the projection.
+Tensor gradient_workspace(int dim, const Tensor& like, int64_t B, int64_t R, int64_t P, int64_t N, int interp, bool pose_gradients, double oversampling, double cutoff) {
+    if (is_f64(like)) return Tensor();
+    const size_t bytes = b200proj_gradient_workspace_bytes(dim, B, R, P, N, interp, pose_gradients ? 1 : 0, oversampling, cutoff);
+    return bytes ? at::empty({(int64_t)bytes}, like.options().dtype(at::kByte)) : Tensor();
+}
 inline void* ws_ptr(const Tensor& ws) { return ws.defined() ? ws.data_ptr() : nullptr; }
 inline size_t ws_size(const Tensor& ws) { return ws.defined() ? (size_t)ws.numel() : 0; }
 
@@ -233,14 +239,14 @@ std::tuple<Tensor, Tensor, Tensor> project_back(int dim, const Tensor& grad_proj
     } else {
         void* s = current_stream(rec);
         const double cut = cutoff_of(cutoff, N);
-        const Tensor ws = need_rot || need_shift ? Tensor() : scatter_workspace(dim, rec, B, p.P, N, interp, false, oversampling, cut);
+        const Tensor ws = gradient_workspace(dim, rec, B, R, p.P, N, interp, need_rot || need_shift, oversampling, cut);
         Tensor order = ws.defined() ? Tensor() : resolve_order(dim, rec, B, p, pose_order);
         int rc;
         if (is_f64(rec)) {
             rc = dim == 2 ? b200proj_project_2d_back_f64(cptr<double>(gp), cptr<double>(rec), B, R, cptr<double>(p.rot), p.B_rot, cptr<double>(p.shifts), p.B_shift, p.P, N, interp, oversampling, cut, mptr<double>(grad_rec), mptr<double>(grad_rot), mptr<double>(grad_sh), s)
                           : b200proj_project_3d_to_2d_back_f64(cptr<double>(gp), cptr<double>(rec), B, R, cptr<double>(p.rot), p.B_rot, cptr<double>(p.shifts), p.B_shift, p.P, N, interp, oversampling, cut, mptr<double>(grad_rec), mptr<double>(grad_rot), mptr<double>(grad_sh), cptr<int32_t>(order), s);
         } else {
-            rc = dim == 2 ? b200proj_project_2d_back(cptr<float>(gp), cptr<float>(rec), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts), p.B_shift, p.P, N, interp, oversampling, cut, mptr<float>(grad_rec), mptr<float>(grad_rot), mptr<float>(grad_sh), s)
+            rc = dim == 2 ? b200proj_project_2d_back_ws(cptr<float>(gp), cptr<float>(rec), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts), p.B_shift, p.P, N, interp, oversampling, cut, mptr<float>(grad_rec), mptr<float>(grad_rot), mptr<float>(grad_sh), ws_ptr(ws), ws_size(ws), s)
                           : b200proj_project_3d_to_2d_back_ws(cptr<float>(gp), cptr<float>(rec), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts), p.B_shift, p.P, N, interp, oversampling, cut, mptr<float>(grad_rec), mptr<float>(grad_rot), mptr<float>(grad_sh), cptr<int32_t>(order), ws_ptr(ws), ws_size(ws), s);
         }
         status(rc, dim == 2 ? "project_2d_back" : "project_3d_to_2d_back");
@@ -339,12 +345,12 @@ std::tuple<Tensor, Tensor, Tensor> project_back_saved(int dim, const Tensor& gra
         if (need_rec_grad) grad_rec.zero_();
     } else {
         const double cut = cutoff_of(cutoff, N);
-        const Tensor ws = need_rec_grad ? scatter_workspace(dim, gp, B, p.P, N, interp, false, oversampling, cut) : Tensor();
+        const Tensor ws = need_rec_grad ? gradient_workspace(dim, gp, B, R, p.P, N, interp, false, oversampling, cut) : Tensor();
         Tensor order = ws.defined() ? Tensor() : resolve_order(dim, reconstruction, B, p, pose_order);
         const int rc = dim == 2
-            ? b200proj_project_2d_back_saved(cptr<float>(gp), cptr<float>(out), cptr<float>(der), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts),
+            ? b200proj_project_2d_back_saved_ws(cptr<float>(gp), cptr<float>(out), cptr<float>(der), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts),
                                              p.B_shift, p.P, N, interp, oversampling, cut, mptr<float>(grad_rec), mptr<float>(grad_rot), mptr<float>(grad_sh),
-                                             current_stream(gp))
+                                                ws_ptr(ws), ws_size(ws), current_stream(gp))
             : b200proj_project_3d_to_2d_back_records(cptr<float>(gp), cptr<float>(out), cptr<float>(der), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts),
                                                    p.B_shift, p.P, N, interp, oversampling, cut, mptr<float>(grad_rec), mptr<float>(grad_rot), mptr<float>(grad_sh),
                                                    cptr<int32_t>(order), ws_ptr(ws), ws_size(ws), current_stream(gp));

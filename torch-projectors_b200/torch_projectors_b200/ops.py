@@ -130,11 +130,9 @@ def set_pose_order_thresholds(min_volume_bytes: int = 96 << 20, min_poses: int =
 # gathering the volume a second time -- and skips the scatter into the volume's gradient altogether
 # when the volume needs none.  Measured on B200, box 512, 4,096 poses of 256 x 256, cubic: forward
 # 6.5 -> 8.9 ms, backward 20.3 -> 15.1 ms (1.9 ms with a fixed volume).
-# When the reconstruction needs a gradient too, the backward pass still scatters, and onto a small
-# reconstruction that scatter is bound by contention, not by the gather beside it (one 128 x 65
-# reference, 65,536 poses, cubic: 9.8 ms either way, while the forward pass pays 1.4 ms for the
-# derivatives): below SAVE_DERIVATIVES_MIN_VOLUME_BYTES per batch item the plain pair stays -- in 3D only
-# up to SAVE_DERIVATIVES_MIN_PIXELS, beyond which the scatter runs brick by brick without that contention.
+# When the reconstruction needs a gradient too, the backward pass still scatters; small calls (below
+# SAVE_DERIVATIVES_MIN_VOLUME_BYTES per batch item and SAVE_DERIVATIVES_MIN_PIXELS pixels) keep the plain
+# pair then, whose gather costs less than the derivatives' way through memory.
 SAVE_DERIVATIVES = True
 SAVE_DERIVATIVES_MAX_BYTES = 16 << 30
 SAVE_DERIVATIVES_MIN_VOLUME_BYTES = 2 << 20
@@ -574,7 +572,7 @@ def _save_derivatives(dim, reconstruction, rotations, output_shape, interpolatio
     N = int(output_shape[0])
     if need_rec and not (interpolation == "cubic" and
                          (reconstruction[0].numel() * 8 >= SAVE_DERIVATIVES_MIN_VOLUME_BYTES or
-                          (dim == 3 and reconstruction.size(0) * rotations.size(1) * N * N >= SAVE_DERIVATIVES_MIN_PIXELS))):
+                          reconstruction.size(0) * rotations.size(1) * N * N >= SAVE_DERIVATIVES_MIN_PIXELS)):
         return _PLAIN
     fits = 8 * (2 if dim == 2 else 4) * reconstruction.size(0) * rotations.size(1) * N * (N // 2 + 1) <= SAVE_DERIVATIVES_MAX_BYTES
     return _KEEP_DERIVATIVES if fits else _PLAIN
