@@ -93,14 +93,14 @@ int b200proj_project_3d_to_2d_forw(const float* rec, int64_t B, int64_t R,
                                    double fourier_radius_cutoff, float* out,
                                    const int32_t* pose_order, void* stream);
 
-/* The 3D projections with scratch: large calls (many slices through each region of the volume) run
- * brick by brick -- a block keeps a piece of the volume in shared memory and handles the pixels of
+/* The projections with scratch: large calls (many slices through each region of the reconstruction) run
+ * brick by brick -- a block keeps a piece of the reconstruction in shared memory and handles the pixels of
  * all slices that fall into it -- which needs a workspace for the slices' records and the list of
  * work items.  b200proj_project_workspace_bytes gives its size, 0 when the call would not gain
  * (small calls; the workspace may then be NULL; records != 0: of _forw_records below).  With too small a workspace, or NULL, the plain
  * kernels run: the results are the same to rounding.  The workspace must be 16-byte aligned and
  * is free again when the call's work has run. */
-size_t b200proj_project_workspace_bytes(int64_t B, int64_t P, int64_t N, int interpolation, int records,
+size_t b200proj_project_workspace_bytes(int dim, int64_t B, int64_t P, int64_t N, int interpolation, int records,
                                         double oversampling, double fourier_radius_cutoff);
 /* The same for the scatters of the 3D operators (b200proj_project_3d_to_2d_back_records and _back_ws with
  * grad_rec, b200proj_backproject_2d_to_3d_accumulate_ws, b200proj_backproject_2d_to_3d_forw; 0: no gain, for
@@ -113,6 +113,18 @@ size_t b200proj_scatter_workspace_bytes(int64_t B, int64_t P, int64_t N, int int
  * half the rate).  pose_gradients != 0: of a _back_ws call that also computes grad_rot or grad_shifts. */
 size_t b200proj_gradient_workspace_bytes(int dim, int64_t B, int64_t R, int64_t P, int64_t N, int interpolation,
                                          int pose_gradients, double oversampling, double fourier_radius_cutoff);
+int b200proj_project_2d_forw_ws(const float* rec, int64_t B, int64_t R,
+                                const float* rot, int64_t B_rot,
+                                const float* shifts, int64_t B_shift,
+                                int64_t P, int64_t N, int interpolation, double oversampling,
+                                double fourier_radius_cutoff, float* out, void* workspace,
+                                size_t workspace_bytes, void* stream);
+int b200proj_project_2d_forw_saving_ws(const float* rec, int64_t B, int64_t R,
+                                       const float* rot, int64_t B_rot,
+                                       const float* shifts, int64_t B_shift,
+                                       int64_t P, int64_t N, int interpolation, double oversampling,
+                                       double fourier_radius_cutoff, float* out, float* derivatives,
+                                       void* workspace, size_t workspace_bytes, void* stream);
 int b200proj_project_3d_to_2d_forw_ws(const float* rec, int64_t B, int64_t R,
                                       const float* rot, int64_t B_rot,
                                       const float* shifts, int64_t B_shift,

@@ -23,10 +23,16 @@ SIZES = [(1, 40, 4, 8, 2.0, None, 1, 1),
          (1, 3, 48, 120, 2.5, 17.0, 1, 1)]
 
 
-def _inputs(size, seed):
+SIZES_2D = SIZES[:5] + [(1, 21, 70, 160, 2.0, 40.0, 1, 1), (2, 300, 130, 130, 1.0, None, 2, 2)]
+
+
+def _inputs(dim, size, seed):
     B, P, N, R, os_, cutoff, B_rot, B_shift = size
-    t = make_inputs(Case("bricks", 3, "cubic", B, P, N, R, os_, cutoff, B_rot, B_shift, shift_range=5.0, seed=seed))
+    t = make_inputs(Case("bricks", dim, "cubic", B, P, N, R, os_, cutoff, B_rot, B_shift, shift_range=5.0, seed=seed))
     lattice = axis_aligned_rotations(torch.Generator().manual_seed(seed))
+    if dim == 2:
+        t["rot"][0, 3] *= 1.2
+        lattice = t["rot"][0, :1].repeat(P + 1, 1, 1)
     if P >= len(lattice):
         t["rot"][0, : len(lattice)] = lattice
         t["rot"][0, len(lattice)] *= 1.2                    # not rotations: these slices take the plain path
@@ -37,46 +43,56 @@ def _inputs(size, seed):
 
 def check(names):
     """Run in a fresh process with the bricks forced on (the library reads the switch once)."""
+    for dim in (3, 2):
+        check_dim(names, dim)
+
+
+def check_dim(names, dim):
     sys.path[:0] = [str(ROOT), str(ROOT / "torch-projectors_b200"), str(ROOT / "tests")]
     import torch_projectors_b200 as tp
     from oracle import port
-    for seed, size in enumerate(SIZES):
+    project, reference, gradient = ((tp.project_3d_to_2d_forw, port.project_3d_to_2d_forw, port.project_3d_to_2d_back) if dim == 3 else
+                                    (tp.project_2d_forw, port.project_2d_forw, port.project_2d_back))
+    backproject, back_reference = ((tp.backproject_2d_to_3d_forw, port.backproject_2d_to_3d_forw) if dim == 3 else
+                                   (tp.backproject_2d_forw, port.backproject_2d_forw))
+    for seed, size in enumerate(SIZES if dim == 3 else SIZES_2D):
         for interp in ("linear", "cubic"):
-            t, kw = _inputs(size, seed)
+            t, kw = _inputs(dim, size, seed)
             N, os_, cutoff = size[2], size[4], size[5]
-            want = port.project_3d_to_2d_forw(t["rec"], t["rot"], t["shifts"], [N, N], interp, os_, cutoff)
+            want = reference(t["rec"], t["rot"], t["shifts"], [N, N], interp, os_, cutoff)
             shifts = t["shifts"].cuda() if t["shifts"] is not None else None
             if "forward" in names:
-                got = tp.project_3d_to_2d_forw(t["rec"].cuda(), t["rot"].cuda(), shifts, interpolation=interp, **kw)
+                got = project(t["rec"].cuda(), t["rot"].cuda(), shifts, interpolation=interp, **kw)
                 assert rel_err(got, want) <= TOL_FORWARD, (size, interp, rel_err(got, want))
             if "gradients" in names:
                 tp.set_save_derivatives(True, min_volume_bytes=0)
                 for fixed in (False, True):
                     rec, rot = t["rec"].cuda().requires_grad_(not fixed), t["rot"].cuda().requires_grad_(True)
                     sh = shifts.clone().requires_grad_(True) if shifts is not None else None
-                    out = tp.project_3d_to_2d_forw(rec, rot, sh, interpolation=interp, **kw)
+                    out = project(rec, rot, sh, interpolation=interp, **kw)
                     assert rel_err(out, want) <= TOL_FORWARD, (size, interp)
                     out.backward(t["proj"].cuda())
-                    grads = port.project_3d_to_2d_back(t["proj"], t["rec"], t["rot"], t["shifts"], interp, os_, cutoff,
+                    grads = gradient(t["proj"], t["rec"], t["rot"], t["shifts"], interp, os_, cutoff,
                                                        need_rot_grad=True, need_shift_grad=shifts is not None)
                     for have, ref, what in ((rec.grad, grads[0], "volume"), (rot.grad, grads[1], "rotations"), (sh.grad if sh is not None else None, grads[2], "shifts")):
                         if have is not None:
                             assert rel_err(have, ref) <= TOL_ATOMIC, (size, interp, what, rel_err(have, ref))
                 rec = t["rec"].cuda().requires_grad_(True)                 # the volume's gradient alone
-                tp.project_3d_to_2d_forw(rec, t["rot"].cuda(), shifts, interpolation=interp, **kw).backward(t["proj"].cuda())
+                project(rec, t["rot"].cuda(), shifts, interpolation=interp, **kw).backward(t["proj"].cuda())
                 assert rel_err(rec.grad, grads[0]) <= TOL_ATOMIC, (size, interp, "volume alone")
             if "backprojection" in names:
                 for weights in (None, t["weights"]):
-                    data, wrec = tp.backproject_2d_to_3d_forw(t["proj"].cuda(), t["rot"].cuda(), weights.cuda() if weights is not None else None, shifts,
+                    data, wrec = backproject(t["proj"].cuda(), t["rot"].cuda(), weights.cuda() if weights is not None else None, shifts,
                                                               interpolation=interp, oversampling=os_, fourier_radius_cutoff=cutoff)
-                    ref, wref = port.backproject_2d_to_3d_forw(t["proj"], weights, t["rot"], t["shifts"], interp, os_, cutoff)
+                    ref, wref = back_reference(t["proj"], weights, t["rot"], t["shifts"], interp, os_, cutoff)
                     assert rel_err(data, ref) <= TOL_ATOMIC, (size, interp, "data", rel_err(data, ref))
-                    if weights is not None:
+                    if weights is not None and dim == 3:
                         acc = tp.new_backprojection_accumulator(size[0], data.shape[-2], "cuda")
                         tp.backproject_2d_to_3d_accumulate_interleaved_(acc, t["proj"].cuda(), t["rot"].cuda(), weights.cuda(), shifts,
                                                                         interpolation=interp, oversampling=os_, fourier_radius_cutoff=cutoff)
                         d2, w2 = tp.fold_backprojection_accumulator(acc)
                         assert rel_err(d2, ref) <= TOL_ATOMIC and rel_err(w2, wref) <= TOL_ATOMIC, (size, interp, "accumulator")
+                    if weights is not None:
                         assert rel_err(wrec, wref) <= TOL_ATOMIC, (size, interp, "weights", rel_err(wrec, wref))
 
 

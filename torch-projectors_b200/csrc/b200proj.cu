@@ -241,12 +241,12 @@ BrickLaunch brick_layout(int64_t B, int64_t P, int64_t N, double os, double cuto
     L.bricks = 1;
     for (int a = 0; a < 3; ++a) {
         L.plan.d[a] = dims[a];
-        L.plan.n[a] = (span + dims[a] - 1) / dims[a];
+        L.plan.n[a] = dims[a] ? (span + dims[a] - 1) / dims[a] : 1;
         L.plan.lo[a] = -((L.plan.n[a] * dims[a]) / 2);
         L.bricks *= L.plan.n[a];
     }
     if (L.bricks * B > (1 << 26) || B * P > (1 << 26)) return L;
-    L.plan.density = (float)((double)D::x * D::y * D::z / (4.0 * os * os));
+    L.plan.density = (float)(D::kDim == 3 ? (double)D::x * D::y * D::z / (4.0 * os * os) : (double)D::x * D::y / (2.0 * os * os));
     double target = pixels / (blocks * 8.0);
     if (target < min_target) target = min_target;
     L.plan.target = (float)target;
@@ -258,7 +258,7 @@ BrickLaunch brick_layout(int64_t B, int64_t P, int64_t N, double os, double cuto
     L.rec_bytes = (size_t)(B * P) * 3 * sizeof(float4);
     L.bytes = 256 + L.item_bytes + L.rec_bytes + (outside ? (size_t)(N * (N / 2 + 1)) * sizeof(int) : 0);
     L.pixels = pixels;
-    L.in_ball = 4.19 * pow(reach + 12.0, 3) / ((double)D::x * D::y * D::z) * (double)B;
+    L.in_ball = (D::kDim == 3 ? 4.19 * pow(reach + 12.0, 3) / ((double)D::x * D::y * D::z) : M_PI * pow(reach + 30.0, 2) / ((double)D::x * D::y)) * (double)B;
     L.forced = force == 1;
     L.use = true;
     return L;
@@ -267,8 +267,15 @@ BrickLaunch brick_layout(int64_t B, int64_t P, int64_t N, double os, double cuto
 // Forward projection: bricks pay once their pixels outweigh staging them, whatever their number, and a fixed cost
 // (measured: 20 us and 26 ns per brick against 33 ps saved per cubic pixel at oversampling 2; dense samples are cheaper
 // for the plain kernels, linear taps save only some 2 ps).
-BrickLaunch gather_plan(int64_t B, int64_t P, int64_t N, bool cubic, bool records, double os, double cutoff) {
-    BrickLaunch L = brick_layout<GatherBrick>(B, P, N, os, cutoff, 148.0 * 3.0, 3000.0, true);
+BrickLaunch gather_plan(int dim, int64_t B, int64_t P, int64_t N, bool cubic, bool records, double os, double cutoff) {
+    if (dim == 2) {
+        // cubic: measured crossings at 2-5 M pixels (27 M: 2.1-2.3x); linear taps are not faster at any size (0.6-1.05x)
+        if (!cubic) return BrickLaunch{};
+        BrickLaunch L = brick_layout<GatherBrick<2>>(B, P, N, os, cutoff, 148.0 * 3.0, 6000.0, true);
+        L.use = L.use && (L.forced || L.pixels > 4.5e6);
+        return L;
+    }
+    BrickLaunch L = brick_layout<GatherBrick<3>>(B, P, N, os, cutoff, 148.0 * 3.0, 3000.0, true);
     const double need = cubic ? (1.2e6 + 900.0 * L.in_ball) * (os < 2.0 ? 2.0 / os : 1.0)
                               : (10e6 + 4000.0 * L.in_ball) * (records ? 0.6 : 1.0);
     // linear taps: small volumes meet a slice in too few pixels per brick (box 38 oversampled twice: 1.8x slower)
@@ -295,23 +302,24 @@ BrickWork brick_work(const BrickLaunch& L, void* workspace) {
     return w;
 }
 
+template <int DIM>
 int brick_setup(const BrickLaunch& bl, const BrickWork& w, const Launch& L, const float* rot, const float* shifts, bool outside, cudaStream_t s) {
     if (int rc = zero_async(w.header, 16, s)) return rc;
     const int64_t clusters = (int64_t)((bl.plan.n[0] + 7) / 8) * ((bl.plan.n[1] + 7) / 8) * ((bl.plan.n[2] + 3) / 4) * L.B;
     const int64_t slices = (L.B * L.P + 255) / 256;
-    brick_setup_kernel<<<(unsigned)(clusters > slices ? clusters : slices) + 1u, 256, 0, s>>>(rot, shifts, w, L.g, bl.plan, (int)L.B, outside ? 1 : 0);
+    brick_setup_kernel<DIM><<<(unsigned)(clusters > slices ? clusters : slices) + 1u, 256, 0, s>>>(rot, shifts, w, L.g, bl.plan, (int)L.B, outside ? 1 : 0);
     return check_launch("brick_setup launch");
 }
 
-template <bool CUBIC, bool SAVE>
+template <int DIM, bool CUBIC, bool SAVE>
 int launch_brick_forw(const Launch& L, const BrickLaunch& bl, void* workspace, const float* rec, const float* rot, const float* shifts,
                       float* out, float* derivs, cudaStream_t s) {
     const BrickWork w = brick_work(bl, workspace);
-    if (int rc = brick_setup(bl, w, L, rot, shifts, true, s)) return rc;
-    constexpr size_t smem = sizeof(float2) * BrickShape<CUBIC>::kVoxels + sizeof(GatherBlock);
-    const cudaError_t e = cudaFuncSetAttribute(brick_forw_kernel<CUBIC, SAVE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (int rc = brick_setup<DIM>(bl, w, L, rot, shifts, true, s)) return rc;
+    constexpr size_t smem = sizeof(float2) * BrickShape<DIM, CUBIC>::kVoxels + sizeof(GatherBlock);
+    const cudaError_t e = cudaFuncSetAttribute(brick_forw_kernel<DIM, CUBIC, SAVE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cuda_fail(e, "brick_forw shared memory");
-    brick_forw_kernel<CUBIC, SAVE><<<148 * 3, kBlockThreads, smem, s>>>((const float2*)rec, rot, shifts, (float2*)out, (float2*)derivs, w, L.g, bl.plan);
+    brick_forw_kernel<DIM, CUBIC, SAVE><<<148 * 3, kBlockThreads, smem, s>>>((const float2*)rec, rot, shifts, (float2*)out, (float2*)derivs, w, L.g, bl.plan);
     return check_launch("brick_forw launch");
 }
 
@@ -320,7 +328,7 @@ int launch_brick_scatter(const Launch& L, const BrickLaunch& bl, void* workspace
                          const float* shifts, float* vol, float* wvol, cudaStream_t s, float4* accum = nullptr) {
     using C = Scatter<WEIGHTS>;
     const BrickWork w = brick_work(bl, workspace);
-    if (int rc = brick_setup(bl, w, L, rot, shifts, false, s)) return rc;
+    if (int rc = brick_setup<3>(bl, w, L, rot, shifts, false, s)) return rc;
     constexpr size_t smem = sizeof(typename C::Shared);
     static_assert((smem + 1024) * C::kBlocks <= 233472, "shared memory of an SM");
     const cudaError_t e = cudaFuncSetAttribute(brick_scatter_kernel<WEIGHTS, DUP, INTERLEAVED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -358,11 +366,12 @@ int project_forw(const Real* rec, int64_t B, int64_t R, const Real* rot, int64_t
     L.g.order = pose_order;
     if (P == 0) return B200PROJ_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    if constexpr (DIM == 3 && std::is_same<Real, float>::value) {
-        const BrickLaunch bl = workspace != nullptr ? gather_plan(B, P, N, interpolation == B200PROJ_CUBIC, false, os, cutoff) : BrickLaunch{};
-        if (bl.use && workspace_bytes >= bl.bytes)
-            return interpolation == B200PROJ_CUBIC ? launch_brick_forw<true, false>(L, bl, workspace, rec, rot, shifts, out, nullptr, s)
-                                                   : launch_brick_forw<false, false>(L, bl, workspace, rec, rot, shifts, out, nullptr, s);
+    if constexpr (std::is_same<Real, float>::value) {
+        const BrickLaunch bl = workspace != nullptr ? gather_plan(DIM, B, P, N, interpolation == B200PROJ_CUBIC, false, os, cutoff) : BrickLaunch{};
+        if (bl.use && workspace_bytes >= bl.bytes) {
+            if (interpolation == B200PROJ_CUBIC) return launch_brick_forw<DIM, true, false>(L, bl, workspace, rec, rot, shifts, out, nullptr, s);
+            if constexpr (DIM == 3) return launch_brick_forw<3, false, false>(L, bl, workspace, rec, rot, shifts, out, nullptr, s);
+        }
     }
     const C2<Real>* v = (const C2<Real>*)rec;
     C2<Real>* o = (C2<Real>*)out;
@@ -428,12 +437,13 @@ int project_forw_saving(const float* rec, int64_t B, int64_t R, const float* rot
     L.g.order = pose_order;
     if (P == 0) return B200PROJ_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    if constexpr (RECORDS) {
-        if ((reinterpret_cast<uintptr_t>(derivatives) & 31u) != 0) return fail(B200PROJ_ERR_ARGUMENT, "records must be 32-byte aligned");
-        const BrickLaunch bl = workspace != nullptr ? gather_plan(B, P, N, interpolation == B200PROJ_CUBIC, true, os, cutoff) : BrickLaunch{};
-        if (bl.use && workspace_bytes >= bl.bytes)
-            return interpolation == B200PROJ_CUBIC ? launch_brick_forw<true, true>(L, bl, workspace, rec, rot, shifts, out, derivatives, s)
-                                                   : launch_brick_forw<false, true>(L, bl, workspace, rec, rot, shifts, out, derivatives, s);
+    if (RECORDS && (reinterpret_cast<uintptr_t>(derivatives) & 31u) != 0) return fail(B200PROJ_ERR_ARGUMENT, "records must be 32-byte aligned");
+    if constexpr (RECORDS || DIM == 2) {
+        const BrickLaunch bl = workspace != nullptr ? gather_plan(DIM, B, P, N, interpolation == B200PROJ_CUBIC, true, os, cutoff) : BrickLaunch{};
+        if (bl.use && workspace_bytes >= bl.bytes) {
+            if (interpolation == B200PROJ_CUBIC) return launch_brick_forw<DIM, true, true>(L, bl, workspace, rec, rot, shifts, out, derivatives, s);
+            if constexpr (DIM == 3) return launch_brick_forw<3, false, true>(L, bl, workspace, rec, rot, shifts, out, derivatives, s);
+        }
     }
     if (interpolation == B200PROJ_CUBIC)
         project_forw_saving_kernel<DIM, true, RECORDS><<<L.grid, kBlockThreads, 0, s>>>((const float2*)rec, rot, shifts, (float2*)out, (float2*)derivatives, L.g);
@@ -847,9 +857,22 @@ size_t b200proj_gradient_workspace_bytes(int dim, int64_t B, int64_t R, int64_t 
     const int copies = workspace_replicas(one, P);
     return copies > 1 ? (size_t)one * (size_t)copies : 0;
 }
-size_t b200proj_project_workspace_bytes(int64_t B, int64_t P, int64_t N, int interpolation, int records, double oversampling, double cutoff) {
-    const BrickLaunch bl = gather_plan(B, P, N, interpolation == B200PROJ_CUBIC, records != 0, oversampling, cutoff);
+size_t b200proj_project_workspace_bytes(int dim, int64_t B, int64_t P, int64_t N, int interpolation, int records, double oversampling, double cutoff) {
+    if (dim != 2 && dim != 3) return 0;
+    const BrickLaunch bl = gather_plan(dim, B, P, N, interpolation == B200PROJ_CUBIC, records != 0, oversampling, cutoff);
     return bl.use ? bl.bytes : 0;
+}
+int b200proj_project_2d_forw_ws(const float* rec, int64_t B, int64_t R, const float* rot,
+                                int64_t B_rot, const float* shifts, int64_t B_shift, int64_t P,
+                                int64_t N, int interpolation, double oversampling, double cutoff,
+                                float* out, void* workspace, size_t workspace_bytes, void* stream) {
+    return project_forw<2>(rec, B, R, rot, B_rot, shifts, B_shift, P, N, interpolation, oversampling, cutoff, out, nullptr, stream, workspace, workspace_bytes);
+}
+int b200proj_project_2d_forw_saving_ws(const float* rec, int64_t B, int64_t R, const float* rot,
+                                       int64_t B_rot, const float* shifts, int64_t B_shift, int64_t P,
+                                       int64_t N, int interpolation, double oversampling, double cutoff,
+                                       float* out, float* derivatives, void* workspace, size_t workspace_bytes, void* stream) {
+    return project_forw_saving<2>(rec, B, R, rot, B_rot, shifts, B_shift, P, N, interpolation, oversampling, cutoff, out, derivatives, nullptr, stream, workspace, workspace_bytes);
 }
 int b200proj_project_3d_to_2d_forw_ws(const float* rec, int64_t B, int64_t R, const float* rot,
                                       int64_t B_rot, const float* shifts, int64_t B_shift, int64_t P,

@@ -1,4 +1,4 @@
-// Brick-stationary kernels of the 3D operators (fp32): the volume is cut into bricks that fit shared
+// Brick-stationary kernels (fp32; 3D, and 2D with cubic taps): the volume is cut into bricks that fit shared
 // memory, a block keeps one brick and walks over the slices, handling the pixels whose sample position
 // lies in its brick.  The plain kernels (fourier_slice_kernels.cuh) keep the pixels and fetch the taps
 // of every pixel through L1: 16 rows of a cubic footprint are 13 cache lines per pixel, and the L1TEX
@@ -22,12 +22,19 @@
 
 namespace b200proj {
 
-// Sample positions of a brick (units of voxels).
+// Sample positions of a brick (units of voxels); Z = 0: a tile of a 2D reconstruction.
 template <int X, int Y, int Z>
 struct BrickDims {
-    static constexpr int x = X, y = Y, z = Z;
+    static constexpr int x = X, y = Y, z = Z, kDim = Z > 0 ? 3 : 2;
 };
-using GatherBrick = BrickDims<17, 17, 16>;
+// 2D tiles of 61 x 61 (64 x 64 with the halo, 32 KB): all slices of a half-plane meet a tile, in rows of some 30 pixels,
+// so that the walk costs less than in 3D (500 slices of 128 x 65 from each of eight references, cubic: 0.755 -> 0.350 ms).
+template <int DIM>
+struct GatherBrickOf { using type = BrickDims<17, 17, 16>; };
+template <>
+struct GatherBrickOf<2> { using type = BrickDims<61, 61, 0>; };
+template <int DIM>
+using GatherBrick = typename GatherBrickOf<DIM>::type;
 constexpr int kBrickSlots = 8;                              // slices a warp takes at a time
 constexpr float kBrickSlack = 0.06f;                        // slack of the linear estimates, in voxels
 
@@ -37,7 +44,7 @@ struct BrickPlan {
     int d[3];               // sample positions of a brick along them
     int lo[3];              // first sample position of the grid
     float ball;             // sample positions of a rotated slice lie inside this radius
-    float density;          // expected pixels per brick and slice at radius r: density / max(r, ...)
+    float density;          // expected pixels per brick and slice: density / max(r, ...) at radius r (2D: density)
     float per_slice;        // pixels of a slice inside the cutoff
     float target;           // pixels a work item should hold
     int max_extra;          // items beyond one per brick that fit the list
@@ -60,7 +67,12 @@ struct SliceRec {           // 48 bytes
 
 // A slice goes through the bricks when the two columns of its matrix that matter are orthonormal to 2e-5
 // (then its pixels stay inside the ball, and plane and half-plane tests with slack hold).
+template <int DIM>
 __device__ __forceinline__ bool brick_slice_ok(const float* __restrict__ rm) {
+    if (DIM == 2) {
+        const float a0 = __ldg(rm + 0), b0 = __ldg(rm + 1), a1 = __ldg(rm + 2), b1 = __ldg(rm + 3);
+        return fabsf(a0 * a0 + a1 * a1 - 1.f) < 2e-5f && fabsf(b0 * b0 + b1 * b1 - 1.f) < 2e-5f && fabsf(a0 * b0 + a1 * b1) < 2e-5f;
+    }
     const float a0 = __ldg(rm + 0), a1 = __ldg(rm + 3), a2 = __ldg(rm + 6);
     const float b0 = __ldg(rm + 1), b1 = __ldg(rm + 4), b2 = __ldg(rm + 7);
     const float aa = a0 * a0 + a1 * a1 + a2 * a2, bb = b0 * b0 + b1 * b1 + b2 * b2, ab = a0 * b0 + a1 * b1 + a2 * b2;
@@ -110,14 +122,16 @@ __device__ __forceinline__ void brick_list_outside(const SliceGeom& g, BrickWork
 // brick plus max_extra, of which a brick takes what is left.
 // Neighbouring bricks are neighbours in the list, so that they run at the same time: the runs of pixels that
 // they write into a row of a slice then meet in L2 before the row's sectors leave it.
+template <int DIM>
 __global__ void __launch_bounds__(256)
 brick_setup_kernel(const float* __restrict__ rot, const float* __restrict__ shifts, BrickWork ws, const SliceGeom g,
                    const BrickPlan pl, int B, int list_outside) {
     const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
     if (t < g.BP) {
         const int b = t / g.P, p = t - b * g.P;
-        const float* rm = pose_rot<3>(g, rot, b, p);
-        const float m00 = __ldg(rm + 0), m01 = __ldg(rm + 1), m10 = __ldg(rm + 3), m11 = __ldg(rm + 4), m20 = __ldg(rm + 6), m21 = __ldg(rm + 7);
+        const float* rm = pose_rot<DIM>(g, rot, b, p);
+        const float m00 = __ldg(rm + 0), m01 = __ldg(rm + 1), m10 = __ldg(rm + DIM), m11 = __ldg(rm + DIM + 1);
+        const float m20 = DIM == 3 ? __ldg(rm + 6) : 0.f, m21 = DIM == 3 ? __ldg(rm + 7) : 0.f;
         float s0 = 0.f, s1 = 0.f;
         if (g.has_shift) {
             const float* s = pose_shift(g, shifts, b, p);
@@ -125,8 +139,8 @@ brick_setup_kernel(const float* __restrict__ rot, const float* __restrict__ shif
             s1 = __ldg(s + 1);
         }
         float nx = m10 * m21 - m20 * m11;
-        const float ny = m20 * m01 - m00 * m21, nz = m00 * m11 - m10 * m01;
-        if (!brick_slice_ok(rm)) nx = __int_as_float(0x7fffffff);
+        const float ny = m20 * m01 - m00 * m21, nz = DIM == 3 ? m00 * m11 - m10 * m01 : 0.f;       // 2D: every tile is in the plane
+        if (!brick_slice_ok<DIM>(rm)) nx = __int_as_float(0x7fffffff);
         ws.recs[3 * t + 0] = make_float4(nx, ny, nz, m00);
         ws.recs[3 * t + 1] = make_float4(m10, m20, m01, m11);
         ws.recs[3 * t + 2] = make_float4(m21, s0, s1, 0.f);
@@ -145,7 +159,7 @@ brick_setup_kernel(const float* __restrict__ rot, const float* __restrict__ shif
     int parts = 0;
     float r;
     if (bx < pl.n[0] && by < pl.n[1] && bz < pl.n[2] && brick_in_ball(pl, bx, by, bz, r)) {
-        const float expected = fminf(pl.density / fmaxf(r, 0.42f * (float)pl.d[0]), pl.per_slice) * (float)g.P;
+        const float expected = fminf(DIM == 3 ? pl.density / fmaxf(r, 0.42f * (float)pl.d[0]) : pl.density, pl.per_slice) * (float)g.P;
         parts = max(1, min((int)(expected / pl.target + 0.5f), (g.P + 31) / 32));
         if (parts > 1) parts = 1 + max(0, min(parts - 1, pl.max_extra - atomicAdd(ws.header + 1, parts - 1)));
     }
@@ -184,10 +198,11 @@ brick_setup_kernel(const float* __restrict__ rot, const float* __restrict__ shif
 // the columns and rows of its footprint in an order that starts at class (l & 3, (l >> 2) & 3), so that at
 // every step the 16 lanes of a half-warp hold 16 different classes = 16 different 8-byte banks, wherever
 // their pixels lie.
-template <bool CUBIC, typename D = GatherBrick>
+template <int DIM, bool CUBIC>
 struct BrickShape {
+    using D = GatherBrick<DIM>;
     static constexpr int T = CUBIC ? 4 : 2;
-    static constexpr int TX = ((D::x + T - 1) + 3) / 4 * 4, TY = ((D::y + T - 1) + 3) / 4 * 4, TZ = D::z + T - 1;
+    static constexpr int TX = ((D::x + T - 1) + 3) / 4 * 4, TY = ((D::y + T - 1) + 3) / 4 * 4, TZ = DIM == 3 ? D::z + T - 1 : 1;
     static constexpr int kRowCells = TX / 4 * 16;            // voxels of four rows
     static constexpr int kPlane = TX * TY;
     static constexpr int kVoxels = kPlane * TZ;
@@ -198,9 +213,9 @@ __device__ __forceinline__ int brick_off_y(int y) { return 4 * (y & 3) + S::kRow
 
 // Stage the brick: voxel (x, y, z) of it is tap (X0 - o + x, Y0 - o + y, Z0 - o + z), o = 1 for cubic, read with
 // the gather's rules (Friedel mirror with conjugation, clamping), so that edges need no further care.
-template <bool CUBIC>
+template <int DIM, bool CUBIC>
 __device__ __forceinline__ void brick_stage(const SliceGeom& g, const float2* __restrict__ vol, float2* sm, int X0, int Y0, int Z0) {
-    using S = BrickShape<CUBIC>;
+    using S = BrickShape<DIM, CUBIC>;
     constexpr int o = CUBIC ? 1 : 0, kRows = kBlockThreads / S::TX;      // rows staged at a time
     const int x = (int)threadIdx.x % S::TX, first = (int)threadIdx.x / S::TX;
     if (first >= kRows) return;
@@ -210,7 +225,7 @@ __device__ __forceinline__ void brick_stage(const SliceGeom& g, const float2* __
     int y = first, z = 0;
 #pragma unroll 4
     for (int n = first; n < S::TY * S::TZ; n += kRows) {
-        const int row = gather_line<CUBIC>(g, Y0 - o + y, m), pln = gather_line<CUBIC>(g, Z0 - o + z, m);
+        const int row = gather_line<CUBIC>(g, Y0 - o + y, m), pln = DIM == 3 ? gather_line<CUBIC>(g, Z0 - o + z, m) : 0;
         float2 v = __ldg(vol + ((pln * g.R + row) * g.Rh + col));
         if (m) v.y = -v.y;
         sm[z * S::kPlane + brick_off_y<S>(y) + ox] = v;
@@ -232,13 +247,13 @@ __device__ __forceinline__ unsigned long long fmul2(unsigned long long a, unsign
 }
 
 // Value (and derivatives) at (lx + fx, ly + fy, lz + fz) of the staged brick, all of it in this lane.
-template <bool CUBIC, bool WITH_DERIV>
+template <int DIM, bool CUBIC, bool WITH_DERIV>
 __device__ __forceinline__ void brick_gather(const float2* sm, int lx, int ly, int lz, float fx, float fy, float fz,
                                              float2& val, float2& gc, float2& gr, float2& gd) {
-    using S = BrickShape<CUBIC>;
+    using S = BrickShape<DIM, CUBIC>;
     using u64 = unsigned long long;
     const int lane = threadIdx.x & 31;
-    constexpr int T = S::T;
+    constexpr int T = S::T, TD = DIM == 3 ? T : 1;
     int ox[T], oy[T];                // byte offsets of the columns and rows, in this lane's order
     u64 wx[T], wy[T], wz[T], dx[T], dy[T], dz[T];
     const int base = (lz * S::kPlane + (ly >> 2) * S::kRowCells + (lx >> 2) * 16) * 8;
@@ -297,22 +312,22 @@ __device__ __forceinline__ void brick_gather(const float2* sm, int lx, int ly, i
             const char* col = smb + (ox[a] + oy[b]);
             u64 s = 0ull, sd = 0ull;
 #pragma unroll
-            for (int k = 0; k < T; ++k) {
+            for (int k = 0; k < TD; ++k) {
                 const u64 v = *reinterpret_cast<const u64*>(col + k * S::kPlane * 8);
-                s = fma2(wz[k], v, s);
-                if (WITH_DERIV) sd = fma2(dz[k], v, sd);
+                s = DIM == 3 ? fma2(wz[k], v, s) : v;
+                if (WITH_DERIV && DIM == 3) sd = fma2(dz[k], v, sd);
             }
             A = fma2(wy[b], s, A);
             if (WITH_DERIV) {
                 Bq = fma2(dy[b], s, Bq);
-                Dq = fma2(wy[b], sd, Dq);
+                if (DIM == 3) Dq = fma2(wy[b], sd, Dq);
             }
         }
         v2 = fma2(wx[a], A, v2);
         if (WITH_DERIV) {
             c2 = fma2(dx[a], A, c2);
             r2 = fma2(wx[a], Bq, r2);
-            d2 = fma2(wx[a], Dq, d2);
+            if (DIM == 3) d2 = fma2(wx[a], Dq, d2);
         }
     }
     unpack2(v2, val.x, val.y);
@@ -360,7 +375,7 @@ __device__ __forceinline__ void brick_walk(const SliceGeom& g, const float4* __r
     const float hx = 0.5f * D::x, hy = 0.5f * D::y, hz = 0.5f * D::z;
     const float cx = (float)X0 + hx, cy = (float)Y0 + hy, cz = (float)Z0 + hz;
     const float osf = (float)g.os, inv_os = 1.f / osf;
-    const int grab = max(1, min(kBrickSlots, (int)(2.f * osf)));       // slices with about 32 rows in the brick
+    const int grab = D::kDim == 3 ? max(1, min(kBrickSlots, (int)(2.f * osf))) : 1;       // slices with about 32 rows in the brick
     for (int k_next = first + part; k_next < last;) {
         if (!kAlone) {
             __syncthreads();
@@ -455,7 +470,7 @@ __device__ __forceinline__ void brick_walk(const SliceGeom& g, const float4* __r
                     };
                     clip(ra.w, rb.z, (float)X0, (float)D::x);
                     clip(rb.x, rb.w, (float)Y0, (float)D::y);
-                    clip(rb.y, m21, (float)Z0, (float)D::z);
+                    if (D::kDim == 3) clip(rb.y, m21, (float)Z0, (float)D::z);
                     ja_i = (int)ceilf(ja);
                     len = jb >= ja ? (int)floorf(jb) - ja_i + 1 : 0;
                 }
@@ -500,11 +515,11 @@ __device__ __forceinline__ void brick_walk(const SliceGeom& g, const float4* __r
                 }
                 px.c = add_rn(mul_rn(ra.w, px.sc), mul_rn(rb.z, px.sr));
                 px.r = add_rn(mul_rn(rb.x, px.sc), mul_rn(rb.w, px.sr));
-                px.d = add_rn(mul_rn(rb.y, px.sc), mul_rn(m21, px.sr));
-                int lx = (int)floorf(px.c) - X0, ly = (int)floorf(px.r) - Y0, lz = (int)floorf(px.d) - Z0;
+                px.d = D::kDim == 3 ? add_rn(mul_rn(rb.y, px.sc), mul_rn(m21, px.sr)) : 0.f;
+                int lx = (int)floorf(px.c) - X0, ly = (int)floorf(px.r) - Y0, lz = D::kDim == 3 ? (int)floorf(px.d) - Z0 : 0;
                 const float rad = add_rn(mul_rn(px.kr, px.kr), mul_rn(px.kc, px.kc));
                 const bool active = k0 + lane < total && (unsigned)lx < (unsigned)D::x && (unsigned)ly < (unsigned)D::y &&
-                                    (unsigned)lz < (unsigned)D::z && !(rad > g.cutoff_sq);
+                                    (D::kDim == 2 || (unsigned)lz < (unsigned)D::z) && !(rad > g.cutoff_sq);
                 if (!active) lx = ly = lz = 0;
                 body(active, slot, kr < 0 ? kr + g.N : kr, j, px, lx, ly, lz);
             }
@@ -518,15 +533,26 @@ __device__ __forceinline__ void brick_walk(const SliceGeom& g, const float4* __r
     }
 }
 
+// A pixel's saved derivatives: a record in 3D, two planes in 2D.
+template <int DIM>
+__device__ __forceinline__ void brick_save(const SliceGeom& g, float2* __restrict__ derivs, size_t pix, float2 gc, float2 gr, float2 gd, float2 v) {
+    if (DIM == 3) {
+        store_record(derivs + 4 * pix, gc, gr, gd, v);
+    } else {
+        __stcg(derivs + pix, gc);
+        __stcg(derivs + (size_t)g.BP * (size_t)g.slice_pixels + pix, gr);
+    }
+}
+
 // What the bricks leave of a slice: zeros outside the cutoff, or -- when its matrix is not (nearly) a rotation, so
 // that its pixels may lie anywhere -- the whole slice, by the plain gather.
-template <bool CUBIC, bool SAVE>
+template <int DIM, bool CUBIC, bool SAVE>
 __device__ __forceinline__ void brick_rest(const SliceGeom& g, const BrickWork& ws, int k, const float2* __restrict__ rec, const float* __restrict__ rot,
                                            const float* __restrict__ shifts, float2* __restrict__ out, float2* __restrict__ derivs) {
     const int b = k / g.P, p = k - b * g.P;
-    const float* rm = pose_rot<3>(g, rot, b, p);
+    const float* rm = pose_rot<DIM>(g, rot, b, p);
     const size_t base = (size_t)k * (size_t)g.slice_pixels;
-    if (brick_slice_ok(rm)) {
+    if (brick_slice_ok<DIM>(rm)) {
         const int n = __ldg(ws.header + 3);
         for (int q = threadIdx.x; q < n; q += kBlockThreads) __stcs(out + (base + (size_t)__ldg(ws.outside + q)), make_float2(0.f, 0.f));
         return;
@@ -537,9 +563,9 @@ __device__ __forceinline__ void brick_rest(const SliceGeom& g, const BrickWork& 
         Pixel px;
         px.c = px.r = px.d = 0.f;
         const bool in_image = i < g.N && j < g.Nh;
-        const bool valid = in_image && pixel_setup<3>(g, rm, i, j, px);
+        const bool valid = in_image && pixel_setup<DIM>(g, rm, i, j, px);
         float2 v, gc, gr, gd;
-        interpolate_any<3, CUBIC, SAVE>(g, rec + (size_t)b * g.vol_elems, px, valid, v, gc, gr, gd);
+        interpolate_any<DIM, CUBIC, SAVE>(g, rec + (size_t)b * g.vol_elems, px, valid, v, gc, gr, gd);
         if (!in_image) continue;
         float2 ph = make_float2(1.f, 0.f);
         if (valid && g.has_shift) {
@@ -549,20 +575,20 @@ __device__ __forceinline__ void brick_rest(const SliceGeom& g, const BrickWork& 
         }
         const size_t pix = base + (size_t)(i * g.Nh + j);
         __stcs(out + pix, v);
-        if (SAVE && valid) store_record(derivs + 4 * pix, g.has_shift ? cmul(gc, ph) : gc, g.has_shift ? cmul(gr, ph) : gr, g.has_shift ? cmul(gd, ph) : gd, v);
+        if (SAVE && valid) brick_save<DIM>(g, derivs, pix, g.has_shift ? cmul(gc, ph) : gc, g.has_shift ? cmul(gr, ph) : gr, DIM == 3 && g.has_shift ? cmul(gd, ph) : gd, v);
     }
 }
 
 using GatherBlock = BrickBlock<kWarps, 1024>;
 
-// Forward projection (SAVE: with the records of project_forw_saving_kernel).
-template <bool CUBIC, bool SAVE>
+// Forward projection (SAVE: with the derivatives of project_forw_saving_kernel, 3D as records).
+template <int DIM, bool CUBIC, bool SAVE>
 __global__ void __launch_bounds__(kBlockThreads, 3)
 brick_forw_kernel(const float2* __restrict__ rec, const float* __restrict__ rot, const float* __restrict__ shifts,
                   float2* __restrict__ out, float2* __restrict__ derivs, BrickWork ws, const SliceGeom g, const BrickPlan pl) {
     extern __shared__ __align__(16) unsigned char dyn[];
     float2* sm = reinterpret_cast<float2*>(dyn);
-    GatherBlock& sb = *reinterpret_cast<GatherBlock*>(dyn + sizeof(float2) * BrickShape<CUBIC>::kVoxels);
+    GatherBlock& sb = *reinterpret_cast<GatherBlock*>(dyn + sizeof(float2) * BrickShape<DIM, CUBIC>::kVoxels);
     const int items = __ldg(ws.header);
     while (true) {
         __syncthreads();
@@ -572,15 +598,15 @@ brick_forw_kernel(const float2* __restrict__ rec, const float* __restrict__ rot,
         if (item >= items) return;
         // beside its brick an item does its share of the slices' rest, whose stores overlap the brick's staging
         for (int k = (int)((long long)g.BP * item / items), k_end = (int)((long long)g.BP * (item + 1) / items); k < k_end; ++k)
-            brick_rest<CUBIC, SAVE>(g, ws, k, rec, rot, shifts, out, derivs);
+            brick_rest<DIM, CUBIC, SAVE>(g, ws, k, rec, rot, shifts, out, derivs);
         const int4 it = __ldg(ws.items + item);
-        const int X0 = pl.lo[0] + (it.x & 1023) * GatherBrick::x, Y0 = pl.lo[1] + ((it.x >> 10) & 1023) * GatherBrick::y, Z0 = pl.lo[2] + (it.x >> 20) * GatherBrick::z;
-        brick_stage<CUBIC>(g, rec + (size_t)it.y * g.vol_elems, sm, X0, Y0, Z0);
+        const int X0 = pl.lo[0] + (it.x & 1023) * GatherBrick<DIM>::x, Y0 = pl.lo[1] + ((it.x >> 10) & 1023) * GatherBrick<DIM>::y, Z0 = pl.lo[2] + (it.x >> 20) * GatherBrick<DIM>::z;
+        brick_stage<DIM, CUBIC>(g, rec + (size_t)it.y * g.vol_elems, sm, X0, Y0, Z0);
         const BrickWarp& sw = sb.warp[threadIdx.x >> 5];
-        brick_walk<GatherBrick>(g, ws.recs, sb, X0, Y0, Z0, it.z, it.w, 0, 1,
+        brick_walk<GatherBrick<DIM>>(g, ws.recs, sb, X0, Y0, Z0, it.z, it.w, 0, 1,
                    [&](bool active, int slot, int i, int j, const Pixel& px, int lx, int ly, int lz) {
             float2 v, gc, gr, gd;
-            brick_gather<CUBIC, SAVE>(sm, lx, ly, lz, px.c - floorf(px.c), px.r - floorf(px.r), px.d - floorf(px.d), v, gc, gr, gd);
+            brick_gather<DIM, CUBIC, SAVE>(sm, lx, ly, lz, px.c - floorf(px.c), px.r - floorf(px.r), DIM == 3 ? px.d - floorf(px.d) : 0.f, v, gc, gr, gd);
             if (!active) return;
             if (g.has_shift) {
                 const float4 rc = sw.slots[slot][2];
@@ -589,12 +615,12 @@ brick_forw_kernel(const float2* __restrict__ rec, const float* __restrict__ rot,
                 if (SAVE) {
                     gc = cmul(gc, ph);
                     gr = cmul(gr, ph);
-                    gd = cmul(gd, ph);
+                    if (DIM == 3) gd = cmul(gd, ph);
                 }
             }
             const size_t pix = (size_t)sw.slice[slot] * (size_t)g.slice_pixels + (size_t)(i * g.Nh + j);
             __stcg(out + pix, v);
-            if (SAVE) store_record(derivs + 4 * pix, gc, gr, gd, v);
+            if (SAVE) brick_save<DIM>(g, derivs, pix, gc, gr, gd, v);
         });
     }
 }

@@ -257,7 +257,7 @@ brick_scatter_kernel(const float2* __restrict__ proj, const float* __restrict__ 
         for (int k = (int)((long long)g.BP * item / items), k_end = (int)((long long)g.BP * (item + 1) / items); k < k_end; ++k) {
             const int b = k / g.P, p = k - b * g.P;
             const float* rm = pose_rot<3>(g, rot, b, p);
-            if (brick_slice_ok(rm)) continue;
+            if (brick_slice_ok<3>(rm)) continue;
             const int nj = (g.Nh + 7) / 8, ni = (g.N + 3) / 4;
             for (int patch = warp; patch < ni * nj; patch += C::kThreads / 32) {
                 BlockWork w;

@@ -155,8 +155,8 @@ Tensor resolve_order(int dim, const Tensor& vol, int64_t B, const Poses& p, cons
 
 // Scratch of the brick-by-brick 3D projection (complex64), undefined when the plain kernels are the better choice.
 Tensor project_workspace(int dim, const Tensor& rec, int64_t P, int64_t N, int interp, bool records, double oversampling, double cutoff) {
-    if (dim != 3 || is_f64(rec)) return Tensor();
-    const size_t bytes = b200proj_project_workspace_bytes(rec.size(0), P, N, interp, records ? 1 : 0, oversampling, cutoff);
+    if (is_f64(rec)) return Tensor();
+    const size_t bytes = b200proj_project_workspace_bytes(dim, rec.size(0), P, N, interp, records ? 1 : 0, oversampling, cutoff);
     return bytes ? at::empty({(int64_t)bytes}, rec.options().dtype(at::kByte)) : Tensor();
 }
 // The same for the 3D scatters.
@@ -200,7 +200,7 @@ Tensor project_forw(int dim, const Tensor& reconstruction, const Tensor& rotatio
         rc = dim == 2 ? b200proj_project_2d_forw_f64(cptr<double>(rec), B, R, cptr<double>(p.rot), p.B_rot, cptr<double>(p.shifts), p.B_shift, p.P, N, interp, oversampling, cut, mptr<double>(out), s)
                       : b200proj_project_3d_to_2d_forw_f64(cptr<double>(rec), B, R, cptr<double>(p.rot), p.B_rot, cptr<double>(p.shifts), p.B_shift, p.P, N, interp, oversampling, cut, mptr<double>(out), cptr<int32_t>(order), s);
     } else {
-        rc = dim == 2 ? b200proj_project_2d_forw(cptr<float>(rec), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts), p.B_shift, p.P, N, interp, oversampling, cut, mptr<float>(out), s)
+        rc = dim == 2 ? b200proj_project_2d_forw_ws(cptr<float>(rec), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts), p.B_shift, p.P, N, interp, oversampling, cut, mptr<float>(out), ws_ptr(ws), ws_size(ws), s)
                       : b200proj_project_3d_to_2d_forw_ws(cptr<float>(rec), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts), p.B_shift, p.P, N, interp, oversampling, cut, mptr<float>(out), cptr<int32_t>(order), ws_ptr(ws), ws_size(ws), s);
     }
     status(rc, dim == 2 ? "project_2d_forw" : "project_3d_to_2d_forw");
@@ -301,8 +301,8 @@ std::tuple<Tensor, Tensor> project_forw_saving(int dim, const Tensor& reconstruc
     const Tensor ws = project_workspace(dim, rec, p.P, N, interp, true, oversampling, cut);
     Tensor order = ws.defined() ? Tensor() : resolve_order(dim, rec, B, p, pose_order);
     const int rc = dim == 2
-        ? b200proj_project_2d_forw_saving(cptr<float>(rec), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts), p.B_shift, p.P, N, interp,
-                                          oversampling, cut, mptr<float>(out), mptr<float>(derivs), current_stream(rec))
+        ? b200proj_project_2d_forw_saving_ws(cptr<float>(rec), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts), p.B_shift, p.P, N, interp,
+                                          oversampling, cut, mptr<float>(out), mptr<float>(derivs), ws_ptr(ws), ws_size(ws), current_stream(rec))
         : b200proj_project_3d_to_2d_forw_records(cptr<float>(rec), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts), p.B_shift, p.P, N, interp,
                                                    oversampling, cut, mptr<float>(out), mptr<float>(derivs), cptr<int32_t>(order), ws_ptr(ws), ws_size(ws), current_stream(rec));
     status(rc, dim == 2 ? "project_2d_forw_saving" : "project_3d_to_2d_forw_saving");
