@@ -102,10 +102,10 @@ int b200proj_project_3d_to_2d_forw(const float* rec, int64_t B, int64_t R,
  * is free again when the call's work has run. */
 size_t b200proj_project_workspace_bytes(int dim, int64_t B, int64_t P, int64_t N, int interpolation, int records,
                                         double oversampling, double fourier_radius_cutoff);
-/* The same for the scatters of the 3D operators (b200proj_project_3d_to_2d_back_records and _back_ws with
- * grad_rec, b200proj_backproject_2d_to_3d_accumulate_ws, b200proj_backproject_2d_to_3d_forw; 0: no gain, for
+/* The same for the scatters (b200proj_project_3d_to_2d_back_records and _back_ws with
+ * grad_rec, b200proj_backproject_2d_to_3d_accumulate_ws, b200proj_backproject_{2d,2d_to_3d}_forw; 0: no gain, for
  * the last of them see there for what else a workspace is good for). */
-size_t b200proj_scatter_workspace_bytes(int64_t B, int64_t P, int64_t N, int interpolation, int has_weights,
+size_t b200proj_scatter_workspace_bytes(int dim, int64_t B, int64_t P, int64_t N, int interpolation, int has_weights,
                                         double oversampling, double fourier_radius_cutoff);
 /* Workspace of the backward passes of the projection (b200proj_project_{2d,3d_to_2d}_back_ws with grad_rec,
  * b200proj_project_2d_back_saved_ws, b200proj_project_3d_to_2d_back_records): the larger calls above, and copies

@@ -20,7 +20,8 @@ SIZES = [(1, 40, 4, 8, 2.0, None, 1, 1),
          (2, 33, 20, 30, 1.5, 7.3, 2, 0),
          (2, 9, 34, 34, 1.0, 20.0, 1, 2),
          (1, 37, 26, 34, 1.3, None, 1, 1),
-         (1, 3, 48, 120, 2.5, 17.0, 1, 1)]
+         (1, 3, 48, 120, 2.5, 17.0, 1, 1),
+         (1, 12, 44, 100, 2.0, 29.0, 1, 1)]          # cutoff beyond Nyquist: corners of the slices
 
 
 SIZES_2D = SIZES[:5] + [(1, 21, 70, 160, 2.0, 40.0, 1, 1), (2, 300, 130, 130, 1.0, None, 2, 2)]

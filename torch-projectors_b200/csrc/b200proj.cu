@@ -284,10 +284,19 @@ BrickLaunch gather_plan(int dim, int64_t B, int64_t P, int64_t N, bool cubic, bo
 }
 
 // Cubic scatter (linear taps keep the plain kernels, see brick_scatter.cuh).
-BrickLaunch scatter_plan(int64_t B, int64_t P, int64_t N, bool cubic, bool weights, double os, double cutoff) {
+template <int DIM, bool WEIGHTS>
+BrickLaunch scatter_layout(int64_t B, int64_t P, int64_t N, double os, double cutoff) {
+    using C = Scatter<DIM, WEIGHTS>;
+    return brick_layout<typename C::Brick>(B, P, N, os, cutoff, 148.0 * C::kBlocks, 3000.0, false);
+}
+BrickLaunch scatter_plan(int dim, int64_t B, int64_t P, int64_t N, bool cubic, bool weights, double os, double cutoff) {
     if (!cubic) return BrickLaunch{};
-    BrickLaunch L = weights ? brick_layout<Scatter<true>::Brick>(B, P, N, os, cutoff, 148.0 * Scatter<true>::kBlocks, 3000.0, false)
-                            : brick_layout<Scatter<false>::Brick>(B, P, N, os, cutoff, 148.0 * Scatter<false>::kBlocks, 3000.0, false);
+    if (dim == 2) {
+        BrickLaunch L = weights ? scatter_layout<2, true>(B, P, N, os, cutoff) : scatter_layout<2, false>(B, P, N, os, cutoff);
+        L.use = L.use && (L.forced || L.pixels > 4.5e6);
+        return L;
+    }
+    BrickLaunch L = weights ? scatter_layout<3, true>(B, P, N, os, cutoff) : scatter_layout<3, false>(B, P, N, os, cutoff);
     // measured crossings with the plain kernels, in M pixels: 0.8 / 1.7 / 5 for box-128 / 256 / 400 gradients, 0.55 / 0.8 / 0.9 with weights
     L.use = L.use && (L.forced || L.pixels > (weights ? 0.6e6 + 45.0 * L.in_ball : 0.75e6 + 430.0 * L.in_ball));
     return L;
@@ -323,17 +332,17 @@ int launch_brick_forw(const Launch& L, const BrickLaunch& bl, void* workspace, c
     return check_launch("brick_forw launch");
 }
 
-template <bool WEIGHTS, bool DUP, bool INTERLEAVED = false>
+template <int DIM, bool WEIGHTS, bool DUP, bool INTERLEAVED = false>
 int launch_brick_scatter(const Launch& L, const BrickLaunch& bl, void* workspace, const float* proj, const float* weights, const float* rot,
                          const float* shifts, float* vol, float* wvol, cudaStream_t s, float4* accum = nullptr) {
-    using C = Scatter<WEIGHTS>;
+    using C = Scatter<DIM, WEIGHTS>;
     const BrickWork w = brick_work(bl, workspace);
-    if (int rc = brick_setup<3>(bl, w, L, rot, shifts, false, s)) return rc;
+    if (int rc = brick_setup<DIM>(bl, w, L, rot, shifts, false, s)) return rc;
     constexpr size_t smem = sizeof(typename C::Shared);
     static_assert((smem + 1024) * C::kBlocks <= 233472, "shared memory of an SM");
-    const cudaError_t e = cudaFuncSetAttribute(brick_scatter_kernel<WEIGHTS, DUP, INTERLEAVED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = cudaFuncSetAttribute(brick_scatter_kernel<DIM, WEIGHTS, DUP, INTERLEAVED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cuda_fail(e, "brick_scatter shared memory");
-    brick_scatter_kernel<WEIGHTS, DUP, INTERLEAVED><<<148 * C::kBlocks, C::kThreads, smem, s>>>((const float2*)proj, weights, rot, shifts, (float2*)vol, wvol, accum, w, L.g, bl.plan);
+    brick_scatter_kernel<DIM, WEIGHTS, DUP, INTERLEAVED><<<148 * C::kBlocks, C::kThreads, smem, s>>>((const float2*)proj, weights, rot, shifts, (float2*)vol, wvol, accum, w, L.g, bl.plan);
     return check_launch("brick_scatter launch");
 }
 
@@ -468,7 +477,7 @@ int project_back_saved(const float* grad_proj, const float* out, const float* de
     cudaStream_t s = (cudaStream_t)stream;
     const bool cubic = interpolation == B200PROJ_CUBIC;
     BrickLaunch bl{};
-    if (RECORDS && P > 0 && grad_rec != nullptr && workspace != nullptr) bl = scatter_plan(B, P, N, cubic, false, os, cutoff);
+    if ((RECORDS || DIM == 2) && P > 0 && grad_rec != nullptr && workspace != nullptr) bl = scatter_plan(DIM, B, P, N, cubic, false, os, cutoff);
     if (workspace_bytes < bl.bytes) bl.use = false;
     const int copies = P > 0 && grad_rec != nullptr && !bl.use ? scatter_copies(L, workspace, workspace_bytes) : 1;
     if (int rc = zero_outputs(s, copies > 1 ? nullptr : grad_rec, L.rec_count * sizeof(float2), grad_rot, (size_t)B_rot * P * DIM * DIM * sizeof(float),
@@ -479,7 +488,7 @@ int project_back_saved(const float* grad_proj, const float* out, const float* de
     const float2* d = (const float2*)derivatives;
     if (bl.use) {
         // large cubic scatter: brick by brick, the pose gradients in a streaming pass of their own
-        if (int rc = launch_brick_scatter<false, false>(L, bl, workspace, grad_proj, nullptr, rot, shifts, grad_rec, nullptr, s)) return rc;
+        if (int rc = launch_brick_scatter<DIM, false, false>(L, bl, workspace, grad_proj, nullptr, rot, shifts, grad_rec, nullptr, s)) return rc;
         if (grad_rot == nullptr && grad_shifts == nullptr) return B200PROJ_OK;
         grad_rec = nullptr;
     }
@@ -510,15 +519,15 @@ int project_back(const Real* grad_proj, const Real* rec, int64_t B, int64_t R, c
         return fail(B200PROJ_ERR_ARGUMENT, "grad_shifts requested but no shifts given");
     cudaStream_t s = (cudaStream_t)stream;
     BrickLaunch bl{};
-    if (DIM == 3 && std::is_same<Real, float>::value && P > 0 && grad_rot == nullptr && grad_shifts == nullptr && workspace != nullptr)
-        bl = scatter_plan(B, P, N, interpolation == B200PROJ_CUBIC, false, os, cutoff);
+    if (std::is_same<Real, float>::value && P > 0 && grad_rot == nullptr && grad_shifts == nullptr && workspace != nullptr)
+        bl = scatter_plan(DIM, B, P, N, interpolation == B200PROJ_CUBIC, false, os, cutoff);
     if (workspace_bytes < bl.bytes) bl.use = false;
     const int copies = P > 0 && std::is_same<Real, float>::value && !bl.use ? scatter_copies(L, workspace, workspace_bytes) : 1;
     if (int rc = zero_outputs(s, copies > 1 ? nullptr : grad_rec, L.rec_count * sizeof(C2<Real>), grad_rot, (size_t)B_rot * P * DIM * DIM * sizeof(Real),
                               grad_shifts, (size_t)(shifts ? B_shift : 0) * P * 2 * sizeof(Real))) return rc;
     if (P == 0) return B200PROJ_OK;
-    if constexpr (DIM == 3 && std::is_same<Real, float>::value)
-        if (bl.use) return launch_brick_scatter<false, false>(L, bl, workspace, grad_proj, nullptr, rot, shifts, grad_rec, nullptr, s);
+    if constexpr (std::is_same<Real, float>::value)
+        if (bl.use) return launch_brick_scatter<DIM, false, false>(L, bl, workspace, grad_proj, nullptr, rot, shifts, grad_rec, nullptr, s);
     if (copies > 1)
         if (int rc = zero_async(workspace, (size_t)copies * L.rec_count * sizeof(float2), s)) return rc;
     C2<Real>* to = copies > 1 ? (C2<Real>*)workspace : (C2<Real>*)grad_rec;
@@ -549,14 +558,14 @@ int backproject_forw(const Real* proj, const Real* weights, int64_t B, int64_t R
     // Interleaved path: data and weight of a voxel share one 16-byte slot of the workspace
     // (one v4 reduction per tap), folded into the outputs afterwards.
     const size_t ws_one = L.rec_count * sizeof(float4);
-    if constexpr (DIM == 3 && std::is_same<Real, float>::value) {
-        const BrickLaunch bl = P > 0 && workspace != nullptr ? scatter_plan(B, P, N, cubic, hw, os, cutoff) : BrickLaunch{};
+    if constexpr (std::is_same<Real, float>::value) {
+        const BrickLaunch bl = P > 0 && workspace != nullptr ? scatter_plan(DIM, B, P, N, cubic, hw, os, cutoff) : BrickLaunch{};
         if (bl.use && workspace_bytes >= bl.bytes && (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0) {
             if (!accumulate) {
                 if (int rc = zero_outputs(s, data_rec, L.rec_count * sizeof(C2<Real>), weight_rec, L.rec_count * sizeof(Real))) return rc;
             }
-            return hw ? launch_brick_scatter<true, true>(L, bl, workspace, proj, weights, rot, shifts, data_rec, weight_rec, s)
-                      : launch_brick_scatter<false, true>(L, bl, workspace, proj, nullptr, rot, shifts, data_rec, nullptr, s);
+            return hw ? launch_brick_scatter<DIM, true, true>(L, bl, workspace, proj, weights, rot, shifts, data_rec, weight_rec, s)
+                      : launch_brick_scatter<DIM, false, true>(L, bl, workspace, proj, nullptr, rot, shifts, data_rec, nullptr, s);
         }
     }
     constexpr bool kIsF32 = std::is_same<Real, float>::value;  // workspace and slab paths exist in fp32 only
@@ -696,8 +705,8 @@ int backproject_accumulate(const float* proj, const float* weights, int64_t B, i
     float4* acc = (float4*)accumulator;
     const bool cubic = interpolation == B200PROJ_CUBIC;
     if (workspace != nullptr && slab_count == plan.slabs) {
-        const BrickLaunch bl = scatter_plan(B, P, N, cubic, true, os, cutoff);
-        if (bl.use && workspace_bytes >= bl.bytes) return launch_brick_scatter<true, true, true>(L, bl, workspace, proj, weights, rot, shifts, nullptr, nullptr, s, acc);
+        const BrickLaunch bl = scatter_plan(3, B, P, N, cubic, true, os, cutoff);
+        if (bl.use && workspace_bytes >= bl.bytes) return launch_brick_scatter<3, true, true, true>(L, bl, workspace, proj, weights, rot, shifts, nullptr, nullptr, s, acc);
     }
     if (plan.slabs > 1) {
         launch_slab_interleaved(L, s, cubic, proj, weights, rot, shifts, acc, plan, slab_first, slab_count);
@@ -844,15 +853,16 @@ int b200proj_project_3d_to_2d_forw(const float* rec, int64_t B, int64_t R, const
     return project_forw<3>(rec, B, R, rot, B_rot, shifts, B_shift, P, N, interpolation, oversampling, cutoff, out, pose_order, stream);
 }
 
-size_t b200proj_scatter_workspace_bytes(int64_t B, int64_t P, int64_t N, int interpolation, int has_weights, double oversampling, double cutoff) {
-    const BrickLaunch bl = scatter_plan(B, P, N, interpolation == B200PROJ_CUBIC, has_weights != 0, oversampling, cutoff);
+size_t b200proj_scatter_workspace_bytes(int dim, int64_t B, int64_t P, int64_t N, int interpolation, int has_weights, double oversampling, double cutoff) {
+    if (dim != 2 && dim != 3) return 0;
+    const BrickLaunch bl = scatter_plan(dim, B, P, N, interpolation == B200PROJ_CUBIC, has_weights != 0, oversampling, cutoff);
     return bl.use ? bl.bytes : 0;
 }
 size_t b200proj_gradient_workspace_bytes(int dim, int64_t B, int64_t R, int64_t P, int64_t N, int interpolation, int pose_gradients,
                                          double oversampling, double cutoff) {
     if ((dim != 2 && dim != 3) || B < 1 || R < 2 || P < 1 || N < 2) return 0;
-    if (dim == 3 && !pose_gradients)
-        if (const size_t bytes = b200proj_scatter_workspace_bytes(B, P, N, interpolation, 0, oversampling, cutoff)) return bytes;
+    if (!pose_gradients)
+        if (const size_t bytes = b200proj_scatter_workspace_bytes(dim, B, P, N, interpolation, 0, oversampling, cutoff)) return bytes;
     const double one = (double)B * (dim == 3 ? R : 1) * R * (R / 2 + 1) * (double)sizeof(float2);
     const int copies = workspace_replicas(one, P);
     return copies > 1 ? (size_t)one * (size_t)copies : 0;

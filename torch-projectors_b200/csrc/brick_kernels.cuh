@@ -454,7 +454,7 @@ __device__ __forceinline__ void brick_walk(const SliceGeom& g, const float4* __r
                 const float m21 = sw.slots[slot][2].x;
                 const float room = g.cutoff_sq - krf * krf;
                 int ja_i = 0, len = 0;
-                if (row0 + lane < rows && room >= 0.f) {
+                if (row0 + lane < rows && room >= 0.f && kr <= g.N / 2) {       // (a slice without rows here still counts one)
                     float ja = 0.f, jb = fminf((float)(g.Nh - 1), sqrtf(room) + 0.01f);
                     auto clip = [&](float a, float b, float lo, float n) {
                         a *= osf;

@@ -1,4 +1,4 @@
-// Brick-stationary scatters of the 3D operators (fp32, cubic taps): gradient of the projection with respect to the volume, and
+// Brick-stationary scatters (fp32, cubic taps): gradient of the projection with respect to the volume, and
 // back-projection.  The plain kernels send every tap to L2 as a reduction and sit on the rate at which reductions
 // leave the SMs.  Here a brick's sums are kept in shared memory and leave once per work item.
 //
@@ -13,7 +13,9 @@
 // An adding warp takes a chunk, one pixel per lane, and every lane its taps in an order that starts at the lane's own
 // class (x & 3, y & 3, z & 3) -- a cubic footprint holds every class once --, two taps a step: the 32 lanes hold 64
 // different classes then, hence 64 different voxels, whatever pixels they hold.  So no two lanes add to the same voxel
-// between two synchronisations of the warp, and no bank conflicts arise.
+// between two synchronisations of the warp, and no bank conflicts arise.  2D reconstructions are cut into tiles; a
+// tile's pixels go to the adding warps in turn, each of which has its own sums (two copies: a 4 x 4 footprint has 16
+// classes, so the halves of the warp are kept apart).
 //
 // Measured on B200: the scatter of 4,096 slices of 256 x 129 into a box-512 gradient 14.4 ms (plain kernel) -> 5.97 ms,
 // 2,501 weighted slices of box 90 into box 180 1.61 -> 0.75 ms.  Bound by the adding warps: a step is a chain of load,
@@ -73,18 +75,22 @@ __device__ __forceinline__ void count_wait(const int* count, int below, int* gav
 
 // ---- sizes --------------------------------------------------------------------------------------------------
 // kX x kY sample positions, kSlabs slabs of kSlab planes of them; kBlocks blocks per SM of kWalkers + kSlabs warps.
-template <bool WEIGHTS>
+template <int DIM, bool WEIGHTS>
 struct ScatterSizes;
-template <> struct ScatterSizes<false> { static constexpr int kX = 13, kY = 13, kSlab = 4, kSlabs = 6, kWalkers = 6, kBlocks = 2, kRing = 4; };
-template <> struct ScatterSizes<true> { static constexpr int kX = 13, kY = 13, kSlab = 4, kSlabs = 4, kWalkers = 6, kBlocks = 2, kRing = 4; };
+template <> struct ScatterSizes<3, false> { static constexpr int kX = 13, kY = 13, kSlab = 4, kSlabs = 6, kWalkers = 6, kBlocks = 2, kRing = 4; };
+template <> struct ScatterSizes<3, true> { static constexpr int kX = 13, kY = 13, kSlab = 4, kSlabs = 4, kWalkers = 6, kBlocks = 2, kRing = 4; };
 
-template <bool WEIGHTS>
-struct Scatter : ScatterSizes<WEIGHTS> {
-    using Z = ScatterSizes<WEIGHTS>;
+// 2D: kSlabs counts adding warps, each with two copies of the tile's sums (kSlab = 0).
+template <> struct ScatterSizes<2, false> { static constexpr int kX = 29, kY = 29, kSlab = 0, kSlabs = 5, kWalkers = 7, kBlocks = 2, kRing = 4; };
+template <> struct ScatterSizes<2, true> { static constexpr int kX = 21, kY = 21, kSlab = 0, kSlabs = 6, kWalkers = 6, kBlocks = 2, kRing = 4; };
+
+template <int DIM, bool WEIGHTS>
+struct Scatter : ScatterSizes<DIM, WEIGHTS> {
+    using Z = ScatterSizes<DIM, WEIGHTS>;
     using Brick = BrickDims<Z::kX, Z::kY, Z::kSlab * Z::kSlabs>;
     static constexpr int kThreads = (Z::kWalkers + Z::kSlabs) * 32;
-    static constexpr int kTX = Z::kX + 3, kTY = Z::kY + 3, kTZ = Z::kSlab + 3;                  // of one slab, halo included
-    static_assert(kTX % 4 == 0 && kTY % 4 == 0 && Z::kSlab >= 3 && Z::kRing >= 2, "whole cells; two slabs share a plane at most");
+    static constexpr int kTX = Z::kX + 3, kTY = Z::kY + 3, kTZ = DIM == 3 ? Z::kSlab + 3 : 2;   // of one slab, halo included
+    static_assert(kTX % 4 == 0 && kTY % 4 == 0 && (DIM == 2 || Z::kSlab >= 3) && Z::kRing >= 2, "whole cells; two slabs share a plane at most");
     static constexpr int kPlane = kTX * kTY, kVoxels = kPlane * kTZ;
     struct Slab {
         float2 sum[kVoxels];
@@ -104,7 +110,7 @@ struct Scatter : ScatterSizes<WEIGHTS> {
         BrickBlock<1, 64> walk[Z::kWalkers];
         int item, done, gave_up;
     };
-    // place of the voxel (x, y, z) of a slab: 4 x 4 cells of a plane are contiguous
+    // place of the voxel (x, y, z) of a slab (2D: copy z): 4 x 4 cells of a plane are contiguous
     __device__ static __forceinline__ int place(int x, int y, int z) { return z * kPlane + 4 * (y & 3) + kTX * 4 * (y >> 2) + x + 12 * (x >> 2); }
 };
 constexpr unsigned kItemEnds = 1u << 24;        // flag of a ring's last entry of an item
@@ -112,8 +118,53 @@ constexpr unsigned kItemEnds = 1u << 24;        // flag of a ring's last entry o
 // ---- adding 32 pixels, one per lane ---------------------------------------------------------------------------
 // A lane without a pixel adds zeros (its classes are its own).
 template <bool WEIGHTS>
-__device__ __forceinline__ void brick_add(typename Scatter<WEIGHTS>::Slab& sb, const float4 a, float2 v, float wv) {
-    using C = Scatter<WEIGHTS>;
+__device__ __forceinline__ void brick_add_2d(typename Scatter<2, WEIGHTS>::Slab& sb, const float4 a, float2 v, float wv) {
+    using C = Scatter<2, WEIGHTS>;
+    using u64 = unsigned long long;
+    const int lane = threadIdx.x & 31;
+    const unsigned at = __float_as_uint(a.w);
+    const int lx = at & 255, ly = at >> 8 & 255, rx = lx & 3, ry = ly & 3;
+    // lanes 16 apart hold the same class: each half of the warp has its own copy
+    const unsigned base = (unsigned)((lane >> 4) * C::kPlane + (ly >> 2) * (C::kTX * 4) + (lx >> 2) * 16) * 8u + smem_addr(sb.sum);
+    unsigned ox[4];
+    float wx[4], wy[4];
+    cubic_weights(a.x, wx);
+    rotate4(wx, (lane - lx) & 3);
+    cubic_weights(a.y, wy);
+    rotate4(wy, ((lane >> 2) - ly) & 3);
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        const int ax = (lane + s) & 3;
+        ox[s] = (unsigned)(ax * 8 + (ax < rx ? 128 : 0)) + base;
+    }
+    const u64 v2 = pack2(v.x, v.y);
+    const unsigned half = (smem_addr(sb.sum) >> 1) - smem_addr(sb.wsum);      // weights: half the distance
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+        const int ay = ((lane >> 2) + b) & 3;
+        const unsigned oy = (unsigned)(ay * 32 + (ay < ry ? C::kTX * 32 : 0));
+        const u64 q = fmul2(pack2(wy[b], wy[b]), v2);
+        const float f = WEIGHTS ? wv * fabsf(wy[b]) : 0.f;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const unsigned s0 = oy + ox[k];
+            const u64 u = lds64(s0);
+            if (WEIGHTS) {
+                const unsigned t0 = (s0 >> 1) - half;
+                const float g0 = lds32(t0);
+                sts64(s0, fma2(pack2(wx[k], wx[k]), q, u));
+                sts32(t0, fmaf(fabsf(wx[k]), f, g0));
+            } else {
+                sts64(s0, fma2(pack2(wx[k], wx[k]), q, u));
+            }
+            __syncwarp();
+        }
+    }
+}
+
+template <bool WEIGHTS>
+__device__ __forceinline__ void brick_add(typename Scatter<3, WEIGHTS>::Slab& sb, const float4 a, float2 v, float wv) {
+    using C = Scatter<3, WEIGHTS>;
     using u64 = unsigned long long;
     constexpr int kPlane = C::kPlane;
     const int lane = threadIdx.x & 31;
@@ -178,10 +229,10 @@ __device__ __forceinline__ void brick_add(typename Scatter<WEIGHTS>::Slab& sb, c
 // Sums of a finished item to the volume, by the scatter's rules (Friedel mirror with conjugation, taps outside the
 // stored half-volume dropped, DUP: the conjugate also to the Friedel partner of a voxel on the c == 0 plane); cleared
 // for the next item.  INTERLEAVED: into 16-byte (re, im, weight, 0) voxels.
-template <bool WEIGHTS, bool DUP, bool INTERLEAVED>
-__device__ __forceinline__ void brick_flush(const SliceGeom& g, typename Scatter<WEIGHTS>::Shared& sh, float2* __restrict__ vol, float* __restrict__ wvol,
+template <int DIM, bool WEIGHTS, bool DUP, bool INTERLEAVED>
+__device__ __forceinline__ void brick_flush(const SliceGeom& g, typename Scatter<DIM, WEIGHTS>::Shared& sh, float2* __restrict__ vol, float* __restrict__ wvol,
                                             float4* __restrict__ accum, int X0, int Y0, int Z0) {
-    using C = Scatter<WEIGHTS>;
+    using C = Scatter<DIM, WEIGHTS>;
     auto add = [&](int off, float re, float im, float w) {
         if (INTERLEAVED) {
             red_add_v4(accum + off, re, im, w, 0.f);
@@ -190,15 +241,13 @@ __device__ __forceinline__ void brick_flush(const SliceGeom& g, typename Scatter
             if (WEIGHTS) red_add(wvol + off, w);
         }
     };
-    // planes that two slabs share are added up first: the first three planes of a slab are the last of the one below
-    for (int t = (int)threadIdx.x; t < (C::kSlab * C::kSlabs + 3) * C::kPlane; t += C::kThreads) {
+    // 3D: planes that two slabs share are added up first (the first three planes of a slab are the last of the one
+    // below); 2D: the copies of all adding warps
+    for (int t = (int)threadIdx.x; t < (DIM == 3 ? C::kSlab * C::kSlabs + 3 : 1) * C::kPlane; t += C::kThreads) {
         const int x = t % C::kTX, row = t / C::kTX, y = row % C::kTY, z = row / C::kTY;
         float2 v = make_float2(0.f, 0.f);
         float w = 0.f;
-        const int last = min(z / C::kSlab, C::kSlabs - 1), first = max(0, z - 3) / C::kSlab;
-        for (int s = first; s <= last; ++s) {
-            typename C::Slab& sb = sh.slab[s];
-            const int at = C::place(x, y, z - s * C::kSlab);
+        auto take = [&](typename C::Slab& sb, int at) {
             const float2 u = sb.sum[at];
             sb.sum[at] = make_float2(0.f, 0.f);
             v.x += u.x;
@@ -207,10 +256,20 @@ __device__ __forceinline__ void brick_flush(const SliceGeom& g, typename Scatter
                 w += sb.wsum[at];
                 sb.wsum[at] = 0.f;
             }
+        };
+        if constexpr (DIM == 3) {
+            const int last = min(z / C::kSlab, C::kSlabs - 1), first = max(0, z - 3) / C::kSlab;
+            for (int s = first; s <= last; ++s) take(sh.slab[s], C::place(x, y, z - s * C::kSlab));
+        } else {
+#pragma unroll
+            for (int s = 0; s < C::kSlabs; ++s) {
+                take(sh.slab[s], C::place(x, y, 0));
+                take(sh.slab[s], C::place(x, y, 1));
+            }
         }
         if (v.x == 0.f && v.y == 0.f && w == 0.f) continue;
         bool m;
-        const int c = scatter_col(g, X0 - 1 + x, m), r = scatter_line(g, Y0 - 1 + y, m), d = scatter_line(g, Z0 - 1 + z, m);
+        const int c = scatter_col(g, X0 - 1 + x, m), r = scatter_line(g, Y0 - 1 + y, m), d = DIM == 3 ? scatter_line(g, Z0 - 1 + z, m) : 0;
         if (c < 0 || r < 0 || d < 0) continue;
         if (m) v.y = -v.y;
         add((d * g.R + r) * g.Rh + c, v.x, v.y, w);
@@ -224,12 +283,12 @@ __device__ __forceinline__ void brick_flush(const SliceGeom& g, typename Scatter
 // No wait can last: a walking warp writes each ring as soon as that ring has room, so the lowest place of a ring that is
 // not written yet waits only for chunks before its own (a ring has more than one), all of which are written and will be
 // taken; the last warp to finish its walk fills every ring up to a whole chunk.
-template <bool WEIGHTS, bool DUP, bool INTERLEAVED>
-__global__ void __launch_bounds__(Scatter<WEIGHTS>::kThreads, Scatter<WEIGHTS>::kBlocks)
+template <int DIM, bool WEIGHTS, bool DUP, bool INTERLEAVED>
+__global__ void __launch_bounds__(Scatter<DIM, WEIGHTS>::kThreads, Scatter<DIM, WEIGHTS>::kBlocks)
 brick_scatter_kernel(const float2* __restrict__ proj, const float* __restrict__ weights, const float* __restrict__ rot,
                      const float* __restrict__ shifts, float2* __restrict__ vol, float* __restrict__ wvol, float4* __restrict__ accum,
                      BrickWork ws, const SliceGeom g, const BrickPlan pl) {
-    using C = Scatter<WEIGHTS>;
+    using C = Scatter<DIM, WEIGHTS>;
     extern __shared__ __align__(16) unsigned char dyn[];
     typename C::Shared& sh = *reinterpret_cast<typename C::Shared*>(dyn);
     constexpr unsigned kFull = 0xffffffffu;
@@ -256,8 +315,8 @@ brick_scatter_kernel(const float2* __restrict__ proj, const float* __restrict__ 
         // the item's share of the slices that are not for the bricks: plain scatter
         for (int k = (int)((long long)g.BP * item / items), k_end = (int)((long long)g.BP * (item + 1) / items); k < k_end; ++k) {
             const int b = k / g.P, p = k - b * g.P;
-            const float* rm = pose_rot<3>(g, rot, b, p);
-            if (brick_slice_ok<3>(rm)) continue;
+            const float* rm = pose_rot<DIM>(g, rot, b, p);
+            if (brick_slice_ok<DIM>(rm)) continue;
             const int nj = (g.Nh + 7) / 8, ni = (g.N + 3) / 4;
             for (int patch = warp; patch < ni * nj; patch += C::kThreads / 32) {
                 BlockWork w;
@@ -270,9 +329,9 @@ brick_scatter_kernel(const float2* __restrict__ proj, const float* __restrict__ 
                 Pixel px;
                 float2 v;
                 float wv;
-                const bool active = backproject_pixel<3, WEIGHTS>(g, w, proj, weights, rot, shifts, px, v, wv);
+                const bool active = backproject_pixel<DIM, WEIGHTS>(g, w, proj, weights, rot, shifts, px, v, wv);
                 const size_t at = (size_t)b * g.vol_elems;
-                scatter_coop<3, true, WEIGHTS, DUP, INTERLEAVED>(g, INTERLEAVED ? nullptr : vol + at, WEIGHTS && !INTERLEAVED ? wvol + at : nullptr,
+                scatter_coop<DIM, true, WEIGHTS, DUP, INTERLEAVED>(g, INTERLEAVED ? nullptr : vol + at, WEIGHTS && !INTERLEAVED ? wvol + at : nullptr,
                                                                   INTERLEAVED ? accum + at : nullptr, px, active, v, wv);
             }
         }
@@ -293,7 +352,7 @@ brick_scatter_kernel(const float2* __restrict__ proj, const float* __restrict__ 
                 if (WEIGHTS) q.w[at] = w;
             };
             // the previous window's pixels, whose values are still on their way from memory
-            int h_slab = -1;
+            int h_slab = -1, turn = warp % C::kSlabs;
             float4 h_a = make_float4(0.f, 0.f, 0.f, 0.f);
             float2 h_v = make_float2(0.f, 0.f), h_ph = make_float2(1.f, 0.f);
             float h_w = 0.f;
@@ -345,10 +404,12 @@ brick_scatter_kernel(const float2* __restrict__ proj, const float* __restrict__ 
                     if (WEIGHTS) w = __ldg(weights + pix);
                 }
                 put();
-                const int s = lz / C::kSlab;
+                int s = 0;
+                if constexpr (DIM == 3) s = lz / C::kSlab;
+                else s = turn = turn + 1 < C::kSlabs ? turn + 1 : 0;                // windows are dealt to the adding warps in turn
                 h_slab = active ? s : -1;
-                h_a = make_float4(px.c - floorf(px.c), px.r - floorf(px.r), px.d - floorf(px.d),
-                                  __uint_as_float((unsigned)(lx | ly << 8 | (lz - s * C::kSlab) << 16)));
+                h_a = make_float4(px.c - floorf(px.c), px.r - floorf(px.r), DIM == 3 ? px.d - floorf(px.d) : 0.f,
+                                  __uint_as_float((unsigned)(lx | ly << 8 | (DIM == 3 ? lz - s * C::kSlab : 0) << 16)));
                 h_v = v;
                 h_w = w;
                 if (g.has_shift) {
@@ -392,13 +453,14 @@ brick_scatter_kernel(const float2* __restrict__ proj, const float* __restrict__ 
                 }
                 if (++slot == C::kRing) { slot = 0; parity ^= 1u; }
                 ends = (__shfl_sync(kFull, __float_as_uint(a.w), 31) & kItemEnds) != 0u;
-                brick_add<WEIGHTS>(sb, a, v, w);
+                if constexpr (DIM == 3) brick_add<WEIGHTS>(sb, a, v, w);
+                else brick_add_2d<WEIGHTS>(sb, a, v, w);
             }
         }
         __syncthreads();
         if (sh.gave_up) break;
         const size_t at = (size_t)it.y * g.vol_elems;
-        brick_flush<WEIGHTS, DUP, INTERLEAVED>(g, sh, INTERLEAVED ? nullptr : vol + at, WEIGHTS && !INTERLEAVED ? wvol + at : nullptr,
+        brick_flush<DIM, WEIGHTS, DUP, INTERLEAVED>(g, sh, INTERLEAVED ? nullptr : vol + at, WEIGHTS && !INTERLEAVED ? wvol + at : nullptr,
                                                       INTERLEAVED ? accum + at : nullptr, X0, Y0, Z0);
     }
     if (threadIdx.x == 0 && sh.gave_up) ws.header[3] = 1;       // never, see above

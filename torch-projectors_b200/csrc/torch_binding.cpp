@@ -153,16 +153,16 @@ Tensor resolve_order(int dim, const Tensor& vol, int64_t B, const Poses& p, cons
     return plane_locality_order(p.rot, B);
 }
 
-// Scratch of the brick-by-brick 3D projection (complex64), undefined when the plain kernels are the better choice.
+// Scratch of the brick-by-brick projection (complex64), undefined when the plain kernels are the better choice.
 Tensor project_workspace(int dim, const Tensor& rec, int64_t P, int64_t N, int interp, bool records, double oversampling, double cutoff) {
     if (is_f64(rec)) return Tensor();
     const size_t bytes = b200proj_project_workspace_bytes(dim, rec.size(0), P, N, interp, records ? 1 : 0, oversampling, cutoff);
     return bytes ? at::empty({(int64_t)bytes}, rec.options().dtype(at::kByte)) : Tensor();
 }
-// The same for the 3D scatters.
+// The same for the scatters.
 Tensor scatter_workspace(int dim, const Tensor& like, int64_t B, int64_t P, int64_t N, int interp, bool weights, double oversampling, double cutoff) {
-    if (dim != 3 || is_f64(like)) return Tensor();
-    const size_t bytes = b200proj_scatter_workspace_bytes(B, P, N, interp, weights ? 1 : 0, oversampling, cutoff);
+    if (is_f64(like)) return Tensor();
+    const size_t bytes = b200proj_scatter_workspace_bytes(dim, B, P, N, interp, weights ? 1 : 0, oversampling, cutoff);
     return bytes ? at::empty({(int64_t)bytes}, like.options().dtype(at::kByte)) : Tensor();
 }
 // The same for the backward passes of the projection.

@@ -101,7 +101,7 @@ def load() -> C.CDLL:
     lib.b200proj_rec_boxsize.restype = _i64
     lib.b200proj_rec_boxsize.argtypes = [_i64, _dbl]
     lib.b200proj_scatter_workspace_bytes.restype = C.c_size_t
-    lib.b200proj_scatter_workspace_bytes.argtypes = [_i64, _i64, _i64, _int, _int, _dbl, _dbl]
+    lib.b200proj_scatter_workspace_bytes.argtypes = [_int, _i64, _i64, _i64, _int, _int, _dbl, _dbl]
     lib.b200proj_backproject_workspace_bytes.restype = C.c_size_t
     lib.b200proj_backproject_workspace_bytes.argtypes = [_int, _i64, _i64, _i64, _i64, _int, _int]
     lib.b200proj_accumulator_bytes.restype = C.c_size_t
@@ -247,7 +247,7 @@ def backproject_accumulate(proj, weights, rot, shifts, interp, oversampling, cut
     B, P, N = proj.shape[0], proj.shape[1], proj.shape[2]
     geom = _geom(B, R, rot, shifts, P, N, interp, oversampling, cutoff)
     if interp == CUBIC:          # large cubic chunks run brick by brick, with scratch
-        n = int(load().b200proj_scatter_workspace_bytes(B, P, N, interp, 1, float(oversampling), float(cutoff)))
+        n = int(load().b200proj_scatter_workspace_bytes(3, B, P, N, interp, 1, float(oversampling), float(cutoff)))
         if n:
             workspace = torch.empty(n, dtype=torch.uint8, device=proj.device)
             _call("b200proj_backproject_2d_to_3d_accumulate_ws", proj, _p(proj), _p(weights), *geom, _p(accumulator), _p(workspace), n)
