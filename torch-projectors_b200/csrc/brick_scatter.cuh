@@ -80,9 +80,11 @@ struct ScatterSizes;
 template <> struct ScatterSizes<3, false> { static constexpr int kX = 13, kY = 13, kSlab = 4, kSlabs = 6, kWalkers = 6, kBlocks = 2, kRing = 4; };
 template <> struct ScatterSizes<3, true> { static constexpr int kX = 13, kY = 13, kSlab = 4, kSlabs = 4, kWalkers = 6, kBlocks = 2, kRing = 4; };
 
-// 2D: kSlabs counts adding warps, each with two copies of the tile's sums (kSlab = 0).
+// 2D: kSlabs counts adding warps, each with two copies of the tile's sums (kSlab = 0).  A pixel has 16 taps there, so the
+// walk weighs more: 27 M pixels of box 128, gradient, 5 + 7 warps 0.73 ms, 4 + 8 0.79, 6 + 6 0.87; weighted 4 + 8 0.97, 5 + 7 on
+// smaller tiles 0.92 (but 1.27 against 0.98 for box 32), 6 + 6 1.02.
 template <> struct ScatterSizes<2, false> { static constexpr int kX = 29, kY = 29, kSlab = 0, kSlabs = 5, kWalkers = 7, kBlocks = 2, kRing = 4; };
-template <> struct ScatterSizes<2, true> { static constexpr int kX = 21, kY = 21, kSlab = 0, kSlabs = 6, kWalkers = 6, kBlocks = 2, kRing = 4; };
+template <> struct ScatterSizes<2, true> { static constexpr int kX = 25, kY = 25, kSlab = 0, kSlabs = 4, kWalkers = 8, kBlocks = 2, kRing = 4; };
 
 template <int DIM, bool WEIGHTS>
 struct Scatter : ScatterSizes<DIM, WEIGHTS> {
