@@ -61,7 +61,7 @@ BACK_BYTES_PER_SLICE = 128 * 65 * 8 + 128 * 65 * 4 + 44 + 2 * (256 * 256 * 129 *
 # DRAM traffic per slice of the dominant kernels (dram__bytes_read.sum + dram__bytes_write.sum) from
 # ncu captures of a smaller launch of the same kernels, scaled by the slices a launch processes
 # (traffic grows in proportion to the slices: the volumes are touched the same way by every slice).
-PROJ_TRAFFIC_PER_SLICE = (48.87e6 + 105.01e6) / 2048      # profiles/project_forw_3d_cubic_box256_2048poses.md (current kernel)
+PROJ_TRAFFIC_PER_SLICE = (416.0e6 + 843.2e6) / 10000      # profiles/brick_kernels_b200.md (a brick writes parts of rows)
 # back-projection: two captures of the slab-ordered kernel (4,096 and 16,384 slices) give a part that grows with the
 # slices and a fixed part (the workspace); the fixed part also holds the zero-fill and the fold of the workspace
 # (profiles/backproject_forw_3d_linear_box256_4096slices.md)
@@ -69,7 +69,7 @@ BACK_TRAFFIC_PER_SLICE = (2506.4e6 - 730.7e6) / (16384 - 4096)
 BACK_TRAFFIC_FIXED = (730.7e6 - 4096 * BACK_TRAFFIC_PER_SLICE) + 135.3e6 + (135.3e6 + 44.2e6)
 # The ceilings the kernels actually sit on (from the same summaries): share of the L1TEX data pipe
 # the cubic gather keeps busy.
-PROJ_L1TEX_DATA_PIPE_FRAC = 0.909
+PROJ_L1TEX_DATA_PIPE_FRAC = 0.755
 
 
 def reduction_ceiling(taps, ms, pattern):
@@ -555,7 +555,7 @@ def autograd_step_workload(args):
             "warmup": args.warmup, "ms_per_step": ms_per_step, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
             "dtype": "f32", "data": "synthetic",
             "config": {"workload": STEP["name"], "l2": "inputs (539 MB volume, 1.08 GB projections) exceed L2; 256 MiB flush before every step"},
-            "kernels_ms": ({"project_forw_saving_kernel<3,cubic>": f, ("project_back_saved_kernel<3,cubic,rot,shift> (+ memsets)" if args.fixed_volume else "project_back_saved_kernel<3,cubic,rot,shift,rec> (+ memsets)"): bw,
+            "kernels_ms": ({"brick_forw_kernel<3,cubic,records> (+ setup)": f, ("pose_grad_saved_kernel" if args.fixed_volume else "brick_scatter_kernel<3> + pose_grad_saved_kernel (+ setup, clears)"): bw,
                             "loss and its gradient (torch elementwise)": ms_per_step - f - bw} if saving else
                            {"project_forw_kernel<3,cubic>": f, "project_back_kernel<3,cubic,rot,shift> (+ memsets)": bw,
                             "loss and its gradient (torch elementwise)": ms_per_step - f - bw}),
@@ -1120,16 +1120,16 @@ def main():
     clocks = sampler.stop()
     ms_per_step = max_over_ranks(sum(ms) / len(ms))
     value = world * PROJ["P"] / (ms_per_step * 1e-3)
-    kernel_ms = max_over_ranks(statistics.median(ms))       # one kernel launch per step
+    kernel_ms = max_over_ranks(statistics.median(ms))       # setup and gather
     achieved = PROJ_BYTES_PER_SLICE * PROJ["P"] / (kernel_ms * 1e-3) / 1e9
-    roofline = {"bound": "hbm", "kernel": "project_forw_kernel<3,cubic>", "achieved": achieved, "peak": peak,
+    roofline = {"bound": "hbm", "kernel": "brick_setup_kernel<3> + brick_forw_kernel<3,cubic>", "achieved": achieved, "peak": peak,
                 "peak_source": peak_kind, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": (PROJ_TRAFFIC_PER_SLICE * PROJ["P"]) if PROJ_TRAFFIC_PER_SLICE else None,
                 "algorithmic_bytes_per_launch": PROJ_BYTES_PER_SLICE * PROJ["P"], "launch_ms": kernel_ms,
-                "secondary": {"bound": "L1TEX data pipe (64 taps x 8 B per pixel, volume L2-resident)",
+                "secondary": {"bound": "L1TEX data pipe (64 taps x 8 B per pixel from shared memory)",
                               "frac": PROJ_L1TEX_DATA_PIPE_FRAC, "unit": "l1tex__data_pipe_lsu_wavefronts, fraction of peak",
                               "gather_taps_per_s": 6490 * 64 * PROJ["P"] / (kernel_ms * 1e-3),
-                              "peak_source": "ncu capture, profiles/project_forw_3d_cubic_box256_2048poses.md"}}
+                              "peak_source": "ncu capture, profiles/brick_kernels_b200.md"}}
     parity = None
     if rank == 0 and not args.skip_cpu:
         parity = check_projection_parity(out_holder["out"], rec, rot, shifts)
@@ -1168,10 +1168,10 @@ def main():
                   "pcie_gbs": (h2d + h_packed.numel() * 8) / (p_ms_per_step * 1e-3) / 1e9,
                   "note": f"{n_inside} of {PROJ['N'] * (PROJ['N'] // 2 + 1)} pixels per slice lie inside the cutoff and are copied"}
     del h_packed
-    # kernels of this package launched so far: one per device-resident step, one per 1000-pose
-    # chunk in every end-to-end step (warm-ups included)
+    # kernels of this package launched so far: two (setup, gather) per device-resident step, at least one per
+    # 1000-pose chunk in every end-to-end step (warm-ups included)
     e2e_chunks = (PROJ["P"] + 999) // 1000
-    launches = args.steps + args.warmup + (len(e2e_ms) + 3) * e2e_chunks + (len(p_ms) + 3) * e2e_chunks
+    launches = 2 * (args.steps + args.warmup) + (len(e2e_ms) + 3) * e2e_chunks + (len(p_ms) + 3) * e2e_chunks
     del h_out, out_holder
     torch.cuda.empty_cache()
 
