@@ -125,6 +125,15 @@ def test_accumulator_and_prep_entries_validate_without_a_device():
     assert lib.b200proj_ifftshift_crop(1, 1, 2, 16, 20, 1, 0) == -1
 
 
+def test_misaligned_records_are_refused_without_a_device():
+    """The backward pass reads records in 16-byte loads: a pointer off that grid is an error, not a device fault."""
+    lib = _abi.load()
+    rc = lib.b200proj_project_3d_to_2d_back_records(16, 16, 24, 1, 16, 16, 1, 0, 0, 1, 8, 0, 2.0, 4.0, 0, 16, 0, 0, 0, 0, 0)
+    assert rc == -1 and "16-byte aligned" in lib.b200proj_last_error().decode()
+    rc = lib.b200proj_project_3d_to_2d_forw_records(16, 1, 16, 16, 1, 0, 0, 1, 8, 0, 2.0, 4.0, 16, 48, 0, 0, 0, 0)
+    assert rc == -1 and "32-byte aligned" in lib.b200proj_last_error().decode()
+
+
 def test_header_is_plain_c(tmp_path):
     """The boundary is a C ABI: the header compiles as C99 with no torch, CUDA or C++ in sight."""
     import shutil

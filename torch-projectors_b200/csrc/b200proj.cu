@@ -305,6 +305,13 @@ BrickLaunch scatter_plan(int dim, int64_t B, int64_t P, int64_t N, bool cubic, b
     return L;
 }
 
+// Scratch a call can use: 16-byte aligned and, for the brick kernels, large enough.  What is not is left alone and the
+// plain kernels run.
+bool scratch_aligned(const void* workspace) { return workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0; }
+bool runs_in(const BrickLaunch& L, const void* workspace, size_t workspace_bytes) {
+    return L.use && scratch_aligned(workspace) && workspace_bytes >= L.bytes;
+}
+
 BrickWork brick_work(const BrickLaunch& L, void* workspace) {
     BrickWork w;
     w.header = (int*)workspace;
@@ -352,7 +359,7 @@ int launch_brick_scatter(const Launch& L, const BrickLaunch& bl, void* workspace
 // Copies of a small complex reconstruction over which the slices of a scatter are spread (see workspace_replicas):
 // as many as the rule wants and the workspace holds; sets the kernels' geometry.
 int scatter_copies(Launch& L, const void* workspace, size_t workspace_bytes) {
-    if (workspace == nullptr || (reinterpret_cast<uintptr_t>(workspace) & 15u) != 0) return 1;
+    if (!scratch_aligned(workspace)) return 1;
     const size_t one = L.rec_count * sizeof(float2);
     int copies = workspace_replicas((double)one, L.P);
     while (copies > 1 && (size_t)copies * one > workspace_bytes) copies /= 2;
@@ -380,7 +387,7 @@ int project_forw(const Real* rec, int64_t B, int64_t R, const Real* rot, int64_t
     cudaStream_t s = (cudaStream_t)stream;
     if constexpr (std::is_same<Real, float>::value) {
         const BrickLaunch bl = workspace != nullptr ? gather_plan(DIM, B, P, N, interpolation == B200PROJ_CUBIC, false, os, cutoff) : BrickLaunch{};
-        if (bl.use && workspace_bytes >= bl.bytes) {
+        if (runs_in(bl, workspace, workspace_bytes)) {
             if (interpolation == B200PROJ_CUBIC) return launch_brick_forw<DIM, true, false>(L, bl, workspace, rec, rot, shifts, out, nullptr, s);
             if constexpr (DIM == 3) return launch_brick_forw<3, false, false>(L, bl, workspace, rec, rot, shifts, out, nullptr, s);
         }
@@ -452,7 +459,7 @@ int project_forw_saving(const float* rec, int64_t B, int64_t R, const float* rot
     if (RECORDS && (reinterpret_cast<uintptr_t>(derivatives) & 31u) != 0) return fail(B200PROJ_ERR_ARGUMENT, "records must be 32-byte aligned");
     if constexpr (RECORDS || DIM == 2) {
         const BrickLaunch bl = workspace != nullptr ? gather_plan(DIM, B, P, N, interpolation == B200PROJ_CUBIC, true, os, cutoff) : BrickLaunch{};
-        if (bl.use && workspace_bytes >= bl.bytes) {
+        if (runs_in(bl, workspace, workspace_bytes)) {
             if (interpolation == B200PROJ_CUBIC) return launch_brick_forw<DIM, true, true>(L, bl, workspace, rec, rot, shifts, out, derivatives, s);
             if constexpr (DIM == 3) return launch_brick_forw<3, false, true>(L, bl, workspace, rec, rot, shifts, out, derivatives, s);
         }
@@ -476,12 +483,13 @@ int project_back_saved(const float* grad_proj, const float* out, const float* de
     if (grad_rot != nullptr && derivatives == nullptr) return fail(B200PROJ_ERR_ARGUMENT, "grad_rotations requested but no saved derivatives given");
     if (grad_shifts != nullptr && (shifts == nullptr || out == nullptr))
         return fail(B200PROJ_ERR_ARGUMENT, "grad_shifts requested but no shifts / saved projections given");
+    if (RECORDS && (reinterpret_cast<uintptr_t>(derivatives) & 15u) != 0) return fail(B200PROJ_ERR_ARGUMENT, "records must be 16-byte aligned");
     if (grad_rec == nullptr && grad_rot == nullptr && grad_shifts == nullptr) return B200PROJ_OK;
     cudaStream_t s = (cudaStream_t)stream;
     const bool cubic = interpolation == B200PROJ_CUBIC;
     BrickLaunch bl{};
     if ((RECORDS || DIM == 2) && P > 0 && grad_rec != nullptr && workspace != nullptr) bl = scatter_plan(DIM, B, P, N, cubic, false, os, cutoff);
-    if (workspace_bytes < bl.bytes) bl.use = false;
+    bl.use = runs_in(bl, workspace, workspace_bytes);
     const int copies = P > 0 && grad_rec != nullptr && !bl.use ? scatter_copies(L, workspace, workspace_bytes) : 1;
     if (int rc = zero_outputs(s, copies > 1 ? nullptr : grad_rec, L.rec_count * sizeof(float2), grad_rot, (size_t)B_rot * P * DIM * DIM * sizeof(float),
                               grad_shifts, (size_t)(shifts ? B_shift : 0) * P * 2 * sizeof(float))) return rc;
@@ -524,7 +532,7 @@ int project_back(const Real* grad_proj, const Real* rec, int64_t B, int64_t R, c
     BrickLaunch bl{};
     if (std::is_same<Real, float>::value && P > 0 && grad_rot == nullptr && grad_shifts == nullptr && workspace != nullptr)
         bl = scatter_plan(DIM, B, P, N, interpolation == B200PROJ_CUBIC, false, os, cutoff);
-    if (workspace_bytes < bl.bytes) bl.use = false;
+    bl.use = runs_in(bl, workspace, workspace_bytes);
     const int copies = P > 0 && std::is_same<Real, float>::value && !bl.use ? scatter_copies(L, workspace, workspace_bytes) : 1;
     if (int rc = zero_outputs(s, copies > 1 ? nullptr : grad_rec, L.rec_count * sizeof(C2<Real>), grad_rot, (size_t)B_rot * P * DIM * DIM * sizeof(Real),
                               grad_shifts, (size_t)(shifts ? B_shift : 0) * P * 2 * sizeof(Real))) return rc;
@@ -563,7 +571,7 @@ int backproject_forw(const Real* proj, const Real* weights, int64_t B, int64_t R
     const size_t ws_one = L.rec_count * sizeof(float4);
     if constexpr (std::is_same<Real, float>::value) {
         const BrickLaunch bl = P > 0 && workspace != nullptr ? scatter_plan(DIM, B, P, N, cubic, hw, os, cutoff) : BrickLaunch{};
-        if (bl.use && workspace_bytes >= bl.bytes && (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0) {
+        if (runs_in(bl, workspace, workspace_bytes)) {
             if (!accumulate) {
                 if (int rc = zero_outputs(s, data_rec, L.rec_count * sizeof(C2<Real>), weight_rec, L.rec_count * sizeof(Real))) return rc;
             }
@@ -573,8 +581,7 @@ int backproject_forw(const Real* proj, const Real* weights, int64_t B, int64_t R
     }
     constexpr bool kIsF32 = std::is_same<Real, float>::value;  // workspace and slab paths exist in fp32 only
     if constexpr (kIsF32) {
-    if (hw && P > 0 && !(DIM == 3 && slab_plan(R, hw).slabs > 1) && workspace != nullptr && workspace_bytes >= ws_one &&
-        (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0) {
+    if (hw && P > 0 && !(DIM == 3 && slab_plan(R, hw).slabs > 1) && scratch_aligned(workspace) && workspace_bytes >= ws_one) {
         // small reconstructions: as many copies as the rule wants and the workspace holds
         int replicas = workspace_replicas((double)ws_one, P);
         while (replicas > 1 && (size_t)replicas * ws_one > workspace_bytes) replicas /= 2;
@@ -709,7 +716,7 @@ int backproject_accumulate(const float* proj, const float* weights, int64_t B, i
     const bool cubic = interpolation == B200PROJ_CUBIC;
     if (workspace != nullptr && slab_count == plan.slabs) {
         const BrickLaunch bl = scatter_plan(3, B, P, N, cubic, true, os, cutoff);
-        if (bl.use && workspace_bytes >= bl.bytes) return launch_brick_scatter<3, true, true, true>(L, bl, workspace, proj, weights, rot, shifts, nullptr, nullptr, s, acc);
+        if (runs_in(bl, workspace, workspace_bytes)) return launch_brick_scatter<3, true, true, true>(L, bl, workspace, proj, weights, rot, shifts, nullptr, nullptr, s, acc);
     }
     if (plan.slabs > 1) {
         launch_slab_interleaved(L, s, cubic, proj, weights, rot, shifts, acc, plan, slab_first, slab_count);

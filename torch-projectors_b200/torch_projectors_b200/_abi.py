@@ -50,12 +50,23 @@ SIGNATURES["b200proj_project_2d_back_saved"] = [_ptr, _ptr, _ptr] + _COMMON + [_
 SIGNATURES["b200proj_project_3d_to_2d_forw_saving"] = [_ptr] + _COMMON + [_ptr, _ptr, _ptr, _ptr]
 SIGNATURES["b200proj_project_3d_to_2d_back_saved"] = [_ptr, _ptr, _ptr] + _COMMON + [_ptr, _ptr, _ptr, _ptr, _ptr]
 SIGNATURES["b200proj_project_3d_to_2d_forw_packed"] = [_ptr] + _COMMON + [_ptr, _ptr, _i64, _ptr, _ptr]
+# the operators with scratch (workspace pointer and bytes before the stream), fp32
+_WS = [_ptr, C.c_size_t, _ptr]
+SIGNATURES["b200proj_project_2d_forw_ws"] = [_ptr] + _COMMON + [_ptr] + _WS
+SIGNATURES["b200proj_project_2d_forw_saving_ws"] = [_ptr] + _COMMON + [_ptr, _ptr] + _WS
+SIGNATURES["b200proj_project_3d_to_2d_forw_ws"] = [_ptr] + _COMMON + [_ptr, _ptr] + _WS
+SIGNATURES["b200proj_project_3d_to_2d_forw_records"] = [_ptr] + _COMMON + [_ptr, _ptr, _ptr] + _WS
+SIGNATURES["b200proj_project_2d_back_ws"] = [_ptr, _ptr] + _COMMON + [_ptr, _ptr, _ptr] + _WS
+SIGNATURES["b200proj_project_2d_back_saved_ws"] = [_ptr, _ptr, _ptr] + _COMMON + [_ptr, _ptr, _ptr] + _WS
+SIGNATURES["b200proj_project_3d_to_2d_back_ws"] = [_ptr, _ptr] + _COMMON + [_ptr, _ptr, _ptr, _ptr] + _WS
+SIGNATURES["b200proj_project_3d_to_2d_back_records"] = [_ptr, _ptr, _ptr] + _COMMON + [_ptr, _ptr, _ptr, _ptr] + _WS
 SIGNATURES["b200proj_reduction_rate_probe"] = [_int, _ptr, C.c_size_t, _int, _int, _ptr]
 SIGNATURES["b200proj_reduction_rate_probe_streaming"] = [_ptr, C.c_size_t, C.c_size_t, _ptr, C.c_size_t, _int, _int, _int, _ptr]
 SIGNATURES["b200proj_backproject_2d_to_3d_accumulate_slabs"] = [_ptr, _ptr] + _COMMON + [_ptr, _int, _int, _ptr]
 EXPORTS = list(SIGNATURES) + ["b200proj_version", "b200proj_last_error", "b200proj_rec_boxsize",
                                 "b200proj_backproject_workspace_bytes", "b200proj_accumulator_bytes",
                                 "b200proj_source_stamp", "b200proj_accumulator_slab_plan", "b200proj_scatter_workspace_bytes",
+                                "b200proj_project_workspace_bytes", "b200proj_gradient_workspace_bytes",
                                 "b200proj_accumulator_slab_voxels", "b200proj_debug_index", "b200proj_cutoff_pack_index"]
 
 _lib: Optional[C.CDLL] = None
@@ -102,6 +113,10 @@ def load() -> C.CDLL:
     lib.b200proj_rec_boxsize.argtypes = [_i64, _dbl]
     lib.b200proj_scatter_workspace_bytes.restype = C.c_size_t
     lib.b200proj_scatter_workspace_bytes.argtypes = [_int, _i64, _i64, _i64, _int, _int, _dbl, _dbl]
+    lib.b200proj_project_workspace_bytes.restype = C.c_size_t
+    lib.b200proj_project_workspace_bytes.argtypes = [_int, _i64, _i64, _i64, _int, _int, _dbl, _dbl]
+    lib.b200proj_gradient_workspace_bytes.restype = C.c_size_t
+    lib.b200proj_gradient_workspace_bytes.argtypes = [_int, _i64, _i64, _i64, _i64, _int, _int, _dbl, _dbl]
     lib.b200proj_backproject_workspace_bytes.restype = C.c_size_t
     lib.b200proj_backproject_workspace_bytes.argtypes = [_int, _i64, _i64, _i64, _i64, _int, _int]
     lib.b200proj_accumulator_bytes.restype = C.c_size_t
