@@ -104,7 +104,9 @@ size_t b200proj_project_workspace_bytes(int dim, int64_t B, int64_t P, int64_t N
                                         double oversampling, double fourier_radius_cutoff);
 /* The same for the scatters (b200proj_project_3d_to_2d_back_records and _back_ws with
  * grad_rec, b200proj_backproject_2d_to_3d_accumulate_ws, b200proj_backproject_{2d,2d_to_3d}_forw; 0: no gain, for
- * the last of them see there for what else a workspace is good for). */
+ * the last of them see there for what else a workspace is good for).  These kernels' warps hand pixels to one another
+ * and wait in doing so, for no longer than some seconds: should a wait ever run out, the parts of the result that lack
+ * sums are NaN and the fourth int of the workspace is 1 (else 0) when the call's work has run. */
 size_t b200proj_scatter_workspace_bytes(int dim, int64_t B, int64_t P, int64_t N, int interpolation, int has_weights,
                                         double oversampling, double fourier_radius_cutoff);
 /* Workspace of the backward passes of the projection (b200proj_project_{2d,3d_to_2d}_back_ws with grad_rec,

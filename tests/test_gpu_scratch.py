@@ -70,3 +70,33 @@ def test_unusable_scratch_is_left_alone():
     r = subprocess.run([sys.executable, "-c", f"import sys; sys.path[:0] = [{str(ROOT / 'tests')!r}, {str(ROOT / 'torch-projectors_b200')!r}, {str(ROOT)!r}]; import test_gpu_scratch as t; t.check()"],
                        env=env, cwd=ROOT, capture_output=True, text=True, timeout=600)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]
+
+
+def check_waits():
+    """In a fresh process, bricks on and a wait that gives up at its first look: what is lost shows as NaN and in the status word."""
+    import torch_projectors_b200 as tp
+    abi, lib = tp._abi, tp._abi.load()
+    for dim in (2, 3):
+        t = {k: v.cuda() for k, v in make_inputs(Case("waits", dim, "cubic", 1, 300, N, R, OS, None, 1, 1, seed=dim)).items()}
+        geom = abi._geom(1, R, t["rot"], t["shifts"], 300, N, abi.CUBIC, OS, N / 2.0)
+        for weights in (0, 1):
+            n = lib.b200proj_scatter_workspace_bytes(dim, 1, 300, N, abi.CUBIC, weights, OS, N / 2.0)
+            ws = torch.zeros(n, dtype=torch.uint8, device="cuda")
+            data, wrec = torch.zeros_like(t["rec"]), torch.zeros_like(t["rec"].real.contiguous())
+            abi._call("b200proj_backproject_2d_forw" if dim == 2 else "b200proj_backproject_2d_to_3d_forw", t["proj"], t["proj"].data_ptr(),
+                      t["weights"].data_ptr() if weights else 0, *geom, data.data_ptr(), wrec.data_ptr() if weights else 0, 0, ws.data_ptr(), n)
+            torch.cuda.synchronize()
+            assert ws[:16].view(torch.int32)[3] == 1
+            assert torch.isnan(data.real).any() and (not weights or torch.isnan(wrec).any())
+        project = tp.project_3d_to_2d_forw if dim == 3 else tp.project_2d_forw
+        rec = t["rec"].requires_grad_(True)
+        project(rec, t["rot"], t["shifts"], output_shape=(N, N), interpolation="cubic", oversampling=OS).backward(t["proj"])
+        assert torch.isnan(rec.grad.real).any()
+
+
+def test_a_wait_that_gives_up_shows_in_the_result():
+    """With no patience the adding warps' first look at an empty ring ends their wait (the kernel returns by itself)."""
+    env = dict(os.environ, B200PROJ_BRICKS="1", B200PROJ_BRICK_WAIT_MS="0")
+    r = subprocess.run([sys.executable, "-c", f"import sys; sys.path[:0] = [{str(ROOT / 'tests')!r}, {str(ROOT / 'torch-projectors_b200')!r}, {str(ROOT)!r}]; import test_gpu_scratch as t; t.check_waits()"],
+                       env=env, cwd=ROOT, capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]

@@ -253,6 +253,8 @@ BrickLaunch brick_layout(int64_t B, int64_t P, int64_t N, double os, double cuto
     L.plan.per_slice = (float)pixels_inside(N, cutoff);
     // the estimate counts bricks that stick out of the ball in full, and a few large ones may each count the whole slice
     L.plan.max_extra = (int)((L.bricks < 64 ? (double)L.bricks : 4.0) * pixels / target) + 64;
+    static const int wait_ms = [] { const char* e = getenv("B200PROJ_BRICK_WAIT_MS"); return e ? atoi(e) : 10000; }();   // for tests
+    L.plan.wait_ms = wait_ms < 0 ? 0 : wait_ms;
     L.items = (size_t)(L.bricks * B) + (size_t)L.plan.max_extra;
     L.item_bytes = (L.items * sizeof(int4) + 255) & ~(size_t)255;
     L.rec_bytes = (size_t)(B * P) * 3 * sizeof(float4);

@@ -48,9 +48,11 @@ struct BrickPlan {
     float per_slice;        // pixels of a slice inside the cutoff
     float target;           // pixels a work item should hold
     int max_extra;          // items beyond one per brick that fit the list
+    int wait_ms;            // after which a scatter's wait gives up
 };
 
-// Workspace layout: int header[4] {items, extra, ticket, pixels outside the cutoff}, int4 items[bricks * B + max_extra],
+// Workspace layout: int header[4] {items, extra, ticket, gathers: pixels outside the cutoff, scatters: 1 when a wait gave
+// up}, int4 items[bricks * B + max_extra],
 // float4 records[3 * B * P], int outside[N * Nh].
 struct BrickWork {
     int* header;

@@ -51,26 +51,47 @@ __device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned coun
 __device__ __forceinline__ void mbar_arrive(unsigned long long* bar, unsigned count) {
     asm volatile("{ .reg .b64 state; mbarrier.arrive.shared::cta.b64 state, [%0], %1; }" ::"r"(smem_addr(bar)), "r"(count) : "memory");
 }
-// Wait for the phase of the given parity.  Every wait ends by construction (see brick_scatter_kernel); should one not,
-// it gives up after some seconds, and all later ones at once, so that the kernel returns.
-__device__ __forceinline__ void mbar_wait(unsigned long long* bar, unsigned parity, int* gave_up) {
-    for (int tries = 0; tries < (1 << 22); ++tries) {
+// Every wait ends by construction (see brick_scatter_kernel).  Should one not, it gives up: the block then writes NaN
+// into the bricks that it could not finish, so that the loss shows in the result, and the kernel returns.  The limit is
+// time spent polling; a gap between two polls counts 1 ms at most (a block that was not running loses no patience).
+struct Patience {
+    unsigned long long last = 0ull, spent = 0ull, limit;
+    __device__ explicit Patience(int ms) : limit((unsigned long long)ms * 1000000ull) {}
+    __device__ __forceinline__ bool over() {
+        unsigned long long now;
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
+        if (last != 0ull) spent += min(now - last, 1000000ull);
+        last = now;
+        return spent >= limit;
+    }
+};
+// Wait for the phase of the given parity; false: given up, by this wait or another of the block.
+__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity, int* gave_up, int limit_ms) {
+    Patience patience(limit_ms);
+    while (true) {
         unsigned ready;
         asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
                      : "=r"(ready) : "r"(smem_addr(bar)), "r"(parity) : "memory");
-        if (ready) return;
-        if ((tries & 1023) == 1023 && *(volatile int*)gave_up) return;
+        if (ready) return true;
+        if (*(volatile int*)gave_up) return false;
+        if (patience.over()) {
+            *(volatile int*)gave_up = 1;
+            return false;
+        }
     }
-    *(volatile int*)gave_up = 1;
 }
 // Wait until *count exceeds `below`, likewise.
-__device__ __forceinline__ void count_wait(const int* count, int below, int* gave_up) {
-    for (int tries = 0; tries < (1 << 24); ++tries) {
-        if (*(const volatile int*)count > below) return;
+__device__ __forceinline__ bool count_wait(const int* count, int below, int* gave_up, int limit_ms) {
+    Patience patience(limit_ms);
+    while (*(const volatile int*)count <= below) {
+        if (*(volatile int*)gave_up) return false;
+        if (patience.over()) {
+            *(volatile int*)gave_up = 1;
+            return false;
+        }
         __nanosleep(32);
-        if ((tries & 1023) == 1023 && *(volatile int*)gave_up) return;
     }
-    *(volatile int*)gave_up = 1;
+    return true;
 }
 
 // ---- sizes --------------------------------------------------------------------------------------------------
@@ -230,10 +251,10 @@ __device__ __forceinline__ void brick_add(typename Scatter<3, WEIGHTS>::Slab& sb
 
 // Sums of a finished item to the volume, by the scatter's rules (Friedel mirror with conjugation, taps outside the
 // stored half-volume dropped, DUP: the conjugate also to the Friedel partner of a voxel on the c == 0 plane); cleared
-// for the next item.  INTERLEAVED: into 16-byte (re, im, weight, 0) voxels.
+// for the next item.  INTERLEAVED: into 16-byte (re, im, weight, 0) voxels.  LOST: sums of the item are missing; NaN.
 template <int DIM, bool WEIGHTS, bool DUP, bool INTERLEAVED>
 __device__ __forceinline__ void brick_flush(const SliceGeom& g, typename Scatter<DIM, WEIGHTS>::Shared& sh, float2* __restrict__ vol, float* __restrict__ wvol,
-                                            float4* __restrict__ accum, int X0, int Y0, int Z0) {
+                                            float4* __restrict__ accum, int X0, int Y0, int Z0, bool lost) {
     using C = Scatter<DIM, WEIGHTS>;
     auto add = [&](int off, float re, float im, float w) {
         if (INTERLEAVED) {
@@ -269,6 +290,7 @@ __device__ __forceinline__ void brick_flush(const SliceGeom& g, typename Scatter
                 take(sh.slab[s], C::place(x, y, 1));
             }
         }
+        if (lost) v.x = v.y = w = __int_as_float(0x7fffffff);
         if (v.x == 0.f && v.y == 0.f && w == 0.f) continue;
         bool m;
         const int c = scatter_col(g, X0 - 1 + x, m), r = scatter_line(g, Y0 - 1 + y, m), d = DIM == 3 ? scatter_line(g, Z0 - 1 + z, m) : 0;
@@ -305,6 +327,7 @@ brick_scatter_kernel(const float2* __restrict__ proj, const float* __restrict__ 
     int slot = 0, taken = 0;                                // adding warps: next chunk of the ring, its parity, chunks taken
     unsigned parity = 0;
     const int items = __ldg(ws.header);
+    bool lost = false;                                      // a wait of this block gave up: its rings are of no use any more
     while (true) {
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -339,7 +362,7 @@ brick_scatter_kernel(const float2* __restrict__ proj, const float* __restrict__ 
         }
         const int4 it = __ldg(ws.items + item);
         const int X0 = pl.lo[0] + (it.x & 1023) * C::Brick::x, Y0 = pl.lo[1] + ((it.x >> 10) & 1023) * C::Brick::y, Z0 = pl.lo[2] + (it.x >> 20) * C::Brick::z;
-        if (warp < C::kWalkers) {
+        if (!lost && warp < C::kWalkers) {
             const BrickWarp& sw = sh.walk[warp].warp[0];
             // places [first, first + n) of a ring are written: its chunks count them
             auto arrive = [&](typename C::Ring& q, int first, int n) {
@@ -380,8 +403,8 @@ brick_scatter_kernel(const float2* __restrict__ proj, const float* __restrict__ 
                     if (n > 0) arrive(sh.ring[lane], first, n);
                     return;
                 }
-                unsigned left = __ballot_sync(kFull, n > 0);
-                for (int tries = 0; left != 0u && tries < (1 << 24); ++tries) {
+                Patience patience(pl.wait_ms);
+                for (unsigned left = __ballot_sync(kFull, n > 0); left != 0u;) {
                     const bool now = (left >> lane & 1u) != 0u && *(volatile int*)&sh.ring[lane].taken > ((first + n - 1) >> 5) - C::kRing;
                     const unsigned ready = __ballot_sync(kFull, now);
                     if (mine && (ready >> h_slab & 1u) != 0u) write(q, place, h_a, h_v, h_w);
@@ -389,11 +412,11 @@ brick_scatter_kernel(const float2* __restrict__ proj, const float* __restrict__ 
                     if (now) arrive(sh.ring[lane], first, n);
                     left &= ~ready;
                     if (ready == 0u) {
-                        __nanosleep(64);
+                        if (patience.over()) *(volatile int*)&sh.gave_up = 1;
                         if (__any_sync(kFull, *(volatile int*)&sh.gave_up != 0)) return;
+                        __nanosleep(64);
                     }
                 }
-                if (left != 0u) *(volatile int*)&sh.gave_up = 1;
             };
             brick_walk<typename C::Brick>(g, ws.recs, sh.walk[warp], X0, Y0, Z0, it.z, it.w, warp, C::kWalkers,
                                           [&](bool active, int slot_, int i, int j, const Pixel& px, int lx, int ly, int lz) {
@@ -433,18 +456,18 @@ brick_scatter_kernel(const float2* __restrict__ proj, const float* __restrict__ 
                     const int first = *(volatile int*)&q.tail, n = 32 - (first & 31);
                     __syncwarp();
                     if (lane == 0) *(volatile int*)&q.tail = first + n;
-                    count_wait(&q.taken, (first >> 5) - C::kRing, &sh.gave_up);
+                    if (!__all_sync(kFull, count_wait(&q.taken, (first >> 5) - C::kRing, &sh.gave_up, pl.wait_ms))) break;
                     if (lane < n) write(q, first + lane, make_float4(0.f, 0.f, 0.f, __uint_as_float(lane == n - 1 ? kItemEnds : 0u)), make_float2(0.f, 0.f), 0.f);
                     __syncwarp();
                     if (lane == 0) arrive(q, first, n);
                 }
             }
-        } else {
+        } else if (!lost) {
             typename C::Ring& q = sh.ring[warp - C::kWalkers];
             typename C::Slab& sb = sh.slab[warp - C::kWalkers];
             bool ends = false;
-            while (!ends && *(volatile int*)&sh.gave_up == 0) {
-                mbar_wait(&q.full[slot], parity, &sh.gave_up);
+            while (!ends) {
+                if (!__all_sync(kFull, mbar_wait(&q.full[slot], parity, &sh.gave_up, pl.wait_ms))) break;
                 const float4 a = q.a[slot * 32 + lane];
                 const float2 v = q.v[slot * 32 + lane];
                 const float w = WEIGHTS ? q.w[slot * 32 + lane] : 0.f;
@@ -460,12 +483,12 @@ brick_scatter_kernel(const float2* __restrict__ proj, const float* __restrict__ 
             }
         }
         __syncthreads();
-        if (sh.gave_up) break;
+        lost = sh.gave_up != 0;
         const size_t at = (size_t)it.y * g.vol_elems;
         brick_flush<DIM, WEIGHTS, DUP, INTERLEAVED>(g, sh, INTERLEAVED ? nullptr : vol + at, WEIGHTS && !INTERLEAVED ? wvol + at : nullptr,
-                                                      INTERLEAVED ? accum + at : nullptr, X0, Y0, Z0);
+                                                      INTERLEAVED ? accum + at : nullptr, X0, Y0, Z0, lost);
     }
-    if (threadIdx.x == 0 && sh.gave_up) ws.header[3] = 1;       // never, see above
+    if (threadIdx.x == 0 && lost) ws.header[3] = 1;
 }
 
 }  // namespace b200proj
