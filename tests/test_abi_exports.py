@@ -134,6 +134,13 @@ def test_misaligned_records_are_refused_without_a_device():
     assert rc == -1 and "32-byte aligned" in lib.b200proj_last_error().decode()
 
 
+def test_operator_layer_shares_libstdcxx_with_libtorch():
+    """With a copy of its own, an operator's error message with a number in it crashes the process."""
+    from torch_projectors_b200 import build
+    data = build.BINDING_PATH.read_bytes()
+    assert b"\0libstdc++.so.6\0" in data, "libstdc++.so.6 is not among the libraries it needs"
+
+
 def test_header_is_plain_c(tmp_path):
     """The boundary is a C ABI: the header compiles as C99 with no torch, CUDA or C++ in sight."""
     import shutil

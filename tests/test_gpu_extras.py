@@ -342,3 +342,14 @@ def test_small_reconstructions_spread_over_workspace_copies(tp, dim, interp, B, 
     fn = tp.backproject_2d_to_3d_forw if dim == 3 else tp.backproject_2d_forw
     d, w = fn(g["proj"], g["rot"], weights=g["weights"], shifts=g["shifts"], interpolation=interp, oversampling=2.0)
     assert rel_err(d, d_want) <= TOL_ATOMIC and rel_err(w, w_want) <= TOL_ATOMIC
+
+
+def test_errors_with_numbers_in_their_text_are_raised(tp):
+    ops = torch.ops.torch_projectors_b200
+    rec, rot = torch.zeros(1, 16, 16, 9, dtype=torch.complex64, device="cuda"), torch.eye(3, device="cuda").repeat(1, 4, 1, 1)
+    with pytest.raises(RuntimeError, match=r"Rotations must be \(B_rot, P, 3, 3\)"):
+        ops.project_3d_to_2d_forw(rec, rot[..., :2], None, [16, 16], "cubic", 1.0, None)
+    with pytest.raises(RuntimeError, match="projection boxsize 2050 exceeds 2048"):
+        ops.project_3d_to_2d_forw(rec, rot[:, :1], None, [2050, 2050], "cubic", 1.0, None)
+    with pytest.raises(RuntimeError, match="of B\\*P = 4 entries"):
+        ops.project_3d_to_2d_forw_ordered(rec, rot, None, [16, 16], "cubic", 1.0, None, torch.zeros(7, dtype=torch.int32, device="cuda"))

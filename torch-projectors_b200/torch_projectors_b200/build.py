@@ -67,7 +67,18 @@ def source_stamp() -> str:
 
 def binding_stamp() -> str:
     import torch
-    return _stamp_of(BINDING_SOURCES + [INCLUDE_DIR / "b200proj.h"]) + "-torch" + torch.__version__
+    return _stamp_of(BINDING_SOURCES + [INCLUDE_DIR / "b200proj.h"]) + "-torch" + torch.__version__ + "-shared-libstdc++"
+
+
+def _libstdcxx_flags(cxx: str) -> list:
+    """Link flags for the libstdc++ that libtorch has loaded, for a compiler that comes with a static one only.  Two
+    copies of it in one process share some of their symbols and not others: an operator that puts a number into an
+    error message then crashes instead of raising it."""
+    found = subprocess.run([cxx, "-print-file-name=libstdc++.so"], capture_output=True, text=True, check=True).stdout.strip()
+    if os.path.isabs(found):
+        return []
+    loaded = [line.split()[-1] for line in open("/proc/self/maps") if "/libstdc++.so" in line]
+    return ["-nostdlib++", loaded[0], "-lm"] if loaded else []
 
 
 def _recorded(path: Path) -> str:
@@ -137,13 +148,14 @@ def build_binding(force: bool = False, verbose: bool = False) -> Path:
         stamp = binding_stamp()
         torch_lib = Path(torch.__file__).resolve().parent / "lib"
         cuda_home = Path(os.environ.get("CUDA_HOME") or "/usr/local/cuda")
-        cmd = [os.environ.get("CXX") or shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared",
+        cxx = os.environ.get("CXX") or shutil.which("g++") or "g++"
+        cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared",
                "-D_GLIBCXX_USE_CXX11_ABI=" + str(int(torch._C._GLIBCXX_USE_CXX11_ABI)),
                f"-I{INCLUDE_DIR}", f"-I{cuda_home / 'include'}"]
         cmd += [f"-I{p}" for p in cpp_extension.include_paths()]
         cmd += [str(s) for s in BINDING_SOURCES]
         cmd += [f"-L{PKG_DIR}", "-lb200proj", f"-L{torch_lib}", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",
-                "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib}"]
+                "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib}"] + _libstdcxx_flags(cxx)
         _run_into_place(cmd, BINDING_PATH, stamp, verbose)
     return BINDING_PATH
 
