@@ -144,3 +144,21 @@ def test_public_api_keeps_one_order_for_forward_and_backward(tp):
     finally:
         tp.set_save_derivatives(True)
     assert torch.equal(plain, out.detach())
+
+
+def test_a_wrong_order_is_refused_by_calls_that_do_not_need_one(tp):
+    """Large cubic calls run brick by brick and ignore the order; a wrong one is an error all the same."""
+    ops = torch.ops.torch_projectors_b200
+    rec, grad = torch.zeros(1, 64, 64, 33, dtype=torch.complex64, device="cuda"), torch.zeros(1, 2500, 64, 33, dtype=torch.complex64, device="cuda")
+    rot, sh = torch.eye(3, device="cuda").repeat(1, 2500, 1, 1), torch.zeros(1, 2500, 2, device="cuda")
+    assert tp._abi.load().b200proj_project_workspace_bytes(3, 1, 2500, 64, tp._abi.CUBIC, 0, 1.0, 32.0) > 0
+    out, der = ops.project_3d_to_2d_forw_saving(rec, rot, sh, [64, 64], "cubic", 1.0, None, None)
+    rot_g = rot.clone().requires_grad_(True)
+    for order in (torch.zeros(2500, dtype=torch.int64, device="cuda"), torch.zeros(7, dtype=torch.int32, device="cuda"), torch.zeros(2500, dtype=torch.int32)):
+        for call in (lambda: ops.project_3d_to_2d_forw_ordered(rec, rot, sh, [64, 64], "cubic", 1.0, None, order),
+                     lambda: ops.project_3d_to_2d_forw_saving(rec, rot, sh, [64, 64], "cubic", 1.0, None, order),
+                     lambda: ops.project_3d_to_2d_back_ordered(grad, rec, rot, sh, "cubic", 1.0, None, order),
+                     lambda: ops.project_3d_to_2d_back_saved(grad, out, der, rec, rot_g, sh, "cubic", 1.0, None, order, True),
+                     lambda: ops.project_3d_to_2d_back_saved(grad, out, der, rec, rot_g, sh, "cubic", 1.0, None, order, False)):
+            with pytest.raises(RuntimeError, match="pose_order must be an int32 CUDA tensor"):
+                call()

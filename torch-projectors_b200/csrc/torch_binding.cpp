@@ -139,8 +139,9 @@ Tensor plane_locality_order(const Tensor& rotations, int64_t batch) {
     return order;
 }
 
-// The order an operator uses: the caller's (checked), or one made here when the volume is large.
-Tensor resolve_order(int dim, const Tensor& vol, int64_t B, const Poses& p, const OptTensor& given) {
+// The order an operator uses: the caller's (checked), or one made here when the volume is large and the call's kernels
+// go slice by slice (`used`).
+Tensor resolve_order(int dim, const Tensor& vol, int64_t B, const Poses& p, const OptTensor& given, bool used = true) {
     if (dim != 3) return Tensor();
     if (given.has_value() && given->defined()) {
         const Tensor& o = *given;
@@ -149,7 +150,7 @@ Tensor resolve_order(int dim, const Tensor& vol, int64_t B, const Poses& p, cons
                     "pose_order must be an int32 CUDA tensor of B*P = ", B * p.P, " entries on the device of the data");
         return o.contiguous();
     }
-    if (p.P < g_order_min_poses.load() || vol[0].numel() * (int64_t)vol.element_size() < g_order_min_bytes.load()) return Tensor();
+    if (!used || p.P < g_order_min_poses.load() || vol[0].numel() * (int64_t)vol.element_size() < g_order_min_bytes.load()) return Tensor();
     return plane_locality_order(p.rot, B);
 }
 
@@ -194,7 +195,7 @@ Tensor project_forw(int dim, const Tensor& reconstruction, const Tensor& rotatio
     void* s = current_stream(rec);
     const double cut = cutoff_of(cutoff, N);
     const Tensor ws = project_workspace(dim, rec, p.P, N, interp, false, oversampling, cut);
-    Tensor order = ws.defined() ? Tensor() : resolve_order(dim, rec, B, p, pose_order);
+    Tensor order = resolve_order(dim, rec, B, p, pose_order, !ws.defined());
     int rc;
     if (is_f64(rec)) {
         rc = dim == 2 ? b200proj_project_2d_forw_f64(cptr<double>(rec), B, R, cptr<double>(p.rot), p.B_rot, cptr<double>(p.shifts), p.B_shift, p.P, N, interp, oversampling, cut, mptr<double>(out), s)
@@ -240,7 +241,7 @@ std::tuple<Tensor, Tensor, Tensor> project_back(int dim, const Tensor& grad_proj
         void* s = current_stream(rec);
         const double cut = cutoff_of(cutoff, N);
         const Tensor ws = gradient_workspace(dim, rec, B, R, p.P, N, interp, need_rot || need_shift, oversampling, cut);
-        Tensor order = ws.defined() ? Tensor() : resolve_order(dim, rec, B, p, pose_order);
+        Tensor order = resolve_order(dim, rec, B, p, pose_order, !ws.defined());
         int rc;
         if (is_f64(rec)) {
             rc = dim == 2 ? b200proj_project_2d_back_f64(cptr<double>(gp), cptr<double>(rec), B, R, cptr<double>(p.rot), p.B_rot, cptr<double>(p.shifts), p.B_shift, p.P, N, interp, oversampling, cut, mptr<double>(grad_rec), mptr<double>(grad_rot), mptr<double>(grad_sh), s)
@@ -299,7 +300,7 @@ std::tuple<Tensor, Tensor> project_forw_saving(int dim, const Tensor& reconstruc
     if (out.numel() == 0) return std::make_tuple(out, derivs);
     const double cut = cutoff_of(cutoff, N);
     const Tensor ws = project_workspace(dim, rec, p.P, N, interp, true, oversampling, cut);
-    Tensor order = ws.defined() ? Tensor() : resolve_order(dim, rec, B, p, pose_order);
+    Tensor order = resolve_order(dim, rec, B, p, pose_order, !ws.defined());
     const int rc = dim == 2
         ? b200proj_project_2d_forw_saving_ws(cptr<float>(rec), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts), p.B_shift, p.P, N, interp,
                                           oversampling, cut, mptr<float>(out), mptr<float>(derivs), ws_ptr(ws), ws_size(ws), current_stream(rec))
@@ -346,7 +347,7 @@ std::tuple<Tensor, Tensor, Tensor> project_back_saved(int dim, const Tensor& gra
     } else {
         const double cut = cutoff_of(cutoff, N);
         const Tensor ws = need_rec_grad ? gradient_workspace(dim, gp, B, R, p.P, N, interp, false, oversampling, cut) : Tensor();
-        Tensor order = ws.defined() ? Tensor() : resolve_order(dim, reconstruction, B, p, pose_order);
+        Tensor order = resolve_order(dim, reconstruction, B, p, pose_order, !ws.defined());
         const int rc = dim == 2
             ? b200proj_project_2d_back_saved_ws(cptr<float>(gp), cptr<float>(out), cptr<float>(der), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts),
                                              p.B_shift, p.P, N, interp, oversampling, cut, mptr<float>(grad_rec), mptr<float>(grad_rot), mptr<float>(grad_sh),
