@@ -353,3 +353,51 @@ def test_errors_with_numbers_in_their_text_are_raised(tp):
         ops.project_3d_to_2d_forw(rec, rot[:, :1], None, [2050, 2050], "cubic", 1.0, None)
     with pytest.raises(RuntimeError, match="of B\\*P = 4 entries"):
         ops.project_3d_to_2d_forw_ordered(rec, rot, None, [16, 16], "cubic", 1.0, None, torch.zeros(7, dtype=torch.int32, device="cuda"))
+
+
+@pytest.mark.parametrize("fixed_volume", [True, False])
+def test_saved_records_survive_copies_that_hooks_make_of_them(tp, fixed_volume):
+    """A hook on saved tensors may hand back a copy with the same strides in other memory; what lay between the elements
+    of the saved tensor is lost then (here: NaN).  The shift gradients must not depend on it."""
+    case = Case("hooks", 3, "cubic", 1, 9, 16, 32, 2.0, None, 1, 1, shift_range=3.0, seed=95)
+    t = {k: v.cuda() for k, v in make_inputs(case).items()}
+
+    def copy(x):
+        span = 1 + sum((n - 1) * s for n, s in zip(x.shape, x.stride()))
+        return torch.full((span + 3,), float("nan"), dtype=x.dtype, device=x.device).as_strided(x.shape, x.stride()).copy_(x)
+
+    grads = []
+    tp.set_save_derivatives(True, min_volume_bytes=0)
+    try:
+        for pack in (lambda x: x, copy, lambda x: x.cpu()):
+            sh, rot = t["shifts"].clone().requires_grad_(True), t["rot"].clone().requires_grad_(True)
+            rec = t["rec"].clone().requires_grad_(not fixed_volume)
+            with torch.autograd.graph.saved_tensors_hooks(pack, lambda x: x.cuda()):
+                out = tp.project_3d_to_2d_forw(rec, rot, sh, output_shape=(16, 16), interpolation="cubic", oversampling=2.0)
+                out.backward(t["proj"])
+            grads.append([g for g in (sh.grad, rot.grad, rec.grad) if g is not None])
+    finally:
+        tp.set_save_derivatives(True)
+    for other in grads[1:]:
+        for a, b in zip(other, grads[0]):
+            assert rel_err(a, b) <= 2e-6
+
+
+@pytest.mark.parametrize("layout", ["view", "planes", "records"])
+def test_shift_gradients_come_from_the_projections_given(tp, layout):
+    """The operator's `projections` argument counts, not what the forward pass left beside the derivatives; records
+    given whole hold their own pixels."""
+    ops = torch.ops.torch_projectors_b200
+    case = Case("given", 3, "cubic", 1, 9, 16, 32, 2.0, None, 1, 1, shift_range=3.0, seed=96)
+    t = {k: v.cuda() for k, v in make_inputs(case).items()}
+    rot, sh = t["rot"].requires_grad_(True), t["shifts"].requires_grad_(True)
+    out, der = ops.project_3d_to_2d_forw_saving(t["rec"], rot, sh, [16, 16], "cubic", 2.0, None, None)
+    if layout == "records":
+        given = der.permute(1, 2, 3, 4, 0).as_strided((1, 9, 16, 9, 4), der.permute(1, 2, 3, 4, 0).stride()).clone()
+        double = given * torch.tensor([1, 1, 1, 2], device="cuda")
+    else:
+        given = double = der if layout == "view" else der.contiguous()
+    for need_rec in (False, True):
+        one = ops.project_3d_to_2d_back_saved(t["proj"], out, given, t["rec"], rot, sh, "cubic", 2.0, None, None, need_rec)
+        two = ops.project_3d_to_2d_back_saved(t["proj"], 2 * out, double, t["rec"], rot, sh, "cubic", 2.0, None, None, need_rec)
+        assert rel_err(two[2], 2 * one[2]) <= 1e-5 and rel_err(two[1], one[1]) <= 1e-5

@@ -483,7 +483,7 @@ int project_back_saved(const float* grad_proj, const float* out, const float* de
     L.g.order = pose_order;
     if (grad_proj == nullptr) return fail(B200PROJ_ERR_ARGUMENT, "grad_projections pointer is NULL");
     if (grad_rot != nullptr && derivatives == nullptr) return fail(B200PROJ_ERR_ARGUMENT, "grad_rotations requested but no saved derivatives given");
-    if (grad_shifts != nullptr && (shifts == nullptr || out == nullptr))
+    if (grad_shifts != nullptr && (shifts == nullptr || (out == nullptr && !(RECORDS && derivatives != nullptr))))
         return fail(B200PROJ_ERR_ARGUMENT, "grad_shifts requested but no shifts / saved projections given");
     if (RECORDS && (reinterpret_cast<uintptr_t>(derivatives) & 15u) != 0) return fail(B200PROJ_ERR_ARGUMENT, "records must be 16-byte aligned");
     if (grad_rec == nullptr && grad_rot == nullptr && grad_shifts == nullptr) return B200PROJ_OK;

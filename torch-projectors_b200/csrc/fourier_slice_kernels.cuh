@@ -376,7 +376,7 @@ project_back_saved_kernel(const float2* __restrict__ grad_proj, const float2* __
             }
         }
         if (NEED_SHIFT) {
-            const float2 o = __ldcs(out + w.pix);
+            const float2 o = __ldcs(!RECORDS || out != nullptr ? out + w.pix : derivs + 4 * w.pix + 3);
             const float cross = u.y * o.x - u.x * o.y;
             acc[2 * DIM + 0] = (float)(g.shift_scale * (double)px.kr) * cross;
             acc[2 * DIM + 1] = (float)(g.shift_scale * (double)px.kc) * cross;
@@ -395,7 +395,7 @@ project_back_saved_kernel(const float2* __restrict__ grad_proj, const float2* __
 // grid.x = slice, grid.y = parts of its pixels; a block walks over its part with consecutive threads on
 // consecutive pixels and four pixels in flight per thread (48 bytes each), and adds its sums once.
 // Bound by DRAM (4,096 slices of 128 x 65: 0.182 ms for 1.06 GB = 5.8 TB/s); as tiles of 16 x 16 pixels
-// with one reduction per tile it took 0.52 ms.  RECORDS: the pixel itself is the record's fourth entry.
+// with one reduction per tile it took 0.52 ms.  RECORDS: without `out` the pixel is the record's fourth entry.
 template <int DIM, bool NEED_ROT, bool NEED_SHIFT, bool RECORDS>
 __global__ void __launch_bounds__(kBlockThreads)
 pose_grad_saved_kernel(const float2* __restrict__ grad_proj, const float2* __restrict__ out, const float2* __restrict__ derivs,
@@ -430,17 +430,23 @@ pose_grad_saved_kernel(const float2* __restrict__ grad_proj, const float2* __res
                 u[h] = __ldcs(grad_proj + pix);
                 if (RECORDS && NEED_ROT) {
                     const float4* rec4 = reinterpret_cast<const float4*>(derivs + 4 * pix);
-                    const float4 x = __ldcs(rec4), y = __ldcs(rec4 + 1);
+                    const float4 x = __ldcs(rec4);
                     d[h][0] = make_float2(x.x, x.y);
                     d[h][1] = make_float2(x.z, x.w);
-                    if (DIM == 3) d[h][DIM - 1] = make_float2(y.x, y.y);
-                    if (NEED_SHIFT) o[h] = make_float2(y.z, y.w);
+                    if (NEED_SHIFT && out == nullptr) {
+                        const float4 y = __ldcs(rec4 + 1);
+                        if (DIM == 3) d[h][DIM - 1] = make_float2(y.x, y.y);
+                        o[h] = make_float2(y.z, y.w);
+                    } else {
+                        if (DIM == 3) d[h][DIM - 1] = __ldcs(reinterpret_cast<const float2*>(rec4 + 1));
+                        if (NEED_SHIFT) o[h] = __ldcs(out + pix);
+                    }
                 } else {
                     if (NEED_ROT) {
 #pragma unroll
                         for (int a = 0; a < DIM; ++a) d[h][a] = __ldcs(derivs + (size_t)a * plane + pix);
                     }
-                    if (NEED_SHIFT) o[h] = __ldcs(out + pix);
+                    if (NEED_SHIFT) o[h] = __ldcs(!RECORDS || out != nullptr ? out + pix : derivs + 4 * pix + 3);
                 }
             }
         }

@@ -257,14 +257,20 @@ std::tuple<Tensor, Tensor, Tensor> project_back(int dim, const Tensor& grad_proj
 }
 
 // The saved derivatives, [dim, B, P, H, W/2+1].  3D: a view of records [B, P, H, W/2+1, 4] (the fourth entry of a
-// record is the pixel itself), which is how the kernels write and read them; 2D: plain planes.
+// record is the pixel itself), which is how the kernels write and read them; 2D: plain planes.  What is seen through the
+// view does not include the fourth entries, and a copy of it need not have them: with it the backward pass takes the
+// pixels from its `projections`; with the records given whole, from the records.
 Tensor empty_derivatives(int dim, int64_t B, int64_t P, int64_t N, const at::TensorOptions& opt) {
     if (dim == 2) return at::empty({2, B, P, N, N / 2 + 1}, opt);
     return at::empty({B, P, N, N / 2 + 1, 4}, opt).permute({4, 0, 1, 2, 3}).narrow(0, 0, 3);
 }
-// Derivatives in the layout the kernels read: as made above, or copied into it.
-Tensor kernel_derivatives(int dim, const Tensor& d, const Tensor& projections) {
+bool whole_records(int dim, const Tensor& d, const Tensor& projections) {
+    return dim == 3 && d.dim() == 5 && d.size(4) == 4 && d.sizes().slice(0, 4) == projections.sizes();
+}
+// Derivatives in the layout the kernels read: as made above, or copied into it (without the fourth entries).
+Tensor kernel_derivatives(int dim, const Tensor& d, bool whole) {
     if (dim == 2) return d.contiguous();
+    if (whole) return d.is_contiguous() && (reinterpret_cast<uintptr_t>(d.data_ptr()) & 31u) == 0 ? d : d.clone(at::MemoryFormat::Contiguous);
     int64_t stride = 4;
     bool records = d.stride(0) == 1 && (reinterpret_cast<uintptr_t>(d.data_ptr()) & 31u) == 0;
     for (int64_t a = 4; a >= 1; --a) {
@@ -274,7 +280,6 @@ Tensor kernel_derivatives(int dim, const Tensor& d, const Tensor& projections) {
     if (records) return d;
     Tensor made = at::empty({d.size(1), d.size(2), d.size(3), d.size(4), 4}, d.options());
     made.narrow(4, 0, 3).copy_(d.permute({1, 2, 3, 4, 0}));
-    made.select(4, 3).copy_(projections);
     return made;
 }
 
@@ -329,14 +334,15 @@ std::tuple<Tensor, Tensor, Tensor> project_back_saved(int dim, const Tensor& gra
                 "saved projections must match grad_projections");
     const bool need_rot = rotations.requires_grad();
     // the derivatives are read for the rotation gradient only: without it an empty tensor will do
-    TORCH_CHECK((!need_rot && derivatives.numel() == 0) ||
+    const bool whole = whole_records(dim, derivatives, grad_projections) && derivatives.scalar_type() == at::kComplexFloat && derivatives.is_cuda();
+    TORCH_CHECK((!need_rot && derivatives.numel() == 0) || whole ||
                 (derivatives.dim() == 5 && derivatives.size(0) == dim && derivatives.sizes().slice(1) == grad_projections.sizes() &&
                  derivatives.scalar_type() == at::kComplexFloat && derivatives.is_cuda()),
-                "saved derivatives must be (dim, B, P, H, W/2+1) complex64");
+                "saved derivatives must be (dim, B, P, H, W/2+1) complex64, or in 3D the records (B, P, H, W/2+1, 4)");
     const bool need_shift = p.shifts.defined() && shifts->requires_grad();
     const Tensor gp = grad_projections.contiguous();
-    const Tensor out = projections.contiguous();
-    const Tensor der = derivatives.numel() ? kernel_derivatives(dim, derivatives, projections) : Tensor();
+    const Tensor out = whole ? projections : projections.contiguous();
+    const Tensor der = derivatives.numel() ? kernel_derivatives(dim, derivatives, whole) : Tensor();
     const int64_t R = reconstruction.size(-2);
     c10::cuda::CUDAGuard guard(gp.device());
     Tensor grad_rec = need_rec_grad ? at::empty(reconstruction.sizes(), gp.options()) : Tensor();
@@ -352,7 +358,7 @@ std::tuple<Tensor, Tensor, Tensor> project_back_saved(int dim, const Tensor& gra
             ? b200proj_project_2d_back_saved_ws(cptr<float>(gp), cptr<float>(out), cptr<float>(der), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts),
                                              p.B_shift, p.P, N, interp, oversampling, cut, mptr<float>(grad_rec), mptr<float>(grad_rot), mptr<float>(grad_sh),
                                                 ws_ptr(ws), ws_size(ws), current_stream(gp))
-            : b200proj_project_3d_to_2d_back_records(cptr<float>(gp), cptr<float>(out), cptr<float>(der), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts),
+            : b200proj_project_3d_to_2d_back_records(cptr<float>(gp), whole && der.defined() ? nullptr : cptr<float>(out), cptr<float>(der), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts),
                                                    p.B_shift, p.P, N, interp, oversampling, cut, mptr<float>(grad_rec), mptr<float>(grad_rot), mptr<float>(grad_sh),
                                                    cptr<int32_t>(order), ws_ptr(ws), ws_size(ws), current_stream(gp));
         status(rc, dim == 2 ? "project_2d_back_saved" : "project_3d_to_2d_back_saved");

@@ -578,6 +578,13 @@ def _save_derivatives(dim, reconstruction, rotations, output_shape, interpolatio
     return _KEEP_DERIVATIVES if fits else _PLAIN
 
 
+def _whole_records(derivatives: torch.Tensor) -> torch.Tensor:
+    """The records [B, P, H, W/2+1, 4] that the derivatives of ``project_3d_to_2d_forw_saving`` are a view of.  They are
+    saved whole: what hooks on saved tensors copy is what they see, and the backward pass needs the fourth entries too."""
+    d = derivatives.permute(1, 2, 3, 4, 0)
+    return d.as_strided(d.shape[:-1] + (4,), d.stride())
+
+
 class _Project2D(torch.autograd.Function):
     @staticmethod
     def forward(ctx, reconstruction, rotations, shifts, output_shape, interpolation, oversampling,
@@ -638,7 +645,7 @@ class _Project3DTo2D(torch.autograd.Function):
         if saving == _KEEP_DERIVATIVES:
             projection, derivatives = _ops.project_3d_to_2d_forw_saving(reconstruction, rotations, shifts, output_shape, interpolation,
                                                                         oversampling, fourier_radius_cutoff, order)
-            ctx.save_for_backward(reconstruction, rotations, shifts, projection, derivatives)
+            ctx.save_for_backward(reconstruction, rotations, shifts, projection, _whole_records(derivatives))
         elif saving == _KEEP_OUTPUT:
             projection = _ops.project_3d_to_2d_forw_ordered(reconstruction, rotations, shifts, output_shape, interpolation,
                                                             oversampling, fourier_radius_cutoff, order)
