@@ -342,3 +342,18 @@ def test_bench_script_refers_to_no_undefined_name():
             defined.add(n.id)
     loaded = {n.id for n in ast.walk(tree) if isinstance(n, ast.Name) and isinstance(n.ctx, ast.Load)}
     assert loaded - defined == set(), sorted(loaded - defined)
+
+
+@pytest.mark.parametrize("dim,poses,kept", [(3, 18_000, True), (3, 21_600, True), (3, 21_800, False), (2, 32_000, True), (2, 33_000, False)])
+def test_derivatives_are_kept_up_to_the_limit_on_the_derivatives_themselves(dim, poses, kept):
+    """16 GiB by default: 256 x 129 slices with three derivatives each up to 21,671 poses, with two up to 32,506."""
+    from torch_projectors_b200 import ops
+
+    class Volume:
+        is_cuda, dtype = True, torch.complex64
+        size = staticmethod(lambda d: 1)
+        __getitem__ = staticmethod(lambda k: torch.empty((512,) * (dim - 1) + (257,), device="meta"))
+
+    rot = torch.empty(1, poses, dim, dim, device="meta")
+    how = ops._save_derivatives(dim, Volume(), rot, (256, 256), "cubic", True, True, True)
+    assert (how == ops._KEEP_DERIVATIVES) == kept

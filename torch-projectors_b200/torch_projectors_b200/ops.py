@@ -126,7 +126,7 @@ def set_pose_order_thresholds(min_volume_bytes: int = 96 << 20, min_poses: int =
 
 # Saved derivatives: when the rotations of a cubic 3D projection need gradients, the forward pass can
 # also write every pixel's derivatives with respect to its sample position (a record of four times
-# the projections' size), and the backward pass then forms the pose gradients from them instead of
+# the projections' size, the projections among it), and the backward pass then forms the pose gradients from them instead of
 # gathering the volume a second time -- and skips the scatter into the volume's gradient altogether
 # when the volume needs none.  Measured on B200, box 512, 4,096 poses of 256 x 256, cubic: forward
 # 6.5 -> 8.9 ms, backward 20.3 -> 15.1 ms (1.9 ms with a fixed volume).
@@ -143,7 +143,8 @@ def set_save_derivatives(enabled: bool = True, max_bytes: int = 16 << 30, min_vo
     """Whether ``project_2d_forw`` / ``project_3d_to_2d_forw`` keep their pixels' derivatives for the
     backward pass when the rotations require gradients (complex64; when the reconstruction needs a
     gradient as well: cubic interpolation and at least `min_volume_bytes` per batch item), and up to
-    which size of that extra tensor (2D: 2 x the projections, 3D: 4 x)."""
+    which size of the derivatives (2D: 2 x the projections, 3D: 3 x).  In 3D they are kept in records of
+    4 x the projections' size, together with the projections, which are then not saved again."""
     global SAVE_DERIVATIVES, SAVE_DERIVATIVES_MAX_BYTES, SAVE_DERIVATIVES_MIN_VOLUME_BYTES
     SAVE_DERIVATIVES, SAVE_DERIVATIVES_MAX_BYTES = bool(enabled), int(max_bytes)
     SAVE_DERIVATIVES_MIN_VOLUME_BYTES = int(min_volume_bytes)
@@ -574,7 +575,8 @@ def _save_derivatives(dim, reconstruction, rotations, output_shape, interpolatio
                          (reconstruction[0].numel() * 8 >= SAVE_DERIVATIVES_MIN_VOLUME_BYTES or
                           reconstruction.size(0) * rotations.size(1) * N * N >= SAVE_DERIVATIVES_MIN_PIXELS)):
         return _PLAIN
-    fits = 8 * (2 if dim == 2 else 4) * reconstruction.size(0) * rotations.size(1) * N * (N // 2 + 1) <= SAVE_DERIVATIVES_MAX_BYTES
+    # the derivatives proper: the fourth entry of a 3D record is the projection, which the step saves nowhere else
+    fits = 8 * dim * reconstruction.size(0) * rotations.size(1) * N * (N // 2 + 1) <= SAVE_DERIVATIVES_MAX_BYTES
     return _KEEP_DERIVATIVES if fits else _PLAIN
 
 
@@ -645,7 +647,7 @@ class _Project3DTo2D(torch.autograd.Function):
         if saving == _KEEP_DERIVATIVES:
             projection, derivatives = _ops.project_3d_to_2d_forw_saving(reconstruction, rotations, shifts, output_shape, interpolation,
                                                                         oversampling, fourier_radius_cutoff, order)
-            ctx.save_for_backward(reconstruction, rotations, shifts, projection, _whole_records(derivatives))
+            ctx.save_for_backward(reconstruction, rotations, shifts, projection.new_empty(0), _whole_records(derivatives))
         elif saving == _KEEP_OUTPUT:
             projection = _ops.project_3d_to_2d_forw_ordered(reconstruction, rotations, shifts, output_shape, interpolation,
                                                             oversampling, fourier_radius_cutoff, order)
@@ -664,6 +666,8 @@ class _Project3DTo2D(torch.autograd.Function):
     def backward(ctx, grad_output):
         if ctx.saving:
             reconstruction, rotations, shifts, projection, derivatives = ctx.saved_tensors
+            if ctx.saving == _KEEP_DERIVATIVES:
+                projection = derivatives.select(-1, 3)
             grad_reconstruction, grad_rotations, grad_shifts = _ops.project_3d_to_2d_back_saved(
                 grad_output.contiguous(), projection, derivatives, reconstruction, rotations, shifts, ctx.interpolation,
                 ctx.oversampling, ctx.fourier_radius_cutoff, ctx.pose_order, ctx.need_rec)
