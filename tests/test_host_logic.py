@@ -357,3 +357,25 @@ def test_derivatives_are_kept_up_to_the_limit_on_the_derivatives_themselves(dim,
     rot = torch.empty(1, poses, dim, dim, device="meta")
     how = ops._save_derivatives(dim, Volume(), rot, (256, 256), "cubic", True, True, True)
     assert (how == ops._KEEP_DERIVATIVES) == kept
+
+
+def test_a_callers_own_volume_size_decides_alone_which_reconstructions_keep_derivatives():
+    from torch_projectors_b200 import ops
+
+    class Volume:
+        is_cuda, dtype = True, torch.complex64
+        size = staticmethod(lambda d: 1)
+        __getitem__ = staticmethod(lambda k: torch.empty((128, 65), device="meta"))
+
+    def kept(poses):
+        return ops._save_derivatives(2, Volume(), torch.empty(1, poses, 2, 2, device="meta"), (128, 128), "cubic", True, True)
+
+    assert kept(200) == ops._PLAIN and kept(300) == ops._KEEP_DERIVATIVES          # 3.3 and 4.9 M pixels
+    try:
+        tp.set_save_derivatives(True, min_volume_bytes=64 << 20)
+        assert kept(300) == ops._PLAIN
+        tp.set_save_derivatives(True, min_volume_bytes=1 << 10)
+        assert kept(200) == ops._KEEP_DERIVATIVES
+    finally:
+        tp.set_save_derivatives(True)
+    assert kept(300) == ops._KEEP_DERIVATIVES

@@ -142,12 +142,13 @@ SAVE_DERIVATIVES_MIN_PIXELS = 1 << 22
 def set_save_derivatives(enabled: bool = True, max_bytes: int = 16 << 30, min_volume_bytes: int = 2 << 20) -> None:
     """Whether ``project_2d_forw`` / ``project_3d_to_2d_forw`` keep their pixels' derivatives for the
     backward pass when the rotations require gradients (complex64; when the reconstruction needs a
-    gradient as well: cubic interpolation and at least `min_volume_bytes` per batch item), and up to
-    which size of the derivatives (2D: 2 x the projections, 3D: 3 x).  In 3D they are kept in records of
+    gradient as well: cubic interpolation and at least `min_volume_bytes` per batch item; left at its
+    default, also calls of 4 M pixels and more), and up to which size of the derivatives (2D: 2 x the projections, 3D: 3 x).  In 3D they are kept in records of
     4 x the projections' size, together with the projections, which are then not saved again."""
-    global SAVE_DERIVATIVES, SAVE_DERIVATIVES_MAX_BYTES, SAVE_DERIVATIVES_MIN_VOLUME_BYTES
+    global SAVE_DERIVATIVES, SAVE_DERIVATIVES_MAX_BYTES, SAVE_DERIVATIVES_MIN_VOLUME_BYTES, SAVE_DERIVATIVES_MIN_PIXELS
     SAVE_DERIVATIVES, SAVE_DERIVATIVES_MAX_BYTES = bool(enabled), int(max_bytes)
     SAVE_DERIVATIVES_MIN_VOLUME_BYTES = int(min_volume_bytes)
+    SAVE_DERIVATIVES_MIN_PIXELS = 1 << 22 if SAVE_DERIVATIVES_MIN_VOLUME_BYTES == 2 << 20 else None
 
 
 def plane_locality_order(rotations: torch.Tensor, batch: int = 1) -> torch.Tensor:
@@ -573,7 +574,8 @@ def _save_derivatives(dim, reconstruction, rotations, output_shape, interpolatio
     N = int(output_shape[0])
     if need_rec and not (interpolation == "cubic" and
                          (reconstruction[0].numel() * 8 >= SAVE_DERIVATIVES_MIN_VOLUME_BYTES or
-                          reconstruction.size(0) * rotations.size(1) * N * N >= SAVE_DERIVATIVES_MIN_PIXELS)):
+                          (SAVE_DERIVATIVES_MIN_PIXELS is not None
+                           and reconstruction.size(0) * rotations.size(1) * N * N >= SAVE_DERIVATIVES_MIN_PIXELS))):
         return _PLAIN
     # the derivatives proper: the fourth entry of a 3D record is the projection, which the step saves nowhere else
     fits = 8 * dim * reconstruction.size(0) * rotations.size(1) * N * (N // 2 + 1) <= SAVE_DERIVATIVES_MAX_BYTES
