@@ -162,3 +162,34 @@ def test_a_wrong_order_is_refused_by_calls_that_do_not_need_one(tp):
                      lambda: ops.project_3d_to_2d_back_saved(grad, out, der, rec, rot_g, sh, "cubic", 1.0, None, order, False)):
             with pytest.raises(RuntimeError, match="pose_order must be an int32 CUDA tensor"):
                 call()
+
+
+@pytest.mark.parametrize("interp,poses,sorted_once", [("cubic", 2500, 0), ("cubic", 90, 1), ("linear", 2500, 1)])
+def test_the_training_step_sorts_poses_only_for_kernels_that_use_the_order(tp, monkeypatch, interp, poses, sorted_once):
+    """2,500 cubic slices of box 64 run brick by brick, 90 do not, nor do linear ones of this box."""
+    from torch_projectors_b200 import ops
+
+    class Spy:
+        calls = 0
+
+        def __getattr__(self, name):
+            Spy.calls += name == "plane_locality_order"
+            return getattr(torch.ops.torch_projectors_b200, name)
+
+    gen = torch.Generator().manual_seed(3)
+    rec = torch.randn(1, 64, 64, 33, dtype=torch.complex64, generator=gen).cuda()
+    base = random_rotations_3d(poses, gen).view(1, poses, 3, 3).cuda()
+    bricks = tp._abi.project_workspace_bytes(3, 1, poses, 64, ops._interp_code(interp), True, 1.0, 32.0) > 0
+    assert bricks == (sorted_once == 0)
+    monkeypatch.setattr(ops, "_ops", Spy())
+    monkeypatch.setattr(ops, "POSE_ORDER_MIN_BYTES", 0)
+    grads = []
+    for order in (None, False):
+        Spy.calls = 0
+        rot = base.clone().requires_grad_(True)
+        out = tp.project_3d_to_2d_forw(rec, rot, None, output_shape=(64, 64), interpolation=interp, oversampling=1.0, pose_order=order)
+        out.abs().square().sum().backward()
+        assert Spy.calls == (sorted_once if order is None else 0)
+        grads.append((out.detach(), rot.grad))
+    for a, b in zip(*grads):
+        assert rel_err(a, b) <= 2e-6

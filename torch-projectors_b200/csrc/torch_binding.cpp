@@ -353,7 +353,8 @@ std::tuple<Tensor, Tensor, Tensor> project_back_saved(int dim, const Tensor& gra
     } else {
         const double cut = cutoff_of(cutoff, N);
         const Tensor ws = need_rec_grad ? gradient_workspace(dim, gp, B, R, p.P, N, interp, false, oversampling, cut) : Tensor();
-        Tensor order = resolve_order(dim, reconstruction, B, p, pose_order, !ws.defined());
+        // (without the volume's gradient the pose gradients are a streaming pass)
+        Tensor order = resolve_order(dim, reconstruction, B, p, pose_order, need_rec_grad && !ws.defined());
         const int rc = dim == 2
             ? b200proj_project_2d_back_saved_ws(cptr<float>(gp), cptr<float>(out), cptr<float>(der), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts),
                                              p.B_shift, p.P, N, interp, oversampling, cut, mptr<float>(grad_rec), mptr<float>(grad_rot), mptr<float>(grad_sh),

@@ -143,6 +143,10 @@ def backproject_workspace_bytes(dim: int, B: int, R: int, P: int, N: int, interp
     return int(load().b200proj_backproject_workspace_bytes(dim, B, R, P, N, interp, int(has_weights)))
 
 
+def project_workspace_bytes(dim: int, B: int, P: int, N: int, interp: int, records: bool, oversampling: float, cutoff: float) -> int:
+    return int(load().b200proj_project_workspace_bytes(dim, B, P, N, interp, int(records), float(oversampling), float(cutoff)))
+
+
 def _p(t: Optional[torch.Tensor]) -> int:
     return 0 if t is None else t.data_ptr()
 

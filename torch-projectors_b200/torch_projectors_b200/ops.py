@@ -174,14 +174,17 @@ def _natural_order(device) -> torch.Tensor:
     return t
 
 
-def _resolve_order(pose_order, vol: torch.Tensor, rotations: torch.Tensor) -> torch.Tensor:
-    """pose_order argument of the public 3D functions -> the tensor handed to the operators (and
+def _resolve_order(pose_order, vol: torch.Tensor, rotations: torch.Tensor, unused=None) -> Optional[torch.Tensor]:
+    """pose_order argument of the public 3D functions -> what is handed to the operators (and
     kept for the backward pass): a given order as it is, ``False`` = natural order, ``None`` = made
-    here when the volume is large enough for it to matter."""
+    here when the volume is large enough for it to matter; but when the forward pass has no use for
+    it (``unused()``), None: an operator of the backward pass that has makes its own."""
     if isinstance(pose_order, torch.Tensor):
         return pose_order
     if pose_order is None and rotations.size(1) >= POSE_ORDER_MIN_POSES and \
             vol[0].numel() * vol.element_size() >= POSE_ORDER_MIN_BYTES and vol.is_cuda:
+        if unused is not None and unused():
+            return None
         return _ops.plane_locality_order(rotations.detach(), vol.size(0))
     return _natural_order(vol.device)
 
@@ -639,11 +642,14 @@ class _Project3DTo2D(torch.autograd.Function):
     def forward(ctx, reconstruction, rotations, shifts, output_shape, interpolation, oversampling,
                 fourier_radius_cutoff, pose_order):
         reconstruction, rotations, shifts = _canon_project(3, reconstruction, rotations, shifts)
-        # the processing order of the slices is settled once here and kept for the backward pass
-        order = _resolve_order(pose_order, reconstruction, rotations)
         need_rec = ctx.needs_input_grad[0]
         saving = _save_derivatives(3, reconstruction, rotations, output_shape, interpolation, need_rec, ctx.needs_input_grad[1],
                                    shifts is not None and ctx.needs_input_grad[2])
+        # the processing order of the slices is settled once here and kept for the backward pass; kernels that go brick by
+        # brick have no use for it (4,096 slices: 9.5 us of sorting by one block)
+        order = _resolve_order(pose_order, reconstruction, rotations, lambda: reconstruction.dtype == torch.complex64 and _abi.project_workspace_bytes(
+            3, reconstruction.size(0), rotations.size(1), int(output_shape[0]), _interp_code(interpolation), saving == _KEEP_DERIVATIVES,
+            oversampling, _cutoff(fourier_radius_cutoff, int(output_shape[0]))) > 0)
         ctx.saving = saving
         ctx.need_rec = need_rec
         if saving == _KEEP_DERIVATIVES:
