@@ -128,3 +128,26 @@ def test_scatters_spread_over_copies_of_a_small_reconstruction(dim, interp, P):
     forw, ref = (tp.backproject_2d_forw, port.backproject_2d_forw) if dim == 2 else (tp.backproject_2d_to_3d_forw, port.backproject_2d_to_3d_forw)
     data, _ = forw(t["proj"].cuda(), t["rot"].cuda(), None, t["shifts"].cuda(), interpolation=interp, oversampling=1.5)
     assert rel_err(data, ref(t["proj"], None, t["rot"], t["shifts"], interp, 1.5, None)[0]) <= TOL_ATOMIC
+
+
+@pytest.mark.parametrize("dim,interp,P,copies", [(2, "linear", 4000, 32), (2, "cubic", 1031, 32), (3, "linear", 1501, 32), (3, "cubic", 257, 8), (3, "cubic", 20, 1)])
+def test_scatters_choose_copies_by_the_reductions_per_byte(dim, interp, P, copies):
+    """At sizes where the copies are chosen by themselves (many slices onto a small reconstruction), and where not:
+    gradients with and without pose gradients and back-projection without weights, against the oracle."""
+    import torch_projectors_b200 as tp
+    from oracle import port
+    t = make_inputs(Case("copies", dim, interp, 1, P, 12, 18, 1.5, None, 1, 1, shift_range=2.0, seed=P))
+    one = 8 * (18 if dim == 3 else 1) * 18 * 10
+    have = tp._abi.load().b200proj_gradient_workspace_bytes(dim, 1, 18, P, 12, tp.ops._interp_code(interp), 0, 1.5, 6.0)
+    assert have == (copies * one if copies > 1 else 0)
+    project, back = (tp.project_2d_forw, port.project_2d_back) if dim == 2 else (tp.project_3d_to_2d_forw, port.project_3d_to_2d_back)
+    want = back(t["proj"], t["rec"], t["rot"], t["shifts"], interp, 1.5, None, need_rot_grad=True, need_shift_grad=True)
+    for poses in (True, False):
+        rec, rot, sh = (t[k].cuda().requires_grad_(k == "rec" or poses) for k in ("rec", "rot", "shifts"))
+        project(rec, rot, sh, output_shape=(12, 12), interpolation=interp, oversampling=1.5).backward(t["proj"].cuda())
+        assert rel_err(rec.grad, want[0]) <= TOL_ATOMIC
+        if poses:
+            assert rel_err(rot.grad, want[1]) <= TOL_ATOMIC and rel_err(sh.grad, want[2]) <= TOL_ATOMIC
+    forw, ref = (tp.backproject_2d_forw, port.backproject_2d_forw) if dim == 2 else (tp.backproject_2d_to_3d_forw, port.backproject_2d_to_3d_forw)
+    data, _ = forw(t["proj"].cuda(), t["rot"].cuda(), None, t["shifts"].cuda(), interpolation=interp, oversampling=1.5)
+    assert rel_err(data, ref(t["proj"], None, t["rot"], t["shifts"], interp, 1.5, None)[0]) <= TOL_ATOMIC

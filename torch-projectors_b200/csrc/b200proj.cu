@@ -177,7 +177,7 @@ SlabPlan slab_plan(int64_t R, bool has_weights, bool interleaved = false, bool e
     return {slabs, planes};
 }
 
-// Copies of a small interleaved workspace over which the slices of one call are spread: reductions
+// Copies of a small reconstruction or interleaved workspace over which the slices of one call are spread: reductions
 // onto less than ~2 MB run at 55-60 % of the rate they reach on a larger target (probe: 146 instead
 // of 254 G taps/s at 128 KB), so a reconstruction of `bytes` bytes gets the power of two of copies
 // that brings it to 2 MiB, at most 32 and at most one per 32 slices.
@@ -231,6 +231,7 @@ BrickLaunch brick_layout(int64_t B, int64_t P, int64_t N, double os, double cuto
     BrickLaunch L{};
     static const int force = [] { const char* e = getenv("B200PROJ_BRICKS"); return e ? atoi(e) : -1; }();   // 0 / 1: never / always, for tests
     if (force == 0 || os < 1.0 || !(cutoff >= 0.0) || P < 1) return L;
+    if (force != 1 && (double)B * (double)P * (double)N * (double)(N / 2 + 1) < 6e5) return L;      // below all lines
     const double corner = sqrt((double)N * N / 2.0);
     const double reach = (cutoff < corner ? cutoff : corner) * os;
     if (reach > 1000.0) return L;
@@ -358,12 +359,27 @@ int launch_brick_scatter(const Launch& L, const BrickLaunch& bl, void* workspace
     return check_launch("brick_scatter launch");
 }
 
-// Copies of a small complex reconstruction over which the slices of a scatter are spread (see workspace_replicas):
-// as many as the rule wants and the workspace holds; sets the kernels' geometry.
-int scatter_copies(Launch& L, const void* workspace, size_t workspace_bytes) {
+// Copies of a small complex reconstruction (all batch items: `one` bytes) over which the slices of a scatter without
+// weights are spread.  They cost a clear, a sum over the copies and two launches (3-5 us; small calls lose up to half), and
+// gain where many reductions meet on few sectors.  In reductions per byte, measured on both sides of the lines: 2D, cubic /
+// linear, 264 KB: 32 a byte 0.95 / 1.0x, 64 1.1 / 1.1x; 3D 461 KB cubic: 5 a byte 0.9x, 22 1.1x; 1.08 MB cubic: 10 0.95x, 32
+// 1.1x; 1.5 MB cubic: 14 0.93x, 43 1.1x.  Linear reductions leave in pairs and gain nothing from 0.7 MB on (0.96-1.04x).  Beside
+// the gather of the pose gradients they weigh less: linear 0.93-1.04x up to 80 a byte, 1.06x and more from 130 on; 2D
+// cubic, 149-264 KB (of one batch item): 0.96x at 65, 1.0x at 300; below 0.1 MB 1.1x at 65.
+int copies_wanted(int dim, double one, int64_t B, int64_t P, int64_t N, bool cubic, bool pose_gradients) {
+    const int t = cubic ? 4 : 2;
+    const double sums = (double)B * (double)P * (double)N * (double)(N / 2 + 1) * (dim == 3 ? t * t * t : t * t);
+    double per_byte = dim == 3 && one <= 1.2e6 ? 15.0 : 36.0;
+    if (pose_gradients && !cubic) per_byte = 120.0;
+    else if (pose_gradients && dim == 2 && one > 1e5 * (double)B) per_byte = 250.0;
+    if (sums < 1e6 || sums < per_byte * one || (!cubic && one > 5.5e5)) return 1;
+    return workspace_replicas(one, P);
+}
+// As many of them as the workspace holds; sets the kernels' geometry.
+int scatter_copies(Launch& L, int dim, bool cubic, bool pose_gradients, const void* workspace, size_t workspace_bytes) {
     if (!scratch_aligned(workspace)) return 1;
     const size_t one = L.rec_count * sizeof(float2);
-    int copies = workspace_replicas((double)one, L.P);
+    int copies = copies_wanted(dim, (double)one, L.B, L.P, L.g.N, cubic, pose_gradients);
     while (copies > 1 && (size_t)copies * one > workspace_bytes) copies /= 2;
     L.g.replicas = copies;
     L.g.replica_stride = copies > 1 ? (long long)L.rec_count : 0;
@@ -492,7 +508,7 @@ int project_back_saved(const float* grad_proj, const float* out, const float* de
     BrickLaunch bl{};
     if ((RECORDS || DIM == 2) && P > 0 && grad_rec != nullptr && workspace != nullptr) bl = scatter_plan(DIM, B, P, N, cubic, false, os, cutoff);
     bl.use = runs_in(bl, workspace, workspace_bytes);
-    const int copies = P > 0 && grad_rec != nullptr && !bl.use ? scatter_copies(L, workspace, workspace_bytes) : 1;
+    const int copies = P > 0 && grad_rec != nullptr && !bl.use ? scatter_copies(L, DIM, cubic, false, workspace, workspace_bytes) : 1;
     if (int rc = zero_outputs(s, copies > 1 ? nullptr : grad_rec, L.rec_count * sizeof(float2), grad_rot, (size_t)B_rot * P * DIM * DIM * sizeof(float),
                               grad_shifts, (size_t)(shifts ? B_shift : 0) * P * 2 * sizeof(float))) return rc;
     if (P == 0) return B200PROJ_OK;
@@ -535,7 +551,7 @@ int project_back(const Real* grad_proj, const Real* rec, int64_t B, int64_t R, c
     if (std::is_same<Real, float>::value && P > 0 && grad_rot == nullptr && grad_shifts == nullptr && workspace != nullptr)
         bl = scatter_plan(DIM, B, P, N, interpolation == B200PROJ_CUBIC, false, os, cutoff);
     bl.use = runs_in(bl, workspace, workspace_bytes);
-    const int copies = P > 0 && std::is_same<Real, float>::value && !bl.use ? scatter_copies(L, workspace, workspace_bytes) : 1;
+    const int copies = P > 0 && std::is_same<Real, float>::value && !bl.use ? scatter_copies(L, DIM, interpolation == B200PROJ_CUBIC, grad_rot != nullptr || grad_shifts != nullptr, workspace, workspace_bytes) : 1;
     if (int rc = zero_outputs(s, copies > 1 ? nullptr : grad_rec, L.rec_count * sizeof(C2<Real>), grad_rot, (size_t)B_rot * P * DIM * DIM * sizeof(Real),
                               grad_shifts, (size_t)(shifts ? B_shift : 0) * P * 2 * sizeof(Real))) return rc;
     if (P == 0) return B200PROJ_OK;
@@ -608,7 +624,7 @@ int backproject_forw(const Real* proj, const Real* weights, int64_t B, int64_t R
     }
     if constexpr (kIsF32) {
         // a small reconstruction without weights: copies of it in the workspace
-        const int copies = !hw && P > 0 ? scatter_copies(L, workspace, workspace_bytes) : 1;
+        const int copies = !hw && P > 0 ? scatter_copies(L, DIM, cubic, false, workspace, workspace_bytes) : 1;
         if (copies > 1) {
             if (int rc = zero_async(workspace, (size_t)copies * L.rec_count * sizeof(float2), s)) return rc;
             if (cubic) backproject_forw_kernel<DIM, true, false><<<L.grid, kBlockThreads, 0, s>>>((const float2*)proj, weights, rot, shifts, (float2*)workspace, weight_rec, L.g);
@@ -825,7 +841,7 @@ size_t b200proj_backproject_workspace_bytes(int dim, int64_t B, int64_t R, int64
     if (taps < 4.0 * voxels) return 0;
     if (dim == 3 && slab_plan(R, has_weights != 0).slabs > 1) return 0;      // beyond-L2 volumes take the slab-ordered path
     const double one = voxels * (double)(has_weights ? sizeof(float4) : sizeof(float2));
-    const int copies = workspace_replicas(one, P);                 // small reconstructions: several copies
+    const int copies = has_weights ? workspace_replicas(one, P) : copies_wanted(dim, one, B, P, N, interpolation == B200PROJ_CUBIC, false);   // small reconstructions: several copies
     return has_weights || copies > 1 ? (size_t)one * (size_t)copies : 0;
 }
 
@@ -876,7 +892,7 @@ size_t b200proj_gradient_workspace_bytes(int dim, int64_t B, int64_t R, int64_t 
     if (!pose_gradients)
         if (const size_t bytes = b200proj_scatter_workspace_bytes(dim, B, P, N, interpolation, 0, oversampling, cutoff)) return bytes;
     const double one = (double)B * (dim == 3 ? R : 1) * R * (R / 2 + 1) * (double)sizeof(float2);
-    const int copies = workspace_replicas(one, P);
+    const int copies = copies_wanted(dim, one, B, P, N, interpolation == B200PROJ_CUBIC, pose_gradients != 0);
     return copies > 1 ? (size_t)one * (size_t)copies : 0;
 }
 size_t b200proj_project_workspace_bytes(int dim, int64_t B, int64_t P, int64_t N, int interpolation, int records, double oversampling, double cutoff) {
