@@ -130,6 +130,45 @@ def test_scatters_spread_over_copies_of_a_small_reconstruction(dim, interp, P):
     assert rel_err(data, ref(t["proj"], None, t["rot"], t["shifts"], interp, 1.5, None)[0]) <= TOL_ATOMIC
 
 
+def _matrices(dim, size, seed):
+    """Poses that are no rotations: magnified (up to and beyond what bricks take), sheared, mirrored, slightly perturbed, singular."""
+    B, P, N, R, os_, cutoff, B_rot, B_shift = size
+    t = make_inputs(Case("matrices", dim, "cubic", B, P, N, R, os_, cutoff, B_rot, B_shift, shift_range=5.0, seed=seed))
+    gen = torch.Generator().manual_seed(seed)
+    for p in range(P):
+        m = t["rot"][:, p]
+        kind = p % 8
+        if kind == 0:
+            m *= (0.05, 0.12, 0.3, 0.7, 1.01, 1.08, 1.3, 1.7, 2.0, 2.3)[p // 8 % 10]
+        elif kind == 1:
+            m += 0.02 * torch.randn(m.shape, generator=gen)
+        elif kind == 2:
+            m[..., 1] += (0.3, 1.0, 4.0)[p // 8 % 3] * m[..., 0]
+        elif kind == 3:
+            m[..., 0] *= -1.0
+        elif kind == 4:
+            m *= torch.tensor([1.25, 0.8, 1.0][:dim])
+        elif kind == 5:
+            m *= 0.0 if p // 8 % 2 else 1.0 + 1e-4
+    return t, dict(output_shape=(N, N), oversampling=os_, fourier_radius_cutoff=cutoff)
+
+
+def check_matrices(names):
+    global _inputs, SIZES, SIZES_2D
+    _inputs = _matrices
+    SIZES = [(1, 100, 18, 36, 2.0, None, 1, 1), (2, 83, 34, 50, 1.5, 13.0, 1, 2), (1, 80, 20, 20, 1.0, 14.0, 1, 0)]
+    SIZES_2D = SIZES + [(1, 90, 70, 160, 2.0, 40.0, 1, 1)]
+    check(names)
+
+
+@pytest.mark.parametrize("names", ["forward", "gradients", "backprojection"])
+def test_bricks_match_the_oracle_for_matrices_that_are_no_rotations(names):
+    env = dict(os.environ, B200PROJ_BRICKS="1")
+    r = subprocess.run([sys.executable, "-c", f"import sys; sys.path.insert(0, {str(ROOT / 'tests')!r}); import test_gpu_bricks as t; t.check_matrices({names!r})"],
+                       env=env, cwd=ROOT, capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]
+
+
 @pytest.mark.parametrize("dim,interp,P,copies", [(2, "linear", 4000, 32), (2, "cubic", 1031, 32), (3, "linear", 1501, 32), (3, "cubic", 257, 8), (3, "cubic", 20, 1)])
 def test_scatters_choose_copies_by_the_reductions_per_byte(dim, interp, P, copies):
     """At sizes where the copies are chosen by themselves (many slices onto a small reconstruction), and where not:

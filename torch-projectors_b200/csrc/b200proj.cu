@@ -208,10 +208,11 @@ bool linear_rows2() {
 // ---- brick-stationary kernels: plan and launch ---------------------------------------------------------
 struct BrickLaunch {
     BrickPlan plan;
-    int64_t bricks;          // of one batch item
+    int64_t bricks;          // of one batch item, for rotations
     size_t items;            // capacity of the item list
     size_t item_bytes, rec_bytes;
     size_t bytes;            // workspace
+    int64_t slices;
     double pixels, in_ball;  // of the call: pixels inside the cutoff, bricks that can hold some
     bool forced, use;
 };
@@ -236,16 +237,22 @@ BrickLaunch brick_layout(int64_t B, int64_t P, int64_t N, double os, double cuto
     const double reach = (cutoff < corner ? cutoff : corner) * os;
     if (reach > 1000.0) return L;
     const double pixels = pixels_inside(N, cutoff) * (double)B * (double)P;
-    L.plan.ball = (float)(reach + 1.0);
-    const int span = 2 * ((int)ceil(reach) + 2);
+    L.slices = B * P;
+    L.plan.reach = (float)reach;
+    L.plan.keep = 1 << 20;
     const int dims[3] = {D::x, D::y, D::z};
-    L.bricks = 1;
-    for (int a = 0; a < 3; ++a) {
-        L.plan.d[a] = dims[a];
-        L.plan.n[a] = dims[a] ? (span + dims[a] - 1) / dims[a] : 1;
-        L.plan.lo[a] = -((L.plan.n[a] * dims[a]) / 2);
-        L.bricks *= L.plan.n[a];
-    }
+    // grid of a shell: that of the first with whole clusters of brick_setup_kernel around it, so that all lie on one lattice
+    auto grid = [&](int shell, int* n) {
+        const int span = 2 * ((int)ceil(reach * brick_stretch(shell)) + 2), inner = 2 * ((int)ceil(reach) + 2), cluster[3] = {8, 8, 4};
+        int64_t cells = 1;
+        for (int a = 0; a < 3; ++a) {
+            n[a] = dims[a] ? (inner + dims[a] - 1) / dims[a] : 1;
+            while (dims[a] && n[a] * dims[a] < span) n[a] += 2 * cluster[a];
+            cells *= n[a];
+        }
+        return cells;
+    };
+    L.bricks = grid(0, L.plan.n);
     if (L.bricks * B > (1 << 26) || B * P > (1 << 26)) return L;
     L.plan.density = (float)(D::kDim == 3 ? (double)D::x * D::y * D::z / (4.0 * os * os) : (double)D::x * D::y / (2.0 * os * os));
     double target = pixels / (blocks * 8.0);
@@ -256,9 +263,24 @@ BrickLaunch brick_layout(int64_t B, int64_t P, int64_t N, double os, double cuto
     L.plan.max_extra = (int)((L.bricks < 64 ? (double)L.bricks : 4.0) * pixels / target) + 64;
     static const int wait_ms = [] { const char* e = getenv("B200PROJ_BRICK_WAIT_MS"); return e ? atoi(e) : 10000; }();   // for tests
     L.plan.wait_ms = wait_ms < 0 ? 0 : wait_ms;
-    L.items = (size_t)(L.bricks * B) + (size_t)L.plan.max_extra;
+    // the shells' lists, as long as those beyond the first stay below 64 MB
+    for (int l = 0; l < kShells; ++l) {
+        int n[3];
+        const double cells = (double)grid(l, n), r = reach * brick_stretch(l) + 1.0 + sqrt((double)dims[0] * dims[0] + (double)dims[1] * dims[1] + (double)dims[2] * dims[2]);
+        const double round = D::kDim == 3 ? 4.19 * r * r * r / ((double)D::x * D::y * D::z) : M_PI * r * r / ((double)D::x * D::y);   // bricks that meet the ball lie in this one
+        const size_t need = (size_t)((round < cells ? ceil(round) : cells) * (double)B) + (size_t)L.plan.max_extra;
+        if (l > 0 && (L.items + need) * sizeof(int4) > (64u << 20)) break;
+        for (int a = 0; a < 3; ++a) L.plan.n[a] = n[a];
+        L.plan.at[l] = (int)L.items;
+        L.plan.shells = l + 1;
+        L.items += need;
+    }
+    for (int a = 0; a < 3; ++a) {
+        L.plan.d[a] = dims[a];
+        L.plan.lo[a] = -((L.plan.n[a] * dims[a]) / 2);
+    }
     L.item_bytes = (L.items * sizeof(int4) + 255) & ~(size_t)255;
-    L.rec_bytes = (size_t)(B * P) * 3 * sizeof(float4);
+    L.rec_bytes = (size_t)(B * P) * (4 * sizeof(float4) + sizeof(float2));
     L.bytes = 256 + L.item_bytes + L.rec_bytes + (outside ? (size_t)(N * (N / 2 + 1)) * sizeof(int) : 0);
     L.pixels = pixels;
     L.in_ball = (D::kDim == 3 ? 4.19 * pow(reach + 12.0, 3) / ((double)D::x * D::y * D::z) : M_PI * pow(reach + 30.0, 2) / ((double)D::x * D::y)) * (double)B;
@@ -282,7 +304,7 @@ BrickLaunch gather_plan(int dim, int64_t B, int64_t P, int64_t N, bool cubic, bo
     const double need = cubic ? (1.2e6 + 900.0 * L.in_ball) * (os < 2.0 ? 2.0 / os : 1.0)
                               : (10e6 + 4000.0 * L.in_ball) * (records ? 0.6 : 1.0);
     // linear taps: small volumes meet a slice in too few pixels per brick (box 38 oversampled twice: 1.8x slower)
-    L.use = L.use && (L.forced || (L.pixels > need && (cubic || L.plan.ball > 85.f)));
+    L.use = L.use && (L.forced || (L.pixels > need && (cubic || L.plan.reach > 84.f)));
     return L;
 }
 
@@ -299,7 +321,7 @@ BrickLaunch scatter_plan(int dim, int64_t B, int64_t P, int64_t N, bool cubic, b
         BrickLaunch L = weights ? scatter_layout<2, true>(B, P, N, os, cutoff) : scatter_layout<2, false>(B, P, N, os, cutoff);
         // measured at 9 M pixels: weighted 1.3-1.4x, else 1.0-1.35x (dense samples 1.5x and more: the plain kernels contend); 27 M: 1.1-1.7x;
         // reconstructions that fill less than a tile gain nothing
-        L.use = L.use && (L.forced || (L.pixels > (weights || os < 1.25 ? 4.5e6 : 9e6) && L.plan.ball > 25.f));
+        L.use = L.use && (L.forced || (L.pixels > (weights || os < 1.25 ? 4.5e6 : 9e6) && L.plan.reach > 24.f));
         return L;
     }
     BrickLaunch L = weights ? scatter_layout<3, true>(B, P, N, os, cutoff) : scatter_layout<3, false>(B, P, N, os, cutoff);
@@ -320,16 +342,17 @@ BrickWork brick_work(const BrickLaunch& L, void* workspace) {
     w.header = (int*)workspace;
     w.items = (int4*)((char*)workspace + 256);
     w.recs = (float4*)((char*)workspace + 256 + L.item_bytes);
+    w.shifts = (float2*)(w.recs + 4 * (size_t)L.slices);
     w.outside = (int*)((char*)workspace + 256 + L.item_bytes + L.rec_bytes);
     return w;
 }
 
 template <int DIM>
 int brick_setup(const BrickLaunch& bl, const BrickWork& w, const Launch& L, const float* rot, const float* shifts, bool outside, cudaStream_t s) {
-    if (int rc = zero_async(w.header, 16, s)) return rc;
+    if (int rc = zero_async(w.header, 80, s)) return rc;
     const int64_t clusters = (int64_t)((bl.plan.n[0] + 7) / 8) * ((bl.plan.n[1] + 7) / 8) * ((bl.plan.n[2] + 3) / 4) * L.B;
     const int64_t slices = (L.B * L.P + 255) / 256;
-    brick_setup_kernel<DIM><<<(unsigned)(clusters > slices ? clusters : slices) + 1u, 256, 0, s>>>(rot, shifts, w, L.g, bl.plan, (int)L.B, outside ? 1 : 0);
+    brick_setup_kernel<DIM><<<(unsigned)(1 + clusters + slices), 256, 0, s>>>(rot, shifts, w, L.g, bl.plan, (int)L.B, outside ? 1 : 0);
     return check_launch("brick_setup launch");
 }
 
@@ -350,7 +373,9 @@ int launch_brick_scatter(const Launch& L, const BrickLaunch& bl, void* workspace
                          const float* shifts, float* vol, float* wvol, cudaStream_t s, float4* accum = nullptr) {
     using C = Scatter<DIM, WEIGHTS>;
     const BrickWork w = brick_work(bl, workspace);
-    if (int rc = brick_setup<DIM>(bl, w, L, rot, shifts, false, s)) return rc;
+    BrickLaunch kept = bl;
+    kept.plan.keep = L.g.half;
+    if (int rc = brick_setup<DIM>(kept, w, L, rot, shifts, false, s)) return rc;
     constexpr size_t smem = sizeof(typename C::Shared);
     static_assert((smem + 1024) * C::kBlocks <= 233472, "shared memory of an SM");
     const cudaError_t e = cudaFuncSetAttribute(brick_scatter_kernel<DIM, WEIGHTS, DUP, INTERLEAVED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -13,7 +13,7 @@
 // pay for finding them.
 //
 // A call runs as two launches:
-//   brick_setup_kernel   per slice a 48-byte record (matrix, shift, plane normal); per brick its work items
+//   brick_setup_kernel   per slice a 64-byte record (plane, half-plane, matrix, its rows); per brick its work items
 //   brick_*_kernel       persistent blocks take items (brick, range of slices) from a ticket counter
 // Nothing waits on another block.
 #pragma once
@@ -38,63 +38,119 @@ using GatherBrick = typename GatherBrickOf<DIM>::type;
 constexpr int kBrickSlots = 8;                              // slices a warp takes at a time
 constexpr float kBrickSlack = 0.06f;                        // slack of the linear estimates, in voxels
 
+// The samples of a rotated slice lie inside a ball, those of a matrix that stretches by s inside one s times as large.  The
+// bricks are listed in shells: 0 for rotations, l for slices that stretch by up to kStretch[l]; the shells beyond 0 are
+// worked on only when a call has slices that need them.  (Rotations alone and all else pixel by pixel, one slice per
+// block: 10,000 cubic slices of 128 x 65, all stretched by 1.01, took 6.84 ms where the plain kernel takes 3.96, from a
+// box-512 volume 14.2 against 3.34.)
+constexpr int kShells = 5;
+__host__ __device__ constexpr float brick_stretch(int shell) { return shell == 0 ? 1.f : shell == 1 ? 1.1f : shell == 2 ? 1.3f : shell == 3 ? 1.6f : 2.f; }
+
 // What the host derives from the sizes (see brick_plan in b200proj.cu).
 struct BrickPlan {
     int n[3];               // bricks along x (column), y (row), z (plane)
     int d[3];               // sample positions of a brick along them
     int lo[3];              // first sample position of the grid
-    float ball;             // sample positions of a rotated slice lie inside this radius
+    float reach;            // distance from the origin of the farthest sample of a rotated slice
+    int shells;             // of the grid
+    int at[kShells];        // where their work items start in the list
+    int keep;               // bricks beyond this coordinate are left out (scatters: nothing of them is stored)
     float density;          // expected pixels per brick and slice: density / max(r, ...) at radius r (2D: density)
     float per_slice;        // pixels of a slice inside the cutoff
     float target;           // pixels a work item should hold
-    int max_extra;          // items beyond one per brick that fit the list
+    int max_extra;          // items beyond one per brick that fit the list of a shell
     int wait_ms;            // after which a scatter's wait gives up
 };
 
-// Workspace layout: int header[4] {items, extra, ticket, gathers: pixels outside the cutoff, scatters: 1 when a wait gave
-// up}, int4 items[bricks * B + max_extra],
-// float4 records[3 * B * P], int outside[N * Nh].
+// Workspace layout: int header[20] {-, -, ticket, gathers: pixels outside the cutoff, scatters: 1 when a wait gave up; last
+// shell in use, -, -, -; items of each shell; extra items of each shell}, int4 items[shells], float4 records[4 * B * P],
+// float2 shifts[B * P], int outside[N * Nh].
 struct BrickWork {
     int* header;
     int4* items;
     float4* recs;
+    float2* shifts;
     int* outside;
 };
 
-struct SliceRec {           // 48 bytes
-    float4 a;               // n.x, n.y, n.z (plane normal; NaN: the slice is not for the bricks), m00
-    float4 b;               // m10, m20, m01, m11
-    float4 c;               // m21, s0, s1, -
+// A slice's record.  The columns a and b of its matrix map a pixel to a sample: x = os (kc a + kr b).
+struct SliceRec {           // 64 bytes
+    float4 a;               // unit normal of the plane (NaN: the slice is not for the bricks), then the unit vector
+    float4 b;               // in the plane along which kc grows at fixed kr b (2 more), a.x, a.y
+    float4 c;               // a.z, b.x, b.y, b.z
+    float4 d;               // v with v.a = 0, v.b = 1: a sample x of the slice is of row v.x / os; -
 };
 
-// A slice goes through the bricks when the two columns of its matrix that matter are orthonormal to 2e-5
-// (then its pixels stay inside the ball, and plane and half-plane tests with slack hold).
+// Plane, half-plane and shell of a slice; -1: not for the bricks.  Any two columns that are far from parallel and stretch by
+// no more than the last shell will do (then the linear estimates of the walk hold with their slack: they lose at most
+// a factor of 25 to cancellation, of 1e-7 of some 2,000 voxels).
 template <int DIM>
-__device__ __forceinline__ bool brick_slice_ok(const float* __restrict__ rm) {
-    if (DIM == 2) {
-        const float a0 = __ldg(rm + 0), b0 = __ldg(rm + 1), a1 = __ldg(rm + 2), b1 = __ldg(rm + 3);
-        return fabsf(a0 * a0 + a1 * a1 - 1.f) < 2e-5f && fabsf(b0 * b0 + b1 * b1 - 1.f) < 2e-5f && fabsf(a0 * b0 + a1 * b1) < 2e-5f;
+__device__ __forceinline__ int brick_slice_fit(const BrickPlan& pl, const float (&a)[3], const float (&b)[3], float (&n)[3], float (&h)[3], float (&v)[3]) {
+    const float aa = a[0] * a[0] + a[1] * a[1] + a[2] * a[2], bb = b[0] * b[0] + b[1] * b[1] + b[2] * b[2], ab = a[0] * b[0] + a[1] * b[1] + a[2] * b[2];
+    const float det = aa * bb - ab * ab, diff = aa - bb;
+    const float most = 0.5f * (aa + bb + sqrtf(diff * diff + 4.f * ab * ab)), least = det / most;       // squared singular values
+    if (!(most <= 4.f && least >= 0.04f * most && least >= 0.01f)) return -1;
+    const float inv = rsqrtf(det), t = ab / bb, len = rsqrtf(det / bb);
+    n[0] = (a[1] * b[2] - a[2] * b[1]) * inv;
+    n[1] = (a[2] * b[0] - a[0] * b[2]) * inv;
+    n[2] = DIM == 3 ? (a[0] * b[1] - a[1] * b[0]) * inv : 0.f;         // 2D: every tile is in the plane
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        h[q] = (a[q] - t * b[q]) * len;
+        v[q] = (aa * b[q] - ab * a[q]) / det;
     }
-    const float a0 = __ldg(rm + 0), a1 = __ldg(rm + 3), a2 = __ldg(rm + 6);
-    const float b0 = __ldg(rm + 1), b1 = __ldg(rm + 4), b2 = __ldg(rm + 7);
-    const float aa = a0 * a0 + a1 * a1 + a2 * a2, bb = b0 * b0 + b1 * b1 + b2 * b2, ab = a0 * b0 + a1 * b1 + a2 * b2;
-    return fabsf(aa - 1.f) < 2e-5f && fabsf(bb - 1.f) < 2e-5f && fabsf(ab) < 2e-5f;
+    const float far = sqrtf(most) * pl.reach;
+    for (int l = 0; l < pl.shells; ++l)
+        if (far <= brick_stretch(l) * pl.reach + 0.9f) return l;
+    return -1;
 }
+__device__ __forceinline__ bool brick_has_slice(const BrickWork& ws, int k) { return !isnan(__ldg(&ws.recs[4 * (size_t)k].x)); }
 
-__device__ __forceinline__ bool brick_in_ball(const BrickPlan& pl, int bx, int by, int bz, float& r_center) {
+// Shell of a brick; -1: none.
+__device__ __forceinline__ int brick_shell(const BrickPlan& pl, int bx, int by, int bz, float& r_center) {
     const int at[3] = {bx, by, bz};
     float near2 = 0.f, mid2 = 0.f;
+    bool out = false;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        const float x = (float)(pl.lo[a] + at[a] * pl.d[a]), n = fmaxf(fmaxf(x, -(x + (float)pl.d[a])), 0.f), c = x + 0.5f * (float)pl.d[a];
+        const int lo = pl.lo[a] + at[a] * pl.d[a];
+        const float x = (float)lo, n = fmaxf(fmaxf(x, -(x + (float)pl.d[a])), 0.f), c = x + 0.5f * (float)pl.d[a];
+        out = out || lo - 1 > pl.keep || lo + pl.d[a] + 1 < -pl.keep;
         near2 += n * n;
         mid2 += c * c;
     }
     r_center = sqrtf(mid2);
-    return near2 <= pl.ball * pl.ball;
+    if (out) return -1;
+    for (int l = 0; l < pl.shells; ++l) {
+        const float ball = brick_stretch(l) * pl.reach + 1.f;
+        if (near2 <= ball * ball) return l;
+    }
+    return -1;
 }
 
-// The pixels outside the cutoff, by one block: their offsets in a slice, row by row.
+// The work items of a call: those of the shells in use.
+__device__ __forceinline__ int brick_items(const BrickWork& ws) {
+    const int last = __ldg(ws.header + 4);
+    int n = 0;
+#pragma unroll
+    for (int l = 0; l < kShells; ++l) {
+        const int here = __ldg(ws.header + 8 + l);
+        n += l <= last ? here : 0;
+    }
+    return n;
+}
+__device__ __forceinline__ int4 brick_item(const BrickWork& ws, const BrickPlan& pl, int item) {
+    int at = -1;
+#pragma unroll
+    for (int l = 0; l < kShells; ++l) {
+        const int n = __ldg(ws.header + 8 + l);
+        if (at < 0 && item < n) at = pl.at[l] + item;
+        item -= n;
+    }
+    return __ldg(ws.items + at);
+}
+
+// The pixels outside the cutoff, by one block of 256 threads: their offsets in a slice, row by row.
 __device__ __forceinline__ void brick_list_outside(const SliceGeom& g, BrickWork ws) {
     __shared__ int row_at[2049];
     // first column outside: rad is monotonic in j, the estimate is at most one column late
@@ -104,84 +160,121 @@ __device__ __forceinline__ void brick_list_outside(const SliceGeom& g, BrickWork
         while (j < g.Nh && !(add_rn(kr2, mul_rn((float)j, (float)j)) > g.cutoff_sq)) ++j;
         return j;
     };
-    for (int i = threadIdx.x; i < g.N; i += blockDim.x) row_at[i + 1] = g.Nh - first_out(i);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        row_at[0] = 0;
-        for (int i = 0; i < g.N; ++i) row_at[i + 1] += row_at[i];
-        ws.header[3] = row_at[g.N];
-    }
-    __syncthreads();
-    for (int i = threadIdx.x >> 5; i < g.N; i += (int)blockDim.x >> 5) {
-        const int at = row_at[i], n = row_at[i + 1] - at;
-        for (int q = threadIdx.x & 31; q < n; q += 32) ws.outside[at + q] = i * g.Nh + g.Nh - n + q;
-    }
-}
-
-// Slice records (one thread per slice) and work items (one thread per brick and batch item).  header[0..2]
-// are zero on entry.  A brick's slices are split over as many items as bring one near pl.target pixels for
-// uniformly distributed poses (the density of pixels falls as 1 / r); the list has room for one item per
-// brick plus max_extra, of which a brick takes what is left.
-// Neighbouring bricks are neighbours in the list, so that they run at the same time: the runs of pixels that
-// they write into a row of a slice then meet in L2 before the row's sectors leave it.
-template <int DIM>
-__global__ void __launch_bounds__(256)
-brick_setup_kernel(const float* __restrict__ rot, const float* __restrict__ shifts, BrickWork ws, const SliceGeom g,
-                   const BrickPlan pl, int B, int list_outside) {
-    const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    if (t < g.BP) {
-        const int b = t / g.P, p = t - b * g.P;
-        const float* rm = pose_rot<DIM>(g, rot, b, p);
-        const float m00 = __ldg(rm + 0), m01 = __ldg(rm + 1), m10 = __ldg(rm + DIM), m11 = __ldg(rm + DIM + 1);
-        const float m20 = DIM == 3 ? __ldg(rm + 6) : 0.f, m21 = DIM == 3 ? __ldg(rm + 7) : 0.f;
-        float s0 = 0.f, s1 = 0.f;
-        if (g.has_shift) {
-            const float* s = pose_shift(g, shifts, b, p);
-            s0 = __ldg(s);
-            s1 = __ldg(s + 1);
-        }
-        float nx = m10 * m21 - m20 * m11;
-        const float ny = m20 * m01 - m00 * m21, nz = DIM == 3 ? m00 * m11 - m10 * m01 : 0.f;       // 2D: every tile is in the plane
-        if (!brick_slice_ok<DIM>(rm)) nx = __int_as_float(0x7fffffff);
-        ws.recs[3 * t + 0] = make_float4(nx, ny, nz, m00);
-        ws.recs[3 * t + 1] = make_float4(m10, m20, m01, m11);
-        ws.recs[3 * t + 2] = make_float4(m21, s0, s1, 0.f);
-    }
-    if (blockIdx.x == gridDim.x - 1) {
-        if (list_outside) brick_list_outside(g, ws);
-        return;
-    }
-    // work items: a block takes a cluster of 8 x 8 x 4 neighbouring bricks of one batch item
-    __shared__ int warp_sum[8], block_at, upto[257], code[256];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int cx = (pl.n[0] + 7) / 8, cy = (pl.n[1] + 7) / 8, cz = (pl.n[2] + 3) / 4;
-    if ((int)blockIdx.x >= cx * cy * cz * B) return;
-    const int b = (int)blockIdx.x / (cx * cy * cz), k = (int)blockIdx.x - b * (cx * cy * cz);
-    const int bx = k % cx * 8 + (threadIdx.x & 7), by = k / cx % cy * 8 + (threadIdx.x >> 3 & 7), bz = k / (cx * cy) * 4 + (threadIdx.x >> 6);
-    int parts = 0;
-    float r;
-    if (bx < pl.n[0] && by < pl.n[1] && bz < pl.n[2] && brick_in_ball(pl, bx, by, bz, r)) {
-        const float expected = fminf(DIM == 3 ? pl.density / fmaxf(r, 0.42f * (float)pl.d[0]) : pl.density, pl.per_slice) * (float)g.P;
-        parts = max(1, min((int)(expected / pl.target + 0.5f), (g.P + 31) / 32));
-        if (parts > 1) parts = 1 + max(0, min(parts - 1, pl.max_extra - atomicAdd(ws.header + 1, parts - 1)));
-    }
-    int incl = parts;
+    // row_at[i + 1] = pixels of rows 0 .. i: 256 threads with a run of rows each
+    __shared__ int warp_rows[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, per = (g.N + 255) / 256, row0 = (int)threadIdx.x * per, row1 = min(row0 + per, g.N);
+    int sum = 0;
+    for (int i = row0; i < row1; ++i) sum += g.Nh - first_out(i);
+    int incl = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const int up = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += up;
     }
-    if (lane == 31) warp_sum[warp] = incl;
+    if (lane == 31) warp_rows[warp] = incl;
     __syncthreads();
-    if (threadIdx.x == 0) {
+    int at = incl - sum;
+    for (int w = 0; w < warp; ++w) at += warp_rows[w];
+    if (threadIdx.x == 0) row_at[0] = 0;
+    for (int i = row0; i < row1; ++i) row_at[i + 1] = at += g.Nh - first_out(i);
+    __syncthreads();
+    if (threadIdx.x == 0) ws.header[3] = row_at[g.N];
+    for (int i = warp; i < g.N; i += 8) {
+        const int first = row_at[i], n = row_at[i + 1] - first;
+        for (int q = lane; q < n; q += 32) ws.outside[first + q] = i * g.Nh + g.Nh - n + q;
+    }
+}
+
+// Slice records (a thread per slice) and work items (a thread per brick and batch item).  The header
+// is zero on entry.  A brick's slices are split over as many items as bring one near pl.target pixels for
+// uniformly distributed poses (the density of pixels falls as 1 / r); a shell's list has room for one item per
+// brick plus max_extra, of which a brick takes what is left.
+// Neighbouring bricks are neighbours in the list, so that they run at the same time: the runs of pixels that
+// they write into a row of a slice then meet in L2 before the row's sectors leave it.
+template <int DIM>
+__global__ void __launch_bounds__(256)
+brick_setup_kernel(const float* __restrict__ rot, const float* __restrict__ shifts, BrickWork ws, const SliceGeom g, const BrickPlan pl, int B, int list_outside) {
+    // block 0: the pixels outside the cutoff; then one block per cluster of bricks and batch item; then the slices
+    if (blockIdx.x == 0) {
+        if (list_outside) brick_list_outside(g, ws);
+        return;
+    }
+    const int cx = (pl.n[0] + 7) / 8, cy = (pl.n[1] + 7) / 8, cz = (pl.n[2] + 3) / 4, clusters = cx * cy * cz * B;
+    if ((int)blockIdx.x > clusters) {
+        const int t = ((int)blockIdx.x - 1 - clusters) * 256 + (int)threadIdx.x;
+        int shell = 0;
+        if (t < g.BP) {
+            const int b = t / g.P, p = t - b * g.P;
+            const float* rm = pose_rot<DIM>(g, rot, b, p);
+            const float ma[3] = {__ldg(rm + 0), __ldg(rm + DIM), DIM == 3 ? __ldg(rm + 6) : 0.f}, mb[3] = {__ldg(rm + 1), __ldg(rm + DIM + 1), DIM == 3 ? __ldg(rm + 7) : 0.f};
+            float n[3] = {0.f, 0.f, 0.f}, h[3] = {0.f, 0.f, 0.f}, v[3] = {0.f, 0.f, 0.f};
+            shell = brick_slice_fit<DIM>(pl, ma, mb, n, h, v);
+            if (shell < 0) n[0] = __int_as_float(0x7fffffff);
+            ws.recs[4 * (size_t)t + 0] = make_float4(n[0], n[1], n[2], h[0]);
+            ws.recs[4 * (size_t)t + 1] = make_float4(h[1], h[2], ma[0], ma[1]);
+            ws.recs[4 * (size_t)t + 2] = make_float4(ma[2], mb[0], mb[1], mb[2]);
+            ws.recs[4 * (size_t)t + 3] = make_float4(v[0], v[1], v[2], 0.f);
+            if (g.has_shift) {
+                const float* s = pose_shift(g, shifts, b, p);
+                ws.shifts[t] = make_float2(__ldg(s), __ldg(s + 1));
+            }
+        }
+        shell = __reduce_max_sync(0xffffffffu, shell);
+        if (shell > 0 && (threadIdx.x & 31) == 0) atomicMax(ws.header + 4, shell);
+        return;
+    }
+    // work items: a block takes a cluster of 8 x 8 x 4 neighbouring bricks of one batch item
+    __shared__ int warp_sum[8], shell_sum[kShells][8], block_at[kShells], upto[257], code[256], start[256];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int b = ((int)blockIdx.x - 1) / (cx * cy * cz), k = (int)blockIdx.x - 1 - b * (cx * cy * cz);
+    const int bx = k % cx * 8 + (threadIdx.x & 7), by = k / cx % cy * 8 + (threadIdx.x >> 3 & 7), bz = k / (cx * cy) * 4 + (threadIdx.x >> 6);
+    int parts = 0;
+    float r;
+    const int mine = bx < pl.n[0] && by < pl.n[1] && bz < pl.n[2] ? brick_shell(pl, bx, by, bz, r) : -1;
+    if (mine >= 0) {
+        const float expected = fminf(DIM == 3 ? pl.density / fmaxf(r, 0.42f * (float)pl.d[0]) : pl.density, pl.per_slice) * (float)g.P;
+        parts = max(1, min((int)(expected / pl.target + 0.5f), (g.P + 31) / 32));
+    }
+    auto scan = [&](int n) {
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int up = __shfl_up_sync(0xffffffffu, n, o);
+            if (lane >= o) n += up;
+        }
+        return n;
+    };
+    // what the list of extra items has room for, and the place of the brick's first item in its shell's list
+    int place = 0;
+    for (int l = 0; l < pl.shells; ++l) {
+        int sum = 0;
+        if (__any_sync(0xffffffffu, mine == l)) {
+            const int extra = mine == l ? parts - 1 : 0, extra_upto = scan(extra);
+            int taken = 0;
+            if (lane == 31 && extra_upto > 0) taken = atomicAdd(ws.header + 8 + kShells + l, extra_upto);
+            taken = __shfl_sync(0xffffffffu, taken, 31) + extra_upto - extra;
+            if (mine == l) parts = 1 + max(0, min(extra, pl.max_extra - taken));
+            const int n = mine == l ? parts : 0, upto_me = scan(n);
+            if (mine == l) place = upto_me - n;
+            sum = __shfl_sync(0xffffffffu, upto_me, 31);
+        }
+        if (lane == l) shell_sum[l][warp] = sum;
+    }
+    const int incl = scan(parts);
+    if (lane == 31) warp_sum[warp] = incl;
+    if (__syncthreads_or(parts) == 0) return;
+    if (threadIdx.x < pl.shells) {
+        int sum = 0;
+        for (int w = 0; w < 8; ++w) { const int n = shell_sum[threadIdx.x][w]; shell_sum[threadIdx.x][w] = sum; sum += n; }
+        if (sum > 0) block_at[threadIdx.x] = pl.at[threadIdx.x] + atomicAdd(ws.header + 8 + threadIdx.x, sum);
+    } else if (threadIdx.x == 32) {
         int sum = 0;
         for (int w = 0; w < 8; ++w) { const int n = warp_sum[w]; warp_sum[w] = sum; sum += n; }
         upto[256] = sum;
-        block_at = atomicAdd(ws.header, sum);
     }
     __syncthreads();
     upto[threadIdx.x] = warp_sum[warp] + incl;
     code[threadIdx.x] = bx | by << 10 | bz << 20;
+    start[threadIdx.x] = mine >= 0 ? block_at[mine] + shell_sum[mine][warp] + place : 0;
     __syncthreads();
     // a brick's slices in `parts` nearly equal shares; all threads write items, a thread finds the brick of its item by search
     for (int o = threadIdx.x; o < upto[256]; o += 256) {
@@ -191,7 +284,7 @@ brick_setup_kernel(const float* __restrict__ rot, const float* __restrict__ shif
             if (upto[t0 + step - 1] <= o) t0 += step;
         const int before = t0 ? upto[t0 - 1] : 0, n = upto[t0] - before, q = o - before;
         const int share = g.P / n, more = g.P - share * n, first = b * g.P + q * share + min(q, more);
-        ws.items[block_at + o] = make_int4(code[t0], b, first, first + share + (q < more ? 1 : 0));
+        ws.items[start[t0] + q] = make_int4(code[t0], b, first, first + share + (q < more ? 1 : 0));
     }
 }
 
@@ -343,7 +436,7 @@ __device__ __forceinline__ void brick_gather(const float2* sm, int lx, int ly, i
 // A warp's working set of the slice walk.
 struct BrickWarp {
     uint2 segs[64];                 // rows of slices: {slot << 16 | (kr & 0xffff), ja << 16 | length}
-    float4 slots[kBrickSlots][3];   // the slices' records
+    float4 slots[kBrickSlots][2];   // the slices' matrices and shifts {a.x, a.y, a.z, b.x}, {b.y, b.z, shift}
     int slice[kBrickSlots];         // and their indices
 };
 
@@ -358,7 +451,7 @@ struct BrickBlock {
 // The slice walk of one work item: calls body(active, slice record slot, i, j, pixel, lx, ly, lz) with all 32
 // lanes for windows of 32 candidate pixels; `active` lanes hold a pixel whose sample position lies in the brick.
 // Every pixel of the item's slices inside the brick is visited exactly once.
-//   1. all threads test the slices' planes (and half-planes: columns j >= 0 only) against the brick,
+//   1. all threads test the slices' planes and half-planes (columns j >= 0) against the brick,
 //   2. a warp takes a few slices from the list of hits and flattens their rows, one row per lane: row kr meets the
 //      brick in one run of columns, clipped with linear estimates plus slack,
 //   3. the non-empty runs of 32 rows are flattened into one index space, so that the windows are full although
@@ -366,7 +459,7 @@ struct BrickBlock {
 // The whole block walks together, or (BLOCK::kWalkers == 1) every warp by itself over each `parts`-th slice,
 // so that it never waits for another warp.
 template <typename D, typename BLOCK, typename Body>
-__device__ __forceinline__ void brick_walk(const SliceGeom& g, const float4* __restrict__ recs, BLOCK& sb,
+__device__ __forceinline__ void brick_walk(const SliceGeom& g, const float4* __restrict__ recs, const float2* __restrict__ shifts, BLOCK& sb,
                                            int X0, int Y0, int Z0, int first, int last, int part, int parts, Body body) {
     constexpr bool kAlone = BLOCK::kWalkers == 1;
     constexpr int kThreads = BLOCK::kWalkers * 32;
@@ -390,10 +483,10 @@ __device__ __forceinline__ void brick_walk(const SliceGeom& g, const float4* __r
                 const int k = k_next + thread * parts;
                 bool hit = false;
                 if (k < last) {
-                    const float4 a = __ldg(recs + 3 * (size_t)k);
+                    const float4 a = __ldg(recs + 4 * (size_t)k);
                     hit = fabsf(a.x * cx + a.y * cy + a.z * cz) <= fabsf(a.x) * hx + fabsf(a.y) * hy + fabsf(a.z) * hz + kBrickSlack;
                     if (hit) {
-                        const float2 e = __ldg(reinterpret_cast<const float2*>(recs + 3 * (size_t)k + 1));
+                        const float2 e = __ldg(reinterpret_cast<const float2*>(recs + 4 * (size_t)k + 1));
                         hit = a.w * cx + e.x * cy + e.y * cz + fabsf(a.w) * hx + fabsf(e.x) * hy + fabsf(e.y) * hz >= -kBrickSlack;
                     }
                 }
@@ -426,12 +519,13 @@ __device__ __forceinline__ void brick_walk(const SliceGeom& g, const float4* __r
             int row_count = 0, k_lo = 0;
             if (lane < slices) {
                 const int slice = sb.hits[h + lane];
-                const float4 a = __ldg(recs + 3 * (size_t)slice), e = __ldg(recs + 3 * (size_t)slice + 1), f = __ldg(recs + 3 * (size_t)slice + 2);
+                const float4 e = __ldg(recs + 4 * (size_t)slice + 1), f = __ldg(recs + 4 * (size_t)slice + 2), v = __ldg(recs + 4 * (size_t)slice + 3);
+                const float2 s = g.has_shift ? __ldg(shifts + slice) : make_float2(0.f, 0.f);
                 sw.slice[lane] = slice;
-                sw.slots[lane][0] = a;
-                sw.slots[lane][1] = e;
-                sw.slots[lane][2] = f;
-                const float mid = e.z * cx + e.w * cy + f.x * cz, reach = fabsf(e.z) * hx + fabsf(e.w) * hy + fabsf(f.x) * hz + kBrickSlack;
+                sw.slots[lane][0] = make_float4(e.z, e.w, f.x, f.y);
+                sw.slots[lane][1] = make_float4(f.z, f.w, s.x, s.y);
+                const float mid = v.x * cx + v.y * cy + v.z * cz;
+                const float reach = fabsf(v.x) * (hx + kBrickSlack) + fabsf(v.y) * (hy + kBrickSlack) + fabsf(v.z) * (hz + kBrickSlack);
                 k_lo = max((int)ceilf((mid - reach) * inv_os), 1 - g.N / 2);
                 row_count = max(1, min((int)floorf((mid + reach) * inv_os), g.N / 2) - k_lo + 1);
             }
@@ -453,7 +547,6 @@ __device__ __forceinline__ void brick_walk(const SliceGeom& g, const float4* __r
                 const int kr = row0 + lane + __shfl_sync(kFull, kr_start, slot);
                 const float krf = (float)kr;
                 const float4 ra = sw.slots[slot][0], rb = sw.slots[slot][1];
-                const float m21 = sw.slots[slot][2].x;
                 const float room = g.cutoff_sq - krf * krf;
                 int ja_i = 0, len = 0;
                 if (row0 + lane < rows && room >= 0.f && kr <= g.N / 2) {       // (a slice without rows here still counts one)
@@ -470,9 +563,9 @@ __device__ __forceinline__ void brick_walk(const SliceGeom& g, const float4* __r
                             jb = fminf(jb, fmaxf(x0, x1));
                         }
                     };
-                    clip(ra.w, rb.z, (float)X0, (float)D::x);
-                    clip(rb.x, rb.w, (float)Y0, (float)D::y);
-                    if (D::kDim == 3) clip(rb.y, m21, (float)Z0, (float)D::z);
+                    clip(ra.x, ra.w, (float)X0, (float)D::x);
+                    clip(ra.y, rb.x, (float)Y0, (float)D::y);
+                    if (D::kDim == 3) clip(ra.z, rb.y, (float)Z0, (float)D::z);
                     ja_i = (int)ceilf(ja);
                     len = jb >= ja ? (int)floorf(jb) - ja_i + 1 : 0;
                 }
@@ -504,7 +597,6 @@ __device__ __forceinline__ void brick_walk(const SliceGeom& g, const float4* __r
                 const int j = k0 + lane + __shfl_sync(kFull, ja_start, src);
                 const int kr = (int)(short)(sk & 0xffffu), slot = (int)(sk >> 16);
                 const float4 ra = sw.slots[slot][0], rb = sw.slots[slot][1];
-                const float m21 = sw.slots[slot][2].x;
                 Pixel px;
                 px.kr = (float)kr;
                 px.kc = (float)j;
@@ -515,9 +607,9 @@ __device__ __forceinline__ void brick_walk(const SliceGeom& g, const float4* __r
                     px.sc = (float)((double)px.kc * g.os);
                     px.sr = (float)((double)px.kr * g.os);
                 }
-                px.c = add_rn(mul_rn(ra.w, px.sc), mul_rn(rb.z, px.sr));
-                px.r = add_rn(mul_rn(rb.x, px.sc), mul_rn(rb.w, px.sr));
-                px.d = D::kDim == 3 ? add_rn(mul_rn(rb.y, px.sc), mul_rn(m21, px.sr)) : 0.f;
+                px.c = add_rn(mul_rn(ra.x, px.sc), mul_rn(ra.w, px.sr));
+                px.r = add_rn(mul_rn(ra.y, px.sc), mul_rn(rb.x, px.sr));
+                px.d = D::kDim == 3 ? add_rn(mul_rn(ra.z, px.sc), mul_rn(rb.y, px.sr)) : 0.f;
                 int lx = (int)floorf(px.c) - X0, ly = (int)floorf(px.r) - Y0, lz = D::kDim == 3 ? (int)floorf(px.d) - Z0 : 0;
                 const float rad = add_rn(mul_rn(px.kr, px.kr), mul_rn(px.kc, px.kc));
                 const bool active = k0 + lane < total && (unsigned)lx < (unsigned)D::x && (unsigned)ly < (unsigned)D::y &&
@@ -546,15 +638,15 @@ __device__ __forceinline__ void brick_save(const SliceGeom& g, float2* __restric
     }
 }
 
-// What the bricks leave of a slice: zeros outside the cutoff, or -- when its matrix is not (nearly) a rotation, so
-// that its pixels may lie anywhere -- the whole slice, by the plain gather.
+// What the bricks leave of a slice: zeros outside the cutoff, or -- when its matrix is nearly singular or stretches
+// beyond the shells -- the whole slice, by the plain gather.
 template <int DIM, bool CUBIC, bool SAVE>
 __device__ __forceinline__ void brick_rest(const SliceGeom& g, const BrickWork& ws, int k, const float2* __restrict__ rec, const float* __restrict__ rot,
                                            const float* __restrict__ shifts, float2* __restrict__ out, float2* __restrict__ derivs) {
     const int b = k / g.P, p = k - b * g.P;
     const float* rm = pose_rot<DIM>(g, rot, b, p);
     const size_t base = (size_t)k * (size_t)g.slice_pixels;
-    if (brick_slice_ok<DIM>(rm)) {
+    if (brick_has_slice(ws, k)) {
         const int n = __ldg(ws.header + 3);
         for (int q = threadIdx.x; q < n; q += kBlockThreads) __stcs(out + (base + (size_t)__ldg(ws.outside + q)), make_float2(0.f, 0.f));
         return;
@@ -591,7 +683,7 @@ brick_forw_kernel(const float2* __restrict__ rec, const float* __restrict__ rot,
     extern __shared__ __align__(16) unsigned char dyn[];
     float2* sm = reinterpret_cast<float2*>(dyn);
     GatherBlock& sb = *reinterpret_cast<GatherBlock*>(dyn + sizeof(float2) * BrickShape<DIM, CUBIC>::kVoxels);
-    const int items = __ldg(ws.header);
+    const int items = brick_items(ws);
     while (true) {
         __syncthreads();
         if (threadIdx.x == 0) sb.item = atomicAdd(ws.header + 2, 1);
@@ -601,18 +693,18 @@ brick_forw_kernel(const float2* __restrict__ rec, const float* __restrict__ rot,
         // beside its brick an item does its share of the slices' rest, whose stores overlap the brick's staging
         for (int k = (int)((long long)g.BP * item / items), k_end = (int)((long long)g.BP * (item + 1) / items); k < k_end; ++k)
             brick_rest<DIM, CUBIC, SAVE>(g, ws, k, rec, rot, shifts, out, derivs);
-        const int4 it = __ldg(ws.items + item);
+        const int4 it = brick_item(ws, pl, item);
         const int X0 = pl.lo[0] + (it.x & 1023) * GatherBrick<DIM>::x, Y0 = pl.lo[1] + ((it.x >> 10) & 1023) * GatherBrick<DIM>::y, Z0 = pl.lo[2] + (it.x >> 20) * GatherBrick<DIM>::z;
         brick_stage<DIM, CUBIC>(g, rec + (size_t)it.y * g.vol_elems, sm, X0, Y0, Z0);
         const BrickWarp& sw = sb.warp[threadIdx.x >> 5];
-        brick_walk<GatherBrick<DIM>>(g, ws.recs, sb, X0, Y0, Z0, it.z, it.w, 0, 1,
+        brick_walk<GatherBrick<DIM>>(g, ws.recs, ws.shifts, sb, X0, Y0, Z0, it.z, it.w, 0, 1,
                    [&](bool active, int slot, int i, int j, const Pixel& px, int lx, int ly, int lz) {
             float2 v, gc, gr, gd;
             brick_gather<DIM, CUBIC, SAVE>(sm, lx, ly, lz, px.c - floorf(px.c), px.r - floorf(px.r), DIM == 3 ? px.d - floorf(px.d) : 0.f, v, gc, gr, gd);
             if (!active) return;
             if (g.has_shift) {
-                const float4 rc = sw.slots[slot][2];
-                const float2 ph = phase_ramp(g, px, rc.y, rc.z);
+                const float4 rc = sw.slots[slot][1];
+                const float2 ph = phase_ramp(g, px, rc.z, rc.w);
                 v = cmul(v, ph);
                 if (SAVE) {
                     gc = cmul(gc, ph);

@@ -326,7 +326,7 @@ brick_scatter_kernel(const float2* __restrict__ proj, const float* __restrict__ 
     if (threadIdx.x == 0) sh.gave_up = 0;
     int slot = 0, taken = 0;                                // adding warps: next chunk of the ring, its parity, chunks taken
     unsigned parity = 0;
-    const int items = __ldg(ws.header);
+    const int items = brick_items(ws);
     bool lost = false;                                      // a wait of this block gave up: its rings are of no use any more
     while (true) {
         __syncthreads();
@@ -340,8 +340,7 @@ brick_scatter_kernel(const float2* __restrict__ proj, const float* __restrict__ 
         // the item's share of the slices that are not for the bricks: plain scatter
         for (int k = (int)((long long)g.BP * item / items), k_end = (int)((long long)g.BP * (item + 1) / items); k < k_end; ++k) {
             const int b = k / g.P, p = k - b * g.P;
-            const float* rm = pose_rot<DIM>(g, rot, b, p);
-            if (brick_slice_ok<DIM>(rm)) continue;
+            if (brick_has_slice(ws, k)) continue;
             const int nj = (g.Nh + 7) / 8, ni = (g.N + 3) / 4;
             for (int patch = warp; patch < ni * nj; patch += C::kThreads / 32) {
                 BlockWork w;
@@ -360,7 +359,7 @@ brick_scatter_kernel(const float2* __restrict__ proj, const float* __restrict__ 
                                                                   INTERLEAVED ? accum + at : nullptr, px, active, v, wv);
             }
         }
-        const int4 it = __ldg(ws.items + item);
+        const int4 it = brick_item(ws, pl, item);
         const int X0 = pl.lo[0] + (it.x & 1023) * C::Brick::x, Y0 = pl.lo[1] + ((it.x >> 10) & 1023) * C::Brick::y, Z0 = pl.lo[2] + (it.x >> 20) * C::Brick::z;
         if (!lost && warp < C::kWalkers) {
             const BrickWarp& sw = sh.walk[warp].warp[0];
@@ -418,7 +417,7 @@ brick_scatter_kernel(const float2* __restrict__ proj, const float* __restrict__ 
                     }
                 }
             };
-            brick_walk<typename C::Brick>(g, ws.recs, sh.walk[warp], X0, Y0, Z0, it.z, it.w, warp, C::kWalkers,
+            brick_walk<typename C::Brick>(g, ws.recs, ws.shifts, sh.walk[warp], X0, Y0, Z0, it.z, it.w, warp, C::kWalkers,
                                           [&](bool active, int slot_, int i, int j, const Pixel& px, int lx, int ly, int lz) {
                 active = active && !(j == 0 && i >= g.N / 2);
                 float2 v = make_float2(0.f, 0.f);
@@ -438,8 +437,8 @@ brick_scatter_kernel(const float2* __restrict__ proj, const float* __restrict__ 
                 h_v = v;
                 h_w = w;
                 if (g.has_shift) {
-                    const float4 rc = sw.slots[slot_][2];
-                    h_ph = phase_ramp(g, px, rc.y, rc.z);
+                    const float4 rc = sw.slots[slot_][1];
+                    h_ph = phase_ramp(g, px, rc.z, rc.w);
                 }
             });
             put();
