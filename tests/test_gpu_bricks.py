@@ -9,7 +9,7 @@ from pathlib import Path
 import pytest
 import torch
 
-from cases import Case, TOL_ATOMIC, TOL_FORWARD, axis_aligned_rotations, make_inputs, rel_err
+from cases import Case, TOL_ATOMIC, TOL_FORWARD, axis_aligned_rotations, make_inputs, random_rotations_2d, random_rotations_3d, rel_err
 
 pytestmark = pytest.mark.gpu
 ROOT = Path(__file__).resolve().parent.parent
@@ -61,6 +61,10 @@ def check_dim(names, dim):
             t, kw = _inputs(dim, size, seed)
             N, os_, cutoff = size[2], size[4], size[5]
             want = reference(t["rec"], t["rot"], t["shifts"], [N, N], interp, os_, cutoff)
+            sizes = (dim, size[0], size[1], N, tp.ops._interp_code(interp))
+            lib, radius = tp._abi.load(), N / 2.0 if cutoff is None else cutoff
+            assert (interp == "linear" and dim == 2) or lib.b200proj_project_workspace_bytes(*sizes, 0, os_, radius) > 0, "the bricks are not forced on"
+            assert interp == "linear" or all(lib.b200proj_scatter_workspace_bytes(*sizes, w, os_, radius) > 0 for w in (0, 1))
             shifts = t["shifts"].cuda() if t["shifts"] is not None else None
             if "forward" in names:
                 got = project(t["rec"].cuda(), t["rot"].cuda(), shifts, interpolation=interp, **kw)
@@ -190,3 +194,63 @@ def test_scatters_choose_copies_by_the_reductions_per_byte(dim, interp, P, copie
     forw, ref = (tp.backproject_2d_forw, port.backproject_2d_forw) if dim == 2 else (tp.backproject_2d_to_3d_forw, port.backproject_2d_to_3d_forw)
     data, _ = forw(t["proj"].cuda(), t["rot"].cuda(), None, t["shifts"].cuda(), interpolation=interp, oversampling=1.5)
     assert rel_err(data, ref(t["proj"], None, t["rot"], t["shifts"], interp, 1.5, None)[0]) <= TOL_ATOMIC
+
+
+def _one_plane(t, share):
+    """Every `share`-th pose becomes an in-plane turn of one and the same plane: a few bricks get all of its pixels."""
+    turns = torch.linspace(0, 6.2, t["rot"][:, ::share].shape[1])
+    t["rot"][:, ::share, :2, :2] = torch.stack([turns.cos(), -turns.sin(), turns.sin(), turns.cos()], 1).view(1, -1, 2, 2)
+    t["rot"][:, ::share, 2] = torch.tensor([0.0, 0.0, 1.0])
+    t["rot"][:, ::share, :, 2] = torch.tensor([0.0, 0.0, 1.0])
+
+
+@pytest.mark.parametrize("os_,P,share", [(2.0, 3000, 1), (2.0, 3001, 3), (1.0, 2999, 2)])
+def test_scatters_that_run_in_bricks_by_themselves_match_the_oracle(os_, P, share):
+    """Cubic 3D calls just above the sizes from which bricks are chosen: several items per brick and per block."""
+    import torch_projectors_b200 as tp
+    from oracle import port
+    N, R = 32, int(32 * os_)
+    t = make_inputs(Case("rings", 3, "cubic", 1, P, N, R, os_, None, 1, 1, shift_range=4.0, seed=P, special_poses=False))
+    _one_plane(t, share)
+    lib, cubic = tp._abi.load(), tp._abi.CUBIC
+    assert all(lib.b200proj_scatter_workspace_bytes(3, 1, P, N, cubic, w, os_, N / 2.0) > 0 for w in (0, 1))
+    c = {k: v.cuda() for k, v in t.items()}
+    kw = dict(interpolation="cubic", oversampling=os_)
+    got = tp.project_3d_to_2d_back(c["proj"], c["rec"], c["rot"], c["shifts"], **kw)
+    assert rel_err(got, port.project_3d_to_2d_back(t["proj"], t["rec"], t["rot"], t["shifts"], "cubic", os_, None)[0]) <= TOL_ATOMIC
+    for weights in (None, "weights"):
+        data, wrec = tp.backproject_2d_to_3d_forw(c["proj"], c["rot"], c[weights] if weights else None, c["shifts"], **kw)
+        ref, wref = port.backproject_2d_to_3d_forw(t["proj"], t[weights] if weights else None, t["rot"], t["shifts"], "cubic", os_, None)
+        assert rel_err(data, ref) <= TOL_ATOMIC and (weights is None or rel_err(wrec, wref) <= TOL_ATOMIC)
+
+
+@pytest.mark.parametrize("dim,N,P", [(3, 64, 12000), (3, 80, 7919), (2, 128, 3001)])
+def test_long_runs_of_the_scatter_rings_match_double_precision(dim, N, P):
+    """Enough slices that a walking warp refills its list of hits and rings and sums are used over many items of a block,
+    against the double-precision kernels (which do not run in bricks).  Their sample positions are not rounded to
+    single precision: up to 4 * 160 * 2^-24 = 4e-5 voxels apart, times slopes of the taps below 1.3, of random signs."""
+    import torch_projectors_b200 as tp
+    lib, cubic = tp._abi.load(), tp._abi.CUBIC
+    gen = torch.Generator("cuda").manual_seed(N)
+    real = lambda *s: torch.rand(*s, generator=gen, device="cuda")  # noqa: E731
+    proj = torch.randn(1, P, N, N // 2 + 1, dtype=torch.complex64, generator=gen, device="cuda")
+    w, sh = real(1, P, N, N // 2 + 1), real(1, P, 2) * 8 - 4
+    rot = {"rot": (random_rotations_3d if dim == 3 else random_rotations_2d)(P, torch.Generator().manual_seed(N)).view(1, P, dim, dim)}
+    if dim == 3:
+        _one_plane(rot, 3)
+    rot = rot["rot"].cuda()
+    assert all(lib.b200proj_scatter_workspace_bytes(dim, 1, P, N, cubic, k, 2.0, N / 2.0) > 0 for k in (0, 1))
+    forw = tp.backproject_2d_to_3d_forw if dim == 3 else tp.backproject_2d_forw
+    back = tp.project_3d_to_2d_back if dim == 3 else tp.project_2d_back
+    kw = dict(interpolation="cubic", oversampling=2.0)
+    d, dw = forw(proj.to(torch.complex128), rot.double(), w.double(), sh.double(), **kw)
+    data, wrec = forw(proj, rot, w, sh, **kw)
+    assert rel_err(data, d) <= TOL_ATOMIC and rel_err(wrec, dw) <= TOL_ATOMIC
+    assert rel_err(forw(proj, rot, None, sh, **kw)[0], d) <= TOL_ATOMIC
+    rec = torch.zeros_like(data)
+    assert rel_err(back(proj, rec, rot, sh, **kw), back(proj.to(torch.complex128), rec.to(torch.complex128), rot.double(), sh.double(), **kw)) <= TOL_ATOMIC
+    if dim == 3:
+        acc = tp.new_backprojection_accumulator(1, 2 * N, "cuda")
+        tp.backproject_2d_to_3d_accumulate_interleaved_(acc, proj, rot, w, sh, **kw)
+        d2, w2 = tp.fold_backprojection_accumulator(acc)
+        assert rel_err(d2, d) <= TOL_ATOMIC and rel_err(w2, dw) <= TOL_ATOMIC
