@@ -557,7 +557,7 @@ def autograd_step_workload(args):
             "config": {"workload": STEP["name"], "l2": "inputs (539 MB volume, 1.08 GB projections) exceed L2; 256 MiB flush before every step"},
             "kernels_ms": ({"brick_forw_kernel<3,cubic,records> (+ setup)": f, ("pose_grad_saved_kernel" if args.fixed_volume else "brick_scatter_kernel<3> + pose_grad_saved_kernel (+ setup, clears)"): bw,
                             "loss and its gradient (torch elementwise)": ms_per_step - f - bw} if saving else
-                           {"project_forw_kernel<3,cubic>": f, "project_back_kernel<3,cubic,rot,shift> (+ memsets)": bw,
+                           {"brick_forw_kernel<3,cubic> (+ setup)": f, "project_back_kernel<3,cubic,rot,shift> (+ clears)": bw,
                             "loss and its gradient (torch elementwise)": ms_per_step - f - bw}),
             "saved_derivatives": saving, "fixed_volume": bool(args.fixed_volume),
             "roofline": {"bound": "hbm", "kernel": "project_forw + project_back (op time only)", "achieved": achieved, "peak": peak,

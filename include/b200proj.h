@@ -111,8 +111,8 @@ size_t b200proj_scatter_workspace_bytes(int dim, int64_t B, int64_t P, int64_t N
                                         double oversampling, double fourier_radius_cutoff);
 /* Workspace of the backward passes of the projection (b200proj_project_{2d,3d_to_2d}_back_ws with grad_rec,
  * b200proj_project_2d_back_saved_ws, b200proj_project_3d_to_2d_back_records): the larger calls above, and copies
- * of a small reconstruction over which the scatter is spread (reductions onto less than ~2 MB run at
- * half the rate).  pose_gradients != 0: of a _back_ws call that also computes grad_rot or grad_shifts. */
+ * of a small reconstruction over which the scatter of many slices is spread (reductions that pile up on few
+ * sectors run at half the rate or less).  pose_gradients != 0: of a _back_ws call that also computes grad_rot or grad_shifts. */
 size_t b200proj_gradient_workspace_bytes(int dim, int64_t B, int64_t R, int64_t P, int64_t N, int interpolation,
                                          int pose_gradients, double oversampling, double fourier_radius_cutoff);
 int b200proj_project_2d_forw_ws(const float* rec, int64_t B, int64_t R,
@@ -230,8 +230,10 @@ int b200proj_project_3d_to_2d_back(const float* grad_proj, const float* rec, int
  * b200proj_backproject_workspace_bytes(...) bytes, or NULL.  With weights and a workspace the
  * kernel accumulates data and weight of each voxel in one 16-byte slot of the workspace (one
  * vector reduction per tap instead of two), then folds the workspace into data_rec /
- * weight_rec; results are the same up to summation order.  Without a workspace (or without
- * weights) it reduces straight into the outputs.  The workspace holds no state between calls.
+ * weight_rec; without weights it spreads many slices onto a small reconstruction over copies of it in
+ * the workspace and adds them up.  Large cubic calls, with or without weights, run brick by brick when the
+ * workspace has b200proj_scatter_workspace_bytes(...) bytes.  Results are the same up to summation order.
+ * Else it reduces straight into the outputs.  The workspace holds no state between calls.
  * replaces: backproject_2d_forw_cuda       csrc/cuda/2d/backprojection_2d_kernels.cu:827-976
  *           backproject_2d_to_3d_forw_cuda csrc/cuda/3d/backprojection_2d_to_3d_kernels.cu:1001-1188 */
 int b200proj_backproject_2d_forw(const float* proj, const float* weights, int64_t B, int64_t R,
@@ -250,8 +252,8 @@ int b200proj_backproject_2d_to_3d_forw(const float* proj, const float* weights, 
                                        void* workspace, size_t workspace_bytes, void* stream);
 
 /* Bytes of workspace with which a back-projection of these sizes runs faster, or 0 when a
- * workspace would not help (no weights, or too few slices to pay for two extra passes over
- * the volume).  dim = 2 or 3.  No counterpart in the reference (its kernels use no scratch). */
+ * workspace would not help (too few slices to pay for the extra passes over the volume, or without
+ * weights a volume that is not small).  dim = 2 or 3.  No counterpart in the reference (its kernels use no scratch). */
 size_t b200proj_backproject_workspace_bytes(int dim, int64_t B, int64_t R, int64_t P, int64_t N,
                                             int interpolation, int has_weights);
 

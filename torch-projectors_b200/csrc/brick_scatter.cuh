@@ -13,14 +13,18 @@
 // An adding warp takes a chunk, one pixel per lane, and every lane its taps in an order that starts at the lane's own
 // class (x & 3, y & 3, z & 3) -- a cubic footprint holds every class once --, two taps a step: the 32 lanes hold 64
 // different classes then, hence 64 different voxels, whatever pixels they hold.  So no two lanes add to the same voxel
-// between two synchronisations of the warp, and no bank conflicts arise.  2D reconstructions are cut into tiles; a
+// between two synchronisations of the warp, and the 8-byte sums meet no bank conflicts (of the 4-byte sums of the weights
+// those of lanes 16 apart can meet in a bank).  2D reconstructions are cut into tiles; a
 // tile's pixels go to the adding warps in turn, each of which has its own sums (two copies: a 4 x 4 footprint has 16
 // classes, so the halves of the warp are kept apart).
 //
 // Measured on B200: the scatter of 4,096 slices of 256 x 129 into a box-512 gradient 14.4 ms (plain kernel) -> 5.97 ms,
-// 2,501 weighted slices of box 90 into box 180 1.61 -> 0.75 ms.  Bound by the adding warps: a step is a chain of load,
-// add, store (58 clocks for 64 taps alone, 70-80 beside the walkers), so what counts is how many slabs fit an SM: 12
-// of 13 x 13 x 4 sample positions (16 x 16 x 7 sums), 8 with weights.  Measured slower for that scatter: 10 slabs of 5
+// 2,501 weighted slices of box 90 into box 180 1.61 -> 0.75 ms.  What bounds it, from timers around the waits, in
+// shares of the kernel's time: without weights the walk (the walking warps walk for 67 % and wait for room for 7 %, the
+// adding warps add for 53 % and wait for chunks for 37 %), with weights the adding (64 % and 24 %, walking warps 43 % and
+// 27 %); flushes are 6-7 %.  A step of 64 taps is a chain of load, add, store: 58 clocks alone, 100 beside the other warps
+// of the SM (126 with weights), which use 56 % of the issue slots.  An SM holds 12 slabs of 13 x 13 x 4 sample
+// positions (16 x 16 x 7 sums), 8 with weights.  Measured slower for that scatter: 10 slabs of 5
 // planes 6.1 ms, 8 slabs of 8 planes 6.4 ms, one block of 14 walkers and 10 slabs 6.6 ms, one adding warp per block
 // with a barrier for each hand-over 7.8 ms, and pixels of a full ring sent to L2 as reductions by the walkers 7.6 ms
 // (that starves the adding warps).  For linear taps (2 x 2 x 2 classes, overlapping pixels one after the other) the

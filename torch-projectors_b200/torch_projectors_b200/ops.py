@@ -129,7 +129,7 @@ def set_pose_order_thresholds(min_volume_bytes: int = 96 << 20, min_poses: int =
 # the projections' size, the projections among it), and the backward pass then forms the pose gradients from them instead of
 # gathering the volume a second time -- and skips the scatter into the volume's gradient altogether
 # when the volume needs none.  Measured on B200, box 512, 4,096 poses of 256 x 256, cubic: forward
-# 6.5 -> 8.9 ms, backward 20.3 -> 15.1 ms (1.9 ms with a fixed volume).
+# 3.0 -> 3.7 ms, backward 19.6 -> 6.6 ms (0.65 ms with a fixed volume).
 # When the reconstruction needs a gradient too, the backward pass still scatters; small calls (below
 # SAVE_DERIVATIVES_MIN_VOLUME_BYTES per batch item and SAVE_DERIVATIVES_MIN_PIXELS pixels) keep the plain
 # pair then, whose gather costs less than the derivatives' way through memory.
