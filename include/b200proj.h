@@ -427,7 +427,7 @@ int b200proj_project_3d_to_2d_back_saved(const float* grad_proj, const float* ou
 /* The 3D pair with one 32-byte record (d/dc, d/dr, d/dd, projection; complex each) per pixel in place of
  * the planes, records = [B,P,N,Nh,4] complex, 32-byte aligned: whole sectors, which is what the
  * brick-by-brick kernel (workspace as for b200proj_project_3d_to_2d_forw_ws) writes best.  The shift gradients
- * are formed from `out`, or, when it is NULL, from the records' fourth entries. */
+ * are formed from `out`, or, when that is `records` itself, from the records' fourth entries. */
 int b200proj_project_3d_to_2d_forw_records(const float* rec, int64_t B, int64_t R, const float* rot,
                                            int64_t B_rot, const float* shifts, int64_t B_shift, int64_t P,
                                            int64_t N, int interpolation, double oversampling,

@@ -130,6 +130,8 @@ def test_misaligned_records_are_refused_without_a_device():
     lib = _abi.load()
     rc = lib.b200proj_project_3d_to_2d_back_records(16, 16, 24, 1, 16, 16, 1, 0, 0, 1, 8, 0, 2.0, 4.0, 0, 16, 0, 0, 0, 0, 0)
     assert rc == -1 and "16-byte aligned" in lib.b200proj_last_error().decode()
+    rc = lib.b200proj_project_3d_to_2d_back_records(16, 0, 32, 1, 16, 16, 1, 16, 1, 1, 8, 0, 2.0, 4.0, 0, 0, 16, 0, 0, 0, 0)
+    assert rc == -1 and "no shifts / saved projections given" in lib.b200proj_last_error().decode()
     rc = lib.b200proj_project_3d_to_2d_forw_records(16, 1, 16, 16, 1, 0, 0, 1, 8, 0, 2.0, 4.0, 16, 48, 0, 0, 0, 0)
     assert rc == -1 and "32-byte aligned" in lib.b200proj_last_error().decode()
 

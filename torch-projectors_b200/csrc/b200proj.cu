@@ -524,7 +524,7 @@ int project_back_saved(const float* grad_proj, const float* out, const float* de
     L.g.order = pose_order;
     if (grad_proj == nullptr) return fail(B200PROJ_ERR_ARGUMENT, "grad_projections pointer is NULL");
     if (grad_rot != nullptr && derivatives == nullptr) return fail(B200PROJ_ERR_ARGUMENT, "grad_rotations requested but no saved derivatives given");
-    if (grad_shifts != nullptr && (shifts == nullptr || (out == nullptr && !(RECORDS && derivatives != nullptr))))
+    if (grad_shifts != nullptr && (shifts == nullptr || out == nullptr))
         return fail(B200PROJ_ERR_ARGUMENT, "grad_shifts requested but no shifts / saved projections given");
     if (RECORDS && (reinterpret_cast<uintptr_t>(derivatives) & 15u) != 0) return fail(B200PROJ_ERR_ARGUMENT, "records must be 16-byte aligned");
     if (grad_rec == nullptr && grad_rot == nullptr && grad_shifts == nullptr) return B200PROJ_OK;
@@ -538,7 +538,7 @@ int project_back_saved(const float* grad_proj, const float* out, const float* de
                               grad_shifts, (size_t)(shifts ? B_shift : 0) * P * 2 * sizeof(float))) return rc;
     if (P == 0) return B200PROJ_OK;
     const float2* gp = (const float2*)grad_proj;
-    const float2* o = (const float2*)out;
+    const float2* o = RECORDS && out == derivatives ? nullptr : (const float2*)out;      // the records themselves: their fourth entries
     const float2* d = (const float2*)derivatives;
     if (bl.use) {
         // large cubic scatter: brick by brick, the pose gradients in a streaming pass of their own

@@ -395,7 +395,7 @@ project_back_saved_kernel(const float2* __restrict__ grad_proj, const float2* __
 // grid.x = slice, grid.y = parts of its pixels; a block walks over its part with consecutive threads on
 // consecutive pixels and four pixels in flight per thread (48 bytes each), and adds its sums once.
 // Bound by DRAM (4,096 slices of 128 x 65: 0.182 ms for 1.06 GB = 5.8 TB/s); as tiles of 16 x 16 pixels
-// with one reduction per tile it took 0.52 ms.  RECORDS: without `out` the pixel is the record's fourth entry.
+// with one reduction per tile it took 0.52 ms.  RECORDS: where `out` is NULL the pixel is the record's fourth entry.
 template <int DIM, bool NEED_ROT, bool NEED_SHIFT, bool RECORDS>
 __global__ void __launch_bounds__(kBlockThreads)
 pose_grad_saved_kernel(const float2* __restrict__ grad_proj, const float2* __restrict__ out, const float2* __restrict__ derivs,

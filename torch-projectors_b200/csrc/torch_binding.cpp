@@ -359,7 +359,7 @@ std::tuple<Tensor, Tensor, Tensor> project_back_saved(int dim, const Tensor& gra
             ? b200proj_project_2d_back_saved_ws(cptr<float>(gp), cptr<float>(out), cptr<float>(der), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts),
                                              p.B_shift, p.P, N, interp, oversampling, cut, mptr<float>(grad_rec), mptr<float>(grad_rot), mptr<float>(grad_sh),
                                                 ws_ptr(ws), ws_size(ws), current_stream(gp))
-            : b200proj_project_3d_to_2d_back_records(cptr<float>(gp), whole && der.defined() ? nullptr : cptr<float>(out), cptr<float>(der), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts),
+            : b200proj_project_3d_to_2d_back_records(cptr<float>(gp), cptr<float>(whole && der.defined() ? der : out), cptr<float>(der), B, R, cptr<float>(p.rot), p.B_rot, cptr<float>(p.shifts),
                                                    p.B_shift, p.P, N, interp, oversampling, cut, mptr<float>(grad_rec), mptr<float>(grad_rot), mptr<float>(grad_sh),
                                                    cptr<int32_t>(order), ws_ptr(ws), ws_size(ws), current_stream(gp));
         status(rc, dim == 2 ? "project_2d_back_saved" : "project_3d_to_2d_back_saved");
