@@ -13,6 +13,7 @@
 #include <type_traits>
 
 #include "brick_scatter.cuh"
+#include "cell_scatter.cuh"
 
 namespace {
 
@@ -384,6 +385,185 @@ int launch_brick_scatter(const Launch& L, const BrickLaunch& bl, void* workspace
     return check_launch("brick_scatter launch");
 }
 
+// ---- pixel lists: plan and launch ---------------------------------------------------------------------------
+struct ListLaunch {
+    ListPlan plan;
+    size_t count_bytes, item_bytes, pose_bytes, inside_bytes, block_bytes, bytes;
+    int64_t slices;          // of the call
+    double pixels;           // of the call
+    bool forced, use;
+};
+
+// Pixels of a slice that a list holds, and an upper bound of their pairs (as list_setup_kernel finds them).
+void listed_pixels(int64_t N, double cutoff, int64_t* pixels, int64_t* pairs) {
+    const float rc = (float)cutoff;
+    const double room = (double)(rc * rc);
+    *pixels = *pairs = 0;
+    for (int64_t kr = 1 - N / 2; kr <= N / 2; ++kr) {
+        const double left = room - (double)(kr * kr);
+        if (!(left >= 0.0)) continue;
+        int64_t j = left >= 4.0 * (double)(N * N) ? N / 2 : (int64_t)sqrt(left);
+        while ((double)((j + 1) * (j + 1)) <= left) ++j;
+        while ((double)(j * j) > left) --j;
+        if (j > N / 2) j = N / 2;
+        *pixels += j + 1;
+        *pairs += j / 2 + 1;
+        if (kr < 0 || kr == N / 2) --*pixels;             // the mirrored half of column 0
+    }
+}
+
+// A grid of bricks over all samples with taps inside a reconstruction of box R.  `blocks` of the kernel fit the GPU.
+ListLaunch list_layout(int dim, int64_t B, int64_t R, int64_t P, int64_t N, double os, double cutoff, double blocks) {
+    ListLaunch L{};
+    static const int force = [] { const char* e = getenv("B200PROJ_LISTS"); return e ? atoi(e) : -1; }();   // 0 / 1: never / always, for tests
+    if (force == 0 || B < 1 || P < 1 || N < 2 || N > 2048 || R < 2 || R > 4096 || !(cutoff >= 0.0) || !(os > 0.0) || (double)(float)os != os) return L;
+    const double rough = (double)B * (double)P * (double)N * (double)(N / 2 + 1);
+    if (force != 1 && rough < 6e5) return L;                     // below all lines
+    ListPlan& p = L.plan;
+    const int log2[3] = {dim == 3 ? ListBrick<3>::kLogX : ListBrick<2>::kLogX, dim == 3 ? ListBrick<3>::kLogY : ListBrick<2>::kLogY, ListBrick<3>::kLogZ};
+    const int64_t far = R / 2 + 2;                               // cells of samples with a tap inside lie below this, from -this on
+    int64_t bricks = B;
+    for (int a = 0; a < 3; ++a) {
+        // a whole number of bricks on either side of 0 (of c: one)
+        const int64_t size = (int64_t)1 << log2[a], above = (far + size - 1) / size, n = a == 0 ? above + 1 : a < dim ? 2 * above : 1;
+        p.n[a] = (int)n;
+        p.lo[a] = a == 0 ? (int)-size : a < dim ? (int)(-above * size) : 0;
+        bricks *= n;
+        while (((int64_t)1 << p.bits) < n) ++p.bits;
+        p.fit[a] = (float)(above * size) - 0.5f;
+        if (a > 0) p.round[a - 1] = kRound - (float)(p.lo[a] / size);
+    }
+    const double corner = sqrt((double)N * (double)N / 2.0);
+    p.row_zero = 8388608.f + (float)(N / 2 - 1);
+    p.reach = (float)((cutoff < corner ? cutoff : corner) * os * 1.00001);
+    while (((int64_t)1 << p.bits_j) < N / 2 + 1) ++p.bits_j;
+    while (((int64_t)1 << p.bits_i) < N) ++p.bits_i;
+    int64_t inside, pairs;
+    listed_pixels(N, cutoff, &inside, &pairs);
+    if (bricks > (1 << 24) || (B << (dim * p.bits)) > (1 << 28) || B * P > (1 << 26) || inside < 1) return L;
+    p.bricks = (int)bricks;
+    p.item_bricks = (int)(bricks / B);
+    p.inside = (int)inside;
+    p.pairs = (int)pairs;
+    L.slices = B * P;
+    L.pixels = (double)inside * (double)L.slices;
+    // slices of one pass over the list: at most 2^30 entries, and what the bits of an entry can name
+    static const int64_t list_entries = [] { const char* e = getenv("B200PROJ_LIST_ENTRIES"); return e && atoll(e) > 0 ? (int64_t)atoll(e) : (int64_t)1 << 30; }();   // for tests
+    const int64_t by_list = list_entries / inside > 1 ? list_entries / inside : 1, by_bits = (int64_t)1 << (32 - p.bits_i - p.bits_j < 26 ? 32 - p.bits_i - p.bits_j : 26);
+    const int64_t most_slices = by_list < by_bits ? by_list : by_bits, passes = (L.slices + most_slices - 1) / most_slices;
+    p.slices = (int)((L.slices + passes - 1) / passes);
+    const int64_t entries = inside * p.slices;
+    p.capacity = (unsigned)entries;
+    const double most = (double)entries / (blocks * 8.0);
+    p.most = most < 4096.0 ? 4096 : most > 8192.0 ? 8192 : (int)most;
+    const size_t up = 255, items = (size_t)(bricks < entries ? bricks : entries) + (size_t)(entries / p.most) + 1;
+    L.count_bytes = ((size_t)bricks * sizeof(unsigned) + up) & ~up;
+    L.item_bytes = (items * sizeof(int4) + up) & ~up;
+    L.pose_bytes = ((size_t)L.slices * 2 * sizeof(float4) + up) & ~up;
+    L.inside_bytes = ((size_t)pairs * sizeof(unsigned) + up) & ~up;
+    if (p.item_bricks <= kListBricks && B <= 65535) {
+        // few bricks: counted in shared memory, a run of slices per block (some 16 blocks per SM)
+        int64_t run = (p.slices + 148 * 16 - 1) / (148 * 16);
+        p.run = (int)(run < 1 ? 1 : run);
+        L.block_bytes = ((size_t)B * (size_t)((P + p.run - 1) / p.run) * (size_t)p.item_bricks * sizeof(unsigned) + up) & ~up;
+        if (L.block_bytes > (64u << 20)) p.run = 0, L.block_bytes = 0;
+    }
+    L.bytes = 256 + L.count_bytes + L.item_bytes + L.pose_bytes + L.inside_bytes + L.block_bytes + (size_t)entries * sizeof(unsigned);
+    L.forced = force == 1;
+    L.use = true;
+    return L;
+}
+
+ListWork list_work(const ListLaunch& L, void* workspace) {
+    ListWork w;
+    char* at = (char*)workspace;
+    w.header = (int*)at;
+    w.count = (unsigned*)(at += 256);
+    w.items = (int4*)(at += L.count_bytes);
+    w.poses = (float4*)(at += L.item_bytes);
+    w.inside = (unsigned*)(at += L.pose_bytes);
+    w.block_count = (unsigned*)(at += L.inside_bytes);
+    w.list = (unsigned*)(at += L.block_bytes);
+    return w;
+}
+
+// Scatters from pixel lists: above a number of pixels that grows with the bricks (a brick costs its latency and its flush
+// however few pixels it has).  Measured crossings with the kernels used otherwise (in M pixels; bricks inside the ball of the samples), with
+// weights / without: 3D cubic, oversampled twice: 134 bricks 3 / 4, 1,072 2.3 / 3.5, 8,578 9 / 8, 68,600 55 / 50; not oversampled 0.5 / 0.8
+// and 1 / 0.9 of 134 and 1,072.  3D linear 10 / 17, 8.5 / 14, 7 / 26, 36 / 40; 3 / 5, 4.3 / 7.  2D cubic, tiles: 6 1.8 / 3, 25 1.4 / 2.2, 100
+// 1.4 / 2.3, 402 2.4 / 4.  2D linear 25 / 40, 10 / 35, 10.5 / 38, 25 / 50.  Far above them 1.25-1.7x (3D), 1.2-1.7x (2D).
+ListLaunch list_scatter_plan(int dim, int64_t B, int64_t R, int64_t P, int64_t N, bool cubic, bool weights, double os, double cutoff) {
+    const ListLaunch L = list_layout(dim, B, R, P, N, os, cutoff, 148.0 * 4);
+    if (!L.use || L.forced) return L;
+    const double r = L.plan.reach < (float)R * 0.5f ? L.plan.reach : (double)R * 0.5;
+    const double bricks = (double)B * (dim == 3 ? 2.094 * r * r * r / 512.0 : 1.571 * r * r / 256.0);
+    const bool dense = os < 1.25;
+    double line;
+    if (dim == 3) line = cubic ? (dense ? 0.9e6 : weights ? 2.5e6 : 3.2e6) + 750.0 * bricks
+                               : (weights ? (dense ? 3.5e6 : 9e6) : (dense ? 6e6 : 16e6)) + (weights ? 400.0 : 800.0) * bricks;
+    else line = cubic ? (weights ? 1.6e6 : 2.4e6) + 4e3 * bricks : (weights ? 11e6 : 36e6) + 3e4 * bricks + 2e8 / bricks;
+    return r > 24.0 && L.pixels > line ? L : ListLaunch{};
+}
+bool runs_in(const ListLaunch& L, const void* workspace, size_t workspace_bytes) {
+    return L.use && scratch_aligned(workspace) && workspace_bytes >= L.bytes;
+}
+
+// For each pass over the list: sort the pixels, then run(work, plan).
+template <int DIM, typename Run>
+int with_lists(const Launch& L, const ListLaunch& ll, void* workspace, const float* rot, const float* shifts, cudaStream_t s, Run run) {
+    const ListWork w = list_work(ll, workspace);
+    ListPlan pl = ll.plan;
+    const int per_pass = pl.slices;
+    for (int64_t first = 0; first < ll.slices; first += per_pass) {
+        pl.first = (int)first;
+        pl.slices = (int)(ll.slices - first < per_pass ? ll.slices - first : per_pass);
+        if (int rc = zero_async(w.header, 256 + ll.count_bytes, s)) return rc;
+        const unsigned tiles = (unsigned)(L.g.tiles_i * ((L.g.Nh + 31) / 32));
+        list_setup_kernel<DIM><<<tiles + (unsigned)((ll.slices + 255) / 256), 256, 0, s>>>(rot, shifts, w, L.g, pl);
+        if (int rc = check_launch("list_setup launch")) return rc;
+        dim3 grid((unsigned)((pl.pairs + kListPairs - 1) / kListPairs), (unsigned)(pl.slices < 32768 ? pl.slices : 32768), (unsigned)((pl.slices + 32767) / 32768));
+        if (pl.run > 0) grid = dim3((unsigned)((L.P + pl.run - 1) / pl.run), (unsigned)L.B, 1);
+        if (pl.run > 0) list_pixels_kernel<DIM, true, true><<<grid, 256, 0, s>>>(w, L.g, pl);
+        else list_pixels_kernel<DIM, true, false><<<grid, 256, 0, s>>>(w, L.g, pl);
+        if (int rc = check_launch("list_pixels (count) launch")) return rc;
+        const int64_t places = L.B << (DIM * pl.bits);
+        list_plan_kernel<DIM><<<(unsigned)((places + 255) / 256), 256, 0, s>>>(w, pl, (int)L.B);
+        if (int rc = check_launch("list_plan launch")) return rc;
+        if (pl.run > 0) list_pixels_kernel<DIM, false, true><<<grid, 256, 0, s>>>(w, L.g, pl);
+        else list_pixels_kernel<DIM, false, false><<<grid, 256, 0, s>>>(w, L.g, pl);
+        if (int rc = check_launch("list_pixels launch")) return rc;
+        if (int rc = run(w, pl)) return rc;
+    }
+    return B200PROJ_OK;
+}
+
+template <int DIM, bool CUBIC, bool WEIGHTS, bool DUP, bool INTERLEAVED>
+int run_list_scatter(const Launch& L, const ListLaunch& ll, void* workspace, const float* proj, const float* weights, const float* rot,
+                     const float* shifts, float* vol, float* wvol, cudaStream_t s, float4* accum) {
+    using C = std::conditional_t<DIM == 3 && CUBIC, CubicSums<WEIGHTS>, CellSums<DIM, CUBIC, WEIGHTS>>;
+    constexpr size_t smem = sizeof(typename C::Shared);
+    static_assert((smem + 1024) * C::kBlocks <= 233472, "shared memory of an SM");
+    auto kernel = [] {
+        if constexpr (DIM == 3 && CUBIC) return cell_cubic_sums_kernel<WEIGHTS, DUP, INTERLEAVED>;
+        else return cell_sums_kernel<DIM, CUBIC, WEIGHTS, DUP, INTERLEAVED>;
+    }();
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return cuda_fail(e, "cell_sums shared memory");
+    const ScatterTarget<WEIGHTS, INTERLEAVED> to{(float2*)vol, wvol, accum};
+    return with_lists<DIM>(L, ll, workspace, rot, shifts, s, [&](const ListWork& w, const ListPlan& pl) {
+        kernel<<<148 * C::kBlocks, C::kThreads, smem, s>>>((const float2*)proj, weights, to, w, L.g, pl);
+        if (int rc = check_launch("cell_sums launch")) return rc;
+        scatter_rest_kernel<DIM, CUBIC, WEIGHTS, DUP><<<148 * 4, 256, 0, s>>>((const float2*)proj, weights, rot, shifts, to, w, L.g, pl);
+        return check_launch("scatter_rest launch");
+    });
+}
+template <int DIM, bool WEIGHTS, bool DUP, bool INTERLEAVED = false>
+int launch_list_scatter(const Launch& L, const ListLaunch& ll, bool cubic, void* workspace, const float* proj, const float* weights, const float* rot,
+                        const float* shifts, float* vol, float* wvol, cudaStream_t s, float4* accum = nullptr) {
+    return cubic ? run_list_scatter<DIM, true, WEIGHTS, DUP, INTERLEAVED>(L, ll, workspace, proj, weights, rot, shifts, vol, wvol, s, accum)
+                 : run_list_scatter<DIM, false, WEIGHTS, DUP, INTERLEAVED>(L, ll, workspace, proj, weights, rot, shifts, vol, wvol, s, accum);
+}
+
 // Copies of a small complex reconstruction (all batch items: `one` bytes) over which the slices of a scatter without
 // weights are spread.  They cost a clear, a sum over the copies and two launches (3-5 us; small calls lose up to half), and
 // gain where many reductions meet on few sectors.  In reductions per byte, measured on both sides of the lines: 2D, cubic /
@@ -531,18 +711,24 @@ int project_back_saved(const float* grad_proj, const float* out, const float* de
     cudaStream_t s = (cudaStream_t)stream;
     const bool cubic = interpolation == B200PROJ_CUBIC;
     BrickLaunch bl{};
-    if ((RECORDS || DIM == 2) && P > 0 && grad_rec != nullptr && workspace != nullptr) bl = scatter_plan(DIM, B, P, N, cubic, false, os, cutoff);
+    ListLaunch ll{};
+    if ((RECORDS || DIM == 2) && P > 0 && grad_rec != nullptr && workspace != nullptr) {
+        ll = list_scatter_plan(DIM, B, R, P, N, cubic, false, os, cutoff);
+        ll.use = runs_in(ll, workspace, workspace_bytes);
+        if (!ll.use) bl = scatter_plan(DIM, B, P, N, cubic, false, os, cutoff);
+    }
     bl.use = runs_in(bl, workspace, workspace_bytes);
-    const int copies = P > 0 && grad_rec != nullptr && !bl.use ? scatter_copies(L, DIM, cubic, false, workspace, workspace_bytes) : 1;
+    const int copies = P > 0 && grad_rec != nullptr && !bl.use && !ll.use ? scatter_copies(L, DIM, cubic, false, workspace, workspace_bytes) : 1;
     if (int rc = zero_outputs(s, copies > 1 ? nullptr : grad_rec, L.rec_count * sizeof(float2), grad_rot, (size_t)B_rot * P * DIM * DIM * sizeof(float),
                               grad_shifts, (size_t)(shifts ? B_shift : 0) * P * 2 * sizeof(float))) return rc;
     if (P == 0) return B200PROJ_OK;
     const float2* gp = (const float2*)grad_proj;
     const float2* o = RECORDS && out == derivatives ? nullptr : (const float2*)out;      // the records themselves: their fourth entries
     const float2* d = (const float2*)derivatives;
-    if (bl.use) {
-        // large cubic scatter: brick by brick, the pose gradients in a streaming pass of their own
-        if (int rc = launch_brick_scatter<DIM, false, false>(L, bl, workspace, grad_proj, nullptr, rot, shifts, grad_rec, nullptr, s)) return rc;
+    if (bl.use || ll.use) {
+        // large scatter: brick by brick, the pose gradients in a streaming pass of their own
+        if (int rc = ll.use ? launch_list_scatter<DIM, false, false>(L, ll, cubic, workspace, grad_proj, nullptr, rot, shifts, grad_rec, nullptr, s)
+                            : launch_brick_scatter<DIM, false, false>(L, bl, workspace, grad_proj, nullptr, rot, shifts, grad_rec, nullptr, s)) return rc;
         if (grad_rot == nullptr && grad_shifts == nullptr) return B200PROJ_OK;
         grad_rec = nullptr;
     }
@@ -573,15 +759,21 @@ int project_back(const Real* grad_proj, const Real* rec, int64_t B, int64_t R, c
         return fail(B200PROJ_ERR_ARGUMENT, "grad_shifts requested but no shifts given");
     cudaStream_t s = (cudaStream_t)stream;
     BrickLaunch bl{};
-    if (std::is_same<Real, float>::value && P > 0 && grad_rot == nullptr && grad_shifts == nullptr && workspace != nullptr)
-        bl = scatter_plan(DIM, B, P, N, interpolation == B200PROJ_CUBIC, false, os, cutoff);
+    ListLaunch ll{};
+    if (std::is_same<Real, float>::value && P > 0 && grad_rot == nullptr && grad_shifts == nullptr && workspace != nullptr) {
+        ll = list_scatter_plan(DIM, B, R, P, N, interpolation == B200PROJ_CUBIC, false, os, cutoff);
+        ll.use = runs_in(ll, workspace, workspace_bytes);
+        if (!ll.use) bl = scatter_plan(DIM, B, P, N, interpolation == B200PROJ_CUBIC, false, os, cutoff);
+    }
     bl.use = runs_in(bl, workspace, workspace_bytes);
-    const int copies = P > 0 && std::is_same<Real, float>::value && !bl.use ? scatter_copies(L, DIM, interpolation == B200PROJ_CUBIC, grad_rot != nullptr || grad_shifts != nullptr, workspace, workspace_bytes) : 1;
+    const int copies = P > 0 && std::is_same<Real, float>::value && !bl.use && !ll.use ? scatter_copies(L, DIM, interpolation == B200PROJ_CUBIC, grad_rot != nullptr || grad_shifts != nullptr, workspace, workspace_bytes) : 1;
     if (int rc = zero_outputs(s, copies > 1 ? nullptr : grad_rec, L.rec_count * sizeof(C2<Real>), grad_rot, (size_t)B_rot * P * DIM * DIM * sizeof(Real),
                               grad_shifts, (size_t)(shifts ? B_shift : 0) * P * 2 * sizeof(Real))) return rc;
     if (P == 0) return B200PROJ_OK;
-    if constexpr (std::is_same<Real, float>::value)
+    if constexpr (std::is_same<Real, float>::value) {
+        if (ll.use) return launch_list_scatter<DIM, false, false>(L, ll, interpolation == B200PROJ_CUBIC, workspace, grad_proj, nullptr, rot, shifts, grad_rec, nullptr, s);
         if (bl.use) return launch_brick_scatter<DIM, false, false>(L, bl, workspace, grad_proj, nullptr, rot, shifts, grad_rec, nullptr, s);
+    }
     if (copies > 1)
         if (int rc = zero_async(workspace, (size_t)copies * L.rec_count * sizeof(float2), s)) return rc;
     C2<Real>* to = copies > 1 ? (C2<Real>*)workspace : (C2<Real>*)grad_rec;
@@ -613,6 +805,14 @@ int backproject_forw(const Real* proj, const Real* weights, int64_t B, int64_t R
     // (one v4 reduction per tap), folded into the outputs afterwards.
     const size_t ws_one = L.rec_count * sizeof(float4);
     if constexpr (std::is_same<Real, float>::value) {
+        const ListLaunch ll = P > 0 && workspace != nullptr ? list_scatter_plan(DIM, B, R, P, N, cubic, hw, os, cutoff) : ListLaunch{};
+        if (runs_in(ll, workspace, workspace_bytes)) {
+            if (!accumulate) {
+                if (int rc = zero_outputs(s, data_rec, L.rec_count * sizeof(C2<Real>), weight_rec, L.rec_count * sizeof(Real))) return rc;
+            }
+            return hw ? launch_list_scatter<DIM, true, true>(L, ll, cubic, workspace, proj, weights, rot, shifts, data_rec, weight_rec, s)
+                      : launch_list_scatter<DIM, false, true>(L, ll, cubic, workspace, proj, nullptr, rot, shifts, data_rec, nullptr, s);
+        }
         const BrickLaunch bl = P > 0 && workspace != nullptr ? scatter_plan(DIM, B, P, N, cubic, hw, os, cutoff) : BrickLaunch{};
         if (runs_in(bl, workspace, workspace_bytes)) {
             if (!accumulate) {
@@ -758,6 +958,8 @@ int backproject_accumulate(const float* proj, const float* weights, int64_t B, i
     float4* acc = (float4*)accumulator;
     const bool cubic = interpolation == B200PROJ_CUBIC;
     if (workspace != nullptr && slab_count == plan.slabs) {
+        const ListLaunch ll = list_scatter_plan(3, B, R, P, N, cubic, true, os, cutoff);
+        if (runs_in(ll, workspace, workspace_bytes)) return launch_list_scatter<3, true, true, true>(L, ll, cubic, workspace, proj, weights, rot, shifts, nullptr, nullptr, s, acc);
         const BrickLaunch bl = scatter_plan(3, B, P, N, cubic, true, os, cutoff);
         if (runs_in(bl, workspace, workspace_bytes)) return launch_brick_scatter<3, true, true, true>(L, bl, workspace, proj, weights, rot, shifts, nullptr, nullptr, s, acc);
     }
@@ -909,13 +1111,19 @@ int b200proj_project_3d_to_2d_forw(const float* rec, int64_t B, int64_t R, const
 size_t b200proj_scatter_workspace_bytes(int dim, int64_t B, int64_t P, int64_t N, int interpolation, int has_weights, double oversampling, double cutoff) {
     if (dim != 2 && dim != 3) return 0;
     const BrickLaunch bl = scatter_plan(dim, B, P, N, interpolation == B200PROJ_CUBIC, has_weights != 0, oversampling, cutoff);
-    return bl.use ? bl.bytes : 0;
+    const ListLaunch ll = list_scatter_plan(dim, B, b200proj_rec_boxsize(N, oversampling), P, N, interpolation == B200PROJ_CUBIC, has_weights != 0, oversampling, cutoff);
+    const size_t lists = ll.use ? ll.bytes : 0, bricks = bl.use ? bl.bytes : 0;
+    return lists > bricks ? lists : bricks;
 }
 size_t b200proj_gradient_workspace_bytes(int dim, int64_t B, int64_t R, int64_t P, int64_t N, int interpolation, int pose_gradients,
                                          double oversampling, double cutoff) {
     if ((dim != 2 && dim != 3) || B < 1 || R < 2 || P < 1 || N < 2) return 0;
-    if (!pose_gradients)
-        if (const size_t bytes = b200proj_scatter_workspace_bytes(dim, B, P, N, interpolation, 0, oversampling, cutoff)) return bytes;
+    if (!pose_gradients) {
+        const ListLaunch ll = list_scatter_plan(dim, B, R, P, N, interpolation == B200PROJ_CUBIC, false, oversampling, cutoff);
+        const BrickLaunch bl = scatter_plan(dim, B, P, N, interpolation == B200PROJ_CUBIC, false, oversampling, cutoff);
+        const size_t lists = ll.use ? ll.bytes : 0, bricks = bl.use ? bl.bytes : 0;
+        if (lists > 0 || bricks > 0) return lists > bricks ? lists : bricks;
+    }
     const double one = (double)B * (dim == 3 ? R : 1) * R * (R / 2 + 1) * (double)sizeof(float2);
     const int copies = copies_wanted(dim, one, B, P, N, interpolation == B200PROJ_CUBIC, pose_gradients != 0);
     return copies > 1 ? (size_t)one * (size_t)copies : 0;

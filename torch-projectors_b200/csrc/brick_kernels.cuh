@@ -335,12 +335,6 @@ __device__ __forceinline__ void rotate4(F (&w)[4], int t0) {      // w[s] <- w[(
     if (t0 & 2) { F x = w[0]; w[0] = w[2]; w[2] = x; x = w[1]; w[1] = w[3]; w[3] = x; }
 }
 
-__device__ __forceinline__ unsigned long long fmul2(unsigned long long a, unsigned long long b) {
-    unsigned long long r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-
 // Value (and derivatives) at (lx + fx, ly + fy, lz + fz) of the staged brick, all of it in this lane.
 template <int DIM, bool CUBIC, bool WITH_DERIV>
 __device__ __forceinline__ void brick_gather(const float2* sm, int lx, int ly, int lz, float fx, float fy, float fz,

@@ -160,17 +160,25 @@ Tensor project_workspace(int dim, const Tensor& rec, int64_t P, int64_t N, int i
     const size_t bytes = b200proj_project_workspace_bytes(dim, rec.size(0), P, N, interp, records ? 1 : 0, oversampling, cutoff);
     return bytes ? at::empty({(int64_t)bytes}, rec.options().dtype(at::kByte)) : Tensor();
 }
+// Scratch that a call can do without: undefined when none is wanted, or when the device has no room for it (pixel lists take 4
+// bytes per pixel, up to 4 GB).
+Tensor scratch(size_t bytes, const Tensor& like) {
+    if (bytes == 0) return Tensor();
+    try {
+        return at::empty({(int64_t)bytes}, like.options().dtype(at::kByte));
+    } catch (const c10::OutOfMemoryError&) {
+        return Tensor();
+    }
+}
 // The same for the scatters.
 Tensor scatter_workspace(int dim, const Tensor& like, int64_t B, int64_t P, int64_t N, int interp, bool weights, double oversampling, double cutoff) {
     if (is_f64(like)) return Tensor();
-    const size_t bytes = b200proj_scatter_workspace_bytes(dim, B, P, N, interp, weights ? 1 : 0, oversampling, cutoff);
-    return bytes ? at::empty({(int64_t)bytes}, like.options().dtype(at::kByte)) : Tensor();
+    return scratch(b200proj_scatter_workspace_bytes(dim, B, P, N, interp, weights ? 1 : 0, oversampling, cutoff), like);
 }
 // The same for the backward passes of the projection.
 Tensor gradient_workspace(int dim, const Tensor& like, int64_t B, int64_t R, int64_t P, int64_t N, int interp, bool pose_gradients, double oversampling, double cutoff) {
     if (is_f64(like)) return Tensor();
-    const size_t bytes = b200proj_gradient_workspace_bytes(dim, B, R, P, N, interp, pose_gradients ? 1 : 0, oversampling, cutoff);
-    return bytes ? at::empty({(int64_t)bytes}, like.options().dtype(at::kByte)) : Tensor();
+    return scratch(b200proj_gradient_workspace_bytes(dim, B, R, P, N, interp, pose_gradients ? 1 : 0, oversampling, cutoff), like);
 }
 inline void* ws_ptr(const Tensor& ws) { return ws.defined() ? ws.data_ptr() : nullptr; }
 inline size_t ws_size(const Tensor& ws) { return ws.defined() ? (size_t)ws.numel() : 0; }

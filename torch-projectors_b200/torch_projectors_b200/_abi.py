@@ -265,10 +265,14 @@ def backproject_accumulate(proj, weights, rot, shifts, interp, oversampling, cut
     of accumulator_bytes(B, R) bytes); see b200proj_backproject_2d_to_3d_accumulate."""
     B, P, N = proj.shape[0], proj.shape[1], proj.shape[2]
     geom = _geom(B, R, rot, shifts, P, N, interp, oversampling, cutoff)
-    if interp == CUBIC:          # large cubic chunks run brick by brick, with scratch
-        n = int(load().b200proj_scatter_workspace_bytes(3, B, P, N, interp, 1, float(oversampling), float(cutoff)))
-        if n:
+    # large chunks are sorted by brick first, in scratch that they can do without
+    n = int(load().b200proj_scatter_workspace_bytes(3, B, P, N, interp, 1, float(oversampling), float(cutoff)))
+    if n:
+        try:
             workspace = torch.empty(n, dtype=torch.uint8, device=proj.device)
+        except torch.cuda.OutOfMemoryError:
+            workspace = None
+        if workspace is not None:
             _call("b200proj_backproject_2d_to_3d_accumulate_ws", proj, _p(proj), _p(weights), *geom, _p(accumulator), _p(workspace), n)
             return
     _call("b200proj_backproject_2d_to_3d_accumulate", proj, _p(proj), _p(weights), *geom, _p(accumulator))

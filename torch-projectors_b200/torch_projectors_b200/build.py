@@ -33,7 +33,7 @@ BINDING_PATH = PKG_DIR / "_C.so"
 
 SOURCES = [CSRC_DIR / "b200proj.cu"]
 HEADERS = [CSRC_DIR / "fourier_slice_device.cuh", CSRC_DIR / "fourier_slice_kernels.cuh", CSRC_DIR / "brick_kernels.cuh",
-           CSRC_DIR / "brick_scatter.cuh",
+           CSRC_DIR / "brick_scatter.cuh", CSRC_DIR / "pixel_lists.cuh", CSRC_DIR / "cell_scatter.cuh",
            INCLUDE_DIR / "b200proj.h"]
 BINDING_SOURCES = [CSRC_DIR / "torch_binding.cpp"]
 
