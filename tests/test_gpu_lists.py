@@ -138,3 +138,22 @@ def test_sizes_that_are_listed_by_themselves_match_double_precision(dim, interp,
     data, wrec = forw(proj, rot, w, sh, **kw)
     assert rel_err(data, d) <= TOL_ATOMIC and rel_err(wrec, dw) <= TOL_ATOMIC
     assert rel_err(forw(proj, rot, None, sh, **kw)[0], d) <= TOL_ATOMIC
+
+
+@pytest.mark.parametrize("dim,N,os_,P,B,cutoff", [(3, 18, 2.0, 300, 1, None), (3, 6, 1.0, 151, 2, 4.0), (2, 34, 1.5, 297, 1, 11.5), (2, 66, 1.0, 100, 3, None)])
+def test_pose_gradients_of_back_projection_by_patches(dim, N, os_, P, B, cutoff):
+    """Linear calls of at least 296 slices take a slice's patches of 8 x 4 pixels in turn: ragged rows and columns, patches
+    outside the cutoff, with and without weights and shifts."""
+    import torch_projectors_b200 as tp
+    from oracle import port
+    R = -(-int(N * os_) // 2) * 2
+    t = make_inputs(Case("patches", dim, "linear", B, P, N, R, os_, cutoff, 1, 1, shift_range=2.0, seed=N))
+    forw, back = (tp.backproject_2d_forw, port.backproject_2d_back) if dim == 2 else (tp.backproject_2d_to_3d_forw, port.backproject_2d_to_3d_back)
+    for shifts in (True, False):
+        c = {k: v.cuda().requires_grad_(k in ("proj", "weights", "rot", "shifts")) for k, v in t.items()}
+        data, wrec = forw(c["proj"], c["rot"], c["weights"], c["shifts"] if shifts else None, interpolation="linear", oversampling=os_, fourier_radius_cutoff=cutoff)
+        torch.autograd.backward([data, wrec], [c["grad_data"], c["grad_weight"]])
+        want = back(t["grad_data"], t["grad_weight"], t["proj"], t["weights"], t["rot"], t["shifts"] if shifts else None, "linear", os_, cutoff, True, shifts)
+        for have, ref, what in zip((c["proj"].grad, c["weights"].grad, c["rot"].grad, c["shifts"].grad if shifts else None), want, ("projections", "weights", "rotations", "shifts")):
+            if have is not None:
+                assert rel_err(have, ref) <= TOL_ATOMIC, (what, shifts, rel_err(have, ref))

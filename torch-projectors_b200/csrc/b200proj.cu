@@ -895,6 +895,20 @@ void launch_backproject_back(const Launch& L, cudaStream_t s, const C2<Real>* gd
                              C2<Real>* grad_proj, Real* grad_weights, Real* grad_rot,
                              Real* grad_shift) {
     const bool nr = grad_rot != nullptr, ns = grad_shift != nullptr;
+    if constexpr (!CUBIC) {
+        // enough slices: patches (a whole slice per block once that is eight blocks per SM); the measurements stand at backproject_back_patches_kernel
+        if (L.g.BP >= 2 * 148 && (nr || ns)) {
+            const int64_t most = (((L.g.N + 3) / 4) * ((L.g.Nh + 7) / 8) + 7) / 8, fill = (148 * 8 + L.g.BP - 1) / L.g.BP;
+            const dim3 grid((unsigned)(fill < most ? fill : most), L.grid.y, L.grid.z);
+#define B200PROJ_BB(NR, NS) \
+    backproject_back_patches_kernel<DIM, NR, NS><<<grid, kBlockThreads, 0, s>>>(gd, gw, proj, rot, shifts, grad_proj, grad_weights, grad_rot, grad_shift, L.g)
+            if (nr && ns) B200PROJ_BB(true, true);
+            else if (nr) B200PROJ_BB(true, false);
+            else B200PROJ_BB(false, true);
+#undef B200PROJ_BB
+            return;
+        }
+    }
 #define B200PROJ_BB(NR, NS) \
     backproject_back_kernel<DIM, CUBIC, NR, NS><<<L.grid, kBlockThreads, 0, s>>>(gd, gw, proj, rot, shifts, grad_proj, grad_weights, grad_rot, grad_shift, L.g)
     if (nr && ns) B200PROJ_BB(true, true);

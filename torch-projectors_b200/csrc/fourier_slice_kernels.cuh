@@ -20,7 +20,7 @@ namespace b200proj {
 
 struct BlockWork {
     int b, p, i, j;
-    bool in_image;
+    bool slice_ok, in_image;
     size_t pix;     // element offset of (b, p, i, j) in a [B, P, N, Nh] tensor
 };
 
@@ -57,6 +57,7 @@ __device__ __forceinline__ BlockWork block_work(const SliceGeom& g) {
     if (!slice_ok) b = p = 0;
     w.b = b;
     w.p = p;
+    w.slice_ok = slice_ok;
     tile_pixel(g, (int)blockIdx.x, w.i, w.j);
     w.in_image = w.i < g.N && w.j < g.Nh && slice_ok;
     // WIDE_PIX: the same offset as one 64-bit expression per thread.  It costs the cubic 3D
@@ -754,18 +755,11 @@ backproject_slab_kernel(const float2* __restrict__ proj, const float* __restrict
 
 // ---- backward of back-projection --------------------------------------------------------
 // reference semantics: csrc/cpu/3d/backprojection_2d_to_3d_kernels.cpp:417-583
-template <int DIM, bool CUBIC, bool NEED_ROT, bool NEED_SHIFT, typename R>
-__global__ void __launch_bounds__(kBlockThreads)
-backproject_back_kernel(const C2<R>* __restrict__ grad_data_rec,
-                        const R* __restrict__ grad_weight_rec,
-                        const C2<R>* __restrict__ proj, const R* __restrict__ rot,
-                        const R* __restrict__ shifts, C2<R>* __restrict__ grad_proj,
-                        R* __restrict__ grad_weights, R* __restrict__ grad_rot,
-                        R* __restrict__ grad_shift, const SliceGeom g) {
-    const BlockWork w = block_work(g);
-    R acc[2 * DIM + 2];
-#pragma unroll
-    for (int q = 0; q < 2 * DIM + 2; ++q) acc[q] = 0.f;
+// Pixel (w.i, w.j) of the block's slice: its outputs, and its share of the pose gradients (PATCHES: added to acc).  By all lanes of a warp.
+template <int DIM, bool CUBIC, bool NEED_ROT, bool NEED_SHIFT, bool PATCHES, typename R>
+__device__ __forceinline__ void backproject_back_pixel(const SliceGeom& g, const BlockWork& w, const C2<R>* __restrict__ grad_data_rec,
+                                                       const R* __restrict__ grad_weight_rec, const C2<R>* __restrict__ proj, const R* __restrict__ rot,
+                                                       const R* __restrict__ shifts, C2<R>* __restrict__ grad_proj, R* __restrict__ grad_weights, R (&acc)[2 * DIM + 2]) {
     PixelT<R> px;
     px.c = px.r = px.d = px.sc = px.sr = px.kr = px.kc = 0.f;
     const bool active = w.in_image &&
@@ -787,8 +781,9 @@ backproject_back_kernel(const C2<R>* __restrict__ grad_data_rec,
     }
     C2<R> raw;
     R dots[4];
-    // cooperative gather: every lane of the warp takes part
-    gather_pose_dots<DIM, CUBIC, NEED_ROT, true>(g, grad_data_rec + (size_t)w.b * g.vol_elems, px, active, pv, dots, &raw);
+    // cooperative gather: every lane of the warp takes part (PATCHES: unless none has a pixel inside the cutoff)
+    if (!PATCHES || __any_sync(0xffffffffu, active))
+        gather_pose_dots<DIM, CUBIC, NEED_ROT, true>(g, grad_data_rec + (size_t)w.b * g.vol_elems, px, active, pv, dots, &raw);
     if (active) {
         __stcs(grad_proj + w.pix, g.has_shift ? cmul(raw, ph) : raw);
         if (write_w)
@@ -797,19 +792,67 @@ backproject_back_kernel(const C2<R>* __restrict__ grad_data_rec,
         if (NEED_ROT) {
 #pragma unroll
             for (int a = 0; a < DIM; ++a) {
-                acc[2 * a + 0] = dots[a] * px.sc;
-                acc[2 * a + 1] = dots[a] * px.sr;
+                const R u = dots[a] * px.sc, v = dots[a] * px.sr;
+                acc[2 * a + 0] = PATCHES ? acc[2 * a + 0] + u : u;
+                acc[2 * a + 1] = PATCHES ? acc[2 * a + 1] + v : v;
             }
         }
         if (NEED_SHIFT) {
-            acc[2 * DIM + 0] = (R)(g.shift_scale * (double)px.kr) * dots[3];
-            acc[2 * DIM + 1] = (R)(g.shift_scale * (double)px.kc) * dots[3];
+            const R u = (R)(g.shift_scale * (double)px.kr) * dots[3], v = (R)(g.shift_scale * (double)px.kc) * dots[3];
+            acc[2 * DIM + 0] = PATCHES ? acc[2 * DIM + 0] + u : u;
+            acc[2 * DIM + 1] = PATCHES ? acc[2 * DIM + 1] + v : v;
         }
     } else if (w.in_image) {
         __stcs(grad_proj + w.pix, make2<R>(0.f, 0.f));
-        if (write_w) __stcs(grad_weights + w.pix, 0.f);
+        if (write_w) __stcs(grad_weights + w.pix, (R)0.f);
     }
+}
+
+// One 16 x 16 tile of a slice per block.
+template <int DIM, bool CUBIC, bool NEED_ROT, bool NEED_SHIFT, typename R>
+__global__ void __launch_bounds__(kBlockThreads)
+backproject_back_kernel(const C2<R>* __restrict__ grad_data_rec,
+                        const R* __restrict__ grad_weight_rec,
+                        const C2<R>* __restrict__ proj, const R* __restrict__ rot,
+                        const R* __restrict__ shifts, C2<R>* __restrict__ grad_proj,
+                        R* __restrict__ grad_weights, R* __restrict__ grad_rot,
+                        R* __restrict__ grad_shift, const SliceGeom g) {
+    const BlockWork w = block_work(g);
+    R acc[2 * DIM + 2];
+#pragma unroll
+    for (int q = 0; q < 2 * DIM + 2; ++q) acc[q] = 0.f;
+    backproject_back_pixel<DIM, CUBIC, NEED_ROT, NEED_SHIFT, false>(g, w, grad_data_rec, grad_weight_rec, proj, rot, shifts, grad_proj, grad_weights, acc);
     if (NEED_ROT || NEED_SHIFT) pose_grad_flush<DIM>(g, acc, grad_rot, grad_shift, w.b, w.p);
+}
+
+// Linear taps, many slices: a block takes a share of a slice's patches of 8 columns x 4 rows, a warp each at a time, and sums its pose
+// gradients up once.  In tiles the block-wide sum of eight values per 256 pixels and the columns beyond N / 2, 31 % of the tiles
+// of box 64, weigh as much as the gather of linear taps: 2,000 slices of 64 x 33 with all gradients 182 us in tiles, 128 in
+// patches; 1,000 2D slices of 130 x 66 185 and 127.  Cubic taps: 108 us for 500 slices, 160 in patches (registers); 60 linear
+// slices of 100 x 51: 15.2 us, 17.5; 300 of them 59.5, 50.  Four blocks per SM (64 registers): three 131 us, five 148.
+template <int DIM, bool NEED_ROT, bool NEED_SHIFT, typename R>
+__global__ void __launch_bounds__(kBlockThreads, sizeof(R) == 4 ? 4 : 1)
+backproject_back_patches_kernel(const C2<R>* __restrict__ grad_data_rec,
+                                const R* __restrict__ grad_weight_rec,
+                                const C2<R>* __restrict__ proj, const R* __restrict__ rot,
+                                const R* __restrict__ shifts, C2<R>* __restrict__ grad_proj,
+                                R* __restrict__ grad_weights, R* __restrict__ grad_rot,
+                                R* __restrict__ grad_shift, const SliceGeom g) {
+    BlockWork w = block_work(g);
+    R acc[2 * DIM + 2];
+#pragma unroll
+    for (int q = 0; q < 2 * DIM + 2; ++q) acc[q] = 0.f;
+    const int lane = threadIdx.x & 31, across = (g.Nh + 7) / 8, patches = w.slice_ok ? across * ((g.N + 3) / 4) : 0;
+#pragma unroll 1
+    for (int patch = (int)blockIdx.x * kWarps + (int)(threadIdx.x >> 5); patch < patches; patch += (int)gridDim.x * kWarps) {
+        const int down = patch / across;
+        w.i = down * 4 + (lane >> 3);
+        w.j = (patch - down * across) * 8 + (lane & 7);
+        w.in_image = w.i < g.N && w.j < g.Nh;
+        w.pix = (size_t)(w.b * g.P + w.p) * (size_t)g.slice_pixels + (size_t)(w.i * g.Nh + w.j);
+        backproject_back_pixel<DIM, false, NEED_ROT, NEED_SHIFT, true>(g, w, grad_data_rec, grad_weight_rec, proj, rot, shifts, grad_proj, grad_weights, acc);
+    }
+    pose_grad_flush<DIM>(g, acc, grad_rot, grad_shift, w.b, w.p);
 }
 
 // out[k] (+)= sum over copies of it (scatters onto a small reconstruction, see scatter_copies)
