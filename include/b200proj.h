@@ -104,9 +104,11 @@ size_t b200proj_project_workspace_bytes(int dim, int64_t B, int64_t P, int64_t N
                                         double oversampling, double fourier_radius_cutoff);
 /* The same for the scatters (b200proj_project_3d_to_2d_back_records and _back_ws with
  * grad_rec, b200proj_backproject_2d_to_3d_accumulate_ws, b200proj_backproject_{2d,2d_to_3d}_forw; 0: no gain, for
- * the last of them see there for what else a workspace is good for).  These kernels' warps hand pixels to one another
- * and wait in doing so, for no longer than some seconds: should a wait ever run out, the parts of the result that lack
- * sums are NaN and the fourth int of the workspace is 1 (else 0) when the call's work has run. */
+ * the last of them see there for what else a workspace is good for).  The largest calls first sort their pixels by brick,
+ * in lists of 4 bytes per pixel inside the cutoff (at most 4 GB: more pixels take several passes), and run without any
+ * wait; a workspace that has no room for the lists is used as if they did not exist.  In cubic calls below those sizes warps
+ * hand pixels to one another and wait in doing so, for no longer than some seconds: should a wait ever run out, the parts of
+ * the result that lack sums are NaN and the fourth int of the workspace is 1 (else 0) when the call's work has run. */
 size_t b200proj_scatter_workspace_bytes(int dim, int64_t B, int64_t P, int64_t N, int interpolation, int has_weights,
                                         double oversampling, double fourier_radius_cutoff);
 /* Workspace of the backward passes of the projection (b200proj_project_{2d,3d_to_2d}_back_ws with grad_rec,
@@ -231,7 +233,7 @@ int b200proj_project_3d_to_2d_back(const float* grad_proj, const float* rec, int
  * kernel accumulates data and weight of each voxel in one 16-byte slot of the workspace (one
  * vector reduction per tap instead of two), then folds the workspace into data_rec /
  * weight_rec; without weights it spreads many slices onto a small reconstruction over copies of it in
- * the workspace and adds them up.  Large cubic calls, with or without weights, run brick by brick when the
+ * the workspace and adds them up.  Large calls run brick by brick when the
  * workspace has b200proj_scatter_workspace_bytes(...) bytes.  Results are the same up to summation order.
  * Else it reduces straight into the outputs.  The workspace holds no state between calls.
  * replaces: backproject_2d_forw_cuda       csrc/cuda/2d/backprojection_2d_kernels.cu:827-976

@@ -44,9 +44,8 @@ struct ListPlan {
     unsigned capacity;      // entries of the list
 };
 
-// Workspace: int header[64] {entries, work items, ticket, pairs, slices that are not listed, 1: some pixel is not finite, slices with
-// samples out of the grid, -}, then what follows, each
-// part on a 256-byte boundary.
+// Workspace: int header[64] {entries, work items, ticket, 0 (the brick scatters' status), slices that are not listed, 1: some pixel is
+// not finite, slices with samples out of the grid, pairs, -}, then what follows, each part on a 256-byte boundary.
 struct ListWork {
     int* header;
     unsigned* count;        // pixels of each brick; after list_plan_kernel: where the next entry goes
@@ -149,7 +148,7 @@ list_setup_kernel(const float* __restrict__ rot, const float* __restrict__ shift
         const bool first = listed(j), second = listed(j + 1);
         const unsigned m = __ballot_sync(0xffffffffu, first || second);
         int at = 0;
-        if (lane == 0 && m != 0u) at = atomicAdd(ws.header + 3, __popc(m));
+        if (lane == 0 && m != 0u) at = atomicAdd(ws.header + 7, __popc(m));
         at = __shfl_sync(0xffffffffu, at, 0);
         if (first || second)
             ws.inside[at + __popc(m & ((1u << lane) - 1u))] = (unsigned)(row + g.N / 2 - 1) << pl.bits_j | (unsigned)j | (first ? 0x40000000u : 0u) | (second ? 0x80000000u : 0u);
@@ -195,7 +194,7 @@ list_pixels_kernel(ListWork ws, const SliceGeom g, const ListPlan pl) {
     const int lane = threadIdx.x & 31, tid = threadIdx.x;
     const unsigned below = (1u << lane) - 1u;
     const bool all_fit = __ldg(ws.header + 6) == 0;
-    int slice, last, begin = 0, end = __ldg(ws.header + 3), b = 0;
+    int slice, last, begin = 0, end = __ldg(ws.header + 7), b = 0;
     unsigned* row = nullptr;
     if (SHARED) {
         // runs do not cross batch items
