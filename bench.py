@@ -462,7 +462,6 @@ SHARD = dict(name="sharded backproject_2d_to_3d_forw: 200000 slices of 400x400 +
 # read once, gradient volume zero-filled and written): 4.32 GB = 1.055 MB per slice
 STEP_BYTES_PER_SLICE = (2 * 512 * 512 * 257 * 8 + 2 * 4096 * 256 * 129 * 8 + 2 * 512 * 512 * 257 * 8) / 4096
 SHARD_BYTES_PER_SLICE = 400 * 201 * 8 + 400 * 201 * 4 + 44
-SHARD_PIXELS_PER_SLICE = 62_814          # pixels inside the default cutoff of a 400x201 slice that are scattered
 BACK_PIXELS_PER_SLICE = 6_426            # the same for a 128x65 slice
 # Reduction ceilings measured by `bench.py --workload red_ceiling` on B200 (L2-resident buffer,
 # 10^9 reductions per second).
@@ -555,7 +554,7 @@ def autograd_step_workload(args):
             "warmup": args.warmup, "ms_per_step": ms_per_step, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
             "dtype": "f32", "data": "synthetic",
             "config": {"workload": STEP["name"], "l2": "inputs (539 MB volume, 1.08 GB projections) exceed L2; 256 MiB flush before every step"},
-            "kernels_ms": ({"brick_forw_kernel<3,cubic,records> (+ setup)": f, ("pose_grad_saved_kernel" if args.fixed_volume else "brick_scatter_kernel<3> + pose_grad_saved_kernel (+ setup, clears)"): bw,
+            "kernels_ms": ({"brick_forw_kernel<3,cubic,records> (+ setup)": f, ("pose_grad_saved_kernel" if args.fixed_volume else "list_pixels_kernel x2 + cell_cubic_sums_kernel + pose_grad_saved_kernel (+ setup, clears)"): bw,
                             "loss and its gradient (torch elementwise)": ms_per_step - f - bw} if saving else
                            {"brick_forw_kernel<3,cubic> (+ setup)": f, "project_back_kernel<3,cubic,rot,shift> (+ clears)": bw,
                             "loss and its gradient (torch elementwise)": ms_per_step - f - bw}),
@@ -665,7 +664,6 @@ def run_sharded_backprojection(dist, rank, world, local_rank, dev, total, overla
     peak, peak_kind = measured_peak_gbs()
     per_rank = hi - lo
     achieved = (SHARD_BYTES_PER_SLICE * per_rank + 2 * vols.flat.numel() * 4) / (total_ms * 1e-3) / 1e9
-    taps = per_rank * SHARD_PIXELS_PER_SLICE * 8
     parity = None
     if rank == 0 and check_slices and final is not None:
         parity = check_sharded_parity(final, check_slices, dev)
@@ -680,10 +678,10 @@ def run_sharded_backprojection(dist, rank, world, local_rank, dev, total, overla
                    "l2": "each 8192-slice chunk (7.9 GB) and the 3.1 GB volumes exceed L2"},
         "scatter_ms": scatter_ms, "fold_and_reduce_ms": tail_ms, "scatter_ms_per_rank": rank_ms, "chunk_ms_rank0": chunk_ms,
         "final_stage_ms_rank0": final_ms,
-        "roofline": {"bound": "hbm", "kernel": "backproject_slab_kernel<linear,weights,interleaved> (+ fold_interleaved_kernel, NCCL reduce)",
+        "roofline": {"bound": "hbm", "kernel": "chunks: list_pixels_kernel x2 + cell_sums_kernel<3,linear,weights>; final stage: backproject_slab_kernel<linear,weights,interleaved> + fold_interleaved_kernel, NCCL reduce",
                      "achieved": achieved, "peak": peak, "peak_source": peak_kind, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": None, "launch_ms": total_ms,
-                     "secondary": reduction_ceiling(taps, scatter_ms, "lane pairs on adjacent 16-byte slots")},
+                     "secondary": None},
         "parity_check": parity,
         "gpu_launches": launches, "clocks": clocks}
 
@@ -1181,10 +1179,13 @@ def main():
         proj, weights, brot, bshifts = make_backprojection_inputs(dev, 4321 + rank, BACK["P"])
         R = tp._abi.rec_boxsize(BACK["N"], BACK["os"])
         vols = sharding.PartialVolumes(1, R, dev, with_weights=True)
-        ws_bytes = tp._abi.backproject_workspace_bytes(3, 1, R, BACK["P"], BACK["N"], tp._abi.LINEAR, True)
+        # the scratch that the public function takes: pixel lists, else an interleaved accumulation volume
+        list_bytes = int(tp._abi.load().b200proj_scatter_workspace_bytes(3, 1, BACK["P"], BACK["N"], tp._abi.LINEAR, 1, BACK["os"], BACK["N"] / 2.0))
+        ws_bytes = list_bytes or tp._abi.backproject_workspace_bytes(3, 1, R, BACK["P"], BACK["N"], tp._abi.LINEAR, True)
         workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=dev) if ws_bytes else None
         scatter_ev = []
-        back_kernel_name = ("memset(workspace) + backproject_forw_interleaved_kernel<3,linear> + fold_interleaved_kernel" if workspace is not None
+        back_kernel_name = ("list_setup_kernel + list_pixels_kernel x2 + list_plan_kernel + cell_sums_kernel<3,linear,weights> + scatter_rest_kernel" if list_bytes else
+                            "memset(workspace) + backproject_forw_interleaved_kernel<3,linear> + fold_interleaved_kernel" if workspace is not None
                             else "memset(volumes) + backproject_forw_kernel<3,linear,weights>")
 
         def back_step():
@@ -1206,13 +1207,14 @@ def main():
                 "config": {"workload": BACK["name"], "collective": "NCCL reduce of data+weight partial volumes to rank 0" if world > 1 else "none"},
                 "roofline": {"bound": "hbm", "kernel": back_kernel_name, "achieved": bach,
                              "peak": peak, "peak_source": peak_kind, "unit": "GB/s", "frac": bach / peak,
-                             "traffic": (BACK_TRAFFIC_FIXED + BACK_TRAFFIC_PER_SLICE * BACK["P"]) if workspace is not None else None,
+                             "traffic": (BACK_TRAFFIC_FIXED + BACK_TRAFFIC_PER_SLICE * BACK["P"]) if workspace is not None and not list_bytes else None,
                              "algorithmic_bytes_per_launch": BACK_BYTES_PER_SLICE * BACK["P"], "launch_ms": scat,
-                             "secondary": reduction_ceiling(BACK["P"] * BACK_PIXELS_PER_SLICE * 8, scat,
+                             # from lists the taps are added up on chip: the reductions' ceiling is not theirs
+                             "secondary": None if list_bytes else reduction_ceiling(BACK["P"] * BACK_PIXELS_PER_SLICE * 8, scat,
                                                             "lane pairs on adjacent 16-byte slots" if workspace is not None else "lane pairs on adjacent 8-byte voxels")}}
         if rank == 0 and not args.skip_cpu:
             back["parity_check"] = check_backprojection_parity(tp, proj, weights, brot, bshifts, dev)
-        launches += (args.steps + args.warmup) * (2 if workspace is not None else 1)     # scatter (+ fold)
+        launches += (args.steps + args.warmup) * (6 if list_bytes else 2 if workspace is not None else 1)     # lists and sums | scatter (+ fold)
         del proj, weights
         torch.cuda.empty_cache()
 

@@ -309,7 +309,7 @@ BrickLaunch gather_plan(int dim, int64_t B, int64_t P, int64_t N, bool cubic, bo
     return L;
 }
 
-// Cubic scatter (linear taps keep the plain kernels, see brick_scatter.cuh).
+// Cubic scatter (below the sizes of pixel lists; linear taps: plain kernels, see brick_scatter.cuh).
 template <int DIM, bool WEIGHTS>
 BrickLaunch scatter_layout(int64_t B, int64_t P, int64_t N, double os, double cutoff) {
     using C = Scatter<DIM, WEIGHTS>;

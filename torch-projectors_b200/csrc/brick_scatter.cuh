@@ -28,7 +28,11 @@
 // planes 6.1 ms, 8 slabs of 8 planes 6.4 ms, one block of 14 walkers and 10 slabs 6.6 ms, one adding warp per block
 // with a barrier for each hand-over 7.8 ms, and pixels of a full ring sent to L2 as reductions by the walkers 7.6 ms
 // (that starves the adding warps).  For linear taps (2 x 2 x 2 classes, overlapping pixels one after the other) the
-// same scheme took 44-46 ps per pixel where the plain kernels take 33: those keep their reductions.
+// same scheme took 44-46 ps per pixel where the plain kernels take 33.
+//
+// Calls with more pixels per brick, linear ones included, run from pixel lists (cell_scatter.cuh), which take 42 instead of 56 ps per
+// pixel of the scatter above; these kernels have the calls whose bricks hold too few pixels for a cell's sums to pay
+// (list_scatter_plan in b200proj.cu), and those whose workspace has no room for a list.
 #pragma once
 
 #include "brick_kernels.cuh"
