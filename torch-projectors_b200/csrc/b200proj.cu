@@ -297,13 +297,14 @@ BrickLaunch gather_plan(int dim, int64_t B, int64_t P, int64_t N, bool cubic, bo
     if (dim == 2) {
         // cubic: measured crossings at 2-5 M pixels (27 M: 2.1-2.3x); linear taps are not faster at any size (0.6-1.05x)
         if (!cubic) return BrickLaunch{};
-        BrickLaunch L = brick_layout<GatherBrick<2>>(B, P, N, os, cutoff, 148.0 * 3.0, 6000.0, true);
+        BrickLaunch L = brick_layout<GatherBrick<2, true>>(B, P, N, os, cutoff, 148.0 * 3.0, 6000.0, true);
         L.use = L.use && (L.forced || L.pixels > 4.5e6);
         return L;
     }
-    BrickLaunch L = brick_layout<GatherBrick<3>>(B, P, N, os, cutoff, 148.0 * 3.0, 3000.0, true);
+    BrickLaunch L = cubic ? brick_layout<GatherBrick<3, true>>(B, P, N, os, cutoff, 148.0 * 3.0, 3000.0, true)
+                          : brick_layout<GatherBrick<3, false>>(B, P, N, os, cutoff, 148.0 * 4.0, 3000.0, true);
     const double need = cubic ? (1.2e6 + 900.0 * L.in_ball) * (os < 2.0 ? 2.0 / os : 1.0)
-                              : (10e6 + 4000.0 * L.in_ball) * (records ? 0.6 : 1.0);
+                              : (10e6 + 3100.0 * L.in_ball) * (records ? 0.6 : 1.0);
     // linear taps: small volumes meet a slice in too few pixels per brick (box 38 oversampled twice: 1.8x slower)
     L.use = L.use && (L.forced || (L.pixels > need && (cubic || L.plan.reach > 84.f)));
     return L;
@@ -365,7 +366,7 @@ int launch_brick_forw(const Launch& L, const BrickLaunch& bl, void* workspace, c
     constexpr size_t smem = sizeof(float2) * BrickShape<DIM, CUBIC>::kVoxels + sizeof(GatherBlock);
     const cudaError_t e = cudaFuncSetAttribute(brick_forw_kernel<DIM, CUBIC, SAVE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cuda_fail(e, "brick_forw shared memory");
-    brick_forw_kernel<DIM, CUBIC, SAVE><<<148 * 3, kBlockThreads, smem, s>>>((const float2*)rec, rot, shifts, (float2*)out, (float2*)derivs, w, L.g, bl.plan);
+    brick_forw_kernel<DIM, CUBIC, SAVE><<<148 * (CUBIC ? 3 : 4), kBlockThreads, smem, s>>>((const float2*)rec, rot, shifts, (float2*)out, (float2*)derivs, w, L.g, bl.plan);
     return check_launch("brick_forw launch");
 }
 

@@ -6,9 +6,9 @@
 // its pixels, of all slices, come from shared memory without bank conflicts, 16 lanes = 128 bytes a
 // wavefront: 4 wavefronts per cubic pixel instead of 13-18.  Measured on B200: 10,000 slices of 128 x 65
 // from a box-256 volume, cubic, 3.95 -> 1.77 ms (62 -> 27 ps per pixel; data pipe 75 %, issue 69 %), with
-// records 8.9 -> 4.0 ms for 4,096 slices of 256 x 129 from a box-512 volume; linear 1.09 -> 1.02 ms.
+// records 8.9 -> 4.0 ms for 4,096 slices of 256 x 129 from a box-512 volume; linear 1.09 -> 0.97 ms.
 //
-// Bricks of 17 x 17 x 16 sample positions: with the halo of cubic taps 20 x 20 x 19 voxels = 61 KB, three
+// Bricks of 17 x 17 x 16 sample positions (cubic): with the halo 20 x 20 x 19 voxels = 61 KB, three
 // blocks (24 warps, 80 registers) per SM.  Smaller bricks meet a slice in too few pixels (here 40) to
 // pay for finding them.
 //
@@ -29,12 +29,17 @@ struct BrickDims {
 };
 // 2D tiles of 61 x 61 (64 x 64 with the halo, 32 KB): all slices of a half-plane meet a tile, in rows of some 30 pixels,
 // so that the walk costs less than in 3D (500 slices of 128 x 65 from each of eight references, cubic: 0.755 -> 0.350 ms).
-template <int DIM>
+// Linear taps have a halo of one voxel, and 64 registers are enough: bricks of 15 x 15 x 16 (16 x 16 x 17 voxels, 35 KB) make room for four
+// blocks per SM.  Linear, 3,001 slices of 180 x 91 478 -> 443 us, 8,000 of 128 x 65 from a box-256 volume 816 -> 777, records of 2,000 of
+// 200 x 101 548 -> 521; 15 x 15 x 20 444, 747, 547; 19 x 19 x 18 and three blocks 473, 770, 563; 23 x 23 x 21 and two 561; 15 x 15 x 13 and five 463.
+template <int DIM, bool CUBIC>
 struct GatherBrickOf { using type = BrickDims<17, 17, 16>; };
 template <>
-struct GatherBrickOf<2> { using type = BrickDims<61, 61, 0>; };
-template <int DIM>
-using GatherBrick = typename GatherBrickOf<DIM>::type;
+struct GatherBrickOf<3, false> { using type = BrickDims<15, 15, 16>; };
+template <bool CUBIC>
+struct GatherBrickOf<2, CUBIC> { using type = BrickDims<61, 61, 0>; };
+template <int DIM, bool CUBIC>
+using GatherBrick = typename GatherBrickOf<DIM, CUBIC>::type;
 constexpr int kBrickSlots = 8;                              // slices a warp takes at a time
 constexpr float kBrickSlack = 0.06f;                        // slack of the linear estimates, in voxels
 
@@ -295,7 +300,7 @@ brick_setup_kernel(const float* __restrict__ rot, const float* __restrict__ shif
 // their pixels lie.
 template <int DIM, bool CUBIC>
 struct BrickShape {
-    using D = GatherBrick<DIM>;
+    using D = GatherBrick<DIM, CUBIC>;
     static constexpr int T = CUBIC ? 4 : 2;
     static constexpr int TX = ((D::x + T - 1) + 3) / 4 * 4, TY = ((D::y + T - 1) + 3) / 4 * 4, TZ = DIM == 3 ? D::z + T - 1 : 1;
     static constexpr int kRowCells = TX / 4 * 16;            // voxels of four rows
@@ -671,7 +676,7 @@ using GatherBlock = BrickBlock<kWarps, 1024>;
 
 // Forward projection (SAVE: with the derivatives of project_forw_saving_kernel, 3D as records).
 template <int DIM, bool CUBIC, bool SAVE>
-__global__ void __launch_bounds__(kBlockThreads, 3)
+__global__ void __launch_bounds__(kBlockThreads, CUBIC ? 3 : 4)
 brick_forw_kernel(const float2* __restrict__ rec, const float* __restrict__ rot, const float* __restrict__ shifts,
                   float2* __restrict__ out, float2* __restrict__ derivs, BrickWork ws, const SliceGeom g, const BrickPlan pl) {
     extern __shared__ __align__(16) unsigned char dyn[];
@@ -688,10 +693,10 @@ brick_forw_kernel(const float2* __restrict__ rec, const float* __restrict__ rot,
         for (int k = (int)((long long)g.BP * item / items), k_end = (int)((long long)g.BP * (item + 1) / items); k < k_end; ++k)
             brick_rest<DIM, CUBIC, SAVE>(g, ws, k, rec, rot, shifts, out, derivs);
         const int4 it = brick_item(ws, pl, item);
-        const int X0 = pl.lo[0] + (it.x & 1023) * GatherBrick<DIM>::x, Y0 = pl.lo[1] + ((it.x >> 10) & 1023) * GatherBrick<DIM>::y, Z0 = pl.lo[2] + (it.x >> 20) * GatherBrick<DIM>::z;
+        const int X0 = pl.lo[0] + (it.x & 1023) * GatherBrick<DIM, CUBIC>::x, Y0 = pl.lo[1] + ((it.x >> 10) & 1023) * GatherBrick<DIM, CUBIC>::y, Z0 = pl.lo[2] + (it.x >> 20) * GatherBrick<DIM, CUBIC>::z;
         brick_stage<DIM, CUBIC>(g, rec + (size_t)it.y * g.vol_elems, sm, X0, Y0, Z0);
         const BrickWarp& sw = sb.warp[threadIdx.x >> 5];
-        brick_walk<GatherBrick<DIM>>(g, ws.recs, ws.shifts, sb, X0, Y0, Z0, it.z, it.w, 0, 1,
+        brick_walk<GatherBrick<DIM, CUBIC>>(g, ws.recs, ws.shifts, sb, X0, Y0, Z0, it.z, it.w, 0, 1,
                    [&](bool active, int slot, int i, int j, const Pixel& px, int lx, int ly, int lz) {
             float2 v, gc, gr, gd;
             brick_gather<DIM, CUBIC, SAVE>(sm, lx, ly, lz, px.c - floorf(px.c), px.r - floorf(px.r), DIM == 3 ? px.d - floorf(px.d) : 0.f, v, gc, gr, gd);
