@@ -458,7 +458,6 @@ ListLaunch list_layout(int dim, int64_t B, int64_t R, int64_t P, int64_t N, doub
     const double most = (double)entries / (blocks * 8.0);
     p.most = most < 4096.0 ? 4096 : most > 8192.0 ? 8192 : (int)most;
     const size_t up = 255, items = (size_t)(bricks < entries ? bricks : entries) + (size_t)(entries / p.most) + 1;
-    L.count_bytes = ((size_t)bricks * sizeof(unsigned) + up) & ~up;
     L.item_bytes = (items * sizeof(int4) + up) & ~up;
     L.pose_bytes = ((size_t)L.slices * 2 * sizeof(float4) + up) & ~up;
     L.inside_bytes = ((size_t)pairs * sizeof(unsigned) + up) & ~up;
@@ -469,6 +468,9 @@ ListLaunch list_layout(int dim, int64_t B, int64_t R, int64_t P, int64_t N, doub
         L.block_bytes = ((size_t)B * (size_t)((P + p.run - 1) / p.run) * (size_t)p.item_bricks * sizeof(unsigned) + up) & ~up;
         if (L.block_bytes > (64u << 20)) p.run = 0, L.block_bytes = 0;
     }
+    // counters of a brick (see list_pixels_kernel): half of the bricks of the grid meet slices
+    for (p.subs = 1; p.run == 0 && p.subs < 8 && 2 * p.subs * bricks <= 80000;) p.subs *= 2;
+    L.count_bytes = ((size_t)bricks * (size_t)p.subs * sizeof(unsigned) + up) & ~up;
     L.bytes = 256 + L.count_bytes + L.item_bytes + L.pose_bytes + L.inside_bytes + L.block_bytes + (size_t)entries * sizeof(unsigned);
     L.forced = force == 1;
     L.use = true;

@@ -40,6 +40,7 @@ struct ListPlan {
     int inside;             // pixels of a slice that are listed
     int pairs;              // room for their pairs
     int most;               // pixels of a work item
+    int subs;               // counters of a brick (a power of two), for slices taken in turn
     int run;                // slices of a block of list_pixels_kernel that counts in shared memory; 0: in global memory
     unsigned capacity;      // entries of the list
 };
@@ -181,7 +182,12 @@ constexpr int kListBricks = 4096;           // bricks of a batch item that a blo
 // between them, in which second pixels join that lie in the brick of their own first pixel or of the next lane's; the few
 // others go by themselves.  (The match instruction holds the SM's only unit for it for 31 clocks: with one per 32 pixels, not per
 // 64, a pass took 3.5 ps per pixel.)
-//   pl.run == 0: counts in global memory.  Grid: x = kListPairs pairs of a slice, (y, z) = the slice.
+//   pl.run == 0: counts in global memory, pl.subs for each brick, which slices use in turn: atomics at the bricks that many slices meet
+//   in would queue up.  But each is a place where the second pass writes, and beyond some 40,000 such places sectors leave L2
+//   half written.  (Passes in us with 1 / 4 / 8 / 16 counters: 2,501 slices of 90 x 46, 3,000 bricks met, 49 + 55 / 26 + 36 / 26 + 36 / 26 + 36;
+//   50,000 of 128 x 65, 8,600 bricks, 1,070 + 1,500 / 886 + 1,444 / 892 + 1,545 / 892 + 1,670; 4,096 of 256 x 129, 68,000 bricks, 280 + 472 /
+//   261 + 582 / 262 + 648 / 261 + 725; 10,000 of 128 x 65 in one plane 1,486 + 1,524 / 525 + 563 / 429 + 465 / 215 + 251.)
+//   Grid: x = kListPairs pairs of a slice, (y, z) = the slice.
 //   else: bricks are few and many slices meet in each (2D: all slices in every tile), so atomics would queue up at a few
 //   addresses.  A block counts pl.run slices of a batch item in shared memory, and keeps its counts for the second pass.
 //   Grid: x = runs of a batch item, y = batch item.
@@ -244,7 +250,7 @@ list_pixels_kernel(ListWork ws, const SliceGeom g, const ListPlan pl) {
                 own[q] = __ballot_sync(kFull, to_own);
                 next[q] = __ballot_sync(kFull, to_next) << 1;       // by the lane whose brick it is
                 at[q] = at2[q] = 0u;
-                unsigned* counts = SHARED ? here : ws.count;
+                unsigned* counts = SHARED ? here : ws.count + (size_t)(slice & (pl.subs - 1)) * (size_t)pl.bricks;
                 if (brick[q] >= 0 && (same[q] & below) == 0u) {
                     const unsigned n = __popc(same[q]) + __popc(same[q] & own[q]) + __popc(same[q] & next[q]);
                     if (COUNT) atomicAdd(counts + brick[q], n);
@@ -297,7 +303,10 @@ list_plan_kernel(ListWork ws, const ListPlan pl, int B) {
     }
     const bool here = b < B && x < pl.n[0] && y < pl.n[1] && z < pl.n[2];
     const int brick = ((b * pl.n[2] + z) * pl.n[1] + y) * pl.n[0] + x;
-    const int n = here ? (int)ws.count[brick] : 0, parts = (n + pl.most - 1) / pl.most;
+    int n = 0;
+    if (here)
+        for (int k = 0; k < pl.subs; ++k) n += (int)ws.count[(size_t)k * (size_t)pl.bricks + brick];
+    const int parts = (n + pl.most - 1) / pl.most;
     int n_upto = n, parts_upto = parts;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -321,7 +330,15 @@ list_plan_kernel(ListWork ws, const ListPlan pl, int B) {
     }
     __syncthreads();
     const int first = base[0] + warp_n[warp] + n_upto - n;
-    if (n > 0) ws.count[brick] = (unsigned)first;
+    if (n > 0) {
+        int at = first;
+        for (int k = 0; k < pl.subs; ++k) {
+            unsigned& c = ws.count[(size_t)k * (size_t)pl.bricks + brick];
+            const int m = (int)c;
+            c = (unsigned)at;
+            at += m;
+        }
+    }
     // Items part by part: the first of all bricks of the block, then the second ...  Neighbours then go through the same
     // slices at the same time, whose sectors they share.
     __shared__ int level[2][8];
