@@ -122,7 +122,10 @@ scatter_rest_kernel(const float2* __restrict__ proj, const float* __restrict__ w
             if ((j == 0 && i >= g.N / 2) || !pixel_setup<DIM>(g, pose_rot<DIM>(g, rot, b, p), i, j, px)) continue;
             float2 v = __ldg(proj + pix);
             const float w = WEIGHTS ? __ldg(weights + pix) : 0.f;
-            if (g.has_shift) v = cmul_conj(v, phase_ramp(g, px, __ldg(pose_shift(g, shifts, b, p)), __ldg(pose_shift(g, shifts, b, p) + 1)));
+            if (g.has_shift) {              // of listed slices as where the sums are formed, so that both find the same pixels finite
+                const float dot = add_rn(mul_rn(px.kr, __ldg(pose_shift(g, shifts, b, p))), mul_rn(px.kc, __ldg(pose_shift(g, shifts, b, p) + 1)));
+                v = cmul_conj(v, all ? phase_of_dot(g, dot) : list_phase(g, dot));
+            }
             if (all || !finite_values(v, w)) scatter_alone<DIM, CUBIC, DUP>(g, to, (long long)b * g.vol_elems, px.c, px.r, px.d, v, w);
         }
     }
