@@ -2,6 +2,8 @@
 and rejects bad arguments with error codes before touching the device."""
 import ctypes as C
 import re
+import subprocess
+import sys
 from pathlib import Path
 
 import pytest
@@ -155,3 +157,18 @@ def test_header_is_plain_c(tmp_path):
     r = subprocess.run([gcc, "-std=c99", "-Wall", "-Wextra", "-pedantic", "-Werror", "-fsyntax-only", f"-I{HEADER.parent}", str(src)],
                        capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
+
+
+@pytest.mark.parametrize("dim,interp", [(2, 0), (2, 1), (3, 0), (3, 1)])
+def test_scratch_queries_end_for_any_cutoff(dim, interp):
+    """Cutoffs beyond the corners of a slice, infinity among them ("no cutoff"), list all of its pixels and take no longer than
+    others.  In a process of its own with a limit: the count of listed pixels once walked up to the cutoff in every row."""
+    code = (f"from torch_projectors_b200 import _abi; lib = _abi.load(); N = 128\n"
+            f"q = lambda c: (lib.b200proj_scatter_workspace_bytes({dim}, 1, 50000, N, {interp}, 1, 2.0, c), lib.b200proj_gradient_workspace_bytes({dim}, 1, 256, 50000, N, {interp}, 0, 2.0, c))\n"
+            "want = q(float(N))\n"
+            "assert min(want) > 4 * 50000 * (N * (N // 2 + 1) - N // 2), want\n"
+            "assert all(q(c) == want for c in (90.6, 1e3, 1e6, 1e9, 1e18, 1e30, 1e300, float('inf'))), [q(c) for c in (1e3, float('inf'))]\n"
+            "assert all(a < b for a, b in zip(q(N / 2.0), want))")
+    root = Path(__file__).resolve().parent.parent
+    r = subprocess.run([sys.executable, "-c", code], cwd=root / "torch-projectors_b200", capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stderr[-2000:]

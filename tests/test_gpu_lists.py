@@ -157,3 +157,20 @@ def test_pose_gradients_of_back_projection_by_patches(dim, N, os_, P, B, cutoff)
         for have, ref, what in zip((c["proj"].grad, c["weights"].grad, c["rot"].grad, c["shifts"].grad if shifts else None), want, ("projections", "weights", "rotations", "shifts")):
             if have is not None:
                 assert rel_err(have, ref) <= TOL_ATOMIC, (what, shifts, rel_err(have, ref))
+
+
+@pytest.mark.parametrize("dim,interp,N,P", [(3, "linear", 64, 9000), (3, "cubic", 48, 4000), (2, "cubic", 128, 900), (2, "linear", 128, 6000)])
+def test_a_listed_call_takes_an_infinite_cutoff(dim, interp, N, P):
+    """The same as a cutoff beyond the corners of the slices (here: several hundred thousand pixels more than within Nyquist)."""
+    import torch_projectors_b200 as tp
+    gen = torch.Generator("cuda").manual_seed(P)
+    proj = torch.randn(1, P, N, N // 2 + 1, dtype=torch.complex64, generator=gen, device="cuda")
+    w = torch.rand(proj.shape, generator=gen, device="cuda")
+    rot = torch.linalg.qr(torch.randn(1, P, dim, dim, generator=gen, device="cuda"))[0].contiguous()
+    assert tp._abi.load().b200proj_scatter_workspace_bytes(dim, 1, P, N, tp.ops._interp_code(interp), 1, 2.0, float("inf")) > 4 * 0.99 * P * N * (N // 2), "not listed"
+    forw = tp.backproject_2d_to_3d_forw if dim == 3 else tp.backproject_2d_forw
+    a, aw = forw(proj, rot, w, interpolation=interp, oversampling=2.0, fourier_radius_cutoff=float("inf"))
+    b, bw = forw(proj, rot, w, interpolation=interp, oversampling=2.0, fourier_radius_cutoff=float(N))
+    assert rel_err(a, b) <= TOL_ATOMIC and rel_err(aw, bw) <= TOL_ATOMIC
+    inner, _ = forw(proj, rot, w, interpolation=interp, oversampling=2.0)
+    assert rel_err(inner, b) > 100 * TOL_ATOMIC

@@ -403,10 +403,10 @@ void listed_pixels(int64_t N, double cutoff, int64_t* pixels, int64_t* pairs) {
     for (int64_t kr = 1 - N / 2; kr <= N / 2; ++kr) {
         const double left = room - (double)(kr * kr);
         if (!(left >= 0.0)) continue;
-        int64_t j = left >= 4.0 * (double)(N * N) ? N / 2 : (int64_t)sqrt(left);
-        while ((double)((j + 1) * (j + 1)) <= left) ++j;
+        // the last column within the cutoff; a cutoff beyond the slice (infinite ones too) is cut to it first
+        int64_t j = left >= (double)(N / 2) * (double)(N / 2) ? N / 2 : (int64_t)sqrt(left);
+        while (j < N / 2 && (double)((j + 1) * (j + 1)) <= left) ++j;
         while ((double)(j * j) > left) --j;
-        if (j > N / 2) j = N / 2;
         *pixels += j + 1;
         *pairs += j / 2 + 1;
         if (kr < 0 || kr == N / 2) --*pixels;             // the mirrored half of column 0
