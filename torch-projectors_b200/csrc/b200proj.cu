@@ -350,11 +350,11 @@ BrickWork brick_work(const BrickLaunch& L, void* workspace) {
 }
 
 template <int DIM>
-int brick_setup(const BrickLaunch& bl, const BrickWork& w, const Launch& L, const float* rot, const float* shifts, bool outside, cudaStream_t s) {
+int brick_setup(const BrickLaunch& bl, const BrickWork& w, const Launch& L, const float* rot, const float* shifts, bool outside, cudaStream_t s, Gate gate = {}) {
     if (int rc = zero_async(w.header, 80, s)) return rc;
     const int64_t clusters = (int64_t)((bl.plan.n[0] + 7) / 8) * ((bl.plan.n[1] + 7) / 8) * ((bl.plan.n[2] + 3) / 4) * L.B;
     const int64_t slices = (L.B * L.P + 255) / 256;
-    brick_setup_kernel<DIM><<<(unsigned)(1 + clusters + slices), 256, 0, s>>>(rot, shifts, w, L.g, bl.plan, (int)L.B, outside ? 1 : 0);
+    brick_setup_kernel<DIM><<<(unsigned)(1 + clusters + slices), 256, 0, s>>>(rot, shifts, w, L.g, bl.plan, (int)L.B, outside ? 1 : 0, gate);
     return check_launch("brick_setup launch");
 }
 
@@ -372,17 +372,17 @@ int launch_brick_forw(const Launch& L, const BrickLaunch& bl, void* workspace, c
 
 template <int DIM, bool WEIGHTS, bool DUP, bool INTERLEAVED = false>
 int launch_brick_scatter(const Launch& L, const BrickLaunch& bl, void* workspace, const float* proj, const float* weights, const float* rot,
-                         const float* shifts, float* vol, float* wvol, cudaStream_t s, float4* accum = nullptr) {
+                         const float* shifts, float* vol, float* wvol, cudaStream_t s, float4* accum = nullptr, Gate gate = {}) {
     using C = Scatter<DIM, WEIGHTS>;
     const BrickWork w = brick_work(bl, workspace);
     BrickLaunch kept = bl;
     kept.plan.keep = L.g.half;
-    if (int rc = brick_setup<DIM>(kept, w, L, rot, shifts, false, s)) return rc;
+    if (int rc = brick_setup<DIM>(kept, w, L, rot, shifts, false, s, gate)) return rc;
     constexpr size_t smem = sizeof(typename C::Shared);
     static_assert((smem + 1024) * C::kBlocks <= 233472, "shared memory of an SM");
     const cudaError_t e = cudaFuncSetAttribute(brick_scatter_kernel<DIM, WEIGHTS, DUP, INTERLEAVED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cuda_fail(e, "brick_scatter shared memory");
-    brick_scatter_kernel<DIM, WEIGHTS, DUP, INTERLEAVED><<<148 * C::kBlocks, C::kThreads, smem, s>>>((const float2*)proj, weights, rot, shifts, (float2*)vol, wvol, accum, w, L.g, bl.plan);
+    brick_scatter_kernel<DIM, WEIGHTS, DUP, INTERLEAVED><<<148 * C::kBlocks, C::kThreads, smem, s>>>((const float2*)proj, weights, rot, shifts, (float2*)vol, wvol, accum, w, L.g, bl.plan, gate);
     return check_launch("brick_scatter launch");
 }
 
@@ -468,6 +468,10 @@ ListLaunch list_layout(int dim, int64_t B, int64_t R, int64_t P, int64_t N, doub
         L.block_bytes = ((size_t)B * (size_t)((P + p.run - 1) / p.run) * (size_t)p.item_bricks * sizeof(unsigned) + up) & ~up;
         if (L.block_bytes > (64u << 20)) p.run = 0, L.block_bytes = 0;
     }
+    // slices of a block that counts in global memory: several make a shorter grid, which a call whose lists are left aside waits for (0.5 ns a
+    // block).  They follow one another, so that the lists keep the order of the slices (persistent blocks that took slices far apart: sums 5 % slower)
+    const int64_t blocks_of = ((pairs + kListPairs - 1) / kListPairs) * p.slices;
+    p.turn = blocks_of < 16384 ? 1 : 4;
     // counters of a brick (see list_pixels_kernel): half of the bricks of the grid meet slices
     for (p.subs = 1; p.run == 0 && p.subs < 8 && 2 * p.subs * bricks <= 80000;) p.subs *= 2;
     L.count_bytes = ((size_t)bricks * (size_t)p.subs * sizeof(unsigned) + up) & ~up;
@@ -490,14 +494,42 @@ ListWork list_work(const ListLaunch& L, void* workspace) {
     return w;
 }
 
+int copies_wanted(int dim, double one, int64_t B, int64_t P, int64_t N, bool cubic, bool pose_gradients);
+// Scratch of the scatter that runs when the lists are left aside (see Gate).  weights: 1 to a volume of their own, 2 into 16-byte voxels.
+size_t without_lists_bytes(int dim, int64_t B, int64_t R, int64_t P, int64_t N, bool cubic, int weights, double os, double cutoff) {
+    const BrickLaunch bl = scatter_plan(dim, B, P, N, cubic, weights != 0, os, cutoff);
+    if (bl.use) return bl.bytes;
+    if (weights == 2 || (dim == 3 && slab_plan(R, weights != 0).slabs > 1)) return 0;
+    const double one = (double)B * (dim == 3 ? R : 1) * R * (R / 2 + 1) * (double)(weights ? sizeof(float4) : sizeof(float2));
+    const int copies = weights ? workspace_replicas(one, P) : copies_wanted(dim, one, B, P, N, cubic, false);
+    return weights || copies > 1 ? (size_t)one * (size_t)copies : 0;
+}
+// When the lists are left aside: calls in which a brick's pixels share fewer than `crowd` of its cells (see list_setup_kernel; 128 lies between the
+// 190 and more of poses that are spread and the 80 and less of those that are not), and only where the scatter without lists is then faster.
+// Measured, without / from lists, weighted (unweighted): 3D linear, 10,000 slices of 128 x 65 oversampled twice: tilt series 1.46 / 1.59 (1.27 / 1.33) ms, in steps of
+// 3 degrees 1.45 / 2.01, one plane 1.33 / 2.69, one pose 2.5 / 4.4, ten poses 2.2 / 3.5, a hundred 2.2 / 2.2 (1.51 / 1.73), half of the slices in one plane 1.75 / 2.63;
+// not oversampled 0.7-1.1x.  2D, all slices turned alike / not turned, oversampled twice, cubic: 4 M pixels 0.77 / 0.46x of the time from lists,
+// 10 M 1.1 / 0.9x, 30 M and more 1.1-1.3x, but 64 x 33 references 0.85x at any number; linear: 22 M 1.0 / 0.79x, 45 M 1.2 / 0.85x, 77 M and
+// more 1.05-1.5x.  3D cubic: 1.1-4x, except one pose and ten poses onto boxes of 64 and 96 (0.75-0.95x), which from here look like one plane (2x).
+void list_crowd_rule(ListLaunch& L, int dim, int64_t B, int64_t R, int64_t P, int64_t N, bool cubic, int weights, double os, double cutoff) {
+    static const float force = [] { const char* e = getenv("B200PROJ_LIST_CROWD"); return e ? (float)atof(e) : -1.f; }();   // number of cells, for tests
+    const bool gains = dim == 3 ? !cubic : cubic ? L.pixels < 7e6 || R <= 72 : L.pixels < 6e7;
+    L.plan.crowd = P < 2 || (dim == 3 && cubic) ? 0.f : force >= 0.f ? force : gains ? 128.f : 0.f;
+    if (L.plan.crowd == 0.f) return;
+    L.plan.probes = dim == 3 ? 256 : 64;
+    const size_t other = 256 + without_lists_bytes(dim, B, R, P, N, cubic, weights, os, cutoff);
+    if (other > L.bytes) L.bytes = other;
+}
 // Scatters from pixel lists: above a number of pixels that grows with the bricks (a brick costs its latency and its flush
 // however few pixels it has).  Measured crossings with the kernels used otherwise (in M pixels; bricks inside the ball of the samples), with
 // weights / without: 3D cubic, oversampled twice: 134 bricks 3 / 4, 1,072 2.3 / 3.5, 8,578 9 / 8, 68,600 55 / 50; not oversampled 0.5 / 0.8
 // and 1 / 0.9 of 134 and 1,072.  3D linear 10 / 17, 8.5 / 14, 7 / 26, 36 / 40; 3 / 5, 4.3 / 7.  2D cubic, tiles: 6 1.8 / 3, 25 1.4 / 2.2, 100
 // 1.4 / 2.3, 402 2.4 / 4.  2D linear 25 / 40, 10 / 35, 10.5 / 38, 25 / 50.  Far above them 1.25-1.7x (3D), 1.2-1.7x (2D).
-ListLaunch list_scatter_plan(int dim, int64_t B, int64_t R, int64_t P, int64_t N, bool cubic, bool weights, double os, double cutoff) {
-    const ListLaunch L = list_layout(dim, B, R, P, N, os, cutoff, 148.0 * 4);
-    if (!L.use || L.forced) return L;
+ListLaunch list_scatter_plan(int dim, int64_t B, int64_t R, int64_t P, int64_t N, bool cubic, int weights, double os, double cutoff) {
+    ListLaunch L = list_layout(dim, B, R, P, N, os, cutoff, 148.0 * 4);
+    if (!L.use) return L;
+    list_crowd_rule(L, dim, B, R, P, N, cubic, weights, os, cutoff);
+    if (L.forced) return L;
     const double r = L.plan.reach < (float)R * 0.5f ? L.plan.reach : (double)R * 0.5;
     const double bricks = (double)B * (dim == 3 ? 2.094 * r * r * r / 512.0 : 1.571 * r * r / 256.0);
     const bool dense = os < 1.25;
@@ -522,9 +554,10 @@ int with_lists(const Launch& L, const ListLaunch& ll, void* workspace, const flo
         pl.slices = (int)(ll.slices - first < per_pass ? ll.slices - first : per_pass);
         if (int rc = zero_async(w.header, 256 + ll.count_bytes, s)) return rc;
         const unsigned tiles = (unsigned)(L.g.tiles_i * ((L.g.Nh + 31) / 32));
-        list_setup_kernel<DIM><<<tiles + (unsigned)((ll.slices + 255) / 256), 256, 0, s>>>(rot, shifts, w, L.g, pl);
+        list_setup_kernel<DIM><<<tiles + (unsigned)((ll.slices + 255) / 256 + pl.probes), 256, 0, s>>>(rot, shifts, w, L.g, pl);
         if (int rc = check_launch("list_setup launch")) return rc;
-        dim3 grid((unsigned)((pl.pairs + kListPairs - 1) / kListPairs), (unsigned)(pl.slices < 32768 ? pl.slices : 32768), (unsigned)((pl.slices + 32767) / 32768));
+        const unsigned across = (unsigned)((pl.pairs + kListPairs - 1) / kListPairs), down = (unsigned)((pl.slices + pl.turn - 1) / pl.turn);
+        dim3 grid(across, down < 32768u ? down : 32768u, (down + 32767u) / 32768u);
         if (pl.run > 0) grid = dim3((unsigned)((L.P + pl.run - 1) / pl.run), (unsigned)L.B, 1);
         if (pl.run > 0) list_pixels_kernel<DIM, true, true><<<grid, 256, 0, s>>>(w, L.g, pl);
         else list_pixels_kernel<DIM, true, false><<<grid, 256, 0, s>>>(w, L.g, pl);
@@ -597,6 +630,89 @@ int add_copies(const Launch& L, const void* workspace, int copies, float* rec, c
     const size_t blocks = (L.rec_count + 255) / 256;
     add_copies_kernel<<<(unsigned)(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, s>>>((const float2*)workspace, (float2*)rec, L.rec_count, copies, accumulate);
     return check_launch("add_copies launch");
+}
+
+// The scatter of a call whose lists are left aside (linear taps, and cubic ones in 2D): what runs calls without lists, behind a gate that is shut
+// unless they are.  The outputs are cleared.  accum: 16-byte voxels instead of vol and wvol.
+template <int DIM, bool WEIGHTS, bool DUP>
+int scatter_without_lists(Launch L, const ListLaunch& ll, bool cubic, void* workspace, size_t workspace_bytes, const float* proj, const float* weights,
+                          const float* rot, const float* shifts, float* vol, float* wvol, float4* accum, double os, double cutoff, bool accumulate, cudaStream_t s) {
+    const Gate gate{(const int*)workspace, ll.plan.crowd};
+    if (gate.crowd == 0.f) return B200PROJ_OK;
+    void* scratch = (char*)workspace + 256;
+    const size_t bytes = workspace_bytes - 256;
+    const BrickLaunch bl = scatter_plan(DIM, L.B, L.P, L.g.N, cubic, WEIGHTS, os, cutoff);
+    if (DIM == 2 && runs_in(bl, scratch, bytes)) return launch_brick_scatter<DIM, WEIGHTS, DUP>(L, bl, scratch, proj, weights, rot, shifts, vol, wvol, s, nullptr, gate);
+    const float2* p = (const float2*)proj;
+    auto zero = [&](size_t n) {
+        gated_zero_kernel<<<148 * 8, 256, 0, s>>>((float4*)scratch, (n + 15) / 16, gate);
+        return check_launch("gated_zero launch");
+    };
+    // several tiles to a block, as long as there are some ten blocks per place on the GPU
+    const int64_t most = (int64_t)L.grid.x * L.g.BP / 8192;
+    const int tiles = (int)(most < 1 ? 1 : most < (int64_t)L.grid.x ? most : L.grid.x);
+    const dim3 grid((L.grid.x + tiles - 1) / tiles, L.grid.y, L.grid.z);
+    if constexpr (WEIGHTS) {
+        if constexpr (DIM == 3) {
+            const SlabPlan apart = slab_plan(L.g.R, true);
+            if (accum == nullptr && apart.slabs > 1) {
+                backproject_slab_kernel<false, true><<<dim3((unsigned)L.g.BP, (unsigned)apart.slabs, 1), kBlockThreads, 0, s>>>(p, weights, rot, shifts, (float2*)vol, wvol, nullptr, L.g, apart.planes, 0, gate);
+                return check_launch("backproject_slab launch");
+            }
+        }
+        float4* to = accum;
+        if (to == nullptr) {
+            const size_t one = L.rec_count * sizeof(float4);
+            L.g.replicas = workspace_replicas((double)one, L.P);
+            while (L.g.replicas > 1 && (size_t)L.g.replicas * one > bytes) L.g.replicas /= 2;
+            L.g.replica_stride = (long long)L.rec_count;
+            to = (float4*)scratch;
+            if (int rc = zero((size_t)L.g.replicas * one)) return rc;
+        }
+        const SlabPlan plan = DIM == 3 ? slab_plan(L.g.R, true, true, accum == nullptr && os >= 1.5) : SlabPlan{1, L.g.R};
+        if (DIM == 3 && plan.slabs > 1)
+            backproject_slab_kernel<false, true, true><<<dim3((unsigned)L.g.BP, (unsigned)plan.slabs, 1), kBlockThreads, 0, s>>>(p, weights, rot, shifts, nullptr, nullptr, to, L.g, plan.planes, 0, gate);
+        else if (DIM == 2 && cubic)
+            gated_interleaved_kernel<2, true><<<grid, kBlockThreads, 0, s>>>(p, weights, rot, shifts, to, L.g, tiles, gate);
+        else
+            gated_interleaved_kernel<DIM, false><<<grid, kBlockThreads, 0, s>>>(p, weights, rot, shifts, to, L.g, tiles, gate);
+        if (int rc = check_launch("gated scatter launch")) return rc;
+        if (accum != nullptr) return B200PROJ_OK;
+        fold_interleaved_kernel<<<148 * 16, 256, 0, s>>>(to, (float2*)vol, wvol, L.rec_count, accumulate ? 1 : 0, L.g.replicas, L.rec_count, gate);
+        return check_launch("fold_interleaved launch");
+    } else {
+        if constexpr (DIM == 3 && DUP) {
+            const SlabPlan plan = slab_plan(L.g.R, false);
+            if (plan.slabs > 1) {
+                backproject_slab_kernel<false, false><<<dim3((unsigned)L.g.BP, (unsigned)plan.slabs, 1), kBlockThreads, 0, s>>>(p, nullptr, rot, shifts, (float2*)vol, nullptr, nullptr, L.g, plan.planes, 0, gate);
+                return check_launch("backproject_slab launch");
+            }
+        }
+        const int copies = scatter_copies(L, DIM, cubic, false, scratch, bytes);
+        if (copies > 1)
+            if (int rc = zero((size_t)copies * L.rec_count * sizeof(float2))) return rc;
+        float2* to = copies > 1 ? (float2*)scratch : (float2*)vol;
+        if (DIM == 2 && cubic) gated_scatter_kernel<2, true, DUP><<<grid, kBlockThreads, 0, s>>>(p, rot, shifts, to, L.g, tiles, gate);
+        else gated_scatter_kernel<DIM, false, DUP><<<grid, kBlockThreads, 0, s>>>(p, rot, shifts, to, L.g, tiles, gate);
+        if (int rc = check_launch("gated scatter launch")) return rc;
+        if (copies == 1) return B200PROJ_OK;
+        add_copies_kernel<<<148 * 16, 256, 0, s>>>((const float2*)scratch, (float2*)vol, L.rec_count, copies, accumulate, gate);
+        return check_launch("add_copies launch");
+    }
+}
+
+// A scatter from lists and, behind the gate, the one without.
+template <int DIM, bool WEIGHTS, bool DUP>
+int scatter_by_lists(const Launch& L, const ListLaunch& ll, bool cubic, void* workspace, size_t workspace_bytes, const float* proj, const float* weights,
+                     const float* rot, const float* shifts, float* vol, float* wvol, float4* accum, double os, double cutoff, bool accumulate, cudaStream_t s) {
+    int rc;
+    if constexpr (DIM == 3 && WEIGHTS) {
+        rc = accum != nullptr ? launch_list_scatter<3, true, true, true>(L, ll, cubic, workspace, proj, weights, rot, shifts, nullptr, nullptr, s, accum)
+                              : launch_list_scatter<3, true, true>(L, ll, cubic, workspace, proj, weights, rot, shifts, vol, wvol, s);
+    } else {
+        rc = launch_list_scatter<DIM, WEIGHTS, DUP>(L, ll, cubic, workspace, proj, weights, rot, shifts, vol, wvol, s);
+    }
+    return rc ? rc : scatter_without_lists<DIM, WEIGHTS, DUP>(L, ll, cubic, workspace, workspace_bytes, proj, weights, rot, shifts, vol, wvol, accum, os, cutoff, accumulate, s);
 }
 
 // ---- operator bodies, templated on the dimensionality and the real type (float | double) ------------------------------------
@@ -716,7 +832,8 @@ int project_back_saved(const float* grad_proj, const float* out, const float* de
     BrickLaunch bl{};
     ListLaunch ll{};
     if ((RECORDS || DIM == 2) && P > 0 && grad_rec != nullptr && workspace != nullptr) {
-        ll = list_scatter_plan(DIM, B, R, P, N, cubic, false, os, cutoff);
+        // (linear: the kernel below, which forms the pose gradients on its way, is as fast where lists are left aside for it)
+        if (cubic) ll = list_scatter_plan(DIM, B, R, P, N, cubic, 0, os, cutoff);
         ll.use = runs_in(ll, workspace, workspace_bytes);
         if (!ll.use) bl = scatter_plan(DIM, B, P, N, cubic, false, os, cutoff);
     }
@@ -730,7 +847,7 @@ int project_back_saved(const float* grad_proj, const float* out, const float* de
     const float2* d = (const float2*)derivatives;
     if (bl.use || ll.use) {
         // large scatter: brick by brick, the pose gradients in a streaming pass of their own
-        if (int rc = ll.use ? launch_list_scatter<DIM, false, false>(L, ll, cubic, workspace, grad_proj, nullptr, rot, shifts, grad_rec, nullptr, s)
+        if (int rc = ll.use ? scatter_by_lists<DIM, false, false>(L, ll, cubic, workspace, workspace_bytes, grad_proj, nullptr, rot, shifts, grad_rec, nullptr, nullptr, os, cutoff, false, s)
                             : launch_brick_scatter<DIM, false, false>(L, bl, workspace, grad_proj, nullptr, rot, shifts, grad_rec, nullptr, s)) return rc;
         if (grad_rot == nullptr && grad_shifts == nullptr) return B200PROJ_OK;
         grad_rec = nullptr;
@@ -764,7 +881,7 @@ int project_back(const Real* grad_proj, const Real* rec, int64_t B, int64_t R, c
     BrickLaunch bl{};
     ListLaunch ll{};
     if (std::is_same<Real, float>::value && P > 0 && grad_rot == nullptr && grad_shifts == nullptr && workspace != nullptr) {
-        ll = list_scatter_plan(DIM, B, R, P, N, interpolation == B200PROJ_CUBIC, false, os, cutoff);
+        ll = list_scatter_plan(DIM, B, R, P, N, interpolation == B200PROJ_CUBIC, 0, os, cutoff);
         ll.use = runs_in(ll, workspace, workspace_bytes);
         if (!ll.use) bl = scatter_plan(DIM, B, P, N, interpolation == B200PROJ_CUBIC, false, os, cutoff);
     }
@@ -774,7 +891,7 @@ int project_back(const Real* grad_proj, const Real* rec, int64_t B, int64_t R, c
                               grad_shifts, (size_t)(shifts ? B_shift : 0) * P * 2 * sizeof(Real))) return rc;
     if (P == 0) return B200PROJ_OK;
     if constexpr (std::is_same<Real, float>::value) {
-        if (ll.use) return launch_list_scatter<DIM, false, false>(L, ll, interpolation == B200PROJ_CUBIC, workspace, grad_proj, nullptr, rot, shifts, grad_rec, nullptr, s);
+        if (ll.use) return scatter_by_lists<DIM, false, false>(L, ll, interpolation == B200PROJ_CUBIC, workspace, workspace_bytes, grad_proj, nullptr, rot, shifts, grad_rec, nullptr, nullptr, os, cutoff, false, s);
         if (bl.use) return launch_brick_scatter<DIM, false, false>(L, bl, workspace, grad_proj, nullptr, rot, shifts, grad_rec, nullptr, s);
     }
     if (copies > 1)
@@ -808,13 +925,13 @@ int backproject_forw(const Real* proj, const Real* weights, int64_t B, int64_t R
     // (one v4 reduction per tap), folded into the outputs afterwards.
     const size_t ws_one = L.rec_count * sizeof(float4);
     if constexpr (std::is_same<Real, float>::value) {
-        const ListLaunch ll = P > 0 && workspace != nullptr ? list_scatter_plan(DIM, B, R, P, N, cubic, hw, os, cutoff) : ListLaunch{};
+        const ListLaunch ll = P > 0 && workspace != nullptr ? list_scatter_plan(DIM, B, R, P, N, cubic, hw ? 1 : 0, os, cutoff) : ListLaunch{};
         if (runs_in(ll, workspace, workspace_bytes)) {
             if (!accumulate) {
                 if (int rc = zero_outputs(s, data_rec, L.rec_count * sizeof(C2<Real>), weight_rec, L.rec_count * sizeof(Real))) return rc;
             }
-            return hw ? launch_list_scatter<DIM, true, true>(L, ll, cubic, workspace, proj, weights, rot, shifts, data_rec, weight_rec, s)
-                      : launch_list_scatter<DIM, false, true>(L, ll, cubic, workspace, proj, nullptr, rot, shifts, data_rec, nullptr, s);
+            return hw ? scatter_by_lists<DIM, true, true>(L, ll, cubic, workspace, workspace_bytes, proj, weights, rot, shifts, data_rec, weight_rec, nullptr, os, cutoff, accumulate != 0, s)
+                      : scatter_by_lists<DIM, false, true>(L, ll, cubic, workspace, workspace_bytes, proj, nullptr, rot, shifts, data_rec, nullptr, nullptr, os, cutoff, accumulate != 0, s);
         }
         const BrickLaunch bl = P > 0 && workspace != nullptr ? scatter_plan(DIM, B, P, N, cubic, hw, os, cutoff) : BrickLaunch{};
         if (runs_in(bl, workspace, workspace_bytes)) {
@@ -975,8 +1092,8 @@ int backproject_accumulate(const float* proj, const float* weights, int64_t B, i
     float4* acc = (float4*)accumulator;
     const bool cubic = interpolation == B200PROJ_CUBIC;
     if (workspace != nullptr && slab_count == plan.slabs) {
-        const ListLaunch ll = list_scatter_plan(3, B, R, P, N, cubic, true, os, cutoff);
-        if (runs_in(ll, workspace, workspace_bytes)) return launch_list_scatter<3, true, true, true>(L, ll, cubic, workspace, proj, weights, rot, shifts, nullptr, nullptr, s, acc);
+        const ListLaunch ll = list_scatter_plan(3, B, R, P, N, cubic, 2, os, cutoff);
+        if (runs_in(ll, workspace, workspace_bytes)) return scatter_by_lists<3, true, true>(L, ll, cubic, workspace, workspace_bytes, proj, weights, rot, shifts, nullptr, nullptr, acc, os, cutoff, true, s);
         const BrickLaunch bl = scatter_plan(3, B, P, N, cubic, true, os, cutoff);
         if (runs_in(bl, workspace, workspace_bytes)) return launch_brick_scatter<3, true, true, true>(L, bl, workspace, proj, weights, rot, shifts, nullptr, nullptr, s, acc);
     }
@@ -1128,7 +1245,7 @@ int b200proj_project_3d_to_2d_forw(const float* rec, int64_t B, int64_t R, const
 size_t b200proj_scatter_workspace_bytes(int dim, int64_t B, int64_t P, int64_t N, int interpolation, int has_weights, double oversampling, double cutoff) {
     if (dim != 2 && dim != 3) return 0;
     const BrickLaunch bl = scatter_plan(dim, B, P, N, interpolation == B200PROJ_CUBIC, has_weights != 0, oversampling, cutoff);
-    const ListLaunch ll = list_scatter_plan(dim, B, b200proj_rec_boxsize(N, oversampling), P, N, interpolation == B200PROJ_CUBIC, has_weights != 0, oversampling, cutoff);
+    const ListLaunch ll = list_scatter_plan(dim, B, b200proj_rec_boxsize(N, oversampling), P, N, interpolation == B200PROJ_CUBIC, has_weights, oversampling, cutoff);
     const size_t lists = ll.use ? ll.bytes : 0, bricks = bl.use ? bl.bytes : 0;
     return lists > bricks ? lists : bricks;
 }
@@ -1136,7 +1253,7 @@ size_t b200proj_gradient_workspace_bytes(int dim, int64_t B, int64_t R, int64_t 
                                          double oversampling, double cutoff) {
     if ((dim != 2 && dim != 3) || B < 1 || R < 2 || P < 1 || N < 2) return 0;
     if (!pose_gradients) {
-        const ListLaunch ll = list_scatter_plan(dim, B, R, P, N, interpolation == B200PROJ_CUBIC, false, oversampling, cutoff);
+        const ListLaunch ll = list_scatter_plan(dim, B, R, P, N, interpolation == B200PROJ_CUBIC, 0, oversampling, cutoff);
         const BrickLaunch bl = scatter_plan(dim, B, P, N, interpolation == B200PROJ_CUBIC, false, oversampling, cutoff);
         const size_t lists = ll.use ? ll.bytes : 0, bricks = bl.use ? bl.bytes : 0;
         if (lists > 0 || bricks > 0) return lists > bricks ? lists : bricks;

@@ -198,7 +198,8 @@ __device__ __forceinline__ void brick_list_outside(const SliceGeom& g, BrickWork
 // they write into a row of a slice then meet in L2 before the row's sectors leave it.
 template <int DIM>
 __global__ void __launch_bounds__(256)
-brick_setup_kernel(const float* __restrict__ rot, const float* __restrict__ shifts, BrickWork ws, const SliceGeom g, const BrickPlan pl, int B, int list_outside) {
+brick_setup_kernel(const float* __restrict__ rot, const float* __restrict__ shifts, BrickWork ws, const SliceGeom g, const BrickPlan pl, int B, int list_outside, Gate gate) {
+    if (gate.shut()) return;
     // block 0: the pixels outside the cutoff; then one block per cluster of bricks and batch item; then the slices
     if (blockIdx.x == 0) {
         if (list_outside) brick_list_outside(g, ws);

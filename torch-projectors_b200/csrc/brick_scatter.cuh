@@ -319,7 +319,8 @@ template <int DIM, bool WEIGHTS, bool DUP, bool INTERLEAVED>
 __global__ void __launch_bounds__(Scatter<DIM, WEIGHTS>::kThreads, Scatter<DIM, WEIGHTS>::kBlocks)
 brick_scatter_kernel(const float2* __restrict__ proj, const float* __restrict__ weights, const float* __restrict__ rot,
                      const float* __restrict__ shifts, float2* __restrict__ vol, float* __restrict__ wvol, float4* __restrict__ accum,
-                     BrickWork ws, const SliceGeom g, const BrickPlan pl) {
+                     BrickWork ws, const SliceGeom g, const BrickPlan pl, Gate gate) {
+    if (gate.shut()) return;
     using C = Scatter<DIM, WEIGHTS>;
     extern __shared__ __align__(16) unsigned char dyn[];
     typename C::Shared& sh = *reinterpret_cast<typename C::Shared*>(dyn);

@@ -18,6 +18,18 @@ namespace b200proj {
 #define PB_MIN_BLOCKS 4
 #endif
 
+// Kernels that run only when a call's pixel lists are left aside (see list_setup_kernel); header NULL: that run anyway.
+struct Gate {
+    const int* header;
+    float crowd;
+    __device__ __forceinline__ bool shut() const { return header != nullptr && !crowded(header, crowd); }
+    // header[8]: pixels that were found in the brick of a pixel of another slice; header[9]: those in its cell
+    static __device__ __forceinline__ bool crowded(const int* header, float crowd) {
+        const int near = __ldg(header + 8), same = __ldg(header + 9);
+        return same >= 32 && (float)near < crowd * (float)same;
+    }
+};
+
 struct BlockWork {
     int b, p, i, j;
     bool slice_ok, in_image;
@@ -31,9 +43,8 @@ struct BlockWork {
 constexpr int kGridYBits = 15;
 
 template <bool WIDE_PIX = false>
-__device__ __forceinline__ BlockWork block_work(const SliceGeom& g) {
+__device__ __forceinline__ BlockWork block_work(const SliceGeom& g, int x, int y, int z) {
     BlockWork w;
-    const int y = (int)blockIdx.y, z = (int)blockIdx.z;
     int b, p;
     if (g.decode == 0) {
         b = 0;
@@ -58,7 +69,7 @@ __device__ __forceinline__ BlockWork block_work(const SliceGeom& g) {
     w.b = b;
     w.p = p;
     w.slice_ok = slice_ok;
-    tile_pixel(g, (int)blockIdx.x, w.i, w.j);
+    tile_pixel(g, x, w.i, w.j);
     w.in_image = w.i < g.N && w.j < g.Nh && slice_ok;
     // WIDE_PIX: the same offset as one 64-bit expression per thread.  It costs the cubic 3D
     // forward kernel 9 registers (57 instead of 48) and that is its purpose: the kernel is bound
@@ -71,6 +82,8 @@ __device__ __forceinline__ BlockWork block_work(const SliceGeom& g) {
         w.pix = (size_t)(b * g.P + p) * (size_t)g.slice_pixels + (size_t)(w.i * g.Nh + w.j);
     return w;
 }
+template <bool WIDE_PIX = false>
+__device__ __forceinline__ BlockWork block_work(const SliceGeom& g) { return block_work<WIDE_PIX>(g, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z); }
 
 template <int DIM, typename R>
 __device__ __forceinline__ const R* pose_rot(const SliceGeom& g, const R* rot, int b, int p) {
@@ -501,30 +514,32 @@ __device__ __forceinline__ bool backproject_pixel(const SliceGeom& g, const Bloc
     return active;
 }
 
+template <int DIM, bool CUBIC, bool WEIGHTS, bool DUP, typename R>
+__device__ __forceinline__ void backproject_forw(const SliceGeom& g, const BlockWork& w, const C2<R>* __restrict__ proj, const R* __restrict__ weights,
+                                                 const R* __restrict__ rot, const R* __restrict__ shifts, C2<R>* __restrict__ data_rec,
+                                                 R* __restrict__ weight_rec) {
+    PixelT<R> px;
+    C2<R> v;
+    R wv;
+    const bool active = backproject_pixel<DIM, WEIGHTS>(g, w, proj, weights, rot, shifts, px, v, wv);
+    scatter_coop<DIM, CUBIC, WEIGHTS, DUP, false>(g, data_rec + copy_of(g, w.p) + (size_t)w.b * g.vol_elems,
+                                                   WEIGHTS ? weight_rec + (size_t)w.b * g.vol_elems : nullptr,
+                                                   nullptr, px, active, v, wv);
+}
 template <int DIM, bool CUBIC, bool WEIGHTS, typename R>
 __global__ void __launch_bounds__(kBlockThreads)
 backproject_forw_kernel(const C2<R>* __restrict__ proj, const R* __restrict__ weights,
                         const R* __restrict__ rot, const R* __restrict__ shifts,
                         C2<R>* __restrict__ data_rec, R* __restrict__ weight_rec,
                         const SliceGeom g) {
-    const BlockWork w = block_work(g);
-    PixelT<R> px;
-    C2<R> v;
-    R wv;
-    const bool active = backproject_pixel<DIM, WEIGHTS>(g, w, proj, weights, rot, shifts, px, v, wv);
-    scatter_coop<DIM, CUBIC, WEIGHTS, true, false>(g, data_rec + copy_of(g, w.p) + (size_t)w.b * g.vol_elems,
-                                                   WEIGHTS ? weight_rec + (size_t)w.b * g.vol_elems : nullptr,
-                                                   nullptr, px, active, v, wv);
+    backproject_forw<DIM, CUBIC, WEIGHTS, true>(g, block_work(g), proj, weights, rot, shifts, data_rec, weight_rec);
 }
 
 // Back-projection with weights into the interleaved accumulation volume (workspace), and
 // the pass that folds it into the caller's data / weight volumes.
 template <int DIM, bool CUBIC>
-__global__ void __launch_bounds__(kBlockThreads)
-backproject_forw_interleaved_kernel(const float2* __restrict__ proj, const float* __restrict__ weights,
-                                    const float* __restrict__ rot, const float* __restrict__ shifts,
-                                    float4* __restrict__ accum, const SliceGeom g) {
-    const BlockWork w = block_work(g);
+__device__ __forceinline__ void backproject_forw_interleaved(const SliceGeom& g, const BlockWork& w, const float2* __restrict__ proj, const float* __restrict__ weights,
+                                                             const float* __restrict__ rot, const float* __restrict__ shifts, float4* __restrict__ accum) {
     Pixel px;
     float2 v;
     float wv;
@@ -532,12 +547,20 @@ backproject_forw_interleaved_kernel(const float2* __restrict__ proj, const float
     scatter_coop<DIM, CUBIC, true, true, true>(g, nullptr, nullptr, accum + copy_of(g, w.p) + (size_t)w.b * g.vol_elems,
                                                px, active, v, wv);
 }
+template <int DIM, bool CUBIC>
+__global__ void __launch_bounds__(kBlockThreads)
+backproject_forw_interleaved_kernel(const float2* __restrict__ proj, const float* __restrict__ weights,
+                                    const float* __restrict__ rot, const float* __restrict__ shifts,
+                                    float4* __restrict__ accum, const SliceGeom g) {
+    backproject_forw_interleaved<DIM, CUBIC>(g, block_work(g), proj, weights, rot, shifts, accum);
+}
 
 // data[k] (+)= sum over copies of accum[k].xy, weight[k] (+)= sum over copies of accum[k].z
 __global__ void __launch_bounds__(256)
 fold_interleaved_kernel(const float4* __restrict__ accum, float2* __restrict__ data,
                         float* __restrict__ weight, size_t n, int accumulate, int replicas = 1,
-                        size_t replica_stride = 0) {
+                        size_t replica_stride = 0, Gate gate = {}) {
+    if (gate.shut()) return;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += stride) {
         float4 a = __ldcs(accum + k);
@@ -612,7 +635,8 @@ __global__ void __launch_bounds__(kBlockThreads)
 backproject_slab_kernel(const float2* __restrict__ proj, const float* __restrict__ weights,
                         const float* __restrict__ rot, const float* __restrict__ shifts,
                         float2* __restrict__ data_rec, float* __restrict__ weight_rec,
-                        float4* __restrict__ accum, const SliceGeom g, int slab_planes, int slab_first) {
+                        float4* __restrict__ accum, const SliceGeom g, int slab_planes, int slab_first, const Gate gate = {}) {
+    if (gate.shut()) return;
     constexpr int T = CUBIC ? 4 : 2;
     constexpr unsigned kFull = 0xffffffffu;
     constexpr float kEps = 0.05f;                    // slack of the linear estimates below
@@ -857,7 +881,8 @@ backproject_back_patches_kernel(const C2<R>* __restrict__ grad_data_rec,
 
 // out[k] (+)= sum over copies of it (scatters onto a small reconstruction, see scatter_copies)
 __global__ void __launch_bounds__(256)
-add_copies_kernel(const float2* __restrict__ copies, float2* __restrict__ out, size_t n, int count, bool accumulate) {
+add_copies_kernel(const float2* __restrict__ copies, float2* __restrict__ out, size_t n, int count, bool accumulate, Gate gate = {}) {
+    if (gate.shut()) return;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += stride) {
         float2 a = __ldcs(copies + k);

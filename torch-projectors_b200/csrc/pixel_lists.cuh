@@ -41,12 +41,15 @@ struct ListPlan {
     int pairs;              // room for their pairs
     int most;               // pixels of a work item
     int subs;               // counters of a brick (a power of two), for slices taken in turn
+    int probes;             // blocks of list_setup_kernel that look at how the pixels crowd
+    float crowd;            // the lists are left aside when that finds fewer cells
     int run;                // slices of a block of list_pixels_kernel that counts in shared memory; 0: in global memory
+    int turn;               // and of one that counts in global memory
     unsigned capacity;      // entries of the list
 };
 
 // Workspace: int header[64] {entries, work items, ticket, 0 (the brick scatters' status), slices that are not listed, 1: some pixel is
-// not finite, slices with samples out of the grid, pairs, -}, then what follows, each part on a 256-byte boundary.
+// not finite, slices with samples out of the grid, pairs, probed pixels of a brick, of a cell, -}, then what follows, each part on a 256-byte boundary.
 struct ListWork {
     int* header;
     unsigned* count;        // pixels of each brick; after list_plan_kernel: where the next entry goes
@@ -130,7 +133,85 @@ __device__ __forceinline__ float2 list_phase(const SliceGeom& g, float dot) {
 }
 __device__ __forceinline__ bool list_has_slice(const ListWork& ws, int k) { return !isnan(__ldg(&ws.poses[2 * (size_t)k].x)); }
 
-// Blocks of 256 threads: one per 16 rows and 32 columns of a slice, then one per 256 slices.  The header is zero on entry.
+// How many of a brick's cells the pixels of a call share: pixels of slices drawn at random, the brick and the cell of each, and
+// the pixels of another slice that lie in this brick (header[8]) and in this cell (header[9]).  Their ratio is the number of cells that
+// would be as crowded if all were alike: 330-570 of 512 for uniform poses, poses about one axis with free in-plane turns, and within 15
+// degrees of one view; 60 for slices of one plane (any turn), 15 for slices of one pose (oversampled twice: one sample in four
+// cells of a plane), 45-70 for a tilt series (200 not oversampled), 90 for a hundred poses, 75 when half the slices share a plane.
+__device__ __forceinline__ unsigned probe_bits(unsigned x) {            // (Wellons' "lowbias32" hash)
+    x ^= x >> 16; x *= 0x7feb352du; x ^= x >> 15; x *= 0x846ca68bu; x ^= x >> 16;
+    return x;
+}
+template <int DIM>
+__device__ __forceinline__ void list_probe(const float* __restrict__ rot, const ListWork& ws, const SliceGeom& g, const ListPlan& pl, int draw) {
+    using L = ListBrick<DIM>;
+    constexpr unsigned kFull = 0xffffffffu;
+    constexpr int kHits = DIM == 3 ? 2 : 1, kFar = 16;         // hits of a warp that are counted; reach of the search, in pixels
+    constexpr float kHalfX = 0.5f * (1 << L::kLogX), kHalfY = 0.5f * (1 << L::kLogY), kHalfZ = DIM == 3 ? 0.5f * (1 << L::kLogZ) : 0.f;
+    constexpr float kDiagonal = DIM == 3 ? 6.94f : 11.33f;      // from the centre of a brick to its corners
+    const int lane = threadIdx.x & 31, half = g.N / 2;
+    auto columns = [&](int k, float4& ra, float4& rb) {
+        const int b = k / g.P;
+        const float* rm = pose_rot<DIM>(g, rot, b, k - b * g.P);
+        ra = make_float4(__ldg(rm), __ldg(rm + DIM), DIM == 3 ? __ldg(rm + 6) : 0.f, __ldg(rm + 1));
+        rb = make_float4(__ldg(rm + DIM + 1), DIM == 3 ? __ldg(rm + 7) : 0.f, 0.f, 0.f);
+    };
+    auto brick = [&](const ListSample& s) { return make_int3(s.x >> L::kLogX, s.y >> L::kLogY, DIM == 3 ? s.z >> L::kLogZ : 0); };
+    auto listed = [&](int kr, int kc) { return kr > -half && kr <= half && kc >= 0 && kc <= half && (float)(kr * kr + kc * kc) <= g.cutoff_sq && !(kc == 0 && (kr < 0 || kr == half)); };
+    const unsigned seed = 4u * (unsigned)draw;
+    const int k = (int)__umulhi(probe_bits(seed), (unsigned)g.BP), first = k - k % g.P;
+    int other = k + 1 + (int)__umulhi(probe_bits(seed + 1u), (unsigned)(g.P - 1));
+    if (other >= first + g.P) other -= g.P;
+    // a pixel within the cutoff, of those in the rows and columns that it reaches
+    const float within = fminf((float)half, sqrtf(g.cutoff_sq));
+    const int reach = (int)within, kr = (int)__umulhi(probe_bits(seed + 2u), 2u * (unsigned)reach + 1u) - reach, kc = (int)__umulhi(probe_bits(seed + 3u), (unsigned)reach + 1u);
+    float4 ra, rb;
+    columns(k, ra, rb);
+    const ListSample s = list_sample<DIM>(g, pl, ra, rb, (unsigned)(kr + half - 1), (unsigned)kc);
+    const int3 at = brick(s);
+    bool hit = listed(kr, kc) && (unsigned)at.x < (unsigned)pl.n[0] && (unsigned)at.y < (unsigned)pl.n[1] && (DIM == 2 || (unsigned)at.z < (unsigned)pl.n[2]);
+    // where the other slice comes closest to the centre of the brick: the least squares solution for its columns
+    columns(other, ra, rb);
+    const float x = (float)(at.x * (1 << L::kLogX) + pl.lo[0]) + kHalfX, y = (float)(at.y * (1 << L::kLogY) + pl.lo[1]) + kHalfY, z = DIM == 3 ? (float)(at.z * (1 << L::kLogZ) + pl.lo[2]) + kHalfZ : 0.f;
+    const float aa = ra.x * ra.x + ra.y * ra.y + ra.z * ra.z, ab = ra.x * ra.w + ra.y * rb.x + ra.z * rb.y, bb = ra.w * ra.w + rb.x * rb.x + rb.y * rb.y;
+    const float u = ra.x * x + ra.y * y + ra.z * z, v = ra.w * x + rb.x * y + rb.y * z, det = aa * bb - ab * ab;
+    const float col = (bb * u - ab * v) / det, row = (aa * v - ab * u) / det, least = 0.5f * (aa + bb - sqrtf((aa - bb) * (aa - bb) + 4.f * ab * ab)),
+                far = ceilf(kDiagonal * rsqrtf(least) / g.os_f + 0.5f);
+    const float dx = ra.x * col + ra.w * row - x, dy = ra.y * col + rb.x * row - y, dz = ra.z * col + rb.y * row - z;
+    hit = hit && det > 0.f && least > 0.f && far <= (float)kFar && dx * dx + dy * dy + dz * dz <= kDiagonal * kDiagonal;
+    const int near_col = hit ? __float2int_rn(col / g.os_f) : 0, near_row = hit ? __float2int_rn(row / g.os_f) : 0, wide = hit ? 2 * (int)far + 1 : 0;
+    int in_brick = 0, in_cell = 0;
+    unsigned hits = __ballot_sync(kFull, hit);
+    for (int q = 0; q < kHits && hits != 0u; ++q, hits &= hits - 1u) {
+        const int from = __ffs(hits) - 1;
+        const float4 fa = make_float4(__shfl_sync(kFull, ra.x, from), __shfl_sync(kFull, ra.y, from), __shfl_sync(kFull, ra.z, from), __shfl_sync(kFull, ra.w, from));
+        const float4 fb = make_float4(__shfl_sync(kFull, rb.x, from), __shfl_sync(kFull, rb.y, from), 0.f, 0.f);
+        const int w = __shfl_sync(kFull, wide, from), c0 = __shfl_sync(kFull, near_col, from) - w / 2, r0 = __shfl_sync(kFull, near_row, from) - w / 2;
+        const int cx = __shfl_sync(kFull, s.x, from), cy = __shfl_sync(kFull, s.y, from), cz = __shfl_sync(kFull, s.z, from);
+        for (int t = lane; t < w * w; t += 32) {
+            // pixels of the half that is not stored are the conjugates of those at the opposite place, which were folded over
+            int c = c0 + t % w, r = r0 + t / w;
+            const bool opposite = c < 0;
+            if (opposite) {
+                c = -c;
+                r = -r;
+            }
+            if (!listed(r, c)) continue;
+            const ListSample o = list_sample<DIM>(g, pl, fa, fb, (unsigned)(r + half - 1), (unsigned)c);
+            if (o.folded != opposite) continue;
+            in_brick += o.x >> L::kLogX == cx >> L::kLogX && o.y >> L::kLogY == cy >> L::kLogY && (DIM == 2 || o.z >> L::kLogZ == cz >> L::kLogZ);
+            in_cell += o.x == cx && o.y == cy && o.z == cz;
+        }
+    }
+    in_brick = __reduce_add_sync(kFull, in_brick);
+    in_cell = __reduce_add_sync(kFull, in_cell);
+    if (lane == 0 && in_brick > 0) {
+        atomicAdd(ws.header + 8, in_brick);
+        if (in_cell > 0) atomicAdd(ws.header + 9, in_cell);
+    }
+}
+
+// Blocks of 256 threads: one per 16 rows and 32 columns of a slice, one per 256 slices, then pl.probes.  The header is zero on entry.
 // Pixels outside the cutoff and the mirrored half of column 0 are left out.  Slices with matrices or shifts that are not
 // finite, or so large that the arithmetic above would not hold, are not listed.
 template <int DIM>
@@ -156,6 +237,10 @@ list_setup_kernel(const float* __restrict__ rot, const float* __restrict__ shift
         return;
     }
     const int t = ((int)blockIdx.x - tiles) * 256 + (int)threadIdx.x;
+    if ((int)blockIdx.x - tiles >= (g.BP + 255) / 256) {
+        list_probe<DIM>(rot, ws, g, pl, t);
+        return;
+    }
     if (t >= g.BP) return;
     const int b = t / g.P, p = t - b * g.P;
     const float* rm = pose_rot<DIM>(g, rot, b, p);
@@ -187,7 +272,7 @@ constexpr int kListBricks = 4096;           // bricks of a batch item that a blo
 //   half written.  (Passes in us with 1 / 4 / 8 / 16 counters: 2,501 slices of 90 x 46, 3,000 bricks met, 49 + 55 / 26 + 36 / 26 + 36 / 26 + 36;
 //   50,000 of 128 x 65, 8,600 bricks, 1,070 + 1,500 / 886 + 1,444 / 892 + 1,545 / 892 + 1,670; 4,096 of 256 x 129, 68,000 bricks, 280 + 472 /
 //   261 + 582 / 262 + 648 / 261 + 725; 10,000 of 128 x 65 in one plane 1,486 + 1,524 / 525 + 563 / 429 + 465 / 215 + 251.)
-//   Grid: x = kListPairs pairs of a slice, (y, z) = the slice.
+//   Grid: x = kListPairs pairs of a slice, y = pl.turn slices, one after the other.
 //   else: bricks are few and many slices meet in each (2D: all slices in every tile), so atomics would queue up at a few
 //   addresses.  A block counts pl.run slices of a batch item in shared memory, and keeps its counts for the second pass.
 //   Grid: x = runs of a batch item, y = batch item.
@@ -199,6 +284,7 @@ list_pixels_kernel(ListWork ws, const SliceGeom g, const ListPlan pl) {
     constexpr unsigned kFull = 0xffffffffu;
     const int lane = threadIdx.x & 31, tid = threadIdx.x;
     const unsigned below = (1u << lane) - 1u;
+    if (Gate::crowded(ws.header, pl.crowd)) return;
     const bool all_fit = __ldg(ws.header + 6) == 0;
     int slice, last, begin = 0, end = __ldg(ws.header + 7), b = 0;
     unsigned* row = nullptr;
@@ -219,15 +305,14 @@ list_pixels_kernel(ListWork ws, const SliceGeom g, const ListPlan pl) {
         }
         __syncthreads();
     } else {
-        slice = (int)blockIdx.y + (int)blockIdx.z * 32768;
-        if (slice >= pl.slices) return;
-        last = slice + 1;
+        slice = ((int)blockIdx.y + (int)blockIdx.z * 32768) * pl.turn;
+        last = min(pl.slices, slice + pl.turn);
         begin = (int)blockIdx.x * kListPairs;
         end = min(end, begin + kListPairs);
-        b = (pl.first + slice) / g.P;
     }
     for (; slice < last; ++slice) {
         const int k = pl.first + slice;
+        if (!SHARED) b = k / g.P;
         const float4 ra = __ldg(ws.poses + 2 * (size_t)k), rb = __ldg(ws.poses + 2 * (size_t)k + 1);
         if (isnan(ra.x)) continue;
         for (int base = begin; base < end; base += kListPairs) {
@@ -292,6 +377,7 @@ list_pixels_kernel(ListWork ws, const SliceGeom g, const ListPlan pl) {
 template <int DIM>
 __global__ void __launch_bounds__(256)
 list_plan_kernel(ListWork ws, const ListPlan pl, int B) {
+    if (Gate::crowded(ws.header, pl.crowd)) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned t = blockIdx.x * 256u + threadIdx.x, place = t & ((1u << (DIM * pl.bits)) - 1u);
     const int b = (int)(t >> (DIM * pl.bits));
