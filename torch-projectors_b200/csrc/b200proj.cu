@@ -461,7 +461,8 @@ ListLaunch list_layout(int dim, int64_t B, int64_t R, int64_t P, int64_t N, doub
     L.item_bytes = (items * sizeof(int4) + up) & ~up;
     L.pose_bytes = ((size_t)L.slices * 2 * sizeof(float4) + up) & ~up;
     L.inside_bytes = ((size_t)pairs * sizeof(unsigned) + up) & ~up;
-    if (p.item_bricks <= kListBricks && B <= 65535) {
+    static const int shared = [] { const char* e = getenv("B200PROJ_LIST_SHARED"); return e ? atoi(e) : kListBricks; }();   // for tests
+    if (p.item_bricks <= (shared < kListBricks ? shared : kListBricks) && B <= 65535) {
         // few bricks: counted in shared memory, a run of slices per block (some 16 blocks per SM)
         int64_t run = (p.slices + 148 * 16 - 1) / (148 * 16);
         p.run = (int)(run < 1 ? 1 : run);
@@ -474,7 +475,12 @@ ListLaunch list_layout(int dim, int64_t B, int64_t R, int64_t P, int64_t N, doub
     p.turn = blocks_of < 16384 ? 1 : 4;
     // counters of a brick (see list_pixels_kernel): half of the bricks of the grid meet slices
     for (p.subs = 1; p.run == 0 && p.subs < 8 && 2 * p.subs * bricks <= 80000;) p.subs *= 2;
-    L.count_bytes = ((size_t)bricks * (size_t)p.subs * sizeof(unsigned) + up) & ~up;
+    // their places: an odd factor near the golden ratio of the power of two of groups sends neighbours far apart
+    unsigned groups = 1;
+    while (8ll * groups < bricks) groups *= 2;
+    p.groups = groups - 1;
+    p.spread = (unsigned)(0.6180339887 * (double)groups) | 1u;
+    L.count_bytes = ((size_t)groups * 8 * (size_t)p.subs * sizeof(unsigned) + up) & ~up;
     L.bytes = 256 + L.count_bytes + L.item_bytes + L.pose_bytes + L.inside_bytes + L.block_bytes + (size_t)entries * sizeof(unsigned);
     L.forced = force == 1;
     L.use = true;

@@ -41,6 +41,7 @@ struct ListPlan {
     int pairs;              // room for their pairs
     int most;               // pixels of a work item
     int subs;               // counters of a brick (a power of two), for slices taken in turn
+    unsigned spread, groups;    // of the counters, see list_counter; groups of 8 less one
     int probes;             // blocks of list_setup_kernel that look at how the pixels crowd
     float crowd;            // the lists are left aside when that finds fewer cells
     int run;                // slices of a block of list_pixels_kernel that counts in shared memory; 0: in global memory
@@ -52,7 +53,7 @@ struct ListPlan {
 // not finite, slices with samples out of the grid, pairs, probed pixels of a brick, of a cell, -}, then what follows, each part on a 256-byte boundary.
 struct ListWork {
     int* header;
-    unsigned* count;        // pixels of each brick; after list_plan_kernel: where the next entry goes
+    unsigned* count;        // pixels of each brick, at list_counter; after list_plan_kernel: where the next entry goes
     int4* items;            // {brick, first entry, entries, -}
     float4* poses;          // per slice of the call: {m00, m10, m20, m01}, {m11, m21, shift}; NaN: the slice is not listed
     unsigned* inside;       // pairs of neighbours in a row: what an entry says of the first pixel, (row frequency + N / 2 - 1) << bits_j
@@ -259,6 +260,12 @@ list_setup_kernel(const float* __restrict__ rot, const float* __restrict__ shift
     ws.poses[2 * (size_t)t + 1] = rb;
 }
 
+// Where the counter of a brick lies: groups of eight bricks (a sector of L2) are spread over the lines.  One after the other, the
+// counters of a plane's bricks share a few dozen lines, where atomics queue up.
+__device__ __forceinline__ unsigned list_counter(const ListPlan& pl, int brick) {
+    return ((((unsigned)brick >> 3) * pl.spread) & pl.groups) << 3 | ((unsigned)brick & 7u);
+}
+
 constexpr int kListRun = 2;                 // pairs of pixels of a thread at a time
 constexpr int kListPairs = 256 * kListRun;  // of a block
 constexpr int kListBricks = 4096;           // bricks of a batch item that a block can count in shared memory
@@ -269,9 +276,10 @@ constexpr int kListBricks = 4096;           // bricks of a batch item that a blo
 // 64, a pass took 3.5 ps per pixel.)
 //   pl.run == 0: counts in global memory, pl.subs for each brick, which slices use in turn: atomics at the bricks that many slices meet
 //   in would queue up.  But each is a place where the second pass writes, and beyond some 40,000 such places sectors leave L2
-//   half written.  (Passes in us with 1 / 4 / 8 / 16 counters: 2,501 slices of 90 x 46, 3,000 bricks met, 49 + 55 / 26 + 36 / 26 + 36 / 26 + 36;
-//   50,000 of 128 x 65, 8,600 bricks, 1,070 + 1,500 / 886 + 1,444 / 892 + 1,545 / 892 + 1,670; 4,096 of 256 x 129, 68,000 bricks, 280 + 472 /
-//   261 + 582 / 262 + 648 / 261 + 725; 10,000 of 128 x 65 in one plane 1,486 + 1,524 / 525 + 563 / 429 + 465 / 215 + 251.)
+//   half written.  (Passes in us with 1 / 4 / 8 / 16 counters, all one after the other: 2,501 slices of 90 x 46, 3,000 bricks met, 49 + 55 / 26 + 36 /
+//   26 + 36 / 26 + 36; 50,000 of 128 x 65, 8,600 bricks, 1,070 + 1,500 / 886 + 1,444 / 892 + 1,545 / 892 + 1,670; 4,096 of 256 x 129, 68,000 bricks,
+//   280 + 472 / 261 + 582 / 262 + 648 / 261 + 725.)  In groups spread over the lines (list_counter), four of them: 10,000 slices of 128 x 65 in one
+//   plane 812 + 852 -> 161 + 255, within 15 degrees of one view 324 + 391 -> 162 + 237, of uniform poses 173 + 272 -> 165 + 251.
 //   Grid: x = kListPairs pairs of a slice, y = pl.turn slices, one after the other.
 //   else: bricks are few and many slices meet in each (2D: all slices in every tile), so atomics would queue up at a few
 //   addresses.  A block counts pl.run slices of a batch item in shared memory, and keeps its counts for the second pass.
@@ -299,7 +307,7 @@ list_pixels_kernel(ListWork ws, const SliceGeom g, const ListPlan pl) {
             unsigned n = 0u;
             if (!COUNT) {
                 n = row[t];
-                if (n != 0u) n = atomicAdd(ws.count + b * pl.item_bricks + t, n);
+                if (n != 0u) n = atomicAdd(ws.count + list_counter(pl, b * pl.item_bricks + t), n);
             }
             here[t] = n;
         }
@@ -335,15 +343,17 @@ list_pixels_kernel(ListWork ws, const SliceGeom g, const ListPlan pl) {
                 own[q] = __ballot_sync(kFull, to_own);
                 next[q] = __ballot_sync(kFull, to_next) << 1;       // by the lane whose brick it is
                 at[q] = at2[q] = 0u;
-                unsigned* counts = SHARED ? here : ws.count + (size_t)(slice & (pl.subs - 1)) * (size_t)pl.bricks;
+                unsigned* counts = SHARED ? here : ws.count + (size_t)(slice & (pl.subs - 1)) * (size_t)(8u * (pl.groups + 1u));
                 if (brick[q] >= 0 && (same[q] & below) == 0u) {
                     const unsigned n = __popc(same[q]) + __popc(same[q] & own[q]) + __popc(same[q] & next[q]);
-                    if (COUNT) atomicAdd(counts + brick[q], n);
-                    else at[q] = atomicAdd(counts + brick[q], n);
+                    unsigned* c = counts + (SHARED ? (unsigned)brick[q] : list_counter(pl, brick[q]));
+                    if (COUNT) atomicAdd(c, n);
+                    else at[q] = atomicAdd(c, n);
                 }
                 if (brick2[q] >= 0 && !to_own && !to_next) {
-                    if (COUNT) atomicAdd(counts + brick2[q], 1u);
-                    else at2[q] = atomicAdd(counts + brick2[q], 1u);
+                    unsigned* c = counts + (SHARED ? (unsigned)brick2[q] : list_counter(pl, brick2[q]));
+                    if (COUNT) atomicAdd(c, 1u);
+                    else at2[q] = atomicAdd(c, 1u);
                 }
             }
             if (COUNT) continue;
@@ -367,7 +377,7 @@ list_pixels_kernel(ListWork ws, const SliceGeom g, const ListPlan pl) {
         for (int t = tid; t < pl.item_bricks; t += 256) {
             const unsigned n = here[t];
             row[t] = n;
-            if (n != 0u) atomicAdd(ws.count + b * pl.item_bricks + t, n);
+            if (n != 0u) atomicAdd(ws.count + list_counter(pl, b * pl.item_bricks + t), n);
         }
     }
 }
@@ -389,9 +399,10 @@ list_plan_kernel(ListWork ws, const ListPlan pl, int B) {
     }
     const bool here = b < B && x < pl.n[0] && y < pl.n[1] && z < pl.n[2];
     const int brick = ((b * pl.n[2] + z) * pl.n[1] + y) * pl.n[0] + x;
+    const unsigned counter = list_counter(pl, brick);
     int n = 0;
     if (here)
-        for (int k = 0; k < pl.subs; ++k) n += (int)ws.count[(size_t)k * (size_t)pl.bricks + brick];
+        for (int k = 0; k < pl.subs; ++k) n += (int)ws.count[(size_t)k * (size_t)(8u * (pl.groups + 1u)) + counter];
     const int parts = (n + pl.most - 1) / pl.most;
     int n_upto = n, parts_upto = parts;
 #pragma unroll
@@ -419,7 +430,7 @@ list_plan_kernel(ListWork ws, const ListPlan pl, int B) {
     if (n > 0) {
         int at = first;
         for (int k = 0; k < pl.subs; ++k) {
-            unsigned& c = ws.count[(size_t)k * (size_t)pl.bricks + brick];
+            unsigned& c = ws.count[(size_t)k * (size_t)(8u * (pl.groups + 1u)) + counter];
             const int m = (int)c;
             c = (unsigned)at;
             at += m;
