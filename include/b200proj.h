@@ -106,17 +106,24 @@ size_t b200proj_project_workspace_bytes(int dim, int64_t B, int64_t P, int64_t N
  * grad_rec, b200proj_backproject_2d_to_3d_accumulate_ws, b200proj_backproject_{2d,2d_to_3d}_forw; 0: no gain, for
  * the last of them see there for what else a workspace is good for).  The largest calls first sort their pixels by brick,
  * in lists of 4 bytes per pixel inside the cutoff (at most 4 GB: more pixels take several passes), and run without any
- * wait; a workspace that has no room for the lists is used as if they did not exist.  In cubic calls below those sizes warps
+ * wait; a workspace that has no room for the lists is used as if they did not exist.  has_weights: 2 for
+ * b200proj_backproject_2d_to_3d_accumulate_ws.  _within: the largest workspace of at most `most` bytes that the call has a
+ * use for, for callers that could not get a larger one.  In cubic calls below those sizes warps
  * hand pixels to one another and wait in doing so, for no longer than some seconds: should a wait ever run out, the parts of
  * the result that lack sums are NaN and the fourth int of the workspace is 1 (else 0) when the call's work has run. */
 size_t b200proj_scatter_workspace_bytes(int dim, int64_t B, int64_t P, int64_t N, int interpolation, int has_weights,
                                         double oversampling, double fourier_radius_cutoff);
+size_t b200proj_scatter_workspace_bytes_within(int dim, int64_t B, int64_t P, int64_t N, int interpolation, int has_weights,
+                                               double oversampling, double fourier_radius_cutoff, size_t most);
 /* Workspace of the backward passes of the projection (b200proj_project_{2d,3d_to_2d}_back_ws with grad_rec,
  * b200proj_project_2d_back_saved_ws, b200proj_project_3d_to_2d_back_records): the larger calls above, and copies
  * of a small reconstruction over which the scatter of many slices is spread (reductions that pile up on few
- * sectors run at half the rate or less).  pose_gradients != 0: of a _back_ws call that also computes grad_rot or grad_shifts. */
+ * sectors run at half the rate or less).  pose_gradients: 1 of a _back_ws call that also computes grad_rot or grad_shifts, 2 of
+ * the calls from saved derivatives (0 will do as well, but may be more than they use). */
 size_t b200proj_gradient_workspace_bytes(int dim, int64_t B, int64_t R, int64_t P, int64_t N, int interpolation,
                                          int pose_gradients, double oversampling, double fourier_radius_cutoff);
+size_t b200proj_gradient_workspace_bytes_within(int dim, int64_t B, int64_t R, int64_t P, int64_t N, int interpolation,
+                                                int pose_gradients, double oversampling, double fourier_radius_cutoff, size_t most);
 int b200proj_project_2d_forw_ws(const float* rec, int64_t B, int64_t R,
                                 const float* rot, int64_t B_rot,
                                 const float* shifts, int64_t B_shift,

@@ -100,3 +100,46 @@ def test_a_wait_that_gives_up_shows_in_the_result():
     r = subprocess.run([sys.executable, "-c", f"import sys; sys.path[:0] = [{str(ROOT / 'tests')!r}, {str(ROOT / 'torch-projectors_b200')!r}, {str(ROOT)!r}]; import test_gpu_scratch as t; t.check_waits()"],
                        env=env, cwd=ROOT, capture_output=True, text=True, timeout=600)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]
+
+
+def check_little_memory():
+    """In a fresh process whose allocator may take 60 MB more: cubic scatters whose lists (77 MB) have no room run brick by brick."""
+    import ctypes as C
+    import torch_projectors_b200 as tp
+    lib, P, N = tp._abi.load(), 12000, 64
+    gen = torch.Generator("cuda").manual_seed(0)
+    proj = torch.randn(1, P, N, N // 2 + 1, dtype=torch.complex64, generator=gen, device="cuda")
+    w, rot = torch.rand(proj.shape, generator=gen, device="cuda"), torch.linalg.qr(torch.randn(1, P, 3, 3, generator=gen, device="cuda"))[0].contiguous()
+    rec = torch.zeros(1, 2 * N, 2 * N, N + 1, dtype=torch.complex64, device="cuda")
+    acc = tp.new_backprojection_accumulator(1, 2 * N, "cuda")
+    kw = dict(interpolation="cubic", oversampling=2.0)
+    none = C.c_size_t(-1).value
+    calls = {"weighted": lambda: tp.backproject_2d_to_3d_forw(proj, rot, w, **kw), "plain": lambda: tp.backproject_2d_to_3d_forw(proj, rot, None, **kw)[0],
+             "gradient": lambda: tp.project_3d_to_2d_back(proj, rec, rot, **kw),
+             "accumulator": lambda: tp.backproject_2d_to_3d_accumulate_interleaved_(acc.zero_(), proj, rot, w, **kw) or acc}
+    want = {k: f() for k, f in calls.items()}
+    want["accumulator"] = acc.clone()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (60 << 20)) / total)
+    for k, f in calls.items():
+        mode = {"weighted": 1, "plain": 0, "gradient": 0, "accumulator": 2}[k]
+        sizes = [lib.b200proj_scatter_workspace_bytes_within(3, 1, P, N, tp._abi.CUBIC, mode, 2.0, N / 2.0, most) for most in (none, 60 << 20)]
+        assert sizes[0] > 77e6 > 20e6 > sizes[1] > 0, sizes
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        got = f()
+        torch.cuda.synchronize()
+        outputs = torch.cuda.memory_allocated() - before
+        scratch = torch.cuda.max_memory_allocated() - before - outputs
+        assert scratch >= sizes[1], (k, scratch, sizes)
+        for a, b in zip(got if isinstance(got, tuple) else (got,), want[k] if isinstance(want[k], tuple) else (want[k],)):
+            assert rel_err(a, b) <= TOL_ATOMIC, (k, rel_err(a, b))
+        del got
+
+
+def test_scatters_without_room_for_lists_take_the_next_smaller_scratch():
+    r = subprocess.run([sys.executable, "-c", f"import sys; sys.path[:0] = [{str(ROOT / 'tests')!r}, {str(ROOT / 'torch-projectors_b200')!r}, {str(ROOT)!r}]; import test_gpu_scratch as t; t.check_little_memory()"],
+                       cwd=ROOT, capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]

@@ -707,6 +707,12 @@ int scatter_without_lists(Launch L, const ListLaunch& ll, bool cubic, void* work
     }
 }
 
+// Of the sizes of scratch that a call has a use for, the larger one that is at most `most` bytes.
+size_t largest_within(size_t most, size_t a, size_t b) {
+    if (a > most) a = 0;
+    if (b > most) b = 0;
+    return a > b ? a : b;
+}
 // A scatter from lists and, behind the gate, the one without.
 template <int DIM, bool WEIGHTS, bool DUP>
 int scatter_by_lists(const Launch& L, const ListLaunch& ll, bool cubic, void* workspace, size_t workspace_bytes, const float* proj, const float* weights,
@@ -1248,25 +1254,31 @@ int b200proj_project_3d_to_2d_forw(const float* rec, int64_t B, int64_t R, const
     return project_forw<3>(rec, B, R, rot, B_rot, shifts, B_shift, P, N, interpolation, oversampling, cutoff, out, pose_order, stream);
 }
 
-size_t b200proj_scatter_workspace_bytes(int dim, int64_t B, int64_t P, int64_t N, int interpolation, int has_weights, double oversampling, double cutoff) {
+size_t b200proj_scatter_workspace_bytes_within(int dim, int64_t B, int64_t P, int64_t N, int interpolation, int has_weights, double oversampling, double cutoff, size_t most) {
     if (dim != 2 && dim != 3) return 0;
     const BrickLaunch bl = scatter_plan(dim, B, P, N, interpolation == B200PROJ_CUBIC, has_weights != 0, oversampling, cutoff);
     const ListLaunch ll = list_scatter_plan(dim, B, b200proj_rec_boxsize(N, oversampling), P, N, interpolation == B200PROJ_CUBIC, has_weights, oversampling, cutoff);
-    const size_t lists = ll.use ? ll.bytes : 0, bricks = bl.use ? bl.bytes : 0;
-    return lists > bricks ? lists : bricks;
+    return largest_within(most, ll.use ? ll.bytes : 0, bl.use ? bl.bytes : 0);
+}
+size_t b200proj_scatter_workspace_bytes(int dim, int64_t B, int64_t P, int64_t N, int interpolation, int has_weights, double oversampling, double cutoff) {
+    return b200proj_scatter_workspace_bytes_within(dim, B, P, N, interpolation, has_weights, oversampling, cutoff, SIZE_MAX);
+}
+size_t b200proj_gradient_workspace_bytes_within(int dim, int64_t B, int64_t R, int64_t P, int64_t N, int interpolation, int pose_gradients,
+                                                double oversampling, double cutoff, size_t most) {
+    if ((dim != 2 && dim != 3) || B < 1 || R < 2 || P < 1 || N < 2) return 0;
+    const bool cubic = interpolation == B200PROJ_CUBIC;
+    if (pose_gradients == 0 || (pose_gradients == 2 && cubic)) {
+        const ListLaunch ll = list_scatter_plan(dim, B, R, P, N, cubic, 0, oversampling, cutoff);
+        const BrickLaunch bl = scatter_plan(dim, B, P, N, cubic, false, oversampling, cutoff);
+        if (const size_t bytes = largest_within(most, ll.use ? ll.bytes : 0, bl.use ? bl.bytes : 0)) return bytes;
+    }
+    const double one = (double)B * (dim == 3 ? R : 1) * R * (R / 2 + 1) * (double)sizeof(float2);
+    const int copies = copies_wanted(dim, one, B, P, N, cubic, pose_gradients == 1);
+    return copies > 1 ? largest_within(most, (size_t)one * (size_t)copies, 0) : 0;
 }
 size_t b200proj_gradient_workspace_bytes(int dim, int64_t B, int64_t R, int64_t P, int64_t N, int interpolation, int pose_gradients,
                                          double oversampling, double cutoff) {
-    if ((dim != 2 && dim != 3) || B < 1 || R < 2 || P < 1 || N < 2) return 0;
-    if (!pose_gradients) {
-        const ListLaunch ll = list_scatter_plan(dim, B, R, P, N, interpolation == B200PROJ_CUBIC, 0, oversampling, cutoff);
-        const BrickLaunch bl = scatter_plan(dim, B, P, N, interpolation == B200PROJ_CUBIC, false, oversampling, cutoff);
-        const size_t lists = ll.use ? ll.bytes : 0, bricks = bl.use ? bl.bytes : 0;
-        if (lists > 0 || bricks > 0) return lists > bricks ? lists : bricks;
-    }
-    const double one = (double)B * (dim == 3 ? R : 1) * R * (R / 2 + 1) * (double)sizeof(float2);
-    const int copies = copies_wanted(dim, one, B, P, N, interpolation == B200PROJ_CUBIC, pose_gradients != 0);
-    return copies > 1 ? (size_t)one * (size_t)copies : 0;
+    return b200proj_gradient_workspace_bytes_within(dim, B, R, P, N, interpolation, pose_gradients, oversampling, cutoff, SIZE_MAX);
 }
 size_t b200proj_project_workspace_bytes(int dim, int64_t B, int64_t P, int64_t N, int interpolation, int records, double oversampling, double cutoff) {
     if (dim != 2 && dim != 3) return 0;

@@ -160,25 +160,29 @@ Tensor project_workspace(int dim, const Tensor& rec, int64_t P, int64_t N, int i
     const size_t bytes = b200proj_project_workspace_bytes(dim, rec.size(0), P, N, interp, records ? 1 : 0, oversampling, cutoff);
     return bytes ? at::empty({(int64_t)bytes}, rec.options().dtype(at::kByte)) : Tensor();
 }
-// Scratch that a call can do without: undefined when none is wanted, or when the device has no room for it (pixel lists take 4
-// bytes per pixel, up to 4 GB).
-Tensor scratch(size_t bytes, const Tensor& like) {
-    if (bytes == 0) return Tensor();
-    try {
-        return at::empty({(int64_t)bytes}, like.options().dtype(at::kByte));
-    } catch (const c10::OutOfMemoryError&) {
-        return Tensor();
+// Scratch that a call can do without: the largest that it has a use for (bytes(most): of at most `most` bytes) and the device has
+// room for (pixel lists take 4 bytes per pixel, up to 4 GB; the kernels below them a few MB), undefined when there is none.
+template <typename Bytes>
+Tensor scratch(const Tensor& like, Bytes bytes) {
+    size_t most = SIZE_MAX;
+    while (const size_t n = bytes(most)) {
+        try {
+            return at::empty({(int64_t)n}, like.options().dtype(at::kByte));
+        } catch (const c10::OutOfMemoryError&) {
+            most = n - 1;
+        }
     }
+    return Tensor();
 }
 // The same for the scatters.
 Tensor scatter_workspace(int dim, const Tensor& like, int64_t B, int64_t P, int64_t N, int interp, bool weights, double oversampling, double cutoff) {
     if (is_f64(like)) return Tensor();
-    return scratch(b200proj_scatter_workspace_bytes(dim, B, P, N, interp, weights ? 1 : 0, oversampling, cutoff), like);
+    return scratch(like, [&](size_t most) { return b200proj_scatter_workspace_bytes_within(dim, B, P, N, interp, weights ? 1 : 0, oversampling, cutoff, most); });
 }
-// The same for the backward passes of the projection.
-Tensor gradient_workspace(int dim, const Tensor& like, int64_t B, int64_t R, int64_t P, int64_t N, int interp, bool pose_gradients, double oversampling, double cutoff) {
+// The same for the backward passes of the projection.  pose_gradients: as in the C interface.
+Tensor gradient_workspace(int dim, const Tensor& like, int64_t B, int64_t R, int64_t P, int64_t N, int interp, int pose_gradients, double oversampling, double cutoff) {
     if (is_f64(like)) return Tensor();
-    return scratch(b200proj_gradient_workspace_bytes(dim, B, R, P, N, interp, pose_gradients ? 1 : 0, oversampling, cutoff), like);
+    return scratch(like, [&](size_t most) { return b200proj_gradient_workspace_bytes_within(dim, B, R, P, N, interp, pose_gradients, oversampling, cutoff, most); });
 }
 inline void* ws_ptr(const Tensor& ws) { return ws.defined() ? ws.data_ptr() : nullptr; }
 inline size_t ws_size(const Tensor& ws) { return ws.defined() ? (size_t)ws.numel() : 0; }
@@ -248,8 +252,9 @@ std::tuple<Tensor, Tensor, Tensor> project_back(int dim, const Tensor& grad_proj
     } else {
         void* s = current_stream(rec);
         const double cut = cutoff_of(cutoff, N);
-        const Tensor ws = gradient_workspace(dim, rec, B, R, p.P, N, interp, need_rot || need_shift, oversampling, cut);
-        Tensor order = resolve_order(dim, rec, B, p, pose_order, !ws.defined());
+        const Tensor ws = gradient_workspace(dim, rec, B, R, p.P, N, interp, need_rot || need_shift ? 1 : 0, oversampling, cut);
+        // (linear: for the scatter that runs when the lists are left aside)
+        Tensor order = resolve_order(dim, rec, B, p, pose_order, !ws.defined() || interp == B200PROJ_LINEAR);
         int rc;
         if (is_f64(rec)) {
             rc = dim == 2 ? b200proj_project_2d_back_f64(cptr<double>(gp), cptr<double>(rec), B, R, cptr<double>(p.rot), p.B_rot, cptr<double>(p.shifts), p.B_shift, p.P, N, interp, oversampling, cut, mptr<double>(grad_rec), mptr<double>(grad_rot), mptr<double>(grad_sh), s)
@@ -360,7 +365,7 @@ std::tuple<Tensor, Tensor, Tensor> project_back_saved(int dim, const Tensor& gra
         if (need_rec_grad) grad_rec.zero_();
     } else {
         const double cut = cutoff_of(cutoff, N);
-        const Tensor ws = need_rec_grad ? gradient_workspace(dim, gp, B, R, p.P, N, interp, false, oversampling, cut) : Tensor();
+        const Tensor ws = need_rec_grad ? gradient_workspace(dim, gp, B, R, p.P, N, interp, 2, oversampling, cut) : Tensor();
         // (without the volume's gradient the pose gradients are a streaming pass)
         Tensor order = resolve_order(dim, reconstruction, B, p, pose_order, need_rec_grad && !ws.defined());
         const int rc = dim == 2

@@ -67,6 +67,7 @@ EXPORTS = list(SIGNATURES) + ["b200proj_version", "b200proj_last_error", "b200pr
                                 "b200proj_backproject_workspace_bytes", "b200proj_accumulator_bytes",
                                 "b200proj_source_stamp", "b200proj_accumulator_slab_plan", "b200proj_scatter_workspace_bytes",
                                 "b200proj_project_workspace_bytes", "b200proj_gradient_workspace_bytes",
+                                "b200proj_scatter_workspace_bytes_within", "b200proj_gradient_workspace_bytes_within",
                                 "b200proj_accumulator_slab_voxels", "b200proj_debug_index", "b200proj_cutoff_pack_index"]
 
 _lib: Optional[C.CDLL] = None
@@ -117,6 +118,10 @@ def load() -> C.CDLL:
     lib.b200proj_project_workspace_bytes.argtypes = [_int, _i64, _i64, _i64, _int, _int, _dbl, _dbl]
     lib.b200proj_gradient_workspace_bytes.restype = C.c_size_t
     lib.b200proj_gradient_workspace_bytes.argtypes = [_int, _i64, _i64, _i64, _i64, _int, _int, _dbl, _dbl]
+    lib.b200proj_scatter_workspace_bytes_within.restype = C.c_size_t
+    lib.b200proj_scatter_workspace_bytes_within.argtypes = lib.b200proj_scatter_workspace_bytes.argtypes + [C.c_size_t]
+    lib.b200proj_gradient_workspace_bytes_within.restype = C.c_size_t
+    lib.b200proj_gradient_workspace_bytes_within.argtypes = lib.b200proj_gradient_workspace_bytes.argtypes + [C.c_size_t]
     lib.b200proj_backproject_workspace_bytes.restype = C.c_size_t
     lib.b200proj_backproject_workspace_bytes.argtypes = [_int, _i64, _i64, _i64, _i64, _int, _int]
     lib.b200proj_accumulator_bytes.restype = C.c_size_t
@@ -141,6 +146,20 @@ def rec_boxsize(N: int, oversampling: float) -> int:
 
 def backproject_workspace_bytes(dim: int, B: int, R: int, P: int, N: int, interp: int, has_weights: bool) -> int:
     return int(load().b200proj_backproject_workspace_bytes(dim, B, R, P, N, interp, int(has_weights)))
+
+
+def scatter_workspace(dim: int, B: int, P: int, N: int, interp: int, weights: int, oversampling: float, cutoff: float, device):
+    """The largest scratch that a scatter has a use for and the device has room for (uint8 tensor from torch's caching
+    allocator), or None.  weights: 0, 1, or 2 for the accumulator's 16-byte voxels."""
+    most = C.c_size_t(-1).value
+    while True:
+        n = int(load().b200proj_scatter_workspace_bytes_within(dim, B, P, N, interp, weights, float(oversampling), float(cutoff), most))
+        if n == 0:
+            return None
+        try:
+            return torch.empty(n, dtype=torch.uint8, device=device)
+        except torch.cuda.OutOfMemoryError:
+            most = n - 1
 
 
 def project_workspace_bytes(dim: int, B: int, P: int, N: int, interp: int, records: bool, oversampling: float, cutoff: float) -> int:
@@ -265,16 +284,11 @@ def backproject_accumulate(proj, weights, rot, shifts, interp, oversampling, cut
     of accumulator_bytes(B, R) bytes); see b200proj_backproject_2d_to_3d_accumulate."""
     B, P, N = proj.shape[0], proj.shape[1], proj.shape[2]
     geom = _geom(B, R, rot, shifts, P, N, interp, oversampling, cutoff)
-    # large chunks are sorted by brick first, in scratch that they can do without
-    n = int(load().b200proj_scatter_workspace_bytes(3, B, P, N, interp, 1, float(oversampling), float(cutoff)))
-    if n:
-        try:
-            workspace = torch.empty(n, dtype=torch.uint8, device=proj.device)
-        except torch.cuda.OutOfMemoryError:
-            workspace = None
-        if workspace is not None:
-            _call("b200proj_backproject_2d_to_3d_accumulate_ws", proj, _p(proj), _p(weights), *geom, _p(accumulator), _p(workspace), n)
-            return
+    # large chunks run from pixel lists or brick by brick, in scratch that they can do without
+    workspace = scatter_workspace(3, B, P, N, interp, 2, oversampling, cutoff, proj.device)
+    if workspace is not None:
+        _call("b200proj_backproject_2d_to_3d_accumulate_ws", proj, _p(proj), _p(weights), *geom, _p(accumulator), _p(workspace), workspace.numel())
+        return
     _call("b200proj_backproject_2d_to_3d_accumulate", proj, _p(proj), _p(weights), *geom, _p(accumulator))
 
 

@@ -99,14 +99,16 @@ def _check_pose_inputs(dim: int, what: str, B: int, rotations, shifts, like: tor
     return P, rotations.contiguous(), shifts
 
 
-def _backproject_workspace(dim, B, R, P, N, interp, weights, device):
-    """Scratch for the interleaved accumulation path of the back-projection kernels (from
-    torch's caching allocator, so nothing is freed behind the stream); None when the
-    library says a workspace would not help."""
-    if weights is not None and weights.dtype != torch.float32:
-        return None                      # the interleaved accumulation path is fp32 only
+def _backproject_workspace(dim, B, R, P, N, interp, weights, oversampling, cutoff, projections):
+    """Scratch of the back-projection kernels (from torch's caching allocator, so nothing is freed behind the stream): for pixel
+    lists or bricks, else for interleaved accumulation; None when the library says a workspace would not help."""
+    if projections.dtype != torch.complex64:
+        return None                      # these paths are fp32 only
+    ws = _abi.scatter_workspace(dim, B, P, N, interp, int(weights is not None), oversampling, cutoff, projections.device)
+    if ws is not None:
+        return ws
     n = _abi.backproject_workspace_bytes(dim, B, R, P, N, interp, weights is not None)
-    return torch.empty(n, dtype=torch.uint8, device=device) if n else None
+    return torch.empty(n, dtype=torch.uint8, device=projections.device) if n else None
 
 
 # Volumes (one batch item) at least this large get a locality-preserving processing order of
@@ -386,10 +388,10 @@ def backproject_2d_to_3d_accumulate_(data_rec: torch.Tensor, weight_rec: Optiona
                and weight_rec.device == projections.device, f"weight_rec must be a contiguous {_REAL_OF[projections.dtype]} tensor of shape {want}")
     if P == 0:
         return
-    _abi.backproject_forw(3, projections.contiguous(), weights, rot, sh, interp, oversampling,
-                          _cutoff(fourier_radius_cutoff, N), data_rec,
+    cutoff = _cutoff(fourier_radius_cutoff, N)
+    _abi.backproject_forw(3, projections.contiguous(), weights, rot, sh, interp, oversampling, cutoff, data_rec,
                           weight_rec if weights is not None else None, True,
-                          _backproject_workspace(3, B, R, P, N, interp, weights, projections.device))
+                          _backproject_workspace(3, B, R, P, N, interp, weights, oversampling, cutoff, projections))
 
 
 def new_backprojection_accumulator(batch: int, box: int, device) -> torch.Tensor:
