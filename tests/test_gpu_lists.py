@@ -144,9 +144,9 @@ def test_sizes_that_are_listed_by_themselves_match_double_precision(dim, interp,
     assert rel_err(forw(proj, rot, None, sh, **kw)[0], d) <= TOL_ATOMIC
 
 
-@pytest.mark.parametrize("dim,N,os_,P,B,cutoff", [(3, 18, 2.0, 300, 1, None), (3, 6, 1.0, 151, 2, 4.0), (2, 34, 1.5, 297, 1, 11.5), (2, 66, 1.0, 100, 3, None)])
+@pytest.mark.parametrize("dim,N,os_,P,B,cutoff", [(3, 18, 2.0, 601, 1, None), (3, 6, 1.0, 1501, 2, 4.0), (2, 34, 1.5, 297, 1, 11.5), (2, 66, 1.0, 100, 3, None), (2, 202, 1.0, 1201, 1, None)])
 def test_pose_gradients_of_back_projection_by_patches(dim, N, os_, P, B, cutoff):
-    """Linear calls of at least 296 slices take a slice's patches of 8 x 4 pixels in turn: ragged rows and columns, patches
+    """Linear calls of at least 296 slices and 6,000 patches take a slice's patches of 8 x 4 pixels in turn: several blocks to a slice and one, ragged rows and columns, patches
     outside the cutoff, with and without weights and shifts."""
     import torch_projectors_b200 as tp
     from oracle import port

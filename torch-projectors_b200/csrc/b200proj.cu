@@ -1028,10 +1028,12 @@ void launch_backproject_back(const Launch& L, cudaStream_t s, const C2<Real>* gd
                              Real* grad_shift) {
     const bool nr = grad_rot != nullptr, ns = grad_shift != nullptr;
     if constexpr (!CUBIC) {
-        // enough slices: patches (a whole slice per block once that is eight blocks per SM); the measurements stand at backproject_back_patches_kernel
-        if (L.g.BP >= 2 * 148 && (nr || ns)) {
-            const int64_t most = (((L.g.N + 3) / 4) * ((L.g.Nh + 7) / 8) + 7) / 8, fill = (148 * 8 + L.g.BP - 1) / L.g.BP;
-            const dim3 grid((unsigned)(fill < most ? fill : most), L.grid.y, L.grid.z);
+        // enough slices and pixels: patches; the measurements stand at backproject_back_patches_kernel
+        const int64_t patches = (int64_t)((L.g.N + 3) / 4) * ((L.g.Nh + 7) / 8);
+        if (L.g.BP >= 2 * 148 && L.g.BP * patches >= 6000 && (sizeof(Real) == 4 || patches >= 64) && (nr || ns)) {
+            // eight blocks per SM, and at most 16 patches a warp: what a block has left at the end is short, and few slices are under way at once
+            const int64_t most = (patches + 7) / 8, fill = (148 * 8 + L.g.BP - 1) / L.g.BP, blocks = fill < most ? fill : most, least = (most + 15) / 16;
+            const dim3 grid((unsigned)(blocks > least ? blocks : least), L.grid.y, L.grid.z);
 #define B200PROJ_BB(NR, NS) \
     backproject_back_patches_kernel<DIM, NR, NS><<<grid, kBlockThreads, 0, s>>>(gd, gw, proj, rot, shifts, grad_proj, grad_weights, grad_rot, grad_shift, L.g)
             if (nr && ns) B200PROJ_BB(true, true);

@@ -854,6 +854,9 @@ backproject_back_kernel(const C2<R>* __restrict__ grad_data_rec,
 // of box 64, weigh as much as the gather of linear taps: 2,000 slices of 64 x 33 with all gradients 182 us in tiles, 128 in
 // patches; 1,000 2D slices of 130 x 66 185 and 127.  Cubic taps: 108 us for 500 slices, 160 in patches (registers); 60 linear
 // slices of 100 x 51: 15.2 us, 17.5; 300 of them 59.5, 50.  Four blocks per SM (64 registers): three 131 us, five 148.
+// In tiles / a whole slice per block / at most 16 patches a warp: 1,185 slices of 256 x 129 from box 512 2,628 / 2,800 / 2,539 us, of 400 x 201 from box 400
+// 3,042 / 3,266 / 2,560, 2,400 of 128 x 65 792 / 570 / 582.  Fewer than 6,000 patches gain nothing (300 slices of 24 x 13: 15 us, 17), nor do
+// small slices in double precision (2,000 of 24 x 13: 60, 62; 1,185 of 64 x 33 175, 140).
 template <int DIM, bool NEED_ROT, bool NEED_SHIFT, typename R>
 __global__ void __launch_bounds__(kBlockThreads, sizeof(R) == 4 ? 4 : 1)
 backproject_back_patches_kernel(const C2<R>* __restrict__ grad_data_rec,
