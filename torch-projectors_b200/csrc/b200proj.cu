@@ -515,11 +515,11 @@ size_t without_lists_bytes(int dim, int64_t B, int64_t R, int64_t P, int64_t N, 
 // Measured, without / from lists, weighted (unweighted): 3D linear, 10,000 slices of 128 x 65 oversampled twice: tilt series 1.46 / 1.59 (1.27 / 1.33) ms, in steps of
 // 3 degrees 1.45 / 2.01, one plane 1.33 / 2.69, one pose 2.5 / 4.4, ten poses 2.2 / 3.5, a hundred 2.2 / 2.2 (1.51 / 1.73), half of the slices in one plane 1.75 / 2.63;
 // not oversampled 0.7-1.1x.  2D, all slices turned alike / not turned, oversampled twice, cubic: 4 M pixels 0.77 / 0.46x of the time from lists,
-// 10 M 1.1 / 0.9x, 30 M and more 1.1-1.3x, but 64 x 33 references 0.85x at any number; linear: 22 M 1.0 / 0.79x, 45 M 1.2 / 0.85x, 77 M and
-// more 1.05-1.5x.  3D cubic: 1.1-4x, except one pose and ten poses onto boxes of 64 and 96 (0.75-0.95x), which from here look like one plane (2x).
+// 10 M 1.1 / 0.9x, 30 M and more 1.1-1.3x, but 64 x 33 references 0.85x at any number; linear: 22 M 1.0 / 0.79x, 45 M 1.2 / 0.85x, 51 M and
+// more 1.0-1.5x / 0.95-1.05x.  3D cubic: 1.1-4x, except one pose and ten poses onto boxes of 64 and 96 (0.75-0.95x), which from here look like one plane (2x).
 void list_crowd_rule(ListLaunch& L, int dim, int64_t B, int64_t R, int64_t P, int64_t N, bool cubic, int weights, double os, double cutoff) {
     static const float force = [] { const char* e = getenv("B200PROJ_LIST_CROWD"); return e ? (float)atof(e) : -1.f; }();   // number of cells, for tests
-    const bool gains = dim == 3 ? !cubic : cubic ? L.pixels < 7e6 || R <= 72 : L.pixels < 6e7;
+    const bool gains = dim == 3 ? !cubic : cubic ? L.pixels < 7e6 || R <= 72 : L.pixels < 5e7;
     L.plan.crowd = P < 2 || (dim == 3 && cubic) ? 0.f : force >= 0.f ? force : gains ? 128.f : 0.f;
     if (L.plan.crowd == 0.f) return;
     L.plan.probes = dim == 3 ? 256 : 64;
@@ -530,7 +530,9 @@ void list_crowd_rule(ListLaunch& L, int dim, int64_t B, int64_t R, int64_t P, in
 // however few pixels it has).  Measured crossings with the kernels used otherwise (in M pixels; bricks inside the ball of the samples), with
 // weights / without: 3D cubic, oversampled twice: 134 bricks 3 / 4, 1,072 2.3 / 3.5, 8,578 9 / 8, 68,600 55 / 50; not oversampled 0.5 / 0.8
 // and 1 / 0.9 of 134 and 1,072.  3D linear 10 / 17, 8.5 / 14, 7 / 26, 36 / 40; 3 / 5, 4.3 / 7.  2D cubic, tiles: 6 1.8 / 3, 25 1.4 / 2.2, 100
-// 1.4 / 2.3, 402 2.4 / 4.  2D linear 25 / 40, 10 / 35, 10.5 / 38, 25 / 50.  Far above them 1.25-1.7x (3D), 1.2-1.7x (2D).
+// 1.4 / 2.3, 402 2.4 / 4.  2D linear 25 / 40, 10 / 35, 10.5 / 38, 25 / 50.  3D linear into 16-byte voxels, whose plain kernel reduces faster: 8,578 bricks 11, 68,600
+// 51, 262,000 185.  Far above them 1.25-1.7x (3D), 1.2-1.7x (2D).  (Uniform poses; for others see list_crowd_rule.)  The pixels are those of one
+// pass over the list: each pass clears, plans and flushes all bricks.
 ListLaunch list_scatter_plan(int dim, int64_t B, int64_t R, int64_t P, int64_t N, bool cubic, int weights, double os, double cutoff) {
     ListLaunch L = list_layout(dim, B, R, P, N, os, cutoff, 148.0 * 4);
     if (!L.use) return L;
@@ -543,7 +545,8 @@ ListLaunch list_scatter_plan(int dim, int64_t B, int64_t R, int64_t P, int64_t N
     if (dim == 3) line = cubic ? (dense ? 0.9e6 : weights ? 2.5e6 : 3.2e6) + 750.0 * bricks
                                : (weights ? (dense ? 3.5e6 : 9e6) : (dense ? 6e6 : 16e6)) + (weights ? 400.0 : 800.0) * bricks;
     else line = cubic ? (weights ? 1.6e6 : 2.4e6) + 4e3 * bricks : (weights ? 11e6 : 36e6) + 3e4 * bricks + 2e8 / bricks;
-    return r > 24.0 && L.pixels > line ? L : ListLaunch{};
+    if (dim == 3 && !cubic && weights == 2 && !dense && line < 6e6 + 680.0 * bricks) line = 6e6 + 680.0 * bricks;
+    return r > 24.0 && (double)L.plan.inside * (double)L.plan.slices > line ? L : ListLaunch{};
 }
 bool runs_in(const ListLaunch& L, const void* workspace, size_t workspace_bytes) {
     return L.use && scratch_aligned(workspace) && workspace_bytes >= L.bytes;
