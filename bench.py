@@ -61,10 +61,9 @@ BACK_BYTES_PER_SLICE = 128 * 65 * 8 + 128 * 65 * 4 + 44 + 2 * (256 * 256 * 129 *
 # DRAM traffic per slice of the dominant kernels (dram__bytes_read.sum + dram__bytes_write.sum) from
 # ncu captures of a smaller launch of the same kernels, scaled by the slices a launch processes
 # (traffic grows in proportion to the slices: the volumes are touched the same way by every slice).
-PROJ_TRAFFIC_PER_SLICE = (416.0e6 + 843.2e6) / 10000      # profiles/brick_kernels_b200.md (a brick writes parts of rows)
+PROJ_TRAFFIC_PER_SLICE = (416.0e6 + 843.2e6) / 10000      # (a brick writes parts of rows)
 # back-projection: two captures of the slab-ordered kernel (4,096 and 16,384 slices) give a part that grows with the
 # slices and a fixed part (the workspace); the fixed part also holds the zero-fill and the fold of the workspace
-# (profiles/backproject_forw_3d_linear_box256_4096slices.md)
 BACK_TRAFFIC_PER_SLICE = (2506.4e6 - 730.7e6) / (16384 - 4096)
 BACK_TRAFFIC_FIXED = (730.7e6 - 4096 * BACK_TRAFFIC_PER_SLICE) + 135.3e6 + (135.3e6 + 44.2e6)
 # The ceilings the kernels actually sit on (from the same summaries): share of the L1TEX data pipe
@@ -78,7 +77,7 @@ def reduction_ceiling(taps, ms, pattern):
     rate = taps / (ms * 1e-3) / 1e9
     return {"bound": "reduction request rate (SM L1TEX-to-crossbar port, measured by the probe)", "achieved": rate, "peak": RED_CEILING_GTAPS[pattern], "unit": "G taps/s",
             "frac": rate / RED_CEILING_GTAPS[pattern], "pattern": pattern,
-            "peak_source": "python bench.py --workload red_ceiling (profiles/red_ceiling_b200.md)"}
+            "peak_source": "python bench.py --workload red_ceiling"}
 
 
 def measured_peak_gbs():
@@ -1127,7 +1126,7 @@ def main():
                 "secondary": {"bound": "L1TEX data pipe (64 taps x 8 B per pixel from shared memory)",
                               "frac": PROJ_L1TEX_DATA_PIPE_FRAC, "unit": "l1tex__data_pipe_lsu_wavefronts, fraction of peak",
                               "gather_taps_per_s": 6490 * 64 * PROJ["P"] / (kernel_ms * 1e-3),
-                              "peak_source": "ncu capture, profiles/brick_kernels_b200.md"}}
+                              "peak_source": "ncu capture of a smaller launch"}}
     parity = None
     if rank == 0 and not args.skip_cpu:
         parity = check_projection_parity(out_holder["out"], rec, rot, shifts)

@@ -224,10 +224,11 @@ def test_scatters_that_run_in_bricks_by_themselves_match_the_oracle(os_, P, shar
         assert rel_err(data, ref) <= TOL_ATOMIC and (weights is None or rel_err(wrec, wref) <= TOL_ATOMIC)
 
 
-@pytest.mark.parametrize("dim,N,P", [(3, 64, 12000), (3, 80, 7919), (2, 128, 3001)])
-def test_long_runs_of_the_scatter_rings_match_double_precision(dim, N, P):
-    """Enough slices that a walking warp refills its list of hits and rings and sums are used over many items of a block,
-    against the double-precision kernels (which do not run in bricks).  Their sample positions are not rounded to
+LONG_RUNS = [(3, 64, 12000), (3, 80, 7919), (2, 128, 3001)]
+
+
+def check_long_runs(dim, N, P, lists):
+    """Against the double-precision kernels (which run neither in bricks nor from lists).  Their sample positions are not rounded to
     single precision: up to 4 * 160 * 2^-24 = 4e-5 voxels apart, times slopes of the taps below 1.3, of random signs."""
     import torch_projectors_b200 as tp
     lib, cubic = tp._abi.load(), tp._abi.CUBIC
@@ -239,7 +240,9 @@ def test_long_runs_of_the_scatter_rings_match_double_precision(dim, N, P):
     if dim == 3:
         _one_plane(rot, 3)
     rot = rot["rot"].cuda()
-    assert all(lib.b200proj_scatter_workspace_bytes(dim, 1, P, N, cubic, k, 2.0, N / 2.0) > 0 for k in (0, 1))
+    # a list holds every pixel within Nyquist (0.39 N^2 a slice), bricks hold records of the slices
+    sizes = [lib.b200proj_scatter_workspace_bytes(dim, 1, P, N, cubic, k, 2.0, N / 2.0) for k in (0, 1)]
+    assert all(n > 0 and (n > 4 * 0.39 * P * N * N) == lists for n in sizes), sizes
     forw = tp.backproject_2d_to_3d_forw if dim == 3 else tp.backproject_2d_forw
     back = tp.project_3d_to_2d_back if dim == 3 else tp.project_2d_back
     kw = dict(interpolation="cubic", oversampling=2.0)
@@ -254,3 +257,17 @@ def test_long_runs_of_the_scatter_rings_match_double_precision(dim, N, P):
         tp.backproject_2d_to_3d_accumulate_interleaved_(acc, proj, rot, w, sh, **kw)
         d2, w2 = tp.fold_backprojection_accumulator(acc)
         assert rel_err(d2, d) <= TOL_ATOMIC and rel_err(w2, dw) <= TOL_ATOMIC
+
+
+@pytest.mark.parametrize("dim,N,P", LONG_RUNS)
+def test_long_runs_of_the_scatter_rings_match_double_precision(dim, N, P):
+    """Enough slices that a walking warp refills its list of hits and rings and sums are used over many items of a block.  In a
+    process of its own: calls of this size run from pixel lists unless these are off."""
+    code = f"import sys; sys.path[:0] = [{str(ROOT / 'tests')!r}, {str(ROOT / 'torch-projectors_b200')!r}, {str(ROOT)!r}]; import test_gpu_bricks as t; t.check_long_runs({dim}, {N}, {P}, False)"
+    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, B200PROJ_LISTS="0"), cwd=ROOT, capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]
+
+
+@pytest.mark.parametrize("dim,N,P", LONG_RUNS)
+def test_the_same_from_pixel_lists(dim, N, P):
+    check_long_runs(dim, N, P, True)

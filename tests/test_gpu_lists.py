@@ -180,6 +180,22 @@ def test_a_listed_call_takes_an_infinite_cutoff(dim, interp, N, P):
     assert rel_err(inner, b) > 100 * TOL_ATOMIC
 
 
+@pytest.mark.parametrize("P", [167000, 180000])
+def test_the_longest_lists(P):
+    """Nearly 2^30 entries in one pass (167,000 slices of 128 x 65), and the first number of slices that takes two by itself: the same
+    as in parts."""
+    import torch_projectors_b200 as tp
+    N, gen = 128, torch.Generator("cuda").manual_seed(P)
+    inside = tp._abi.cutoff_pack_index(N, N / 2.0, "cuda")[1] - (N // 2)         # (less the mirrored half of column 0)
+    assert (inside * P <= 1 << 30) == (P < 170000) and inside * P > 0.99 * (1 << 30)
+    proj = torch.randn(1, P, N, N // 2 + 1, dtype=torch.complex64, generator=gen, device="cuda")
+    rot = torch.linalg.qr(torch.randn(1, P, 3, 3, generator=gen, device="cuda"))[0].contiguous()
+    kw = dict(interpolation="linear", oversampling=1.0)
+    whole = tp.backproject_2d_to_3d_forw(proj, rot, None, **kw)[0]
+    parts = sum(tp.backproject_2d_to_3d_forw(proj[:, k::3], rot[:, k::3], None, **kw)[0] for k in range(3))
+    assert rel_err(whole, parts) <= TOL_ATOMIC
+
+
 def _one_view(dim, P, gen):
     """Poses that share a plane; in 2D, all slices turned alike."""
     a = torch.rand(P, generator=gen, device="cuda") * 6.2832 if dim == 3 else torch.full((P,), 0.7, device="cuda")

@@ -65,8 +65,10 @@ def check():
                 assert kind == "small" or not scratch.any(), "a misaligned workspace is left alone"
 
 
-def test_unusable_scratch_is_left_alone():
-    env = dict(os.environ, B200PROJ_BRICKS="1")
+@pytest.mark.parametrize("lists", ["0", "1"])
+def test_unusable_scratch_is_left_alone(lists):
+    """Without and with pixel lists, in whose place bricks run when the scratch is too small for a list."""
+    env = dict(os.environ, B200PROJ_BRICKS="1", B200PROJ_LISTS=lists)
     r = subprocess.run([sys.executable, "-c", f"import sys; sys.path[:0] = [{str(ROOT / 'tests')!r}, {str(ROOT / 'torch-projectors_b200')!r}, {str(ROOT)!r}]; import test_gpu_scratch as t; t.check()"],
                        env=env, cwd=ROOT, capture_output=True, text=True, timeout=600)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]
