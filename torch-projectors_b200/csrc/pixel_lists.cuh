@@ -9,7 +9,7 @@
 // for which the grid starts a brick below.
 //
 // A call runs as
-//   list_setup_kernel    the pixels inside the cutoff, in patches of 16 x 4; a 32-byte record per slice
+//   list_setup_kernel    the pixels inside the cutoff, in patches of 16 x 4; a 32-byte record per slice; whether the poses crowd
 //   list_pixels_kernel   counts the pixels of each brick (COUNT), later writes their entries
 //   list_plan_kernel     a place in the list for each brick, work items of at most `most` pixels of one brick
 #pragma once
