@@ -657,6 +657,7 @@ int scatter_without_lists(Launch L, const ListLaunch& ll, bool cubic, void* work
         gated_zero_kernel<<<148 * 8, 256, 0, s>>>((float4*)scratch, (n + 15) / 16, gate);
         return check_launch("gated_zero launch");
     };
+    const unsigned by_slices = (unsigned)((L.g.BP + kGatedSlices - 1) / kGatedSlices);
     // several tiles to a block, as long as there are some ten blocks per place on the GPU
     const int64_t most = (int64_t)L.grid.x * L.g.BP / 8192;
     const int tiles = (int)(most < 1 ? 1 : most < (int64_t)L.grid.x ? most : L.grid.x);
@@ -665,8 +666,8 @@ int scatter_without_lists(Launch L, const ListLaunch& ll, bool cubic, void* work
         if constexpr (DIM == 3) {
             const SlabPlan apart = slab_plan(L.g.R, true);
             if (accum == nullptr && apart.slabs > 1) {
-                backproject_slab_kernel<false, true><<<dim3((unsigned)L.g.BP, (unsigned)apart.slabs, 1), kBlockThreads, 0, s>>>(p, weights, rot, shifts, (float2*)vol, wvol, nullptr, L.g, apart.planes, 0, gate);
-                return check_launch("backproject_slab launch");
+                gated_slab_kernel<true, false><<<dim3(by_slices, (unsigned)apart.slabs, 1), kBlockThreads, 0, s>>>(p, weights, rot, shifts, (float2*)vol, wvol, nullptr, L.g, apart.planes, gate);
+                return check_launch("gated_slab launch");
             }
         }
         float4* to = accum;
@@ -680,7 +681,7 @@ int scatter_without_lists(Launch L, const ListLaunch& ll, bool cubic, void* work
         }
         const SlabPlan plan = DIM == 3 ? slab_plan(L.g.R, true, true, accum == nullptr && os >= 1.5) : SlabPlan{1, L.g.R};
         if (DIM == 3 && plan.slabs > 1)
-            backproject_slab_kernel<false, true, true><<<dim3((unsigned)L.g.BP, (unsigned)plan.slabs, 1), kBlockThreads, 0, s>>>(p, weights, rot, shifts, nullptr, nullptr, to, L.g, plan.planes, 0, gate);
+            gated_slab_kernel<true, true><<<dim3(by_slices, (unsigned)plan.slabs, 1), kBlockThreads, 0, s>>>(p, weights, rot, shifts, nullptr, nullptr, to, L.g, plan.planes, gate);
         else if (DIM == 2 && cubic)
             gated_interleaved_kernel<2, true><<<grid, kBlockThreads, 0, s>>>(p, weights, rot, shifts, to, L.g, tiles, gate);
         else
@@ -693,8 +694,8 @@ int scatter_without_lists(Launch L, const ListLaunch& ll, bool cubic, void* work
         if constexpr (DIM == 3 && DUP) {
             const SlabPlan plan = slab_plan(L.g.R, false);
             if (plan.slabs > 1) {
-                backproject_slab_kernel<false, false><<<dim3((unsigned)L.g.BP, (unsigned)plan.slabs, 1), kBlockThreads, 0, s>>>(p, nullptr, rot, shifts, (float2*)vol, nullptr, nullptr, L.g, plan.planes, 0, gate);
-                return check_launch("backproject_slab launch");
+                gated_slab_kernel<false, false><<<dim3(by_slices, (unsigned)plan.slabs, 1), kBlockThreads, 0, s>>>(p, nullptr, rot, shifts, (float2*)vol, nullptr, nullptr, L.g, plan.planes, gate);
+                return check_launch("gated_slab launch");
             }
         }
         const int copies = scatter_copies(L, DIM, cubic, false, scratch, bytes);

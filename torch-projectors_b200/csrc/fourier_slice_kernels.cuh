@@ -630,19 +630,15 @@ __device__ __forceinline__ void clip_run(float a, float inv_a, float b, float lo
 
 // INTERLEAVED: reductions go to a 16-byte-per-voxel (re, im, w, 0) accumulator `accum` (one v4
 // reduction per tap) instead of data_rec / weight_rec.
-template <bool CUBIC, bool WEIGHTS, bool INTERLEAVED = false>
-__global__ void __launch_bounds__(kBlockThreads)
-backproject_slab_kernel(const float2* __restrict__ proj, const float* __restrict__ weights,
-                        const float* __restrict__ rot, const float* __restrict__ shifts,
-                        float2* __restrict__ data_rec, float* __restrict__ weight_rec,
-                        float4* __restrict__ accum, const SliceGeom g, int slab_planes, int slab_first, const Gate gate = {}) {
-    if (gate.shut()) return;
+template <bool CUBIC, bool WEIGHTS, bool INTERLEAVED>
+__device__ __forceinline__ void backproject_slab(const SliceGeom& g, int bp, int slab, const float2* __restrict__ proj, const float* __restrict__ weights,
+                                                 const float* __restrict__ rot, const float* __restrict__ shifts, float2* __restrict__ data_rec,
+                                                 float* __restrict__ weight_rec, float4* __restrict__ accum, int slab_planes) {
     constexpr int T = CUBIC ? 4 : 2;
     constexpr unsigned kFull = 0xffffffffu;
     constexpr float kEps = 0.05f;                    // slack of the linear estimates below
-    const int bp = blockIdx.x;
     const int b = bp / g.P, p = bp - b * g.P;
-    const int z_lo = -g.half + 1 + ((int)blockIdx.y + slab_first) * slab_planes;
+    const int z_lo = -g.half + 1 + slab * slab_planes;
     const int z_hi = min(z_lo + slab_planes, g.half + 1);
     const float* rm = pose_rot<3>(g, rot, b, p);
     // linear estimates of the sample position along a row: d ~ ad*j + bd*kr, c ~ ac*j + bc*kr
@@ -775,6 +771,24 @@ backproject_slab_kernel(const float2* __restrict__ proj, const float* __restrict
             scatter_pixel(active, px, v, wv);
         }
     }
+}
+template <bool CUBIC, bool WEIGHTS, bool INTERLEAVED = false>
+__global__ void __launch_bounds__(kBlockThreads)
+backproject_slab_kernel(const float2* __restrict__ proj, const float* __restrict__ weights,
+                        const float* __restrict__ rot, const float* __restrict__ shifts,
+                        float2* __restrict__ data_rec, float* __restrict__ weight_rec,
+                        float4* __restrict__ accum, const SliceGeom g, int slab_planes, int slab_first) {
+    backproject_slab<CUBIC, WEIGHTS, INTERLEAVED>(g, (int)blockIdx.x, (int)blockIdx.y + slab_first, proj, weights, rot, shifts, data_rec, weight_rec, accum, slab_planes);
+}
+// Linear taps behind a gate: kGatedSlices slices to a block, as idle blocks cost time (see cell_scatter.cuh).
+constexpr int kGatedSlices = 4;
+template <bool WEIGHTS, bool INTERLEAVED>
+__global__ void __launch_bounds__(kBlockThreads)
+gated_slab_kernel(const float2* __restrict__ proj, const float* __restrict__ weights, const float* __restrict__ rot, const float* __restrict__ shifts,
+                  float2* __restrict__ data_rec, float* __restrict__ weight_rec, float4* __restrict__ accum, const SliceGeom g, int slab_planes, const Gate gate) {
+    if (gate.shut()) return;
+    for (int bp = (int)blockIdx.x * kGatedSlices, end = min(bp + kGatedSlices, g.BP); bp < end; ++bp)
+        backproject_slab<false, WEIGHTS, INTERLEAVED>(g, bp, (int)blockIdx.y, proj, weights, rot, shifts, data_rec, weight_rec, accum, slab_planes);
 }
 
 // ---- backward of back-projection --------------------------------------------------------
