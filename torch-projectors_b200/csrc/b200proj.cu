@@ -657,7 +657,10 @@ int scatter_without_lists(Launch L, const ListLaunch& ll, bool cubic, void* work
         gated_zero_kernel<<<148 * 8, 256, 0, s>>>((float4*)scratch, (n + 15) / 16, gate);
         return check_launch("gated_zero launch");
     };
-    const unsigned by_slices = (unsigned)((L.g.BP + kGatedSlices - 1) / kGatedSlices);
+    // slab passes: up to four slices to a block, as long as a slab that all slices lie in has some 2,000 blocks (2,048 slices of one plane, box 800: 4.74 ms,
+    // with four to a block 5.0; idle blocks 0.06 ms of 6.4)
+    const int per = L.g.BP < 4096 ? 1 : L.g.BP < 8192 ? 2 : 4;
+    const unsigned by_slices = (unsigned)((L.g.BP + per - 1) / per);
     // several tiles to a block, as long as there are some ten blocks per place on the GPU
     const int64_t most = (int64_t)L.grid.x * L.g.BP / 8192;
     const int tiles = (int)(most < 1 ? 1 : most < (int64_t)L.grid.x ? most : L.grid.x);
@@ -666,7 +669,7 @@ int scatter_without_lists(Launch L, const ListLaunch& ll, bool cubic, void* work
         if constexpr (DIM == 3) {
             const SlabPlan apart = slab_plan(L.g.R, true);
             if (accum == nullptr && apart.slabs > 1) {
-                gated_slab_kernel<true, false><<<dim3(by_slices, (unsigned)apart.slabs, 1), kBlockThreads, 0, s>>>(p, weights, rot, shifts, (float2*)vol, wvol, nullptr, L.g, apart.planes, gate);
+                gated_slab_kernel<true, false><<<dim3(by_slices, (unsigned)apart.slabs, 1), kBlockThreads, 0, s>>>(p, weights, rot, shifts, (float2*)vol, wvol, nullptr, L.g, apart.planes, per, gate);
                 return check_launch("gated_slab launch");
             }
         }
@@ -681,7 +684,7 @@ int scatter_without_lists(Launch L, const ListLaunch& ll, bool cubic, void* work
         }
         const SlabPlan plan = DIM == 3 ? slab_plan(L.g.R, true, true, accum == nullptr && os >= 1.5) : SlabPlan{1, L.g.R};
         if (DIM == 3 && plan.slabs > 1)
-            gated_slab_kernel<true, true><<<dim3(by_slices, (unsigned)plan.slabs, 1), kBlockThreads, 0, s>>>(p, weights, rot, shifts, nullptr, nullptr, to, L.g, plan.planes, gate);
+            gated_slab_kernel<true, true><<<dim3(by_slices, (unsigned)plan.slabs, 1), kBlockThreads, 0, s>>>(p, weights, rot, shifts, nullptr, nullptr, to, L.g, plan.planes, per, gate);
         else if (DIM == 2 && cubic)
             gated_interleaved_kernel<2, true><<<grid, kBlockThreads, 0, s>>>(p, weights, rot, shifts, to, L.g, tiles, gate);
         else
@@ -694,7 +697,7 @@ int scatter_without_lists(Launch L, const ListLaunch& ll, bool cubic, void* work
         if constexpr (DIM == 3 && DUP) {
             const SlabPlan plan = slab_plan(L.g.R, false);
             if (plan.slabs > 1) {
-                gated_slab_kernel<false, false><<<dim3(by_slices, (unsigned)plan.slabs, 1), kBlockThreads, 0, s>>>(p, nullptr, rot, shifts, (float2*)vol, nullptr, nullptr, L.g, plan.planes, gate);
+                gated_slab_kernel<false, false><<<dim3(by_slices, (unsigned)plan.slabs, 1), kBlockThreads, 0, s>>>(p, nullptr, rot, shifts, (float2*)vol, nullptr, nullptr, L.g, plan.planes, per, gate);
                 return check_launch("gated_slab launch");
             }
         }

@@ -780,14 +780,13 @@ backproject_slab_kernel(const float2* __restrict__ proj, const float* __restrict
                         float4* __restrict__ accum, const SliceGeom g, int slab_planes, int slab_first) {
     backproject_slab<CUBIC, WEIGHTS, INTERLEAVED>(g, (int)blockIdx.x, (int)blockIdx.y + slab_first, proj, weights, rot, shifts, data_rec, weight_rec, accum, slab_planes);
 }
-// Linear taps behind a gate: kGatedSlices slices to a block, as idle blocks cost time (see cell_scatter.cuh).
-constexpr int kGatedSlices = 4;
+// Linear taps behind a gate: `slices` slices to a block, as idle blocks cost time (see cell_scatter.cuh).
 template <bool WEIGHTS, bool INTERLEAVED>
 __global__ void __launch_bounds__(kBlockThreads)
 gated_slab_kernel(const float2* __restrict__ proj, const float* __restrict__ weights, const float* __restrict__ rot, const float* __restrict__ shifts,
-                  float2* __restrict__ data_rec, float* __restrict__ weight_rec, float4* __restrict__ accum, const SliceGeom g, int slab_planes, const Gate gate) {
+                  float2* __restrict__ data_rec, float* __restrict__ weight_rec, float4* __restrict__ accum, const SliceGeom g, int slab_planes, int slices, const Gate gate) {
     if (gate.shut()) return;
-    for (int bp = (int)blockIdx.x * kGatedSlices, end = min(bp + kGatedSlices, g.BP); bp < end; ++bp)
+    for (int bp = (int)blockIdx.x * slices, end = min(bp + slices, g.BP); bp < end; ++bp)
         backproject_slab<false, WEIGHTS, INTERLEAVED>(g, bp, (int)blockIdx.y, proj, weights, rot, shifts, data_rec, weight_rec, accum, slab_planes);
 }
 
