@@ -512,8 +512,9 @@ size_t without_lists_bytes(int dim, int64_t B, int64_t R, int64_t P, int64_t N, 
 }
 // When the lists are left aside: calls in which a brick's pixels share fewer than `crowd` of its cells (see list_setup_kernel; 128 lies between the
 // 190 and more of poses that are spread and the 80 and less of those that are not), and only where the scatter without lists is then faster.
-// Measured, without / from lists, weighted (unweighted): 3D linear, 10,000 slices of 128 x 65 oversampled twice: tilt series 1.46 / 1.59 (1.27 / 1.33) ms, in steps of
-// 3 degrees 1.45 / 2.01, one plane 1.33 / 2.69, one pose 2.5 / 4.4, ten poses 2.2 / 3.5, a hundred 2.2 / 2.2 (1.51 / 1.73), half of the slices in one plane 1.75 / 2.63;
+// Measured, without / from lists, weighted (unweighted): 3D linear, 10,000 slices of 128 x 65 oversampled twice: tilt series 1.46 / 1.58 (1.22 / 1.29) ms, in steps of
+// 3 degrees 1.46 / 1.98 (1.22 / 1.56), one plane 1.39 / 1.41 (1.08 / 1.25), one pose 2.6 / 3.7 (2.1 / 2.8), ten poses 2.2 / 3.8, a hundred 2.2 / 2.3 (1.45 / 1.78), half of the
+// slices in one plane 1.78 / 1.43 (1.27 / 1.25); 4,096 of 400 x 201 into volumes of their own: tilt series 7.3 / 7.5, in steps 7.4 / 10.1, one plane 8.9 / 5.3, ten poses 12.6 / 13.9;
 // not oversampled 0.7-1.1x.  2D, all slices turned alike / not turned, oversampled twice, cubic: 4 M pixels 0.77 / 0.46x of the time from lists,
 // 10 M 1.1 / 0.9x, 30 M and more 1.1-1.3x, but 64 x 33 references 0.85x at any number; linear: 22 M 1.0 / 0.79x, 45 M 1.2 / 0.85x, 51 M and
 // more 1.0-1.5x / 0.95-1.05x.  3D cubic: 1.1-4x, except one pose and ten poses onto boxes of 64 and 96 (0.75-0.95x), which from here look like one plane (2x).

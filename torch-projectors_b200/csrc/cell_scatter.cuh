@@ -575,8 +575,8 @@ cell_cubic_sums_kernel(const float2* __restrict__ proj, const float* __restrict_
 // lists are faster (their reductions fall on few sectors).  The poses are on the device, so list_setup_kernel finds out, the kernels above
 // return at once and the ones here run instead (Gate).  Plain kernels take several tiles to a block, as a grid whose blocks return at
 // once takes 0.5-1 ns a block (0.2 ms for the 400,000 tiles of 10,000 slices of 128 x 65); persistent blocks that draw tickets are 5-18 % slower
-// where they run.  10,000 slices of 128 x 65, weighted, linear, turned within one plane: lists 2.64 ms,
-// without 1.33; tilt series in steps of 3 degrees 2.01 and 1.45; of one pose 4.41 and 2.40.
+// where they run.  10,000 slices of 128 x 65, weighted, linear: ten poses from lists
+// 3.77 ms, without 2.19; tilt series in steps of 3 degrees 1.98 and 1.46; of one pose 3.71 and 2.60.
 // x = `tiles` tiles of a slice, (y, z) = the slice.
 template <int DIM, bool CUBIC, bool DUP>
 __global__ void __launch_bounds__(kBlockThreads)
